@@ -39,6 +39,7 @@ NKB_DEV void world_inv_inertia(Q4 pose_q, Q4 inertial_q, V3 inv_i, float* out) {
 NKB_DEV void stage_bodies(Env& e, bool kick) {
     const TemplateView& t = *e.t;
     const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
+#pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         const uint32_t link = __ldg(t.body_to_link + b);
         float* bp = sm_bpose(e, b);
@@ -88,6 +89,7 @@ NKB_DEV float motion_radius(float base, float dt, float sa, float sb) { return b
 NKB_DEV void stage_aabbs(Env& e) {
     const TemplateView& t = *e.t;
     const float margin = fmaxf(t.cfg.contact_margin, 0.0005f), reach = query_reach(t.cfg);
+#pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         const float* bp = sm_bpose(e, b);
         const float* p = t.shape_params + 4u * b;
@@ -130,6 +132,7 @@ NKB_DEV uint32_t stage_pairs(Env& e) {
     const uint32_t cap = t.cfg.max_pairs != 0u && t.cfg.max_pairs < t.cfg.max_contacts ? t.cfg.max_pairs : t.cfg.max_contacts;
     uint32_t count = 0u;
     uint32_t* pairs = sm_pairs(e);
+#pragma unroll 1
     for (uint32_t base = 0u; base < t.n_adm; base += 32u) {
         const uint32_t k = base + e.lane;
         bool hit = false;
@@ -155,6 +158,7 @@ NKB_DEV void stage_store_contacts(Env& e, uint32_t pair_count) {
     const uint32_t S = t.cfg.max_contacts;
     if (e.s->pair_count == nullptr || S == 0u) return;
     if (e.lane == 0u) e.s->pair_count[e.env] = pair_count;
+#pragma unroll 1
     for (uint32_t s = e.lane; s < S; s += 32u) {
         const size_t gs = (size_t)e.env * S + s;
         const uint32_t ab = s < pair_count ? sm_pairs(e)[s] : 0u;

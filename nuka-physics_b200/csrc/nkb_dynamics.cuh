@@ -27,6 +27,7 @@ struct Env {
     uint32_t dof_link[2], dof_comp[2];   // comp == kNoLink for scalar joints
     float vel0[2];           // step-start coordinate velocity
     uint32_t status;
+    bool branching;          // a contact of this step acts on two branches of the articulation's tree
     uint32_t vstride;        // words per shared-memory vector: 32 x coordinates per lane
     // team mode: word offsets from the env's Newton scratch (matrix, block mass, staged rows) and solver vectors to this
     // warp's private copies; zero for the env's lead warp
@@ -108,7 +109,7 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
         if (dof && __ldg(t.jtype + e.dof_link[r]) == kFloating) e.dof_comp[r] = c - __ldg(t.link_dof + e.dof_link[r]);
         e.vel0[r] = 0.f;
     }
-    e.status = 0u;
+    e.status = 0u; e.branching = false;
 #ifdef NKB_STAGE_TAPS
     e.cyc = p.s.dbg_cycles != nullptr ? p.s.dbg_cycles + (size_t)env * 32u : nullptr;
     e.t0 = clock64();
@@ -133,6 +134,7 @@ NKB_DEV void stage_fk(Env& e) {
             rpos = rpos + qrot(rrot, e.axis * e.q);
         }
     }
+#pragma unroll 1
     for (uint32_t d = 0; d <= t.max_depth; ++d) {
         if (link && e.depth == d) {
             float* out = sm_pose(e, l);
@@ -246,6 +248,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
         st3(sm_vel(e, l), vw); st3(sm_vel(e, l) + 3, vv);
     }
     __syncwarp();
+#pragma unroll 1
     for (uint32_t d = 0; d <= t.max_depth; ++d) {
         if (link && e.depth == d && !froot) {
             V3 pw = mk3(0.f, 0.f, 0.f), pv = pw;
@@ -268,6 +271,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     }
     // accelerations root to leaf with gravity injected at the root
     V3 aw = mk3(0.f, 0.f, 0.f), av = aw;
+#pragma unroll 1
     for (uint32_t d = 0; d <= t.max_depth; ++d) {
         if (link && e.depth == d) {
             if (e.parent != kNoLink) xf_motion(E, r, ld3(sm_acc(e, e.parent)), ld3(sm_acc(e, e.parent) + 3), aw, av);
@@ -291,10 +295,12 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     }
     __syncwarp();
     // leaf to root: bias forces and composite inertias, children in list order
+#pragma unroll 1
     for (uint32_t rem = t.max_depth + 1u; rem > 0u; --rem) {
         if (link && e.depth == rem - 1u) {
             const uint32_t cb = __ldg(t.child_begin + l), ce = __ldg(t.child_begin + l + 1u);
             float* ic = sm_ic(e, l);
+#pragma unroll 1
             for (uint32_t c = cb; c < ce; ++c) {
                 const uint32_t child = __ldg(t.children + c);
                 V3 cn, cf;
@@ -344,6 +350,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     }
     // mass matrix, ops/articulation_mass.cuh:124-253
     float* M = sm_mass(e);
+#pragma unroll 1
     for (uint32_t k = l; k < n * ld; k += 32u) M[k] = 0.f;
     __syncwarp();
     if (t.floating_root && l < 6u) {
@@ -370,6 +377,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
         diag += dt * e.drive_dissipation;
         M[di * ld + di] = diag;
         uint32_t walk = l;
+#pragma unroll 1
         for (;;) {
             const uint32_t p = __ldg(t.parent + walk);
             if (p == kNoLink) break;
@@ -396,6 +404,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     __syncwarp();
     if (e.s->dbg_mass != nullptr) {
         float* out = e.s->dbg_mass + (size_t)e.env * n * n;
+#pragma unroll 1
         for (uint32_t k = l; k < n * n; k += 32u) out[k] = M[(k / n) * ld + k % n];
     }
     // L D L^T, unit lower triangle with D on the diagonal and pivot floor 1e-6 (articulation_mass.cuh:269-335).
@@ -404,6 +413,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     // and the pivots read ahead of one short dependent chain instead of a read-modify-write per term.
     float* F = sm_factor(e);
     float* piv = sm_vec(e, kVecTmp);
+#pragma unroll 1
     for (uint32_t k = l; k < n * ld; k += 32u) F[k] = M[k];
     __syncwarp();
 #pragma unroll 1
@@ -426,6 +436,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
                     const float4 a = Fr4[c], b4 = Fk4[c], p = piv4[c];
                     acc -= a.x * b4.x * p.x; acc -= a.y * b4.y * p.y; acc -= a.z * b4.z * p.z; acc -= a.w * b4.w * p.w;
                 }
+#pragma unroll 1
                 for (uint32_t j = full << 2; j < k; ++j) acc -= Fr[j] * Fk[j] * piv[j];
                 v[r] = acc;
             }
@@ -445,6 +456,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     float x[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) x[r] = dof[r] ? rhs[r] : 0.f;
+#pragma unroll 1
     for (uint32_t j = 0; j < n; ++j) {
         const float xj = coord_bcast<NR>(x, j);
 #pragma unroll
@@ -452,6 +464,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (dof[r]) x[r] /= F[row * ld + row]; }
+#pragma unroll 1
     for (uint32_t jj = n; jj > 0u; --jj) {
         const uint32_t j = jj - 1u;
         const float xj = coord_bcast<NR>(x, j);
@@ -505,10 +518,12 @@ struct TorqueOut { float tau, command; uint32_t status; uint32_t applied; };
 // k < n carries row k of the matrix and of the eigenvector table through each rotation, lane 0 closes the 2 x 2 block,
 // and the n x n entries of the result are spread over the lanes.  `vectors` is 36 words of scratch beside the matrix.
 static __device__ __noinline__ void task_metric_pseudoinverse(float* a, float* vectors, uint32_t n, float* inverse, uint32_t lane) {
+#pragma unroll 1
     for (uint32_t i = lane; i < 36u; i += 32u) vectors[i] = (i / 6u == i % 6u && i / 6u < n) ? 1.0f : 0.f;
     __syncwarp();
     for (uint32_t sweep = 0u; sweep < 24u; ++sweep) {
         bool changed = false;
+#pragma unroll 1
         for (uint32_t p = 0u; p < n; ++p) for (uint32_t q = p + 1u; q < n; ++q) {
             const float app = a[p * 6u + p], aqq = a[q * 6u + q], apq = a[p * 6u + q];
             if (fabsf(apq) <= FLT_EPSILON * (fabsf(app) + fabsf(aqq))) continue;       // the same words in every lane: a uniform branch
@@ -538,11 +553,14 @@ static __device__ __noinline__ void task_metric_pseudoinverse(float* a, float* v
         if (!changed) break;
     }
     float largest = 0.f;
+#pragma unroll 1
     for (uint32_t i = 0u; i < n; ++i) largest = fmaxf(largest, a[i * 6u + i]);
     const float tolerance = largest * (8.0f * FLT_EPSILON);
+#pragma unroll 1
     for (uint32_t i = lane; i < n * n; i += 32u) {
         const uint32_t r = i / n, c = i % n;
         double v = 0.0;
+#pragma unroll 1
         for (uint32_t k = 0u; k < n; ++k) {
             const float eigenvalue = a[k * 6u + k];
             if (eigenvalue > tolerance) v += (double)vectors[r * 6u + k] * vectors[c * 6u + k] / eigenvalue;
@@ -569,6 +587,7 @@ static __device__ __noinline__ void task_right_hand_side(TorqueIn e, const float
     float jq[6];
     for (uint32_t r = 0u; r < 6u; ++r) {
         float sum = 0.f;
+#pragma unroll 1
         for (uint32_t i = 0u; i < n; ++i) sum += J[r * n + i] * qdd[i];
         jq[r] = sum;
     }
@@ -642,10 +661,13 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     // bias = -d qd - H qdd_free, lane = actuated joint
     if (column) {
         double b = passive[l];
+#pragma unroll 1
         for (uint32_t c = 0u; c < active; ++c) b -= (double)H[l * active + c] * free_acc[c];
         bias[l] = (float)b;
     }
+#pragma unroll 1
     for (uint32_t i = l; i < 6u * n; i += 32u) J[i] = 0.f;
+#pragma unroll 1
     for (uint32_t i = l; i < n; i += 32u) chain[i] = 0.f;
     __syncwarp();
     // Jacobian columns, lane = link on the chain from the task link to the root
@@ -679,30 +701,42 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     // B: M x = J_r^T through the L D L^T factor, lane = task row
     if (l < rows) {
         float x[32 * NR];
+#pragma unroll 1
         for (uint32_t i = 0u; i < n; ++i) x[i] = J[l * n + i];
+#pragma unroll 1
         for (uint32_t j = 0u; j < n; ++j)
+#pragma unroll 1
             for (uint32_t i = j + 1u; i < n; ++i) x[i] -= F[i * ld + j] * x[j];
+#pragma unroll 1
         for (uint32_t i = 0u; i < n; ++i) x[i] /= F[i * ld + i];
+#pragma unroll 1
         for (uint32_t end = n; end > 0u; --end) {
             const uint32_t i = end - 1u;
             float sum = x[i];
+#pragma unroll 1
             for (uint32_t j = i + 1u; j < n; ++j) sum -= F[j * ld + i] * x[j];
             x[i] = sum;
         }
+#pragma unroll 1
         for (uint32_t c = 0u; c < active; ++c) resp[l * active + c] = x[dofs[c]];
     }
     __syncwarp();
     if (column)
+#pragma unroll 1
         for (uint32_t r = 0u; r < rows; ++r) {
             double v = 0.0;
+#pragma unroll 1
             for (uint32_t a = 0u; a < active; ++a) v += (double)H[l * active + a] * resp[r * active + a];
             tmap[r * active + l] = (float)v;
         }
+#pragma unroll 1
     for (uint32_t i = l; i < 72u; i += 32u) metric[i] = 0.f;      // metric and inverse
     __syncwarp();
+#pragma unroll 1
     for (uint32_t i = l; i < rows * rows; i += 32u) {
         const uint32_t r = i / rows, c = i % rows;
         double v = 0.0;
+#pragma unroll 1
         for (uint32_t a = 0u; a < active; ++a) v += (double)resp[r * active + a] * tmap[c * active + a];
         metric[r * 6u + c] = (float)v;
     }
@@ -720,6 +754,7 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     __syncwarp();
     if (column) {
         double v = 0.0;
+#pragma unroll 1
         for (uint32_t c = 0u; c < active; ++c) v += (double)H[l * active + c] * prhs[c];
         const bool off_chain = chain[dofs[l]] == 0.f;
         if (off_chain) v += own[l];
@@ -728,12 +763,14 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     __syncwarp();
     if (l < rows) {
         float rhs = trhs[l];
+#pragma unroll 1
         for (uint32_t a = 0u; a < active; ++a) rhs -= resp[l * active + a] * (bias[a] - passive[a] + posture[a]);
         trhs[l] = rhs;
     }
     __syncwarp();
     if (l < rows) {
         float sum = 0.f;
+#pragma unroll 1
         for (uint32_t c = 0u; c < rows; ++c) sum += inverse[l * 6u + c] * trhs[c];
         force[l] = sum;
     }
@@ -741,6 +778,7 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     float value = 0.f;
     if (column) {
         double v = bias[l] + posture[l];
+#pragma unroll 1
         for (uint32_t r = 0u; r < rows; ++r) v += (double)tmap[r * active + l] * force[r];
         value = (float)v;
     }
@@ -802,6 +840,7 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) osc_in.acc0[k] = a0[k];
         float* keep = H + active * active;
+#pragma unroll 1
         for (uint32_t i = l; i < n; i += 32u) keep[i] = vecs[vs * kVecAcc + i];
     }
     __syncwarp();
@@ -817,20 +856,28 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     float x[32 * NR];
     // S M^-1 S^T, column by column: M x = e_dof(c) through the L D L^T factor (articulation_mass.cuh:357-411)
     if (column) {
+#pragma unroll 1
         for (uint32_t i = 0u; i < n; ++i) x[i] = i == dofs[l] ? 1.0f : 0.0f;
+#pragma unroll 1
         for (uint32_t j = 0u; j < n; ++j)
+#pragma unroll 1
             for (uint32_t i = j + 1u; i < n; ++i) x[i] -= F[i * ld + j] * x[j];
+#pragma unroll 1
         for (uint32_t i = 0u; i < n; ++i) x[i] /= F[i * ld + i];
+#pragma unroll 1
         for (uint32_t end = n; end > 0u; --end) {
             const uint32_t i = end - 1u;
             float s = x[i];
+#pragma unroll 1
             for (uint32_t j = i + 1u; j < n; ++j) s -= F[j * ld + i] * x[j];
             x[i] = s;
         }
+#pragma unroll 1
         for (uint32_t r = 0u; r < active; ++r) A[r * active + l] = x[dofs[r]];
     }
     __syncwarp();
     if (column)
+#pragma unroll 1
         for (uint32_t c = 0u; c < l; ++c) {
             const float v = 0.5f * (A[l * active + c] + A[c * active + l]);
             A[l * active + c] = v; A[c * active + l] = v;
@@ -838,14 +885,17 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     __syncwarp();
     // L D L^T of the actuated block (FactorControlMass): every lane follows the pivots, lane i owns row i
     bool definite = true;
+#pragma unroll 1
     for (uint32_t j = 0u; j < active; ++j) {
         double pivot = A[j * active + j];
+#pragma unroll 1
         for (uint32_t k = 0u; k < j; ++k) { const double v = A[j * active + k]; pivot -= v * v * diag[k]; }
         if (!(pivot > 0.0) || !isfinite(pivot)) { definite = false; break; }
         __syncwarp();
         if (l == 0u) diag[j] = (float)pivot;
         if (column && l > j) {
             double v = A[l * active + j];
+#pragma unroll 1
             for (uint32_t k = 0u; k < j; ++k) v -= (double)A[l * active + k] * A[j * active + k] * diag[k];
             A[l * active + j] = (float)(v / pivot);
         }
@@ -854,18 +904,24 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     if (!definite) { out.status = kStatusControlFailure; return out; }
     // H = inverse, column by column (SolveControlMass on unit vectors)
     if (column) {
+#pragma unroll 1
         for (uint32_t i = 0u; i < active; ++i) {
             double v = i == l ? 1.0 : 0.0;
+#pragma unroll 1
             for (uint32_t j = 0u; j < i; ++j) v -= (double)A[i * active + j] * x[j];
             x[i] = (float)v;
         }
+#pragma unroll 1
         for (uint32_t i = 0u; i < active; ++i) x[i] /= diag[i];
+#pragma unroll 1
         for (uint32_t ii = active; ii > 0u; --ii) {
             const uint32_t i = ii - 1u;
             double v = x[i];
+#pragma unroll 1
             for (uint32_t j = i + 1u; j < active; ++j) v -= (double)A[j * active + i] * x[j];
             x[i] = (float)v;
         }
+#pragma unroll 1
         for (uint32_t r = 0u; r < active; ++r) H[r * active + l] = x[r];
     }
     __syncwarp();
@@ -879,8 +935,10 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     float value = 0.f;
     if (column) {
         double b = passive[l];
+#pragma unroll 1
         for (uint32_t c = 0u; c < active; ++c) b -= (double)H[l * active + c] * free_acc[c];
         double v = (double)(float)b;
+#pragma unroll 1
         for (uint32_t c = 0u; c < active; ++c) v += (double)H[l * active + c] * rhs[c];
         value = (float)v;
     }
@@ -942,6 +1000,7 @@ NKB_DEV void stage_link_velocities(Env& e) {
     if (link) joint_xform(e, E, r);
     V3 jw = mk3(0.f, 0.f, 0.f), jv = jw;
     if (e.jtype == kRevolute) jw = e.axis * e.qd; else if (e.jtype == kPrismatic) jv = e.axis * e.qd;
+#pragma unroll 1
     for (uint32_t d = 0; d <= t.max_depth; ++d) {
         if (link && e.depth == d && !froot) {
             V3 pw = mk3(0.f, 0.f, 0.f), pv = pw;
@@ -964,9 +1023,11 @@ NKB_DEV void stage_store_links(Env& e) {
     }
     float* gp = e.s->link_pose + (size_t)e.env * L * 7u;
     const float* sp = e.sm + e.lay->pose;
+#pragma unroll 1
     for (uint32_t k = l; k < L * 7u; k += 32u) gp[k] = sp[k];
     float* gv = e.s->link_vel + (size_t)e.env * L * 6u;
     const float* sv = e.sm + e.lay->vel;
+#pragma unroll 1
     for (uint32_t k = l; k < L * 6u; k += 32u) gv[k] = sv[k];
 }
 

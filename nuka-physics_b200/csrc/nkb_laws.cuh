@@ -6,29 +6,16 @@
 
 namespace nkb {
 
-struct Resp { float dual_scale, residual_scale; };
 struct STerm { float impulse, curvature; };
 
-NKB_DEV Resp scalar_response(float cap, float compliance) {
-    const float product = cap * compliance;
-    Resp r;
-    if (product >= 1.0f) { r.dual_scale = 0.0f; r.residual_scale = 1.0f / compliance; }
-    else { r.dual_scale = 1.0f - product; r.residual_scale = cap; }
-    return r;
-}
-
-NKB_DEV STerm scalar_impulse(float dual, float rho, float residual, float lower, float upper, Resp rs) {
+// A rigid row's response (zero compliance, the only kind on this path: the reference's dual scale is 1 and its residual
+// scale the penalty).  NaN inputs pass through.
+NKB_DEV STerm scalar_impulse(float dual, float rho, float residual, float lower, float upper) {
     STerm t; t.impulse = 0.f; t.curvature = 0.f;
     if (rho <= 0.0f) return t;
-    if (dual != dual || rho != rho || residual != residual || lower != lower || upper != upper) {
-        const float invalid = dual + rho + residual + lower + upper;
-        t.impulse = t.curvature = invalid;
-        return t;
-    }
-    const float k = rs.residual_scale;
-    const float x = fmaf(k, residual, rs.dual_scale * dual);
+    const float x = fmaf(rho, residual, dual);
     t.impulse = x < lower ? lower : (x > upper ? upper : x);
-    t.curvature = x != x ? x : (lower < upper && x >= lower && x <= upper ? k : 0.0f);
+    t.curvature = x != x ? x : (lower < upper && x >= lower && x <= upper ? rho : 0.0f);
     return t;
 }
 
@@ -75,18 +62,17 @@ NKB_DEV V3 relax_contact_impulse_fast(V3 dual, V3 next, Relax& last) {
     last.step = step; last.weight = weight; last.point = dual;
     return mk3(dual.x + weight * step.x, dual.y + weight * step.y, dual.z + weight * step.z);
 }
-NKB_DEV void multiplier_steps_iso(V3 dual, V3 next, float scale, float dual_scale, float rho, float mu, float& normal, float& tangent) {
-    normal = scale > 0.0f && dual_scale != 0.0f ? __fdividef(fabsf(next.x - dual.x), scale) : 0.0f;
+NKB_DEV void multiplier_steps_iso(V3 dual, V3 next, float rho, float mu, float& normal, float& tangent) {
+    normal = rho > 0.0f ? __fdividef(fabsf(next.x - dual.x), rho) : 0.0f;
     const float dy = next.y - dual.y, dz = next.z - dual.z;
     tangent = mu > 0.0f && rho > 0.0f ? __fdividef(sqrtf(fmaf(dy, dy, dz * dz)), rho) : 0.0f;
 }
-// sum over axes of (point - next)(next - base) / metric, metric = (scale, rho, rho) for a cone head with mu > 0
-NKB_DEV double momentum_restart_iso(V3 point, V3 next, V3 base, float scale, float rho, bool cone) {
-    double r = 0.0;
-    if (scale > 0.0f) r += ((double)point.x - next.x) * ((double)next.x - base.x) * (double)__frcp_rn(scale);
-    if (cone && rho > 0.0f)
-        r += (((double)point.y - next.y) * ((double)next.y - base.y) + ((double)point.z - next.z) * ((double)next.z - base.z)) * (double)__frcp_rn(rho);
-    return r;
+// sum over axes of (point - next)(next - base) / rho, the tangential axes for a cone head with mu > 0
+NKB_DEV double momentum_restart_iso(V3 point, V3 next, V3 base, float rho, bool cone) {
+    if (!(rho > 0.0f)) return 0.0;
+    double r = ((double)point.x - next.x) * ((double)next.x - base.x);
+    if (cone) r += ((double)point.y - next.y) * ((double)next.y - base.y) + ((double)point.z - next.z) * ((double)next.z - base.z);
+    return r * (double)__frcp_rn(rho);
 }
 NKB_DEV V3 extrapolate_dual_iso(V3 base, V3 next, float beta, float lower, float upper, bool contact, float mu) {
     if (beta == 0.0f) return next;

@@ -70,6 +70,7 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     const LbvhScratch s = lbvh_bind(e, B);
     // ---- scene bound of the box centres (min and max fold exactly in any order) ----
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+#pragma unroll 1
     for (uint32_t b = lane; b < B; b += 32u) {
         const float* a = sm_aabb(e, b);
 #pragma unroll
@@ -82,6 +83,7 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     float inv[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) inv[k] = mx[k] > mn[k] ? 1.0f / (mx[k] - mn[k]) : 0.0f;
+#pragma unroll 1
     for (uint32_t b = lane; b < P; b += 32u) {
         uint32_t code = 0xffffffffu;            // padding sorts to the end
         if (b < B) {
@@ -92,8 +94,11 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     }
     __syncwarp();
     // ---- bitonic sort of (code, body row): ascending, ties by row, i.e. the order a stable radix sort of the codes gives ----
+#pragma unroll 1
     for (uint32_t k = 2u; k <= P; k <<= 1u)
+#pragma unroll 1
         for (uint32_t j = k >> 1u; j > 0u; j >>= 1u) {
+#pragma unroll 1
             for (uint32_t x = lane; x < P; x += 32u) {
                 const uint32_t y = x ^ j;
                 if (y > x) {
@@ -106,11 +111,13 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
         }
     // ---- internal nodes (Karras 2012) ----
     const int n = (int)B;
+#pragma unroll 1
     for (uint32_t i0 = lane; i0 < I; i0 += 32u) {
         const int i = (int)i0;
         const int d = lbvh_delta(s.code, i, i + 1, n) >= lbvh_delta(s.code, i, i - 1, n) ? 1 : -1;
         const int delta_min = lbvh_delta(s.code, i, i - d, n);
         int l_max = 2;
+#pragma unroll 1
         while (lbvh_delta(s.code, i, i + l_max * d, n) > delta_min) l_max <<= 1;
         int l = 0;
         for (int step = l_max >> 1; step >= 1; step >>= 1)
@@ -132,8 +139,10 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     }
     __syncwarp();
     // ---- bounds: a node merges its children once both are final; passes repeat until the root is (height of the tree) ----
+#pragma unroll 1
     for (uint32_t pass = 0u; pass < B; ++pass) {
         bool changed = false;
+#pragma unroll 1
         for (uint32_t i0 = lane; i0 < I; i0 += 32u) {
             if (s.ready[i0] != 0u) continue;
             const uint32_t c0 = s.child[2u * i0], c1 = s.child[2u * i0 + 1u];
@@ -149,6 +158,7 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
         }
         __syncwarp();
         // boxes written in this pass become visible to the next one only: a node never reads a sibling written in the same pass
+#pragma unroll 1
         for (uint32_t i0 = lane; i0 < I; i0 += 32u) if (s.ready[i0] == 1u) s.ready[i0] = 2u;
         __syncwarp();
         if (!__any_sync(NKB_FULL, changed)) break;
@@ -156,6 +166,7 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     // ---- walk: lane = sorted leaf; on a miss or after a leaf the walk jumps to the right child of the node whose split lies after
     //      the subtree's last leaf, so no stack is kept ----
     const uint32_t kEnd = 0xffffffffu;
+#pragma unroll 1
     for (uint32_t k0 = 0u; k0 < B; k0 += 32u) {
         const uint32_t k = k0 + lane;
         if (k < B) {
@@ -163,10 +174,12 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
             const float* q = sm_aabb(e, a);
             const float q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
             uint32_t* row = s.partners + a * W;
+#pragma unroll 1
             for (uint32_t w = 0u; w < W; ++w) row[w] = 0u;
             const uint32_t* adm = t.adm_mask + a * W;
             uint32_t node = 0u;                     // the root
             uint32_t guard = 4u * B;                // a walk visits each node at most once
+#pragma unroll 1
             while (node != kEnd && guard-- != 0u) {
                 const bool leaf = node >= I;
                 const uint32_t last = leaf ? node - I : s.range[2u * node + 1u];
@@ -185,6 +198,7 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
     // ---- emit: bodies in row order, partners in bit order ----
     uint32_t count = 0u;
     uint32_t* pairs = sm_pairs(e);
+#pragma unroll 1
     for (uint32_t a0 = 0u; a0 < B; a0 += 32u) {
         const uint32_t a = a0 + lane;
         uint32_t mine = 0u;
@@ -194,8 +208,10 @@ NKB_DEV uint32_t stage_pairs_lbvh(Env& e) {
         for (int o = 1; o < 32; o <<= 1) { const uint32_t up = __shfl_up_sync(NKB_FULL, scan, o); if ((int)lane >= o) scan += up; }
         uint32_t at = count + scan - mine;
         if (a < B)
+#pragma unroll 1
             for (uint32_t w = 0u; w < W; ++w) {
                 uint32_t bits = s.partners[a * W + w];
+#pragma unroll 1
                 while (bits != 0u) {
                     const uint32_t b = 32u * w + (uint32_t)__ffs(bits) - 1u;
                     bits &= bits - 1u;

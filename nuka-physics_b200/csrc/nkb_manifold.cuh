@@ -258,6 +258,7 @@ NKB_DEV uint32_t pair_class(uint32_t ka, uint32_t kb) {
 
 // The lowest `want` set bits of `mask`: lane index of the g-th (g < want), or 32.
 NKB_DEV uint32_t nth_set_bit(uint32_t mask, uint32_t g) {
+#pragma unroll 1
     for (uint32_t k = 0u; k < g; ++k) mask &= mask - 1u;
     return mask != 0u ? (uint32_t)__ffs(mask) - 1u : 32u;
 }
@@ -539,6 +540,7 @@ static __device__ __noinline__ void box_box_group(PairCtx c, bool active, uint32
 NKB_DEV void narrowphase_frames(Env& e) {
     const TemplateView& t = *e.t;
     const PairCtx c = pair_ctx(e, 0.f);
+#pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         const float* bp = sm_bpose(e, b);
         const Q4 q = ldq(bp + 3);
@@ -557,6 +559,7 @@ NKB_DEV void narrowphase_range(Env& e, uint32_t pair_count, uint32_t first, uint
     const uint32_t S = t.slot_cap, lane = e.lane;          // slots past the admissible-pair count can never fill and have no storage
     PairCtx c = pair_ctx(e, separation);
     c.stage_shift = 64u * first;
+#pragma unroll 1
     for (uint32_t base = 32u * first; base < S; base += 32u * stride) {
         const uint32_t s = base + lane;
         const bool live = s < pair_count;
@@ -581,6 +584,7 @@ NKB_DEV void narrowphase_range(Env& e, uint32_t pair_count, uint32_t first, uint
             ctx_count(c)[s] = count;
         }
         // box on plane: four pairs per pass, eight lanes each
+#pragma unroll 1
         for (uint32_t todo = __ballot_sync(NKB_FULL, cls == kClassBoxPlane); todo != 0u;) {
             const uint32_t owner = nth_set_bit(todo, lane >> 3);
             const bool active = owner < 32u;
@@ -591,6 +595,7 @@ NKB_DEV void narrowphase_range(Env& e, uint32_t pair_count, uint32_t first, uint
             for (int k = 0; k < 4 && todo != 0u; ++k) todo &= todo - 1u;
         }
         // cylinder on plane: two pairs per pass, sixteen lanes each
+#pragma unroll 1
         for (uint32_t todo = __ballot_sync(NKB_FULL, cls == kClassCylinderPlane); todo != 0u;) {
             const uint32_t owner = nth_set_bit(todo, lane >> 4);
             const bool active = owner < 32u;
@@ -601,6 +606,7 @@ NKB_DEV void narrowphase_range(Env& e, uint32_t pair_count, uint32_t first, uint
             for (int k = 0; k < 2 && todo != 0u; ++k) todo &= todo - 1u;
         }
         // box on box: two pairs per pass, sixteen lanes each
+#pragma unroll 1
         for (uint32_t todo = __ballot_sync(NKB_FULL, cls == kClassBoxBox); todo != 0u;) {
             const uint32_t owner = nth_set_bit(todo, lane >> 4);
             const bool active = owner < 32u;

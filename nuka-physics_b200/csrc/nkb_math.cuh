@@ -207,6 +207,23 @@ NKB_DEV float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
     return v;
 }
+NKB_DEV double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
+    return v;
+}
+// Two sums over the warp at the price of one and two broadcasts: the halves of the warp carry one each after the first exchange.
+NKB_DEV void warp_sum2(float& a, float& b, uint32_t lane) {
+    const bool upper = (lane & 16u) != 0u;
+    float keep = upper ? b : a;
+    keep += __shfl_xor_sync(NKB_FULL, upper ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(NKB_FULL, keep, o);
+    a = __shfl_sync(NKB_FULL, keep, 0);
+    b = __shfl_sync(NKB_FULL, keep, 16);
+}
+// Largest of non-negative values (their bit patterns order like the values).
+NKB_DEV float warp_max_positive(float v) { return __uint_as_float(__reduce_max_sync(NKB_FULL, __float_as_uint(v))); }
 NKB_DEV float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(NKB_FULL, v, o));

@@ -9,25 +9,30 @@
 
 namespace nkb {
 
-// head fields (word offsets inside a head record)
+// Head fields (word offsets inside a head record).  A record is 15 groups of four words: every vector starts on a 16-byte
+// boundary and the scalars that are read with it fill its fourth word, so a row evaluation takes a head in four or five
+// vector loads.  60 words put the eight lanes of a quarter warp in distinct bank groups for such loads.
 enum HeadField : uint32_t {
-    HF_FLAGS = 0, HF_OWNER, HF_REF, HF_JOFF, HF_UNITV,
-    HF_RHO, HF_RSD, HF_RSR, HF_LOWER, HF_UPPER, HF_MU, HF_NB, HF_PEN, HF_RHS,
-    HF_DUAL, HF_BASE = HF_DUAL + 3, HF_RES = HF_BASE + 3, HF_MOVE = HF_RES + 3, HF_STEP = HF_MOVE + 3,
-    HF_RXS = HF_STEP + 3, HF_RXW = HF_RXS + 3, HF_RXP,
-    HF_N = HF_RXP + 3, HF_T1 = HF_N + 3, HF_T2 = HF_T1 + 3, HF_RA = HF_T2 + 3, HF_RB = HF_RA + 3,
-    HF_LAM = HF_RB + 3,          // physical multipliers after the velocity solve
-    HF_F = HF_LAM + 3,           // response impulse, curvature (xx, yy, zz, yz) and noise scale at the current move
-    HF_C = HF_F + 3, HF_NZ = HF_C + 4,
-    HF_COUNT = HF_NZ + 3
+    HF_DUAL = 0, HF_RHO = 3, HF_RES = 4, HF_MU = 7, HF_MOVE = 8, HF_LOWER = 11, HF_STEP = 12, HF_UPPER = 15,
+    HF_F = 16,                   // response impulse at the current move,
+    HF_C = 19,                   // its curvature (xx, yy, zz, yz)
+    HF_NZ = 23,                  // and its noise scale
+    HF_FLAGS = 26, HF_OWNER = 27,
+    HF_N = 28, HF_PEN = 31, HF_T1 = 32, HF_RHS = 35, HF_T2 = 36, HF_JOFF = 39, HF_RA = 40, HF_REF = 43, HF_RB = 44, HF_RXW = 47,
+    HF_BASE = 48, HF_LAMX = 51, HF_RXS = 52, HF_LAMY = 55, HF_RXP = 56, HF_LAMZ = 59,    // LAM: physical multipliers after the velocity solve
+    HF_COUNT = 60,
+    HF_UNITV = HF_N              // a single-coordinate row's entry; such a row has no contact frame
 };
 constexpr uint32_t kNoBlock16 = 0xffffu;
 constexpr uint32_t kUnitRow = 0x80000000u;   // HF_JOFF: unit row on coordinate (value & 0xffff)
 
-// heads are records of kHeadStride words (odd, so one lane per head is conflict-free and fields are immediate offsets)
 NKB_DEV float& hf(const Env& e, uint32_t field, uint32_t h) { return e.sm[e.lay->heads + h * kHeadStride + field]; }
 NKB_DEV uint32_t& hu(const Env& e, uint32_t field, uint32_t h) { return reinterpret_cast<uint32_t*>(e.sm)[e.lay->heads + h * kHeadStride + field]; }
-NKB_DEV V3 hf3(const Env& e, uint32_t field, uint32_t h) { return mk3(hf(e, field, h), hf(e, field + 1u, h), hf(e, field + 2u, h)); }
+// the group of four words that starts at `field` (a multiple of 4)
+NKB_DEV float4& hq(const Env& e, uint32_t field, uint32_t h) { return *reinterpret_cast<float4*>(&hf(e, field, h)); }
+NKB_DEV V3 hf3(const Env& e, uint32_t field, uint32_t h) { const float4 q = hq(e, field, h); return mk3(q.x, q.y, q.z); }
+NKB_DEV V3 head_lambda(const Env& e, uint32_t h) { return mk3(hf(e, HF_LAMX, h), hf(e, HF_LAMY, h), hf(e, HF_LAMZ, h)); }
+NKB_DEV void set_head_lambda(const Env& e, uint32_t h, V3 v) { hf(e, HF_LAMX, h) = v.x; hf(e, HF_LAMY, h) = v.y; hf(e, HF_LAMZ, h) = v.z; }
 NKB_DEV void hst3(const Env& e, uint32_t field, uint32_t h, V3 v) { hf(e, field, h) = v.x; hf(e, field + 1u, h) = v.y; hf(e, field + 2u, h) = v.z; }
 NKB_DEV float* sm_jpool(const Env& e) { return e.sm + e.lay->jpool; }
 
@@ -63,6 +68,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
     const bool position_pass = t.cfg.pos_iters > 0u;
     uint32_t nheads = 0u, npoints = 0u;
     // contact heads in slot order
+#pragma unroll 1
     for (uint32_t base = 0u; base < S; base += 32u) {
         const uint32_t s = base + lane;
         const uint32_t cnt = (s < S && s < pair_count) ? sm_ccount(e)[s] : 0u;
@@ -79,6 +85,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             if (oa < t.B) com_a = ld3(sm_bpose(e, a)) + qrot(ldq(sm_bpose(e, a) + 3), ld3(t.inertial_pos + 3u * a));
             if (ob < t.B) com_b = ld3(sm_bpose(e, b)) + qrot(ldq(sm_bpose(e, b) + 3), ld3(t.inertial_pos + 3u * b));
             const float mu = fmaxf(__ldg(t.mu + a), __ldg(t.mu + b));
+#pragma unroll 1
             for (uint32_t p = 0u; p < cnt; ++p) {
                 const uint32_t h = first + p, at = s * 4u + p;
                 if (h >= t.head_cap || h >= t.point_cap) { e.status |= kStatusHeadOverflow; continue; }
@@ -98,7 +105,6 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
                 hu(e, HF_OWNER, h) = oa | (own1 << 16);
                 hu(e, HF_REF, h) = at | (la != kNoLink ? (la << 16) : 0xffff0000u);
                 hu(e, HF_JOFF, h) = lb != kNoLink ? lb : 0xffffu;      // side-b link, pool offset is filled below
-                hf(e, HF_UNITV, h) = 0.f;
                 hf(e, HF_LOWER, h) = 0.f; hf(e, HF_UPPER, h) = FLT_MAX; hf(e, HF_MU, h) = mu;
                 hf(e, HF_PEN, h) = depth;
                 hf(e, HF_RHS, h) = (fminf(depth, 0.0f) + (position_pass ? 0.0f : fminf(fmaxf(cd, 0.0f), t.cfg.overlap_recovery_velocity * dt))) / (dt * dt);
@@ -141,8 +147,13 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             }
         }
         float* pool = sm_jpool(e);
+#pragma unroll 1
         for (uint32_t h = 0u; h < ncontact; ++h) {
             const uint32_t ref = hu(e, HF_REF, h), la = ref >> 16, lb = hu(e, HF_JOFF, h) & 0xffffu;
+            if (la != 0xffffu && lb != 0xffffu) {
+                const uint32_t ma = __ldg(t.anc_mask + la), mb = __ldg(t.anc_mask + lb);
+                e.branching |= (ma & ~mb) != 0u && (mb & ~ma) != 0u;
+            }
             __syncwarp();      // every lane has read the side-b link before lane 0 replaces it with the pool offset
             const uint32_t n4 = (n + 3u) & ~3u, joff = h * 3u * n4;
             const V3 point = ld3(sm_cpoint(e, ref & 0xffffu));
@@ -176,6 +187,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
     }
     __syncwarp();
     // joint rows, lane = link: limit lower/upper, dry friction, drive (ops/assemble_rows.cu:805-971)
+#pragma unroll 1
     for (uint32_t kind = 0u; kind < 4u; ++kind) {
         bool emit = false;
         float lower = 0.f, upper = 0.f, rhs = 0.f, pen = 0.f, unitv = 1.f, lambda = 0.f;
@@ -207,6 +219,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(NKB_FULL, incl, o); if ((int)lane >= o) incl += v; }
             const uint32_t first = nheads + incl - cnt;
             const uint32_t total = __shfl_sync(NKB_FULL, incl, 31);
+#pragma unroll 1
             for (uint32_t side = 0u; side < 2u; ++side) {
                 if (!(lf & (1u << side))) continue;
                 const uint32_t h = first + ((side == 1u && (lf & 1u)) ? 1u : 0u);
@@ -227,7 +240,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
                 // :366-383 covers the contact rows alone)
                 const float carried = e.s->limit_lambda[((size_t)e.env * L + lane) * 2u + side];
                 hst3(e, HF_DUAL, h, mk3(carried, 0.f, 0.f));
-                hst3(e, HF_LAM, h, mk3(carried, 0.f, 0.f));
+                set_head_lambda(e, h, mk3(carried, 0.f, 0.f));
             }
             nheads = min(nheads + total, t.head_cap);
             ++kind;       // kind 1 handled here
@@ -263,6 +276,7 @@ NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t 
     const TemplateView& t = *e.t;
     const uint32_t npts = t.cfg.max_contacts * 4u;
     const CacheEntry* cache = e.s->cache + (size_t)e.env * npts;
+#pragma unroll 1
     for (uint32_t h = first; h < nheads; h += stride) {
         if (!(hu(e, HF_FLAGS, h) & kHeadContact)) break;     // contact heads come first
         const uint32_t at = hu(e, HF_REF, h) & 0xffffu;
@@ -271,6 +285,7 @@ NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t 
         const unsigned long long feat = (unsigned long long)f[0] | ((unsigned long long)f[1] << 32);
         // an earlier current point with the same identity owns the match
         bool dup = false;
+#pragma unroll 1
         for (uint32_t base = 0u; base < h; base += 32u) {
             const uint32_t j = base + e.lane;
             bool same = false;
@@ -282,6 +297,7 @@ NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t 
         }
         if (dup) continue;
         uint32_t found = 0xffffffffu;
+#pragma unroll 1
         for (uint32_t base = 0u; base < npts && found == 0xffffffffu; base += 32u) {
             const uint32_t c = base + e.lane;
             const bool hit = c < npts && cache[c].pair == pair && cache[c].feature == feat && cache[c].age < 2u;
@@ -310,11 +326,13 @@ NKB_DEV void cache_owners_range(Env& e, uint32_t ncontact, uint32_t first, uint3
     const TemplateView& t = *e.t;
     const uint32_t stage_cap = min(t.point_cap, t.slot_cap * 4u);
     uint32_t* owner = reinterpret_cast<uint32_t*>(reinterpret_cast<CacheEntry*>(e.sm + e.lay->cstage) + stage_cap);
+#pragma unroll 1
     for (uint32_t h = first; h < ncontact; h += stride) {
         const uint32_t at = hu(e, HF_REF, h) & 0xffffu;
         const uint32_t pair = head_pair(e, h);
         const uint32_t* f = sm_cfeat(e, at);
         bool dup = false;
+#pragma unroll 1
         for (uint32_t base = 0u; base < h; base += 32u) {
             const uint32_t j = base + e.lane;
             bool same = false;
@@ -339,10 +357,12 @@ NKB_DEV void stage_cache_commit(Env& e, uint32_t nheads, Owners&& owners) {
     const uint32_t nown = t.slot_cap * 4u;
     const uint32_t stage_cap = min(t.point_cap, nown);
     uint32_t* owner = reinterpret_cast<uint32_t*>(stage + stage_cap);
+#pragma unroll 1
     for (uint32_t c = e.lane; c < nown; c += 32u) owner[c] = 0xffffffffu;
     __syncwarp();
     // owners: first current point of each identity
     uint32_t ncontact = 0u;
+#pragma unroll 1
     for (uint32_t base = 0u; base < nheads; base += 32u) {          // contact heads come first
         const uint32_t h = base + e.lane;
         const uint32_t m = __ballot_sync(NKB_FULL, h < nheads && (hu(e, HF_FLAGS, h) & kHeadContact) != 0u);
@@ -353,6 +373,7 @@ NKB_DEV void stage_cache_commit(Env& e, uint32_t nheads, Owners&& owners) {
     __syncwarp();
     // retained old entries in ascending cache order
     uint32_t nret = 0u;
+#pragma unroll 1
     for (uint32_t base = 0u; base < npts; base += 32u) {
         const uint32_t c = base + e.lane;
         bool keep = false;
@@ -361,10 +382,12 @@ NKB_DEV void stage_cache_commit(Env& e, uint32_t nheads, Owners&& owners) {
         if (c < npts) {
             en = cache[c];
             keep = en.pair != 0xffffffffu && en.age < 1u;
+#pragma unroll 1
             for (uint32_t h = 0u; h < ncontact && keep; ++h) {
                 const uint32_t* f = sm_cfeat(e, hu(e, HF_REF, h) & 0xffffu);
                 if (head_pair(e, h) == en.pair && (((unsigned long long)f[1] << 32) | f[0]) == en.feature) keep = false;
             }
+#pragma unroll 1
             for (uint32_t d = 0u; d < c && keep; ++d) if (cache[d].pair == en.pair && cache[d].feature == en.feature) keep = false;
         }
         const uint32_t m = __ballot_sync(NKB_FULL, keep);
@@ -375,6 +398,7 @@ NKB_DEV void stage_cache_commit(Env& e, uint32_t nheads, Owners&& owners) {
     __syncwarp();
     // write the new cache: owners at their own point, retained entries into the free points in order
     uint32_t free_seen = 0u;
+#pragma unroll 1
     for (uint32_t base = 0u; base < npts; base += 32u) {
         const uint32_t c = base + e.lane;
         const bool is_free = c < npts && (c >= nown || owner[c] == 0xffffffffu);
@@ -385,7 +409,7 @@ NKB_DEV void stage_cache_commit(Env& e, uint32_t nheads, Owners&& owners) {
                 const uint32_t h = owner[c];
                 const uint32_t* f = sm_cfeat(e, c);
                 en.pair = head_pair(e, h); en.feature = ((unsigned long long)f[1] << 32) | f[0]; en.age = 0u;
-                const V3 lam = hf3(e, HF_LAM, h);
+                const V3 lam = head_lambda(e, h);
                 en.lambda[0] = lam.x; en.lambda[1] = lam.y; en.lambda[2] = lam.z;
                 const V3 nn = ld3(sm_cnormal(e, c));
                 en.normal[0] = nn.x; en.normal[1] = nn.y; en.normal[2] = nn.z;

@@ -10,10 +10,11 @@
 #pragma once
 #include "nkb_laws.cuh"
 #include "nkb_rows.cuh"
+#include "nkb_tree.cuh"
 
 namespace nkb {
 
-static_assert(HF_COUNT == kHeadWords, "head field count must match the host layout");
+static_assert(HF_COUNT == kHeadStride, "head record must match the host layout");
 
 constexpr uint32_t kNewtonSteps = 16u, kLineSteps = 32u;
 constexpr float kLineTol = 1.0e-6f, kRoundings = 8.0f;
@@ -137,8 +138,10 @@ NKB_DEV float mass_coupling_unit(const Env& e, uint32_t at, float value) {
     const float* F = sm_factor(e);
     float y[32 * NR];
     float r = 0.f;
+#pragma unroll 1
     for (uint32_t i = at; i < n; ++i) {
         float a = i == at ? value : 0.f;
+#pragma unroll 1
         for (uint32_t j = at; j < i; ++j) a -= F[i * ld + j] * y[j];
         y[i] = a;
         r += a * a / F[i * ld + i];
@@ -148,7 +151,7 @@ NKB_DEV float mass_coupling_unit(const Env& e, uint32_t at, float value) {
 
 // The same for dense rows (contact rows against the articulation), all lanes on one row at a time: lane = coordinate
 // in the forward solve, then lane = row adds its row's terms in coordinate order, so the sum is the sequential one.
-// Results land in HF_RSD of each head (a field init_heads fills afterwards).
+// Results land in HF_RHO of each head (a field init_heads fills afterwards).
 template <int NR>
 NKB_DEV void mass_coupling_dense(Env& e, const Tile& tile) {
     const TemplateView& t = *e.t;
@@ -160,6 +163,7 @@ NKB_DEV void mass_coupling_dense(Env& e, const Tile& tile) {
     float diag[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) { const uint32_t c = l + 32u * r; diag[r] = c < n ? F[c * ld + c] : 1.f; }
+#pragma unroll 1
     for (uint32_t base = 0u; base < tile.nheads; base += 32u) {
         const uint32_t h = base + l;
         bool dense = false;
@@ -168,6 +172,7 @@ NKB_DEV void mass_coupling_dense(Env& e, const Tile& tile) {
             dense = ((o & 0xffffu) == t.B || (o >> 16) == t.B) && !(hu(e, HF_JOFF, h) & kUnitRow);
         }
         uint32_t todo = __ballot_sync(NKB_FULL, dense);
+#pragma unroll 1
         while (todo != 0u) {
             uint32_t in_batch = 0u, mine = 0xffffffffu;
 #pragma unroll 1
@@ -191,8 +196,9 @@ NKB_DEV void mass_coupling_dense(Env& e, const Tile& tile) {
             __syncwarp();
             if (mine != 0xffffffffu) {
                 float r = 0.f;
+#pragma unroll 1
                 for (uint32_t i = 0u; i < n; ++i) r += terms[mine * n + i];
-                hf(e, HF_RSD, h) = r;
+                hf(e, HF_RHO, h) = r;
             }
             __syncwarp();
         }
@@ -204,18 +210,20 @@ template <int NR>
 NKB_DEV void init_heads(Env& e, const Tile& tile) {
     const TemplateView& t = *e.t;
     mass_coupling_dense<NR>(e, tile);
+#pragma unroll 1
     for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
         float shares[2] = {0.f, 0.f};
         const uint32_t fl = hu(e, HF_FLAGS, h);
         const uint32_t jo = hu(e, HF_JOFF, h);
         bool valid = true;
+#pragma unroll 1
         for (uint32_t side = 0u; side < 2u; ++side) {
             const uint32_t ob = head_owner(e, h, side);
             float c = 0.f;
             if (ob == kNoBlock16) { /* static or kinematic side: no response */ }
             else if (ob == t.B) {
                 if (jo & kUnitRow) c = mass_coupling_unit<NR>(e, jo & 0xffffu, hf(e, HF_UNITV, h));
-                else c = hf(e, HF_RSD, h);
+                else c = hf(e, HF_RHO, h);
             } else {
                 const V3 dir = hf3(e, HF_N, h) * (side == 0u ? 1.f : -1.f);
                 const V3 ang = cross(hf3(e, side == 0u ? HF_RA : HF_RB, h), dir);
@@ -230,9 +238,7 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
         const float cap = 100.0f / largest;
         float rho = response > 0.f ? fminf(cap, coupled) : 0.f;
         if (!(response == 0.f || (response > 0.f && rho > 0.f && rho <= FLT_MAX))) { e.status |= kStatusSolverFailure; rho = nanf(""); }
-        const Resp rs = scalar_response(rho, 0.0f);
-        hf(e, HF_RHO, h) = rho; hf(e, HF_RSD, h) = rs.dual_scale; hf(e, HF_RSR, h) = rs.residual_scale;
-        hf(e, HF_NB, h) = 0.f;
+        hf(e, HF_RHO, h) = rho;
         hst3(e, HF_BASE, h, hf3(e, HF_DUAL, h));
         hst3(e, HF_RES, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_STEP, h, mk3(0.f, 0.f, 0.f));
         hst3(e, HF_RXS, h, mk3(0.f, 0.f, 0.f)); hf(e, HF_RXW, h) = 0.f; hst3(e, HF_RXP, h, mk3(0.f, 0.f, 0.f));
@@ -246,8 +252,10 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
     const uint32_t nb = tile.nblocks;
     uint32_t* inc = blk_inc(e, nb);
     uint32_t at = 0u;
+#pragma unroll 1
     for (uint32_t b = 0u; b < nb; ++b) {
         if (e.lane == 0u) blk_inc_begin(e, nb, b) = at;
+#pragma unroll 1
         for (uint32_t base = 0u; base < tile.nheads; base += 32u) {
             const uint32_t h = base + e.lane;
             bool hit = false;
@@ -259,8 +267,10 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
     }
     if (e.lane == 0u) blk_inc_begin(e, nb, nb) = at;
     uint16_t* utab = unit_table(e, nb);
+#pragma unroll 1
     for (uint32_t k = e.lane; k < 4u * e.vstride; k += 32u) utab[k] = (uint16_t)kNoUnitHead;
     __syncwarp();
+#pragma unroll 1
     for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
         const uint32_t jo = hu(e, HF_JOFF, h), o = hu(e, HF_OWNER, h), fl = hu(e, HF_FLAGS, h);
         if (!(jo & kUnitRow) || ((o & 0xffffu) != e.t->B && (o >> 16) != e.t->B)) continue;
@@ -275,6 +285,7 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
         if (blk_dim(e, b) == 0u) { if (e.lane == 0u) blk_color(e, nb, b) = 0xffffffffu; continue; }
         uint32_t taken = 0u;
         const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
+#pragma unroll 1
         for (uint32_t k = ib + e.lane; k < ie; k += 32u) {
             const uint32_t o = hu(e, HF_OWNER, inc[k]);
             const uint32_t first = o & 0xffffu, second = o >> 16;
@@ -309,11 +320,14 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
 NKB_DEV void init_residuals(Env& e, const Tile& tile) {
     const TemplateView& t = *e.t;
     const float dt = t.cfg.dt;
+#pragma unroll 1
     for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
         const uint32_t axes = head_axes(e, h);
         V3 res = mk3(0.f, 0.f, 0.f);
+#pragma unroll 1
         for (uint32_t ax = 0u; ax < axes; ++ax) {
             float along = 0.f;
+#pragma unroll 1
             for (uint32_t side = 0u; side < 2u; ++side) {
                 const uint32_t b = head_owner(e, h, side);
                 if (b == kNoBlock16) continue;
@@ -333,23 +347,24 @@ NKB_DEV uint32_t pad_ld(uint32_t n) { const uint32_t ld = (n + 3u) & ~3u; return
 // Register copy of one head for the row evaluations.
 struct HeadRegs {
     V3 dual, res, move, step;
-    float rho, lower, upper, rsd, rsr, mu, nb;
-    bool cone;      // three-axis contact head
+    float rho, lower, upper, mu;
+    bool cone;      // contact head with friction (the position pass clears the coefficient of its scalar rows)
 };
 NKB_DEV HeadRegs load_head(const Env& e, uint32_t h) {
     HeadRegs r;
-    r.dual = hf3(e, HF_DUAL, h); r.res = hf3(e, HF_RES, h); r.move = hf3(e, HF_MOVE, h); r.step = hf3(e, HF_STEP, h);
-    r.rho = hf(e, HF_RHO, h); r.lower = hf(e, HF_LOWER, h); r.upper = hf(e, HF_UPPER, h);
-    r.rsd = hf(e, HF_RSD, h); r.rsr = hf(e, HF_RSR, h); r.mu = hf(e, HF_MU, h); r.nb = hf(e, HF_NB, h);
-    r.cone = head_axes(e, h) == 3u;
+    const float4 dual = hq(e, HF_DUAL, h), res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h), step = hq(e, HF_STEP, h);
+    r.dual = mk3(dual.x, dual.y, dual.z); r.res = mk3(res.x, res.y, res.z);
+    r.move = mk3(move.x, move.y, move.z); r.step = mk3(step.x, step.y, step.z);
+    r.rho = dual.w; r.mu = res.w; r.lower = move.w; r.upper = step.w;
+    r.cone = r.mu > 0.f;
     return r;
 }
+// The friction cone's radius follows the head's normal multiplier at the start of the descent, which the descent leaves as it is.
 NKB_DEV void respond(const HeadRegs& r, V3 move, V3& f, float& cxx, float& cyy, float& czz, float& cyz) {
-    const Resp rs = {r.rsd, r.rsr};
-    const STerm n = scalar_impulse(r.dual.x, r.rho, r.res.x - move.x, r.lower, r.upper, rs);
+    const STerm n = scalar_impulse(r.dual.x, r.rho, r.res.x - move.x, r.lower, r.upper);
     f = mk3(n.impulse, 0.f, 0.f);
     cxx = n.curvature; cyy = czz = cyz = 0.f;
-    if (r.cone) cone_impulse(r.dual, r.rho, r.res.y - move.y, r.res.z - move.z, r.nb, r.mu, f.y, f.z, cyy, czz, cyz);
+    if (r.cone) cone_impulse(r.dual, r.rho, r.res.y - move.y, r.res.z - move.z, r.dual.x, r.mu, f.y, f.z, cyy, czz, cyz);
 }
 
 // Row steps J d of a block's incident heads (block_descent_tile.cuh:2019-2044); lane = head, d staged in shared
@@ -552,11 +567,11 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         Mr[r] = artic ? sm_mass(e) + (coord[r] ? c : 0u) * e.lay->ld : m6 + (coord[r] ? c : 0u) * 12u;
     }
     bool coupled = false;
+#pragma unroll 1
     for (uint32_t k = ib + l; k < ie; k += 32u) {
         const uint32_t h = inc[k];
         const uint32_t o = hu(e, HF_OWNER, h);
         coupled |= (o & 0xffffu) != kNoBlock16 && (o >> 16) != kNoBlock16;
-        hf(e, HF_NB, h) = hf(e, HF_DUAL, h);
         hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f));
     }
     coupled = __any_sync(NKB_FULL, coupled);
@@ -654,7 +669,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                     const uint32_t hs = inc[k];
                     const uint32_t jo = hu(e, HF_JOFF, hs);
                     if (artic && (jo & kUnitRow)) continue;
-                    const V3 f = hf3(e, HF_F, hs), nz = hf3(e, HF_NZ, hs);
+                    const V3 f = hf3(e, HF_F, hs), nz = mk3(hf(e, HF_NZ, hs), hf(e, HF_NZ + 1u, hs), hf(e, HF_NZ + 2u, hs));
                     const float c0 = hf(e, HF_C, hs), c1 = hf(e, HF_C + 1u, hs), c2 = hf(e, HF_C + 2u, hs), c12 = hf(e, HF_C + 3u, hs);
                     if (!(f.x != 0.f || f.y != 0.f || f.z != 0.f || c0 != 0.f || c1 != 0.f || c2 != 0.f || c12 != 0.f || nz.x != 0.f || nz.y != 0.f || nz.z != 0.f)) continue;
                     const float* jr; uint32_t js;
@@ -858,6 +873,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         apply_moves(e, tile, b, alpha);
         if (rounded) break;
     }
+#pragma unroll 1
     for (uint32_t k = ib + l; k < ie; k += 32u) {
         const uint32_t h = inc[k];
         const V3 res = hf3(e, HF_RES, h), move = hf3(e, HF_MOVE, h);
@@ -873,6 +889,355 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     tile.residual = fmaxf(tile.residual, fmaxf(primal, coupled ? moved : 0.f));
 #pragma unroll
     for (int r = 0; r < NR; ++r) if (coord[r]) velocity[l + 32u * r] = u[r];
+    __syncwarp();
+}
+
+// One evaluation of a block's constraint rows at step length alpha (lane = head, as many passes as the block has heads):
+// sums the line's slope, curvature and rounding magnitude, and leaves every head's impulse, curvature and noise scale at the
+// trial point in its record, where the assembly of the next Newton system finds them.
+NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint32_t ie, float alpha, double& slope, float& curvature, float& magnitude) {
+    slope = 0.0; curvature = 0.f; magnitude = 0.f;
+#pragma unroll 1
+    for (uint32_t k = ib + e.lane; k < ie; k += 32u) {
+        const uint32_t h = inc[k];
+        const float4 dual = hq(e, HF_DUAL, h), res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h), step = hq(e, HF_STEP, h);
+        const float rho = dual.w, lower = move.w, upper = step.w;
+        const V3 trial = mk3(fmaf(alpha, step.x, move.x), fmaf(alpha, step.y, move.y), fmaf(alpha, step.z, move.z));
+        const STerm n = scalar_impulse(dual.x, rho, res.x - trial.x, lower, upper);
+        V3 f = mk3(n.impulse, 0.f, 0.f), noise = mk3(fabsf(n.impulse) + n.curvature * (fabsf(res.x) + fabsf(trial.x)), 0.f, 0.f);
+        float cyy = 0.f, czz = 0.f, cyz = 0.f;
+        slope = fma((double)f.x, (double)step.x, slope);
+        curvature = fmaf(n.curvature * step.x, step.x, curvature);
+        magnitude += fabsf(f.x * step.x);
+        if (res.w > 0.f) {
+            cone_impulse(mk3(dual.x, dual.y, dual.z), rho, res.y - trial.y, res.z - trial.z, dual.x, res.w, f.y, f.z, cyy, czz, cyz);
+            noise.y = fabsf(f.y) + cyy * (fabsf(res.y) + fabsf(trial.y));
+            noise.z = fabsf(f.z) + czz * (fabsf(res.z) + fabsf(trial.z));
+            slope = fma((double)f.y, (double)step.y, slope); slope = fma((double)f.z, (double)step.z, slope);
+            curvature += cyy * step.y * step.y + czz * step.z * step.z + 2.0f * cyz * step.y * step.z;
+            magnitude += fabsf(f.y * step.y) + fabsf(f.z * step.z);
+        }
+        hq(e, HF_F, h) = make_float4(f.x, f.y, f.z, n.curvature);
+        hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
+        *reinterpret_cast<float2*>(&hf(e, HF_NZ + 1u, h)) = make_float2(noise.y, noise.z);
+    }
+    slope = warp_sum(slope);
+    warp_sum2(curvature, magnitude, e.lane);
+}
+
+// The articulation's descent with the Newton system kept in the sparsity of its tree (nkb_tree.cuh).  Same model, stopping
+// rules and exact line search as descend_block; valid while every contact row acts along one root path (Env::branching is
+// false): a row between two branches would fill the matrix in.
+//
+// What bounds it is instruction supply: an SM keeps 32 KB of instructions close and fetches the rest from further away at a
+// half to a sixth of the rate (measured with straight-line code), and the warps of an SM are at different places of their
+// solves.  So the loop is written to be short: one copy of the row evaluation serves the start of a descent, the line search
+// and the next Newton system (it leaves impulses and curvatures in the head records), one pass over the mass matrix per step
+// serves the curvature along the direction and, added up, the inertial force.
+//
+// The block velocity u and the inertial force M (u - u_free) are carried in double for the descent, updated by the step along
+// d and along M d, so that neither has to be recomputed; sums that descend_block compensates in float run in double, one fused
+// multiply-add on the FP64 pipe (half the FP32 rate on this GPU) in place of ten FP32 operations.
+template <int NR>
+NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
+    const TemplateView& t = *e.t;
+    const uint32_t l = e.lane, nb = tile.nblocks, b = t.B, dim = t.ndof;
+    const uint32_t* inc = blk_inc(e, nb);
+    const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
+    if (position && ib == ie) return;
+    const uint32_t chunks = (dim + 3u) >> 2, js = chunks << 2;
+    float* velocity = block_vel(e, b, position);
+    double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
+    float* flat = sm_vec(e, kVecS2);
+    const bool floating = t.floating_root != 0u;
+    const TreeLane tl = tree_lane(e);
+    bool coupled = false;
+#pragma unroll 1
+    for (uint32_t k = ib + l; k < ie; k += 32u) {
+        const uint32_t h = inc[k];
+        const uint32_t o = hu(e, HF_OWNER, h);
+        coupled |= (o & 0xffffu) != kNoBlock16 && (o >> 16) != kNoBlock16;
+        hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_STEP, h, mk3(0.f, 0.f, 0.f));
+    }
+    coupled = __any_sync(NKB_FULL, coupled);
+    // a direction is either a Newton step (step >= 0) or one of the two ways to begin: the first velocity sweep searches
+    // toward the free velocity (-1), the others only need M (u - u_free) and the rows at the start (-2)
+    int step = tile.iteration == 0u && !position ? -1 : -2;
+    bool coord[NR];
+    double u[NR], dir[NR], inertial[NR];
+    float force[NR];
+    uint32_t units[NR][2];              // this coordinate's single-coordinate rows: heads by slot, two per word
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const uint32_t c = l + 32u * r;
+        coord[r] = c < dim;
+        u[r] = coord[r] ? velocity[c] : 0.0;
+        const double fr = coord[r] && !position ? (double)block_free(e, b)[c] : 0.0;
+        dir[r] = step == -1 ? fr - u[r] : u[r] - fr;
+        inertial[r] = 0.0; force[r] = 0.f;
+        const uint16_t* utab = unit_table(e, nb) + c;
+        units[r][0] = utab[0] | ((uint32_t)utab[e.vstride] << 16);
+        units[r][1] = utab[2u * e.vstride] | ((uint32_t)utab[3u * e.vstride] << 16);
+    }
+    bool failure = false;
+    float primal = FLT_MAX;
+    tick(e, 15);
+#pragma unroll 1
+    for (;;) {
+        // ---- M d, the line's quadratic part ----
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < NR; ++r) { wide[l + 32u * r] = dir[r]; flat[l + 32u * r] = (float)dir[r]; }
+        __syncwarp();
+        double md[NR], along = 0.0, cur = 0.0, slo = 0.0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            double s0 = 0.0, s1 = 0.0;
+            if (coord[r]) {
+                const float4* m4 = reinterpret_cast<const float4*>(sm_mass(e) + (l + 32u * r) * e.lay->ld);
+                const double2* d2 = reinterpret_cast<const double2*>(wide);
+#pragma unroll 1
+                for (uint32_t c = 0u; c < chunks; ++c) {
+                    const float4 m = m4[c];
+                    const double2 a = d2[2u * c], z = d2[2u * c + 1u];
+                    s0 = fma((double)m.x, a.x, s0); s1 = fma((double)m.y, a.y, s1); s0 = fma((double)m.z, z.x, s0); s1 = fma((double)m.w, z.y, s1);
+                }
+            }
+            md[r] = s0 + s1;
+            cur = fma(dir[r], md[r], cur);
+            slo = fma(inertial[r], dir[r], slo);
+            along = fma((double)force[r], dir[r], along);
+        }
+        bool search = step > -2;
+        double icurv = 0.0, islope = 0.0;
+        float initial = 0.f, alpha = 0.f;
+        if (search) {
+            icurv = warp_sum(cur);
+            if (step < 0) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) inertial[r] = -md[r];
+                islope = -icurv;
+                search = icurv > 0.0 && icurv <= FLT_MAX;
+            } else {
+                // d solves H d = force, so the slope at alpha = 0 is -(force . d)
+                initial = -(float)warp_sum(along);
+                islope = warp_sum(slo);
+                if (!isfinite(initial) || !(fabs(islope) <= FLT_MAX) || !(icurv <= FLT_MAX)) { failure = true; break; }
+                if (!(initial < 0.f)) break;
+                alpha = 1.f;
+            }
+            tick(e, 20);
+            row_steps<true>(e, tile, b, flat);
+            tick(e, 21);
+        } else {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) inertial[r] = md[r];
+        }
+        // ---- exact line search (block_descent_tile.cuh:2048-2125); without a search one evaluation at the start ----
+        {
+            float low = 0.f, high = 0.f;
+            bool bounded = false;
+            int trials = 0;
+#pragma unroll 1
+            for (;;) {
+                double rows; float curvature, magnitude;
+                evaluate_line(e, inc, ib, ie, alpha, rows, curvature, magnitude);
+                tick_count(e, 28);
+                if (!search) break;
+                const float slope = (float)(islope + (double)alpha * icurv - rows);
+                curvature += (float)icurv;
+                if (initial == 0.f) {                      // the first sweep's search starts by measuring its initial slope
+                    initial = slope;
+                    if (!(initial < 0.f)) break;
+                    alpha = 1.f;
+                    continue;
+                }
+                magnitude += fabsf((float)islope) + alpha * (float)icurv;
+                bool give_up = ++trials >= (int)kLineSteps;
+                if (isfinite(slope) && isfinite(curvature)) {
+                    if (fabsf(slope) <= fmaxf(kLineTol * -initial, kRoundings * FLT_EPSILON * magnitude)) break;
+                    if (slope < 0.f) low = alpha; else { high = alpha; bounded = true; }
+                    give_up |= bounded && high - low <= FLT_EPSILON * high;
+                    const float next = alpha - __fdividef(slope, curvature);
+                    alpha = next > low && (!bounded || next < high) ? next : bounded ? 0.5f * (low + high) : 2.0f * alpha;
+                } else { high = alpha; bounded = true; alpha = 0.5f * (low + high); }
+                if (give_up) { alpha = low; search = false; }       // one more evaluation, at the point returned
+            }
+        }
+        tick(e, 22);
+        tick_count(e, 23);
+        // ---- take the step ----
+        bool fin = true, rounded = true;
+        float longest = 0.f;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const double after = fma((double)alpha, step == -2 ? 0.0 : dir[r], u[r]);
+            fin &= fabs(after) <= FLT_MAX;
+            rounded &= (float)after == (float)u[r];
+            longest = fmaxf(longest, fabsf(alpha * (float)dir[r]));
+            u[r] = after;
+            inertial[r] = fma((double)alpha, step == -2 ? 0.0 : md[r], inertial[r]);
+            force[r] = 0.f;
+        }
+        if (alpha != 0.f)
+#pragma unroll 1
+            for (uint32_t k = ib + l; k < ie; k += 32u) {
+                const uint32_t h = inc[k];
+                const float4 s = hq(e, HF_STEP, h), m = hq(e, HF_MOVE, h);
+                hq(e, HF_MOVE, h) = make_float4(fmaf(alpha, s.x, m.x), fmaf(alpha, s.y, m.y), fmaf(alpha, s.z, m.z), m.w);
+            }
+        if (step >= 0) {
+            if (!__all_sync(NKB_FULL, fin)) { failure = true; break; }
+            rounded = __all_sync(NKB_FULL, rounded);
+            primal = rounded ? 0.f : warp_max_positive(longest);
+            if (!(alpha > 0.f) || rounded || step + 1 == (int)kNewtonSteps) break;
+        }
+        step = step < 0 ? 0 : step + 1;
+        // ---- the next Newton system at the new velocity: this lane's row of H, its entry of the force balance ----
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < NR; ++r) flat[l + 32u * r] = (float)u[r];
+        TreeRow row;
+        tree_load_row(e, tl, sm_mass(e), e.lay->ld, row);
+        float base_row[kTreeBase];
+        if (NR > 1) {
+#pragma unroll
+            for (int k = 0; k < kTreeBase; ++k) base_row[k] = floating && l < 6u ? sm_mass(e)[l * e.lay->ld + k] : 0.f;
+        }
+        double g[NR];
+        float scale[NR], diag[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            g[r] = -inertial[r]; scale[r] = fabsf((float)inertial[r]); diag[r] = 0.f;
+            // rows on a single coordinate only touch that coordinate (block_descent_tile.cuh:1555-1568)
+#pragma unroll 1
+            for (uint32_t pair = 0u; pair < 2u; ++pair) {
+                uint32_t two = pair == 0u ? units[r][0] : units[r][1];
+#pragma unroll 1
+                while (two != (kNoUnitHead | (kNoUnitHead << 16))) {
+                    const bool first = (two & 0xffffu) != kNoUnitHead;
+                    const uint32_t h = first ? two & 0xffffu : two >> 16;
+                    two |= first ? kNoUnitHead : kNoUnitHead << 16;
+                    const float v = hf(e, HF_UNITV, h);
+                    diag[r] += v * hf(e, HF_C, h) * v;
+                    g[r] = fma((double)v, (double)hf(e, HF_F, h), g[r]);
+                    scale[r] += fabsf(v) * hf(e, HF_NZ, h);
+                }
+            }
+        }
+        const int depth = (int)t.tree_depth;
+        __syncwarp();
+        tick(e, 16);
+#pragma unroll 1
+        for (uint32_t k = ib; k < ie; ++k) {
+            const uint32_t h = inc[k];
+            const uint32_t jo = hu(e, HF_JOFF, h);
+            if (jo & kUnitRow) break;                        // contact heads come first
+            const float4 f = hq(e, HF_F, h), c4 = hq(e, HF_C + 1u, h);
+            const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
+            const float c0 = f.w, c1 = c4.x, c2 = c4.y, c12 = c4.z;
+            if (c0 + c1 + c2 + c4.w + nz.x + nz.y == 0.f) continue;        // no impulse, no stiffness
+            const float* jr = sm_jpool(e) + jo;
+            float a0 = 0.f, a1 = 0.f, a2 = 0.f, b0 = 0.f, b1 = 0.f, b2 = 0.f;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const uint32_t c = l + 32u * r;
+                const float j0 = coord[r] ? jr[c] : 0.f, j1 = coord[r] ? jr[js + c] : 0.f, j2 = coord[r] ? jr[2u * js + c] : 0.f;
+                g[r] = fma((double)j0, (double)f.x, g[r]); g[r] = fma((double)j1, (double)f.y, g[r]); g[r] = fma((double)j2, (double)f.z, g[r]);
+                scale[r] += fabsf(j0) * c4.w + fabsf(j1) * nz.x + fabsf(j2) * nz.y;
+                const float p0 = j0 * c0, p1 = j1 * c1 + j2 * c12, p2 = j2 * c2 + j1 * c12;
+                diag[r] += p0 * j0 + p1 * j1 + p2 * j2;
+                if (r == 0) { a0 = b0 = p0; a1 = b1 = p1; a2 = b2 = p2; }
+                else if (l < 6u) { a0 = p0; a1 = p1; a2 = p2; }
+            }
+            if (floating) {
+                const float4 x = *reinterpret_cast<const float4*>(jr), y = *reinterpret_cast<const float4*>(jr + js), z = *reinterpret_cast<const float4*>(jr + 2u * js);
+                const float2 x2 = *reinterpret_cast<const float2*>(jr + 4), y2 = *reinterpret_cast<const float2*>(jr + js + 4), z2 = *reinterpret_cast<const float2*>(jr + 2u * js + 4);
+                row.base[0] += a0 * x.x + a1 * y.x + a2 * z.x; row.base[1] += a0 * x.y + a1 * y.y + a2 * z.y;
+                row.base[2] += a0 * x.z + a1 * y.z + a2 * z.z; row.base[3] += a0 * x.w + a1 * y.w + a2 * z.w;
+                row.base[4] += a0 * x2.x + a1 * y2.x + a2 * z2.x; row.base[5] += a0 * x2.y + a1 * y2.y + a2 * z2.y;
+                if (NR > 1) {
+                    base_row[0] += b0 * x.x + b1 * y.x + b2 * z.x; base_row[1] += b0 * x.y + b1 * y.y + b2 * z.y;
+                    base_row[2] += b0 * x.z + b1 * y.z + b2 * z.z; base_row[3] += b0 * x.w + b1 * y.w + b2 * z.w;
+                    base_row[4] += b0 * x2.x + b1 * y2.x + b2 * z2.x; base_row[5] += b0 * x2.y + b1 * y2.y + b2 * z2.y;
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < kTreeLevels; p += 2) {
+                if (p >= depth - 1) break;
+#pragma unroll
+                for (int q = p; q < p + 2; ++q) {
+                    const uint32_t at = tl.ancestor(q);
+                    row.limb[q] += a0 * jr[at] + a1 * jr[js + at] + a2 * jr[2u * js + at];
+                }
+            }
+        }
+        tick(e, 17);
+        // the rounding scale: force terms, and what the row's own stiffness makes of the velocities along its root path
+        const bool high = NR > 1 && l < 6u && floating;          // this lane's joint is its second coordinate
+        row.diag += high ? diag[NR - 1] : diag[0];
+        {
+            float path = fabsf(row.diag * flat[tl.coord]);
+            if (floating) {
+                const float4 v = *reinterpret_cast<const float4*>(flat);
+                const float2 v2 = *reinterpret_cast<const float2*>(flat + 4);
+                path += fabsf(row.base[0] * v.x) + fabsf(row.base[1] * v.y) + fabsf(row.base[2] * v.z) + fabsf(row.base[3] * v.w) + fabsf(row.base[4] * v2.x) + fabsf(row.base[5] * v2.y);
+                if (NR > 1)
+                    scale[0] += high ? fabsf(base_row[0] * v.x) + fabsf(base_row[1] * v.y) + fabsf(base_row[2] * v.z) + fabsf(base_row[3] * v.w) + fabsf(base_row[4] * v2.x) + fabsf(base_row[5] * v2.y) : 0.f;
+            }
+            if (high) scale[NR - 1] += path; else scale[0] += path;
+        }
+        bool finite = true, small = true;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            force[r] = coord[r] ? (float)g[r] : 0.f;
+            finite &= isfinite(force[r]);
+            small &= !coord[r] || fabsf(force[r]) <= kRoundings * FLT_EPSILON * scale[r];
+        }
+        if (!__all_sync(NKB_FULL, finite)) { failure = true; break; }
+        bool converged = __all_sync(NKB_FULL, small);
+        if (converged && tile.tol > 0.f) {
+            float d[NR];
+            solve_block_mass<NR>(e, b, force, d);
+            bool still = true;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) still &= !coord[r] || fabsf(d[r]) < tile.tol;
+            converged = __all_sync(NKB_FULL, still);
+        }
+        if (converged) { primal = 0.f; break; }
+        tick(e, 18);
+        // ---- d = H^-1 g ----
+        if (NR == 1) {
+#pragma unroll
+            for (int k = 0; k < kTreeBase; ++k) base_row[k] = row.base[k];
+        }
+        float x, base_x[kTreeBase];
+        if (!tree_solve<NR>(e, tl, row, high ? force[NR - 1] : force[0], base_row, force[0], e.sm + e.lay->chol, x, base_x)) { failure = true; break; }
+        dir[NR - 1] = 0.0;
+        if (high) dir[NR - 1] = coord[NR - 1] ? x : 0.f; else dir[0] = coord[0] ? x : 0.f;
+        if (floating && l < 6u) dir[0] = l == 0u ? base_x[0] : l == 1u ? base_x[1] : l == 2u ? base_x[2] : l == 3u ? base_x[3] : l == 4u ? base_x[4] : base_x[5];
+        tick(e, 19);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t k = ib + l; k < ie; k += 32u) {
+        const uint32_t h = inc[k];
+        const float4 res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h);
+        hq(e, HF_RES, h) = make_float4(__fsub_rn(res.x, move.x), __fsub_rn(res.y, move.y), __fsub_rn(res.z, move.z), res.w);
+    }
+    if (failure) e.status |= kStatusSolverFailure;
+    float moved = failure ? FLT_MAX : 0.f;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+        if (coord[r]) {
+            const float now = (float)u[r], before = velocity[l + 32u * r];
+            moved = fmaxf(moved, residual_abs(now - before));
+            velocity[l + 32u * r] = now;
+        }
+    moved = warp_max_positive(moved);
+    tile.momentum = fmaxf(tile.momentum, moved);
+    if (failure) primal = FLT_MAX;
+    tile.residual = fmaxf(tile.residual, fmaxf(primal, coupled ? moved : 0.f));
     __syncwarp();
 }
 
@@ -930,8 +1295,10 @@ NKB_DEV bool team_collect(float* sm, const SmemLayout& lay, uint32_t lane, uint3
     // every lane polls the same word, so the warp never splits over a wait
     bool answered = true;
     const long long begin = clock64();
+#pragma unroll 1
     for (uint32_t m = 1u; m < lay.team && answered; ++m) {
         const uint32_t* done = reinterpret_cast<const uint32_t*>(team_result(sm, lay, m)) + 3;
+#pragma unroll 1
         while (team_peek(done) != seq) {
             if (clock64() - begin > kTeamPatience) { answered = false; break; }
             __nanosleep(40);
@@ -952,7 +1319,7 @@ NKB_DEV Env bare_env(float* sm, const SmemLayout* lay, const TemplateView* t, co
     e.axis = mk3(0.f, 0.f, 0.f);
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
     e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink; e.vel0[0] = e.vel0[1] = 0.f;
-    e.status = 0u; e.vstride = vstride; e.newton_shift = 0u; e.vec_shift = 0u;
+    e.status = 0u; e.branching = false; e.vstride = vstride; e.newton_shift = 0u; e.vec_shift = 0u;
 #ifdef NKB_STAGE_TAPS
     e.cyc = nullptr; e.t0 = 0;
 #endif
@@ -1012,6 +1379,7 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
     const uint32_t seq = team_post(e.sm, *e.lay, e.lane, op, count, 0u, false, none);
     work(0u, team);
     if (team_collect(e.sm, *e.lay, e.lane, seq)) {
+#pragma unroll 1
         for (uint32_t m = 1u; m < team; ++m) e.status |= reinterpret_cast<const uint32_t*>(team_result(e.sm, *e.lay, m))[2];
     } else {
         // a helper did not answer: flag the env, stop using the team, and do the whole range here (the stages dealt out
@@ -1023,6 +1391,14 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
     }
 }
 
+// The articulation's block: on its tree where the rows in force keep the tree's sparsity, dense otherwise (root paths of more
+// than kTreeLevels joints, a contact between two branches of the tree).
+template <int NR, bool kRigid>
+NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
+    if (e.t->tree_depth != 0u && !e.branching) descend_tree<NR>(e, tile, position);
+    else descend_block<NR, kRigid, 0>(e, tile, e.t->B, position);
+}
+
 // Blocks descend colour by colour, blocks of one colour in index order (block_descent_tile.cuh:2749-2820).
 template <int NR, bool kRigid>
 NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
@@ -1031,7 +1407,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
     const uint32_t count = order[nb];
     if constexpr (!kRigid) {
 #pragma unroll 1
-        for (uint32_t k = 0u; k < count; ++k) descend_block<NR, false, 0>(e, tile, e.t->B, position);
+        for (uint32_t k = 0u; k < count; ++k) descend_articulation<NR, false>(e, tile, position);
     } else {
         const uint32_t team = e.lay->team;
         RigidRun run;
@@ -1040,10 +1416,11 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
 #pragma unroll 1
         for (uint32_t k = 0u; k < count;) {
             const uint32_t b = order[k];
-            if (b == e.t->B) { descend_block<NR, kRigid, 0>(e, tile, b, position); ++k; continue; }
+            if (b == e.t->B) { descend_articulation<NR, kRigid>(e, tile, position); ++k; continue; }
             // the run of rigid blocks that share b's colour (a rigid block's 6 coordinates: one per lane)
             const uint32_t colour = blk_color(e, nb, b);
             uint32_t k_end = k + 1u;
+#pragma unroll 1
             while (k_end < count && order[k_end] != e.t->B && blk_color(e, nb, order[k_end]) == colour) ++k_end;
             // colour 31 is the overflow colour (index_blocks hands it to every block past the 31st colour): not a set of
             // independent blocks, so it stays with the lead
@@ -1069,6 +1446,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
                 if (shared_out && share == 0u) {
                     collected = team_collect(e.sm, *e.lay, e.lane, seq);
                     if (collected) {
+#pragma unroll 1
                         for (uint32_t m = 1u; m < team; ++m) {
                             const float* r = team_result(e.sm, *e.lay, m);
                             mine.momentum = fmaxf(mine.momentum, r[0]); mine.residual = fmaxf(mine.residual, r[1]);
@@ -1097,14 +1475,14 @@ struct DualMomentum { float t, beta; };
 NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velocity, bool commit, float out[3]) {
     float cn = 0.f, ct = 0.f, cj = 0.f;
     double restart = 0.0;
+#pragma unroll 1
     for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
         const uint32_t fl = hu(e, HF_FLAGS, h);
         const bool contact = (fl & (kHeadContact | kHeadScalar)) == kHeadContact;
         const V3 tdual = commit ? hf3(e, HF_DUAL, h) : hf3(e, HF_BASE, h);
         const V3 res = hf3(e, HF_RES, h);
         const float rho = hf(e, HF_RHO, h), lower = hf(e, HF_LOWER, h), upper = hf(e, HF_UPPER, h), mu = hf(e, HF_MU, h);
-        const Resp rs = {hf(e, HF_RSD, h), hf(e, HF_RSR, h)};
-        const float normal = scalar_impulse(tdual.x, rho, res.x, lower, upper, rs).impulse;
+        const float normal = scalar_impulse(tdual.x, rho, res.x, lower, upper).impulse;
         Relax rx;
         rx.step = hf3(e, HF_RXS, h); rx.weight = hf(e, HF_RXW, h); rx.point = hf3(e, HF_RXP, h);
         if (!commit) { rx.step = mk3(0.f, 0.f, 0.f); rx.weight = 0.f; rx.point = rx.step; }
@@ -1116,8 +1494,7 @@ NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velo
             dual = relax_contact_impulse_fast(tdual, mk3(normal, iy, iz), rx);
         }
         float sn, st;
-        multiplier_steps_iso(tdual, dual, rs.residual_scale, rs.dual_scale, rho, contact ? mu : 0.f, sn, st);
-        if (!commit && rs.residual_scale > 0.f) sn = __fdividef(fabsf(dual.x - tdual.x), rs.residual_scale);
+        multiplier_steps_iso(tdual, dual, rho, contact ? mu : 0.f, sn, st);
         const V3 physical = commit ? dual : tdual;
         if (!contact) {
             const bool normal_row = (fl & kHeadContactNormal) != 0u;
@@ -1132,10 +1509,9 @@ NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velo
             ct = fmaxf(ct, residual_abs(fmaxf(st, fmaxf(along_axis(physical.y, v.y), along_axis(physical.z, v.z)))));
         }
         if (!commit) continue;
-        if (velocity) hst3(e, HF_LAM, h, dual);
-        const bool extrapolate = contact || rs.dual_scale != 0.f;
+        if (velocity) set_head_lambda(e, h, dual);
         const V3 base = hf3(e, HF_BASE, h);
-        if (extrapolate) restart += momentum_restart_iso(tdual, dual, base, rs.residual_scale, rho, contact && mu > 0.f);
+        restart += momentum_restart_iso(tdual, dual, base, rho, contact && mu > 0.f);
         if (mom != nullptr) hst3(e, HF_MOVE, h, base);
         hst3(e, HF_DUAL, h, dual);
         hst3(e, HF_BASE, h, dual);
@@ -1149,11 +1525,11 @@ NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velo
         const float tn = 0.5f * (1.0f + sqrtf(fmaf(4.0f * mom->t, mom->t, 1.0f)));
         mom->beta = (mom->t - 1.0f) / tn;
         mom->t = tn;
+#pragma unroll 1
         for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
             const bool contact = head_axes(e, h) == 3u;
-            const bool extrapolate = contact || hf(e, HF_RSD, h) != 0.f;
             const float mu = hf(e, HF_MU, h);
-            hst3(e, HF_DUAL, h, extrapolate_dual_iso(hf3(e, HF_MOVE, h), hf3(e, HF_BASE, h), extrapolate ? mom->beta : 0.f,
+            hst3(e, HF_DUAL, h, extrapolate_dual_iso(hf3(e, HF_MOVE, h), hf3(e, HF_BASE, h), mom->beta,
                                                      hf(e, HF_LOWER, h), hf(e, HF_UPPER, h), contact, mu));
         }
         __syncwarp();
@@ -1193,7 +1569,7 @@ NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
 #pragma unroll 1
                 for (uint32_t slot = 0u; slot < 4u; ++slot) {
                     const uint32_t h = utab[slot * vs + c];
-                    if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAM, h);
+                    if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAMX, h);
                 }
             }
 #pragma unroll 1
@@ -1201,7 +1577,7 @@ NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
                 const uint32_t h = inc[k];
                 const uint32_t jo = hu(e, HF_JOFF, h);
                 if (jo & kUnitRow) continue;
-                const V3 lam = hf3(e, HF_LAM, h);
+                const V3 lam = head_lambda(e, h);
                 const float* jr = sm_jpool(e) + jo;
                 const bool cone = head_axes(e, h) == 3u;
 #pragma unroll
@@ -1218,7 +1594,8 @@ NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
             for (uint32_t k = ib; k < ie; ++k) {
                 const uint32_t h = inc[k];
                 const uint32_t side = head_owner(e, h, 0u) == b ? 0u : 1u, axes = head_axes(e, h);
-                const V3 lam = hf3(e, HF_LAM, h);
+                const V3 lam = head_lambda(e, h);
+#pragma unroll 1
                 for (uint32_t ax = 0u; ax < axes; ++ax) {
                     const float imp = comp(lam, (int)ax);
                     if (imp == 0.f) continue;
@@ -1259,6 +1636,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     tile.nheads = nheads; tile.nblocks = B + (n != 0u ? 1u : 0u); tile.iteration = 0u;
     tile.momentum = tile.residual = 0.f; tile.tol = t.cfg.velocity_tolerance;
     // rigid blocks: free velocity, mass, carried constraint velocity (block_descent_rigid.cuh:4-48)
+#pragma unroll 1
     for (uint32_t b = l; b < B; b += 32u) {
         float* bv = sm_bvel(e, b);
         float* bf = sm_bfree(e, b);
@@ -1320,6 +1698,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     enum { kPhaseVelocity, kPhaseHandOver, kPhasePosition, kPhaseDone };
     int phase = kPhaseVelocity;
     bool reindex = true;
+#pragma unroll 1
     while (phase != kPhaseDone) {
         if (reindex) {
             index_blocks(e, tile, phase == kPhaseVelocity);
@@ -1342,6 +1721,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
                 }
                 if (l < t.L && joint_dofs(e.jtype) == 1u) e.qd = U[e.link_dof];
             }
+#pragma unroll 1
             for (uint32_t b = l; b < B; b += 32u) {
                 float* carry = e.s->carry_rigid + ((size_t)e.env * B + b) * 6u;
                 const float* bv = sm_bvel(e, b);
@@ -1354,6 +1734,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
             // split-impulse position pass: every head becomes a scalar push-out row (ops/block_descent.cu:1734-1753)
             if (t.cfg.pos_iters != 0u && nheads != 0u) {
                 bool push = false, coupled = false;
+#pragma unroll 1
                 for (uint32_t h = l; h < nheads; h += 32u) {
                     const uint32_t fl = hu(e, HF_FLAGS, h);
                     const bool spec = (fl & kHeadSpeculative) != 0u;
@@ -1369,6 +1750,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
                             const double correction = t.cfg.pos_beta * fmax(depth, 0.0) + reserve;
                             const double target = fmin(depth, 0.0) + correction;
                             double velocity = 0.0;
+#pragma unroll 1
                             for (uint32_t side = 0u; side < 2u; ++side) {
                                 const uint32_t b = head_owner(e, h, side);
                                 if (b == kNoBlock16) continue;
@@ -1385,8 +1767,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
                     coupled |= (o & 0xffffu) != kNoBlock16 && (o >> 16) != kNoBlock16;
                     hu(e, HF_FLAGS, h) = fl | kHeadScalar;
                     hf(e, HF_LOWER, h) = 0.f; hf(e, HF_UPPER, h) = FLT_MAX;
-                    const Resp rs = scalar_response(hf(e, HF_RHO, h), 0.f);
-                    hf(e, HF_RSD, h) = rs.dual_scale; hf(e, HF_RSR, h) = rs.residual_scale;
+                    hf(e, HF_MU, h) = 0.f;
                     hst3(e, HF_RES, h, mk3(bias, 0.f, 0.f));
                     hst3(e, HF_DUAL, h, mk3(0.f, 0.f, 0.f));
                     push |= bias > rounding;
@@ -1407,6 +1788,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         if (phase == kPhasePosition) continue;
         tick(e, 24);
         // momentum balance: plain measure, reconstruction when only the primal lags, re-measure after it
+#pragma unroll 1
         for (int stage = 0; stage < 3; ++stage) {
             const float worst_row = fmaxf(fmaxf(rows[0], rows[1]), rows[2]);
             bool run = true;

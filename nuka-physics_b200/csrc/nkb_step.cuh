@@ -79,6 +79,7 @@ NKB_DEV bool solve_free_rotation(V3 w0, V3 inv_i, float dt, V3& mid_out) {
 NKB_DEV void stage_integrate_bodies(Env& e, bool use_pseudo) {
     const TemplateView& t = *e.t;
     const float dt = t.cfg.dt;
+#pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         if (!(__ldg(t.inv_mass + b) > 0.f) || __ldg(t.body_to_link + b) != kNoLink) continue;
         float* pose = sm_bpose(e, b);
@@ -117,11 +118,12 @@ NKB_DEV void stage_readout_drives(Env& e, uint32_t nheads) {
     uint32_t* has = reinterpret_cast<uint32_t*>(sm_vec(e, kVecTmp2));
     has[e.lane] = 0u;
     __syncwarp();
+#pragma unroll 1
     for (uint32_t h = e.lane; h < nheads; h += 32u) {
         const uint32_t fl = hu(e, HF_FLAGS, h);
-        if (fl & kHeadDrive) { const uint32_t link = hu(e, HF_REF, h); tmp[link] = hf(e, HF_LAM, h); has[link] = 1u; }
+        if (fl & kHeadDrive) { const uint32_t link = hu(e, HF_REF, h); tmp[link] = hf(e, HF_LAMX, h); has[link] = 1u; }
         // a limit row's slot keeps the multiplier of the velocity solve for the next step (block_descent_tile.cuh:2556)
-        if (fl & kHeadLimit) e.s->limit_lambda[((size_t)e.env * t.L + hu(e, HF_REF, h)) * 2u + (hf(e, HF_UNITV, h) < 0.f ? 1u : 0u)] = hf(e, HF_LAM, h);
+        if (fl & kHeadLimit) e.s->limit_lambda[((size_t)e.env * t.L + hu(e, HF_REF, h)) * 2u + (hf(e, HF_UNITV, h) < 0.f ? 1u : 0u)] = hf(e, HF_LAMX, h);
     }
     __syncwarp();
     float applied = 0.f;
@@ -134,8 +136,10 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
     const TemplateView& t = *e.t;
     float* gp = e.s->body_pose + (size_t)e.env * t.B * 7u;
     const float* sp = e.sm + e.lay->bpose;
+#pragma unroll 1
     for (uint32_t k = e.lane; k < t.B * 7u; k += 32u) gp[k] = sp[k];
     if (!velocities) return;
+#pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         if (__ldg(t.body_to_link + b) != kNoLink || !(__ldg(t.inv_mass + b) > 0.f)) continue;     // only free dynamic bodies move
         const size_t gb = (size_t)e.env * t.B + b;
@@ -168,6 +172,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     const bool has_artic = t.L != 0u, has_bodies = t.B != 0u;
     const bool has_collidables = has_bodies && t.cfg.max_contacts != 0u;
     const bool use_pseudo = t.cfg.pos_iters != 0u && (t.cfg.max_contacts != 0u || t.L != 0u);
+#pragma unroll 1
     for (uint32_t step = 0u; step < p.steps; ++step) {
         Env e;
         env_begin<NR>(e, p, sm, env, lane);
@@ -176,6 +181,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             if (has_bodies) { stage_bodies(e, false); stage_store_bodies(e, false); }
             if (has_artic) {
                 float* gp = p.s.link_pose + (size_t)env * t.L * 7u;
+#pragma unroll 1
                 for (uint32_t k = lane; k < t.L * 7u; k += 32u) gp[k] = sm[p.sm.pose + k];
             }
             return;
@@ -240,6 +246,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         if (has_artic) { stage_fk(e); stage_link_velocities(e); stage_store_links(e); }
         if (has_bodies) {
             // link mirrors follow the new link poses; free bodies keep their integrated pose
+#pragma unroll 1
             for (uint32_t b = lane; b < t.B; b += 32u) {
                 const uint32_t link = __ldg(t.body_to_link + b);
                 if (link == kNoLink) continue;
@@ -291,6 +298,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
         uint32_t seq = last;
         {
             const long long begin = clock64();
+#pragma unroll 1
             while ((seq = team_peek(&cmd->seq)) == last) {
                 if (clock64() - begin > kTeamPatience) break;
                 __nanosleep(100);

@@ -11,6 +11,11 @@ namespace nkb {
 constexpr uint32_t kNoLink = 0xffffffffu;
 constexpr uint32_t kMaxLinks = 32u;     // one warp lane per link
 constexpr uint32_t kMaxDof = 64u;       // a warp lane owns coordinates lane and lane + 32
+constexpr int kTreeLevels = 12;         // joints on one root path that the tree-structured solve covers (a multiple of 4)
+constexpr uint32_t kTreeLaneWords = 2u + kTreeLevels / 4u;   // table words per lane: coordinate and depth, descendants, ancestors
+// Row stride (words) and scratch words of the tree-structured solve for `rows` joint lanes and root paths of `depth` joints.
+inline uint32_t tree_row_stride(uint32_t depth) { return depth <= 5u ? 12u : 20u; }
+inline uint32_t tree_scratch_words(uint32_t rows, uint32_t depth) { return rows * tree_row_stride(depth) + 48u + 28u; }
 constexpr uint32_t kMaxBodies = 256u;   // collidable rows per env (the env's shared-memory slice is the practical limit)
 constexpr uint32_t kPtsPerSlot = 4u;
 
@@ -25,8 +30,7 @@ enum : uint32_t { kStatusPairOverflow = 1u << 0, kStatusDofOverflow = 1u << 2, k
 enum : uint32_t { kHeadContact = 1u << 0, kHeadContactNormal = 1u << 1, kHeadSpeculative = 1u << 2,
                   kHeadVelocityOnly = 1u << 3, kHeadDrive = 1u << 4, kHeadLimit = 1u << 5, kHeadFriction = 1u << 6,
                   kHeadScalar = 1u << 7 /* position pass: only the normal axis */ };
-constexpr uint32_t kHeadWords = 64u;
-constexpr uint32_t kHeadStride = kHeadWords + 1u;   // odd record stride in shared memory    // words of shared memory per solver head
+constexpr uint32_t kHeadStride = 60u;   // words of shared memory per solver head: groups of four, 28 mod 32 for conflict-free vector access
 
 // Scratch words of the tree broadphase for B collidable rows (nkb_lbvh.cuh): sorted keys, internal nodes (children, range,
 // box), split table, ready flags and one partner bit row per body.
@@ -62,6 +66,8 @@ struct TemplateView {
     uint32_t slot_cap;          // candidate slots one step can fill: min(max_contacts, admissible pairs)
     const uint32_t *parent, *jtype, *depth, *child_begin, *children, *link_dof, *link_body, *geom_kind, *limit_flags;
     const uint32_t *dof_link, *anc_mask;
+    const uint32_t *tree_lanes;         // 32 x kTreeLaneWords: a lane's place in the coordinate tree (nkb_tree.cuh)
+    uint32_t tree_depth, tree_stride;   // joints on the longest root path (0: deeper than kTreeLevels, dense solve only), row stride
     const float *axis, *offset, *local_quat, *inertia10, *damping, *armature, *frictionloss, *stiffness, *spring_ref;
     const float *limit_lower, *limit_upper, *geom_pos, *geom_quat;
     const uint32_t *body_geom_kind;     // B: nonzero when the row's shape has its own frame in the link

@@ -201,6 +201,29 @@ HostTemplate HostTemplate::Parse(const void* blob_in, size_t bytes) {
     }
     if (t.ndof > kMaxDof) throw Error(kNotSupported, "more than 64 articulation coordinates per env");
     t.floating_root = (L > 0 && t.jtype[0] == kFloating) ? 1u : 0u;
+    {   // the coordinate tree by lane: a joint coordinate c sits on lane c & 31 (beyond 32 coordinates the base's lanes take
+        // the rest: at most 31 joints beside a base of six)
+        const uint32_t base = t.floating_root ? 6u : 0u;
+        t.tree_lanes.assign(32u * kTreeLaneWords, 0u);
+        uint32_t deepest = 0;
+        std::vector<std::vector<uint32_t>> paths(t.ndof);         // ancestor joint coordinates, root side first
+        for (uint32_t c = base; c < t.ndof; ++c) {
+            for (uint32_t l = t.parent[t.dof_link[c]]; l != kNoLink; l = t.parent[l])
+                if (JointDofs(t.jtype[l]) == 1u) paths[c].insert(paths[c].begin(), t.link_dof[l]);
+            deepest = std::max(deepest, static_cast<uint32_t>(paths[c].size()) + 1u);
+        }
+        t.tree_depth = deepest <= static_cast<uint32_t>(kTreeLevels) ? deepest : 0u;
+        for (uint32_t lane = 0; lane < 32u; ++lane) {
+            uint32_t* w = t.tree_lanes.data() + lane * kTreeLaneWords;
+            const uint32_t c = lane < base || lane >= t.ndof ? lane + 32u : lane;
+            const bool joint = t.tree_depth != 0u && c >= base && c < t.ndof;
+            const uint32_t own = joint ? c : (lane < t.ndof ? lane : 0u);
+            w[0] = own | ((joint ? static_cast<uint32_t>(paths[c].size()) : 0xffu) << 8);
+            for (uint32_t p = 0; p < static_cast<uint32_t>(kTreeLevels); ++p)
+                w[2 + p / 4] |= (joint && p < paths[c].size() ? paths[c][p] : own) << (8 * (p % 4));
+            if (joint) for (uint32_t a : paths[c]) t.tree_lanes[(a & 31u) * kTreeLaneWords + 1] |= 1u << lane;
+        }
+    }
     t.child_begin.assign(L + 1, 0);
     for (uint32_t l = 0; l < L; ++l) {
         t.child_begin[l] = static_cast<uint32_t>(t.children.size());
@@ -337,7 +360,9 @@ void World::BuildLayout() {
     s.xrot = take(9 * L); s.xtr = take(3 * L); s.vbias = 0; s.acc = take(6 * L); s.pbias = take(6 * L); s.ic = take(10 * L);
     const uint32_t dynamics_end = at;
     if (std::getenv("NUKA_B200_NO_OVERLAY") == nullptr) at = overlay;
-    s.chol = take(hn * pad_ld(hn)); s.bm6 = take(72 + 24);
+    tv.tree_depth = t.tree_depth; tv.tree_stride = tree_row_stride(t.tree_depth);
+    const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
+    s.chol = take(std::max(hn * pad_ld(hn), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u)); s.bm6 = take(72 + 24);
     s.rjac_heads = t.n_free ? std::min(tv.head_cap, 32u) : 0u;
     s.rjac = take(24 * s.rjac_heads);
     at = std::max(at, dynamics_end);
@@ -438,6 +463,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.parent = Upload(t.parent); v.jtype = Upload(t.jtype); v.depth = Upload(t.depth); v.child_begin = Upload(t.child_begin);
         v.children = Upload(t.children); v.link_dof = Upload(t.link_dof); v.link_body = Upload(t.link_body);
         v.geom_kind = Upload(t.geom_kind); v.limit_flags = Upload(t.limit_flags); v.dof_link = Upload(t.dof_link); v.anc_mask = Upload(t.anc_mask);
+        v.tree_lanes = Upload(t.tree_lanes);
         v.axis = Upload(t.axis); v.offset = Upload(t.offset); v.local_quat = Upload(t.local_quat); v.inertia10 = Upload(t.inertia10);
         v.damping = Upload(t.damping); v.armature = Upload(t.armature); v.frictionloss = Upload(t.frictionloss);
         v.stiffness = Upload(t.stiffness); v.spring_ref = Upload(t.spring_ref); v.limit_lower = Upload(t.limit_lower);

@@ -23,6 +23,8 @@ struct HostTemplate {
     uint32_t L = 0, B = 0, ndof = 0, max_depth = 0, floating_root = 0;
     Config cfg{};
     std::vector<uint32_t> parent, jtype, depth, child_begin, children, link_dof, link_body, geom_kind, limit_flags, dof_link, anc_mask;
+    std::vector<uint32_t> tree_lanes;      // per lane: joint coordinate and depth, descendant lanes, ancestor coordinates
+    uint32_t tree_depth = 0;
     std::vector<float> axis, offset, local_quat, inertia10, damping, armature, frictionloss, stiffness, spring_ref;
     std::vector<float> limit_lower, limit_upper, geom_pos, geom_quat, q0, base_pose0, kp0, kd0, force_limit0;
     std::vector<uint32_t> shape_kind, contype, conaffinity, group, body_to_link;
