@@ -430,12 +430,24 @@ void World::BuildLayout() {
     if (const char* forced = std::getenv("NUKA_B200_SLIM")) slim_ = has_slim && std::atoi(forced) != 0;     // variant experiments and tests
     const size_t* fits = resident[slim_ ? 1 : 0];
     const size_t most = best[slim_ ? 1 : 0];
-    // Block shape: the one that keeps the most warps resident (228 KB shared memory, 1 KB reserved per block); among
-    // equals a multiple of 4 warps (one per scheduler, measured 0.5 % faster than 6-warp blocks at the same residency on
-    // the quadruped), else the largest.
+    // Block shape: the warps of a block go through the step side by side (align_block), so that they share instruction
+    // fetches; the largest block among those that keep the most warps resident (228 KB shared memory, 1 KB reserved per
+    // block) serves that best.  Two exceptions.  Where an SM holds four warps or fewer, fetches are no bottleneck and waiting
+    // for one another only costs (2048 humanoids, 3 per SM: 13.6 ms in blocks of 3, 10.7 ms in blocks of 1).  And a batch that
+    // does not fill the SMs is spread over all of them in blocks of about two fifths of an SM's share (1000 quadrupeds, 6.8
+    // per SM: 2.66 ms in blocks of 1, 2.39 of 3, 2.50 of 5 and 7; 300: 2.07 of 1, 2.30 of 5).
     warps_per_block_ = team;
     for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) if (fits[w] == most) warps_per_block_ = w;
-    for (uint32_t w = 4; w <= kWarpsPerBlockMax; w += 4) if (w % team == 0u && fits[w] == most) warps_per_block_ = w;
+    if (team == 1u) {
+        int sms = 148;
+        Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
+        const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
+        if (most <= 4u) warps_per_block_ = 1u;
+        else if (share < most) {            // the largest such block that still lets the whole batch in at once
+            const uint32_t cap = std::max(1u, (2u * share + 2u) / 5u);
+            for (uint32_t w = 1u; w <= cap; ++w) if (fits[w] >= share) warps_per_block_ = w;
+        }
+    }
     if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // block-shape experiments
         const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
         if (w >= 1u && w <= kWarpsPerBlockMax && w % team == 0u && fits[w] != 0u) warps_per_block_ = w;
