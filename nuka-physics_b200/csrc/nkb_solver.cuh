@@ -434,7 +434,11 @@ NKB_DEV void line_terms(const HeadRegs& r, float alpha, CSum& rs, float& rc, flo
     V3 f; float cxx, cyy, czz, cyz;
     respond(r, trial, f, cxx, cyy, czz, cyz);
     csum_addp(rs, f.x, r.step.x); csum_addp(rs, f.y, r.step.y); csum_addp(rs, f.z, r.step.z);
-    rm += fabsf(f.x * r.step.x) + fabsf(f.y * r.step.y) + fabsf(f.z * r.step.z);
+    // what rounding can make of the slope: an impulse is rho (residual - move) + multiplier, so its own rounding error scales
+    // with those terms even where they cancel.  A bound made of |f| alone sat below that noise at the end of a descent, and
+    // one search in six then halved its interval down to the last bit (26 evaluations).
+    rm += (fabsf(f.x) + cxx * (fabsf(r.res.x) + fabsf(trial.x))) * fabsf(r.step.x) + (fabsf(f.y) + cyy * (fabsf(r.res.y) + fabsf(trial.y))) * fabsf(r.step.y) +
+          (fabsf(f.z) + czz * (fabsf(r.res.z) + fabsf(trial.z))) * fabsf(r.step.z);
     rc += cxx * r.step.x * r.step.x + cyy * r.step.y * r.step.y + czz * r.step.z * r.step.z + 2.0f * cyz * r.step.y * r.step.z;
 }
 
@@ -908,14 +912,14 @@ NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint3
         float cyy = 0.f, czz = 0.f, cyz = 0.f;
         slope = fma((double)f.x, (double)step.x, slope);
         curvature = fmaf(n.curvature * step.x, step.x, curvature);
-        magnitude += fabsf(f.x * step.x);
+        magnitude = fmaf(noise.x, fabsf(step.x), magnitude);
         if (res.w > 0.f) {
             cone_impulse(mk3(dual.x, dual.y, dual.z), rho, res.y - trial.y, res.z - trial.z, dual.x, res.w, f.y, f.z, cyy, czz, cyz);
             noise.y = fabsf(f.y) + cyy * (fabsf(res.y) + fabsf(trial.y));
             noise.z = fabsf(f.z) + czz * (fabsf(res.z) + fabsf(trial.z));
             slope = fma((double)f.y, (double)step.y, slope); slope = fma((double)f.z, (double)step.z, slope);
             curvature += cyy * step.y * step.y + czz * step.z * step.z + 2.0f * cyz * step.y * step.z;
-            magnitude += fabsf(f.y * step.y) + fabsf(f.z * step.z);
+            magnitude += noise.y * fabsf(step.y) + noise.z * fabsf(step.z);
         }
         hq(e, HF_F, h) = make_float4(f.x, f.y, f.z, n.curvature);
         hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
