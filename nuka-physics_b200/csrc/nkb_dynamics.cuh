@@ -6,115 +6,9 @@
 // (position integration), :647-689 (link velocities), :1561-1596 (world poses) and
 // ops/articulation_mass.cuh:124-396 (mass matrix, factor, solve).
 #pragma once
-#include "nkb_math.cuh"
-#include "nkb_types.h"
+#include "nkb_tree.cuh"
 
 namespace nkb {
-
-// Per-warp view of one env: template, state, shared-memory slice and this lane's registers.
-struct Env {
-    const TemplateView* t;
-    const StateView* s;
-    const SmemLayout* lay;
-    float* sm;
-    uint32_t env, lane;
-    // lane = link
-    uint32_t parent, jtype, depth, link_dof;
-    float q, qd, qdd, tau;
-    V3 axis;                 // unit joint axis in the link frame
-    float drive_command, drive_dissipation, drive_lower, drive_upper;
-    // lane = dof: a lane owns coordinates lane and lane + 32 (the second only when the articulation has more than 32)
-    uint32_t dof_link[2], dof_comp[2];   // comp == kNoLink for scalar joints
-    float vel0[2];           // step-start coordinate velocity
-    uint32_t status;
-    bool branching;          // a contact of this step acts on two branches of the articulation's tree
-    uint32_t vstride;        // words per shared-memory vector: 32 x coordinates per lane
-    // team mode: word offsets from the env's Newton scratch (matrix, block mass, staged rows) and solver vectors to this
-    // warp's private copies; zero for the env's lead warp
-    uint32_t newton_shift, vec_shift;
-#ifdef NKB_STAGE_TAPS
-    uint32_t* cyc;           // stage cycle counters of this env, or null
-    long long t0;
-#endif
-};
-
-// Stage cycle counters are a build-time instrument (-DNKB_STAGE_TAPS); the shipped kernel carries none of it.
-#ifdef NKB_STAGE_TAPS
-// Adds the cycles since the last tick to stage counter k.
-NKB_DEV void tick(Env& e, int k) {
-    if (e.cyc == nullptr) return;
-    const long long now = clock64();
-    if (e.lane == 0u) e.cyc[k] += (uint32_t)(now - e.t0);
-    e.t0 = now;
-}
-NKB_DEV void tick_count(Env& e, int k) { if (e.cyc != nullptr && e.lane == 0u) e.cyc[k] += 1u; }
-#else
-NKB_DEV void tick(Env&, int) {}
-NKB_DEV void tick_count(Env&, int) {}
-#endif
-
-NKB_DEV float* sm_pose(const Env& e, uint32_t l) { return e.sm + e.lay->pose + 7u * l; }
-NKB_DEV float* sm_xrot(const Env& e, uint32_t l) { return e.sm + e.lay->xrot + 9u * l; }
-NKB_DEV float* sm_xtr(const Env& e, uint32_t l) { return e.sm + e.lay->xtr + 3u * l; }
-NKB_DEV float* sm_vel(const Env& e, uint32_t l) { return e.sm + e.lay->vel + 6u * l; }
-NKB_DEV float* sm_acc(const Env& e, uint32_t l) { return e.sm + e.lay->acc + 6u * l; }
-NKB_DEV float* sm_pbias(const Env& e, uint32_t l) { return e.sm + e.lay->pbias + 6u * l; }
-NKB_DEV float* sm_ic(const Env& e, uint32_t l) { return e.sm + e.lay->ic + 10u * l; }
-NKB_DEV float* sm_mass(const Env& e) { return e.sm + e.lay->mass; }
-NKB_DEV float* sm_factor(const Env& e) { return e.sm + e.lay->factor; }
-NKB_DEV float* sm_vec(const Env& e, uint32_t k) { return e.sm + e.lay->vecs + e.vec_shift + e.vstride * k; }   // 32 or 64 words per vector
-// value of coordinate j from per-lane registers x[r] (coordinate lane + 32 r)
-template <int NR>
-NKB_DEV float coord_bcast(const float (&x)[NR], uint32_t j) {
-    if (NR == 1) return __shfl_sync(NKB_FULL, x[0], j);
-    return __shfl_sync(NKB_FULL, j < 32u ? x[0] : x[NR - 1], j & 31u);
-}
-// vector slots
-enum { kVecAcc = 0, kVecFree = 1, kVecU = 2, kVecPseudo = 3, kVecTmp = 4, kVecTmp2 = 5,
-       // Newton-loop scratch shares slots whose other users run before or after the solve
-       kVecS0 = kVecTmp, kVecS1 = kVecTmp2, kVecS2 = kVecAcc,
-       // the Newton direction is staged after the last read of S0 in an iteration and consumed before the next write
-       kVecD = kVecS0, kVecCount = 6 };
-
-NKB_DEV uint32_t joint_dofs(uint32_t t) { return (t == kRevolute || t == kPrismatic) ? 1u : t == kFloating ? 6u : t == kSpherical ? 3u : 0u; }
-
-template <int NR>
-NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uint32_t lane) {
-    e.t = &p.t; e.s = &p.s; e.lay = &p.sm; e.sm = sm; e.env = env; e.lane = lane;
-    const TemplateView& t = p.t;
-    const bool link = lane < t.L;
-    e.parent = link ? __ldg(t.parent + lane) : kNoLink;
-    e.jtype = link ? __ldg(t.jtype + lane) : (uint32_t)kFixed;
-    e.depth = link ? __ldg(t.depth + lane) : 0xffffu;
-    e.link_dof = link ? __ldg(t.link_dof + lane) : 0u;
-    e.axis = mk3(0.f, 0.f, 0.f);
-    if (link) {
-        V3 a = ld3(t.axis + 3u * lane);
-        const float ls = dot(a, a);
-        e.axis = ls > 1.0e-12f ? a * rsqrtf(ls) : mk3(0.f, 0.f, 0.f);
-    }
-    const size_t at = (size_t)env * t.L + lane;
-    e.q = link ? p.s.q[at] : 0.f;
-    e.qd = link ? p.s.qdot[at] : 0.f;
-    e.qdd = 0.f; e.tau = 0.f;
-    e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
-    e.vstride = 32u * NR; e.newton_shift = 0u; e.vec_shift = 0u;
-    e.dof_link[1] = 0u; e.dof_comp[1] = kNoLink; e.vel0[1] = 0.f;
-#pragma unroll
-    for (uint32_t r = 0u; r < (uint32_t)NR; ++r) {
-        const uint32_t c = lane + 32u * r;
-        const bool dof = c < t.ndof;
-        e.dof_link[r] = dof ? __ldg(t.dof_link + c) : 0u;
-        e.dof_comp[r] = kNoLink;
-        if (dof && __ldg(t.jtype + e.dof_link[r]) == kFloating) e.dof_comp[r] = c - __ldg(t.link_dof + e.dof_link[r]);
-        e.vel0[r] = 0.f;
-    }
-    e.status = 0u; e.branching = false;
-#ifdef NKB_STAGE_TAPS
-    e.cyc = p.s.dbg_cycles != nullptr ? p.s.dbg_cycles + (size_t)env * 32u : nullptr;
-    e.t0 = clock64();
-#endif
-}
 
 // World poses of every link, ops/articulation.cu:1561-1596 with kinematics.cuh:25-42 joint frames.
 NKB_DEV void stage_fk(Env& e) {
@@ -407,69 +301,82 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
 #pragma unroll 1
         for (uint32_t k = l; k < n * n; k += 32u) out[k] = M[(k / n) * ld + k % n];
     }
-    // L D L^T, unit lower triangle with D on the diagonal and pivot floor 1e-6 (articulation_mass.cuh:269-335).
-    // Column by column, lane = row: entry (row, k) = (M[row][k] - sum_{j<k} L[row][j] L[k][j] d_j) / d_k, the terms
-    // subtracted in ascending j exactly as the reference's in-place elimination subtracts them, but with both rows
-    // and the pivots read ahead of one short dependent chain instead of a read-modify-write per term.
-    float* F = sm_factor(e);
-    float* piv = sm_vec(e, kVecTmp);
-#pragma unroll 1
-    for (uint32_t k = l; k < n * ld; k += 32u) F[k] = M[k];
-    __syncwarp();
-#pragma unroll 1
-    for (uint32_t k = 0; k < n; ++k) {
-        const float* Fk = F + k * ld;
-        float v[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const uint32_t row = l + 32u * r;
-            v[r] = 0.f;
-            if (row >= k && row < n) {
-                const float* Fr = F + row * ld;
-                const float4* Fr4 = reinterpret_cast<const float4*>(Fr);
-                const float4* Fk4 = reinterpret_cast<const float4*>(Fk);
-                const float4* piv4 = reinterpret_cast<const float4*>(piv);
-                float acc = Fr[k];
-                const uint32_t full = k >> 2;
-#pragma unroll 1
-                for (uint32_t c = 0u; c < full; ++c) {
-                    const float4 a = Fr4[c], b4 = Fk4[c], p = piv4[c];
-                    acc -= a.x * b4.x * p.x; acc -= a.y * b4.y * p.y; acc -= a.z * b4.z * p.z; acc -= a.w * b4.w * p.w;
-                }
-#pragma unroll 1
-                for (uint32_t j = full << 2; j < k; ++j) acc -= Fr[j] * Fk[j] * piv[j];
-                v[r] = acc;
-            }
-        }
-        const float dk = fmaxf(coord_bcast<NR>(v, k), 1.0e-6f);
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const uint32_t row = l + 32u * r;
-            if (row == k) { F[row * ld + k] = dk; piv[k] = dk; }
-            else if (row > k && row < n) F[row * ld + k] = v[r] / dk;
-        }
-        __syncwarp();
-    }
-    // the strict upper triangle keeps M's entries; only the lower triangle and the diagonal are read below
-    // solve L D L^T x = rhs, lane = coordinate (articulation_mass.cuh:357-396)
     float x[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) x[r] = dof[r] ? rhs[r] : 0.f;
+    if (t.mass_tree != 0u) {
+        // factor on the tree's sparsity and solve in the same pass (nkb_tree.cuh); the factor stays for the constraint solve
+        const TreeLane tl = tree_lane(e);
+        const bool high = NR > 1 && t.floating_root != 0u && l < 6u;         // this lane's joint is its second coordinate
+        TreeRow row;
+        tree_load_row(e, tl, M, ld, row);
+        float base_row[kTreeBase], base_x[kTreeBase], joint;
+#pragma unroll
+        for (int k = 0; k < kTreeBase; ++k) base_row[k] = NR == 1 ? row.base[k] : t.floating_root != 0u && l < 6u ? M[l * ld + k] : 0.f;
+        tree_solve<NR, true>(e, tl, row, high ? x[NR - 1] : x[0], base_row, x[0], sm_factor(e), joint, base_x);
+        tree_scatter<NR>(e, joint, base_x, x);
+    } else {
+        // L D L^T, unit lower triangle with D on the diagonal and pivot floor 1e-6 (articulation_mass.cuh:269-335).
+        // Column by column, lane = row: entry (row, k) = (M[row][k] - sum_{j<k} L[row][j] L[k][j] d_j) / d_k, the terms
+        // subtracted in ascending j exactly as the reference's in-place elimination subtracts them, but with both rows
+        // and the pivots read ahead of one short dependent chain instead of a read-modify-write per term.
+        float* F = sm_factor(e);
+        float* piv = sm_vec(e, kVecTmp);
 #pragma unroll 1
-    for (uint32_t j = 0; j < n; ++j) {
-        const float xj = coord_bcast<NR>(x, j);
-#pragma unroll
-        for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (row > j && row < n) x[r] -= F[row * ld + j] * xj; }
-    }
-#pragma unroll
-    for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (dof[r]) x[r] /= F[row * ld + row]; }
+        for (uint32_t k = l; k < n * ld; k += 32u) F[k] = M[k];
+        __syncwarp();
 #pragma unroll 1
-    for (uint32_t jj = n; jj > 0u; --jj) {
-        const uint32_t j = jj - 1u;
-        const float xj = coord_bcast<NR>(x, j);
+        for (uint32_t k = 0; k < n; ++k) {
+            const float* Fk = F + k * ld;
+            float v[NR];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (row < j) x[r] -= F[j * ld + row] * xj; }
+            for (int r = 0; r < NR; ++r) {
+                const uint32_t row = l + 32u * r;
+                v[r] = 0.f;
+                if (row >= k && row < n) {
+                    const float* Fr = F + row * ld;
+                    const float4* Fr4 = reinterpret_cast<const float4*>(Fr);
+                    const float4* Fk4 = reinterpret_cast<const float4*>(Fk);
+                    const float4* piv4 = reinterpret_cast<const float4*>(piv);
+                    float acc = Fr[k];
+                    const uint32_t full = k >> 2;
+#pragma unroll 1
+                    for (uint32_t c = 0u; c < full; ++c) {
+                        const float4 a = Fr4[c], b4 = Fk4[c], p = piv4[c];
+                        acc -= a.x * b4.x * p.x; acc -= a.y * b4.y * p.y; acc -= a.z * b4.z * p.z; acc -= a.w * b4.w * p.w;
+                    }
+#pragma unroll 1
+                    for (uint32_t j = full << 2; j < k; ++j) acc -= Fr[j] * Fk[j] * piv[j];
+                    v[r] = acc;
+                }
+            }
+            const float dk = fmaxf(coord_bcast<NR>(v, k), 1.0e-6f);
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const uint32_t row = l + 32u * r;
+                if (row == k) { F[row * ld + k] = dk; piv[k] = dk; }
+                else if (row > k && row < n) F[row * ld + k] = v[r] / dk;
+            }
+            __syncwarp();
+        }
+        // the strict upper triangle keeps M's entries; only the lower triangle and the diagonal are read below
+        // solve L D L^T x = rhs, lane = coordinate (articulation_mass.cuh:357-396)
+#pragma unroll 1
+        for (uint32_t j = 0; j < n; ++j) {
+            const float xj = coord_bcast<NR>(x, j);
+#pragma unroll
+            for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (row > j && row < n) x[r] -= F[row * ld + j] * xj; }
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (dof[r]) x[r] /= F[row * ld + row]; }
+#pragma unroll 1
+        for (uint32_t jj = n; jj > 0u; --jj) {
+            const uint32_t j = jj - 1u;
+            const float xj = coord_bcast<NR>(x, j);
+#pragma unroll
+            for (int r = 0; r < NR; ++r) { const uint32_t row = l + 32u * r; if (row < j) x[r] -= F[j * ld + row] * xj; }
+        }
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r) if (dof[r]) sm_vec(e, kVecAcc)[l + 32u * r] = x[r];

@@ -182,7 +182,12 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
                     pool[joff + c] = ent[0]; pool[joff + n4 + c] = ent[1]; pool[joff + 2u * n4 + c] = ent[2];
                 } else if (c < n4) { pool[joff + c] = 0.f; pool[joff + n4 + c] = 0.f; pool[joff + 2u * n4 + c] = 0.f; }
             }
-            if (lane == 0u) hu(e, HF_JOFF, h) = joff;
+            if (lane == 0u) {
+                hu(e, HF_JOFF, h) = joff;
+                // the deepest joint coordinate the row acts on, for its coupling (init_heads turns the field into the penalty)
+                const uint32_t deep = la == 0xffffu || (lb != 0xffffu && ((__ldg(t.anc_mask + lb) >> la) & 1u)) ? lb : la;
+                hu(e, HF_RHO, h) = deep == 0xffffu ? 0xffu : __ldg(t.link_leaf + deep);
+            }
         }
     }
     __syncwarp();

@@ -10,7 +10,6 @@
 #pragma once
 #include "nkb_laws.cuh"
 #include "nkb_rows.cuh"
-#include "nkb_tree.cuh"
 
 namespace nkb {
 
@@ -18,6 +17,12 @@ static_assert(HF_COUNT == kHeadStride, "head record must match the host layout")
 
 constexpr uint32_t kNewtonSteps = 16u, kLineSteps = 32u;
 constexpr float kLineTol = 1.0e-6f, kRoundings = 8.0f;
+// An impulse is rho (residual - move) + multiplier, so its own rounding error, half an ulp each of the move, the difference
+// and the sum, scales with those terms even where they cancel: up to eps (|f| + rho (|residual| + |move|)).  The line search
+// accepts a slope below that bound once (kRoundings x this factor = 1): nothing smaller can be told from zero.  With |f| alone
+// in the bound one search in six ended below the noise and above the bound, and halved its interval down to the last bit
+// (26 evaluations instead of 1 to 3).
+constexpr float kImpulseRounding = 1.0f / kRoundings;
 
 struct Tile {
     uint32_t nheads, nblocks, iteration;
@@ -101,6 +106,13 @@ template <int NR>
 NKB_DEV void solve_block_mass(const Env& e, uint32_t block, const float (&g)[NR], float (&x)[NR]) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane;
+    if (block == t.B && t.mass_tree != 0u) {
+        const bool high = NR > 1 && t.floating_root != 0u && l < 6u;
+        float joint, base_x[kTreeBase];
+        tree_mass_solve<NR>(e, tree_lane(e), sm_factor(e), high ? g[NR - 1] : g[0], g[0], joint, base_x);
+        tree_scatter<NR>(e, joint, base_x, x);
+        return;
+    }
     if (block == t.B) {
         const uint32_t n = t.ndof, ld = e.lay->ld;
         const float* F = sm_factor(e);
@@ -205,11 +217,33 @@ NKB_DEV void mass_coupling_dense(Env& e, const Tile& tile) {
     }
 }
 
+// The same for contact rows between two branches of the tree, through a whole solve with the tree's factor.
+template <int NR>
+NKB_DEV void mass_coupling_branching(Env& e, const Tile& tile) {
+    const TemplateView& t = *e.t;
+#pragma unroll 1
+    for (uint32_t h = 0u; h < tile.nheads; ++h) {
+        const uint32_t o = hu(e, HF_OWNER, h), jo = hu(e, HF_JOFF, h);
+        if (((o & 0xffffu) != t.B && (o >> 16) != t.B) || (jo & kUnitRow)) continue;
+        const float* row = sm_jpool(e) + jo;
+        float g[NR], x[NR], sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) g[r] = e.lane + 32u * r < t.ndof ? row[e.lane + 32u * r] : 0.f;
+        solve_block_mass<NR>(e, t.B, g, x);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) sum = fmaf(g[r], x[r], sum);
+        sum = warp_sum(sum);
+        if (e.lane == 0u) hf(e, HF_RHO, h) = sum;
+        __syncwarp();
+    }
+}
+
 // Head setup: penalty, response scales (block_descent_tile.cuh:743-797).
 template <int NR>
 NKB_DEV void init_heads(Env& e, const Tile& tile) {
     const TemplateView& t = *e.t;
-    mass_coupling_dense<NR>(e, tile);
+    if (t.mass_tree == 0u) mass_coupling_dense<NR>(e, tile);
+    else if (e.branching) mass_coupling_branching<NR>(e, tile);
 #pragma unroll 1
     for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
         float shares[2] = {0.f, 0.f};
@@ -222,7 +256,10 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
             float c = 0.f;
             if (ob == kNoBlock16) { /* static or kinematic side: no response */ }
             else if (ob == t.B) {
-                if (jo & kUnitRow) c = mass_coupling_unit<NR>(e, jo & 0xffffu, hf(e, HF_UNITV, h));
+                const bool unit = (jo & kUnitRow) != 0u;
+                if (t.mass_tree != 0u && (unit || !e.branching))
+                    c = tree_coupling<NR>(e, sm_factor(e), unit ? nullptr : sm_jpool(e) + jo, unit ? jo & 0xffffu : hu(e, HF_RHO, h), hf(e, HF_UNITV, h));
+                else if (unit) c = mass_coupling_unit<NR>(e, jo & 0xffffu, hf(e, HF_UNITV, h));
                 else c = hf(e, HF_RHO, h);
             } else {
                 const V3 dir = hf3(e, HF_N, h) * (side == 0u ? 1.f : -1.f);
@@ -434,11 +471,9 @@ NKB_DEV void line_terms(const HeadRegs& r, float alpha, CSum& rs, float& rc, flo
     V3 f; float cxx, cyy, czz, cyz;
     respond(r, trial, f, cxx, cyy, czz, cyz);
     csum_addp(rs, f.x, r.step.x); csum_addp(rs, f.y, r.step.y); csum_addp(rs, f.z, r.step.z);
-    // what rounding can make of the slope: an impulse is rho (residual - move) + multiplier, so its own rounding error scales
-    // with those terms even where they cancel.  A bound made of |f| alone sat below that noise at the end of a descent, and
-    // one search in six then halved its interval down to the last bit (26 evaluations).
-    rm += (fabsf(f.x) + cxx * (fabsf(r.res.x) + fabsf(trial.x))) * fabsf(r.step.x) + (fabsf(f.y) + cyy * (fabsf(r.res.y) + fabsf(trial.y))) * fabsf(r.step.y) +
-          (fabsf(f.z) + czz * (fabsf(r.res.z) + fabsf(trial.z))) * fabsf(r.step.z);
+    rm += (fabsf(f.x) + kImpulseRounding * cxx * (fabsf(r.res.x) + fabsf(trial.x))) * fabsf(r.step.x) +
+          (fabsf(f.y) + kImpulseRounding * cyy * (fabsf(r.res.y) + fabsf(trial.y))) * fabsf(r.step.y) +
+          (fabsf(f.z) + kImpulseRounding * czz * (fabsf(r.res.z) + fabsf(trial.z))) * fabsf(r.step.z);
     rc += cxx * r.step.x * r.step.x + cyy * r.step.y * r.step.y + czz * r.step.z * r.step.z + 2.0f * cyz * r.step.y * r.step.z;
 }
 
@@ -912,14 +947,14 @@ NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint3
         float cyy = 0.f, czz = 0.f, cyz = 0.f;
         slope = fma((double)f.x, (double)step.x, slope);
         curvature = fmaf(n.curvature * step.x, step.x, curvature);
-        magnitude = fmaf(noise.x, fabsf(step.x), magnitude);
+        magnitude += (fabsf(f.x) + kImpulseRounding * (noise.x - fabsf(f.x))) * fabsf(step.x);
         if (res.w > 0.f) {
             cone_impulse(mk3(dual.x, dual.y, dual.z), rho, res.y - trial.y, res.z - trial.z, dual.x, res.w, f.y, f.z, cyy, czz, cyz);
             noise.y = fabsf(f.y) + cyy * (fabsf(res.y) + fabsf(trial.y));
             noise.z = fabsf(f.z) + czz * (fabsf(res.z) + fabsf(trial.z));
             slope = fma((double)f.y, (double)step.y, slope); slope = fma((double)f.z, (double)step.z, slope);
             curvature += cyy * step.y * step.y + czz * step.z * step.z + 2.0f * cyz * step.y * step.z;
-            magnitude += noise.y * fabsf(step.y) + noise.z * fabsf(step.z);
+            magnitude += (fabsf(f.y) + kImpulseRounding * (noise.y - fabsf(f.y))) * fabsf(step.y) + (fabsf(f.z) + kImpulseRounding * (noise.z - fabsf(f.z))) * fabsf(step.z);
         }
         hq(e, HF_F, h) = make_float4(f.x, f.y, f.z, n.curvature);
         hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
@@ -1216,10 +1251,11 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             for (int k = 0; k < kTreeBase; ++k) base_row[k] = row.base[k];
         }
         float x, base_x[kTreeBase];
-        if (!tree_solve<NR>(e, tl, row, high ? force[NR - 1] : force[0], base_row, force[0], e.sm + e.lay->chol, x, base_x)) { failure = true; break; }
-        dir[NR - 1] = 0.0;
-        if (high) dir[NR - 1] = coord[NR - 1] ? x : 0.f; else dir[0] = coord[0] ? x : 0.f;
-        if (floating && l < 6u) dir[0] = l == 0u ? base_x[0] : l == 1u ? base_x[1] : l == 2u ? base_x[2] : l == 3u ? base_x[3] : l == 4u ? base_x[4] : base_x[5];
+        if (!tree_solve<NR, false>(e, tl, row, high ? force[NR - 1] : force[0], base_row, force[0], e.sm + e.lay->chol, x, base_x)) { failure = true; break; }
+        float d[NR];
+        tree_scatter<NR>(e, x, base_x, d);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) dir[r] = d[r];
         tick(e, 19);
     }
     __syncwarp();

@@ -14,7 +14,7 @@
 // columns; the ancestors of that depth pull their multiplier and the row from there.  Row strides of 12 and 20 words keep
 // float4 reads of different rows free of bank conflicts.
 #pragma once
-#include "nkb_dynamics.cuh"
+#include "nkb_env.cuh"
 
 namespace nkb {
 
@@ -66,16 +66,28 @@ NKB_DEV void tree_load_row(const Env& e, const TreeLane& t, const float* matrix,
     row.diag = src[t.coord];
 }
 
+// Reciprocal square root of a pivot that is positive and normal (the hardware's, 2 ulp; no denormal path).
+NKB_DEV float rsqrt_normal(float v) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
+NKB_DEV bool pivot_valid(float v) { return v >= FLT_MIN && v <= FLT_MAX; }
+constexpr float kMassPivotFloor = 1.0e-6f;       // articulation_mass.cuh:269-335
+
+// Rows of the tree in shared memory: joint lanes first .. first + rows.  With one coordinate per lane the base's lanes hold no
+// joint and get no row.
+template <int NR> NKB_DEV uint32_t tree_first(const Env& e) { return NR == 1 && e.t->floating_root ? 6u : 0u; }
+template <int NR> NKB_DEV uint32_t tree_rows(const Env& e) { return NR == 1 ? e.t->ndof - tree_first<NR>(e) : 32u; }
+
 // Solves A x = g.  `row` and `g` are the joint lanes' rows and right-hand sides; lanes 0..5 carry the base's rows in
 // `base_row` (lower triangle) and its right-hand sides in `base_g`.  `scratch` holds tree_scratch_words.  On return `x` is the
 // joint lanes' solution and `base_x` (every lane) the base's.  False when a pivot is not positive and finite.
-template <int NR>
+// kKeep leaves the factor in `scratch` for tree_mass_solve and tree_coupling: the scaled rows with their reciprocal pivot roots
+// in word 7, the base block's triangle and reciprocal roots in the 28 words behind the base rows; pivots are held to the mass
+// matrix's floor.
+template <int NR, bool kKeep>
 NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, const float (&base_row)[kTreeBase], float base_g,
                         float* scratch, float& x, float (&base_x)[kTreeBase]) {
     const uint32_t stride = e.t->tree_stride, lane = e.lane;
     const int depth = (int)e.t->tree_depth;
-    // rows are indexed by joint lane; with one coordinate per lane the base's lanes hold no joint and get no row
-    const uint32_t first = NR == 1 && e.t->floating_root ? 6u : 0u, rows = NR == 1 ? e.t->ndof - first : 32u;
+    const uint32_t first = tree_first<NR>(e), rows = tree_rows<NR>(e);
     float* mine = scratch + (lane - first) * stride;
     float inverse = 1.f, y = 0.f;
     bool valid = true;
@@ -90,14 +102,15 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
     for (int p = depth - 1; p >= 0; --p) {
         const uint32_t pivots = __ballot_sync(NKB_FULL, t.level == (uint32_t)p);
         if (t.level == (uint32_t)p) {
-            valid = row.diag > 0.f && row.diag <= FLT_MAX;
-            inverse = rsqrtf(valid ? row.diag : 1.0f);
+            if (kKeep) row.diag = fmaxf(row.diag, kMassPivotFloor);
+            valid = pivot_valid(row.diag);
+            inverse = rsqrt_normal(row.diag);
             y = g * inverse;
 #pragma unroll
             for (int k = 0; k < kTreeBase; ++k) row.base[k] *= inverse;
             float4* out = reinterpret_cast<float4*>(mine);
             out[0] = make_float4(row.base[0], row.base[1], row.base[2], row.base[3]);
-            out[1] = make_float4(row.base[4], row.base[5], y, 0.f);
+            out[1] = make_float4(row.base[4], row.base[5], y, inverse);
 #pragma unroll
             for (int k = 0; k < kTreeLevels; k += 4) {
                 if (k >= 4 * quads) break;
@@ -162,13 +175,14 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
         float a[28];
 #pragma unroll
         for (int k = 0; k < 7; ++k) { const float4 v = reinterpret_cast<const float4*>(entries)[k]; a[4 * k] = v.x; a[4 * k + 1] = v.y; a[4 * k + 2] = v.z; a[4 * k + 3] = v.w; }
+        if (kKeep) __syncwarp();
         float inv[kTreeBase];
 #pragma unroll
         for (int k = 0; k < kTreeBase; ++k) {
-            const float pivot = a[k * (k + 1) / 2 + k];
-            const bool good = pivot > 0.f && pivot <= FLT_MAX;
-            valid &= good;
-            inv[k] = rsqrtf(good ? pivot : 1.0f);
+            float pivot = a[k * (k + 1) / 2 + k];
+            if (kKeep) pivot = fmaxf(pivot, kMassPivotFloor);
+            valid &= pivot_valid(pivot);
+            inv[k] = rsqrt_normal(pivot);
             a[21 + k] *= inv[k];
 #pragma unroll
             for (int i = k + 1; i < kTreeBase; ++i) a[i * (i + 1) / 2 + k] *= inv[k];
@@ -178,6 +192,13 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
 #pragma unroll
                 for (int j = k + 1; j <= i; ++j) a[i * (i + 1) / 2 + j] = fmaf(-a[i * (i + 1) / 2 + k], a[j * (j + 1) / 2 + k], a[i * (i + 1) / 2 + j]);
             }
+        }
+        if (kKeep && lane == 0u) {          // every lane holds the block; nobody reads the entries any more
+            float4* out = reinterpret_cast<float4*>(entries);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) out[k] = make_float4(a[4 * k], a[4 * k + 1], a[4 * k + 2], a[4 * k + 3]);
+            out[5] = make_float4(a[20], inv[0], inv[1], inv[2]);
+            out[6] = make_float4(inv[3], inv[4], inv[5], 0.f);
         }
 #pragma unroll
         for (int k = kTreeBase - 1; k >= 0; --k) {
@@ -189,7 +210,7 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
 #pragma unroll
         for (int k = 0; k < kTreeBase; ++k) acc = fmaf(-row.base[k], base_x[k], acc);
     }
-    if (!__all_sync(NKB_FULL, valid)) return false;
+    if (!kKeep && !__all_sync(NKB_FULL, valid)) return false;
     // joints root to leaf: a depth's solution reaches its descendants by shuffle
 #pragma unroll
     for (int p = 0; p < kTreeLevels - 1; ++p) {
@@ -199,6 +220,135 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
     }
     x = acc * inverse;
     return true;
+}
+
+// Spreads a solution over the lanes' coordinates: joints from their lanes, the base's from the replicated copy.
+template <int NR>
+NKB_DEV void tree_scatter(const Env& e, float joint, const float (&base_x)[kTreeBase], float (&x)[NR]) {
+    const uint32_t l = e.lane, n = e.t->ndof;
+    if (e.t->floating_root && l < 6u) {
+        if (NR > 1) x[NR - 1] = l + 32u < n ? joint : 0.f;
+        x[0] = l == 0u ? base_x[0] : l == 1u ? base_x[1] : l == 2u ? base_x[2] : l == 3u ? base_x[3] : l == 4u ? base_x[4] : base_x[5];
+    } else {
+        if (NR > 1) x[NR - 1] = 0.f;
+        x[0] = l < n ? joint : 0.f;
+    }
+}
+
+// x = M^-1 g with the kept factor: g and x are the joint lanes' entries, base_g / base_x the base's (lane k of the first six
+// carries base_g of coordinate k; base_x in every lane).
+template <int NR>
+NKB_DEV void tree_mass_solve(const Env& e, const TreeLane& t, float* factor, float g, float base_g, float& x, float (&base_x)[kTreeBase]) {
+    const uint32_t stride = e.t->tree_stride, lane = e.lane, first = tree_first<NR>(e), rows = tree_rows<NR>(e);
+    const int depth = (int)e.t->tree_depth;
+    const bool joint = t.level != kTreeNone;
+    float* mine = factor + (joint ? lane - first : 0u) * stride;
+    const float inverse = joint ? mine[7] : 1.f;
+    float y = 0.f;
+    __syncwarp();
+#pragma unroll 1
+    for (int p = depth - 1; p >= 0; --p) {
+        const uint32_t pivots = __ballot_sync(NKB_FULL, t.level == (uint32_t)p);
+        if (t.level == (uint32_t)p) { y = g * inverse; mine[6] = y; }
+        __syncwarp();
+        uint32_t below = t.level < (uint32_t)p ? (t.desc & pivots) : 0u;
+#pragma unroll 1
+        while (below != 0u) {
+            const float* src = factor + ((uint32_t)__ffs(below) - 1u - first) * stride;
+            below &= below - 1u;
+            g = fmaf(-src[8u + t.level], src[6], g);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kTreeBase; ++k) base_x[k] = 0.f;
+    float acc = y;
+    if (e.t->floating_root) {
+        float* block = factor + rows * stride;
+        if (lane < 6u) {
+            const float* src = factor;
+            float s = base_g;
+#pragma unroll 1
+            for (uint32_t k = 0u; k < rows; ++k, src += stride) s = fmaf(-src[lane], src[6], s);
+            block[lane] = s;
+        }
+        __syncwarp();
+        float a[28], z[8];
+#pragma unroll
+        for (int k = 0; k < 7; ++k) { const float4 v = reinterpret_cast<const float4*>(block + 48)[k]; a[4 * k] = v.x; a[4 * k + 1] = v.y; a[4 * k + 2] = v.z; a[4 * k + 3] = v.w; }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) { const float4 v = reinterpret_cast<const float4*>(block)[k]; z[4 * k] = v.x; z[4 * k + 1] = v.y; z[4 * k + 2] = v.z; z[4 * k + 3] = v.w; }
+#pragma unroll
+        for (int k = 0; k < kTreeBase; ++k) {
+            z[k] *= a[21 + k];
+#pragma unroll
+            for (int i = k + 1; i < kTreeBase; ++i) z[i] = fmaf(-a[i * (i + 1) / 2 + k], z[k], z[i]);
+        }
+#pragma unroll
+        for (int k = kTreeBase - 1; k >= 0; --k) {
+            base_x[k] = z[k] * a[21 + k];
+#pragma unroll
+            for (int i = 0; i < k; ++i) z[i] = fmaf(-a[k * (k + 1) / 2 + i], base_x[k], z[i]);
+        }
+        const float4 b0 = reinterpret_cast<const float4*>(mine)[0];
+        const float2 b1 = reinterpret_cast<const float2*>(mine)[2];
+        acc = fmaf(-b0.x, base_x[0], acc); acc = fmaf(-b0.y, base_x[1], acc); acc = fmaf(-b0.z, base_x[2], acc);
+        acc = fmaf(-b0.w, base_x[3], acc); acc = fmaf(-b1.x, base_x[4], acc); acc = fmaf(-b1.y, base_x[5], acc);
+    }
+#pragma unroll 1
+    for (int p = 0; p < depth - 1; ++p) {
+        const uint32_t word = p < 4 ? t.anc[0] : p < 8 ? t.anc[1] : t.anc[2];
+        const float xp = __shfl_sync(NKB_FULL, acc * inverse, (word >> (8 * (p & 3))) & 31u);
+        if (joint && t.level > (uint32_t)p) acc = fmaf(-mine[8 + p], xp, acc);
+    }
+    x = acc * inverse;
+}
+
+// J M^-1 J^T = |L^-1 J^T|^2 of one row per lane, for rows that act on the base and along one root path: `row` is the row's
+// dense entries (or null for a row with the single entry `unit` at coordinate `leaf`), `leaf` the deepest coordinate of its
+// path (0xff: the base alone).  The forward solve only touches the path and the base, so lanes work on rows of their own.
+template <int NR>
+NKB_DEV float tree_coupling(const Env& e, const float* factor, const float* row, uint32_t leaf, float unit) {
+    const uint32_t stride = e.t->tree_stride, first = tree_first<NR>(e), rows = tree_rows<NR>(e);
+    float z[kTreeBase], total = 0.f;
+    const bool floating = e.t->floating_root != 0u;
+#pragma unroll
+    for (int k = 0; k < kTreeBase; ++k) z[k] = row != nullptr && floating ? row[k] : 0.f;
+    if (leaf != 0xffu) {
+        const uint32_t* table = e.t->tree_lanes + (leaf & 31u) * kTreeLaneWords;
+        const int level = (int)((__ldg(table) >> 8) & 0xffu);
+        float path[kTreeLevels];                             // remaining right-hand side along the path
+#pragma unroll
+        for (int p = 0; p < kTreeLevels; ++p) {
+            path[p] = 0.f;
+            if (row != nullptr && p < level) path[p] = row[(__ldg(table + 2 + (p >> 2)) >> (8 * (p & 3))) & 0xffu];
+        }
+        float g = row != nullptr ? row[leaf] : unit;
+        uint32_t at = leaf;
+#pragma unroll 1
+        for (int p = level; p >= 0; --p) {
+            const float* src = factor + ((at & 31u) - first) * stride;
+            const float y = g * src[7];
+            total = fmaf(y, y, total);
+#pragma unroll
+            for (int k = 0; k < kTreeBase; ++k) z[k] = fmaf(-src[k], y, z[k]);
+            g = 0.f;
+#pragma unroll
+            for (int q = 0; q < kTreeLevels - 1; ++q)
+                if (q < p) { path[q] = fmaf(-src[8 + q], y, path[q]); if (q == p - 1) g = path[q]; }
+            if (p > 0) at = (__ldg(table + 2 + ((p - 1) >> 2)) >> (8 * ((p - 1) & 3))) & 0xffu;
+        }
+    }
+    if (floating) {
+        const float* a = factor + rows * stride + 48;
+#pragma unroll
+        for (int k = 0; k < kTreeBase; ++k) {
+            z[k] *= a[21 + k];
+            total = fmaf(z[k], z[k], total);
+#pragma unroll
+            for (int i = k + 1; i < kTreeBase; ++i) z[i] = fmaf(-a[i * (i + 1) / 2 + k], z[k], z[i]);
+        }
+    }
+    return total;
 }
 
 }  // namespace nkb

@@ -66,6 +66,8 @@ struct TemplateView {
     uint32_t slot_cap;          // candidate slots one step can fill: min(max_contacts, admissible pairs)
     const uint32_t *parent, *jtype, *depth, *child_begin, *children, *link_dof, *link_body, *geom_kind, *limit_flags;
     const uint32_t *dof_link, *anc_mask;
+    const uint32_t *link_leaf;          // L: the deepest joint coordinate on a link's root path, 0xff when there is none
+    uint32_t mass_tree;                 // 1: the mass matrix's factor is kept on the tree, 0: dense L D L^T
     const uint32_t *tree_lanes;         // 32 x kTreeLaneWords: a lane's place in the coordinate tree (nkb_tree.cuh)
     uint32_t tree_depth, tree_stride;   // joints on the longest root path (0: deeper than kTreeLevels, dense solve only), row stride
     const float *axis, *offset, *local_quat, *inertia10, *damping, *armature, *frictionloss, *stiffness, *spring_ref;

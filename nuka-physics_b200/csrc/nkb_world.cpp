@@ -224,6 +224,9 @@ HostTemplate HostTemplate::Parse(const void* blob_in, size_t bytes) {
             if (joint) for (uint32_t a : paths[c]) t.tree_lanes[(a & 31u) * kTreeLaneWords + 1] |= 1u << lane;
         }
     }
+    t.link_leaf.assign(L, 0xffu);
+    for (uint32_t l = 0; l < L; ++l)
+        t.link_leaf[l] = JointDofs(t.jtype[l]) == 1u ? t.link_dof[l] : t.parent[l] != kNoLink ? t.link_leaf[t.parent[l]] : 0xffu;
     t.child_begin.assign(L + 1, 0);
     for (uint32_t l = 0; l < L; ++l) {
         t.child_begin[l] = static_cast<uint32_t>(t.children.size());
@@ -361,12 +364,16 @@ void World::BuildLayout() {
     const uint32_t dynamics_end = at;
     if (std::getenv("NUKA_B200_NO_OVERLAY") == nullptr) at = overlay;
     tv.tree_depth = t.tree_depth; tv.tree_stride = tree_row_stride(t.tree_depth);
+    // The mass matrix's factor on the tree: where the tree branches.  On a single chain it is as long as the dense one and its
+    // steps cost more (7-link arm, 32 steps: 3.98 ms against 3.56 ms; quadruped, depth 3 of 18: 3.26 against 3.76).  The
+    // controllers of modes 3 and 4 work on the dense factor.
+    tv.mass_tree = t.tree_depth != 0u && 2u * t.tree_depth <= n && t.cfg.control_mode != 3u && t.cfg.control_mode != 4u ? 1u : 0u;
     const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
     s.chol = take(std::max(hn * pad_ld(hn), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u)); s.bm6 = take(72 + 24);
     s.rjac_heads = t.n_free ? std::min(tv.head_cap, 32u) : 0u;
     s.rjac = take(24 * s.rjac_heads);
     at = std::max(at, dynamics_end);
-    s.mass = take(n * s.ld); s.factor = take(n * s.ld); s.vstride = n > 32u ? 64u : 32u;
+    s.mass = take(n * s.ld); s.factor = take(tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld); s.vstride = n > 32u ? 64u : 32u;
     s.vecs = take(6 * s.vstride);
     const uint32_t slots = B ? t.n_free + 1u : 0u;
     s.bpose = take(7 * B); s.bvel = take(6 * slots);
@@ -475,7 +482,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.parent = Upload(t.parent); v.jtype = Upload(t.jtype); v.depth = Upload(t.depth); v.child_begin = Upload(t.child_begin);
         v.children = Upload(t.children); v.link_dof = Upload(t.link_dof); v.link_body = Upload(t.link_body);
         v.geom_kind = Upload(t.geom_kind); v.limit_flags = Upload(t.limit_flags); v.dof_link = Upload(t.dof_link); v.anc_mask = Upload(t.anc_mask);
-        v.tree_lanes = Upload(t.tree_lanes);
+        v.tree_lanes = Upload(t.tree_lanes); v.link_leaf = Upload(t.link_leaf);
         v.axis = Upload(t.axis); v.offset = Upload(t.offset); v.local_quat = Upload(t.local_quat); v.inertia10 = Upload(t.inertia10);
         v.damping = Upload(t.damping); v.armature = Upload(t.armature); v.frictionloss = Upload(t.frictionloss);
         v.stiffness = Upload(t.stiffness); v.spring_ref = Upload(t.spring_ref); v.limit_lower = Upload(t.limit_lower);

@@ -24,6 +24,7 @@ struct HostTemplate {
     Config cfg{};
     std::vector<uint32_t> parent, jtype, depth, child_begin, children, link_dof, link_body, geom_kind, limit_flags, dof_link, anc_mask;
     std::vector<uint32_t> tree_lanes;      // per lane: joint coordinate and depth, descendant lanes, ancestor coordinates
+    std::vector<uint32_t> link_leaf;       // per link: deepest joint coordinate on its root path, 0xff when there is none
     uint32_t tree_depth = 0;
     std::vector<float> axis, offset, local_quat, inertia10, damping, armature, frictionloss, stiffness, spring_ref;
     std::vector<float> limit_lower, limit_upper, geom_pos, geom_quat, q0, base_pose0, kp0, kd0, force_limit0;
