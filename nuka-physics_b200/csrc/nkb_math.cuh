@@ -212,6 +212,43 @@ NKB_DEV double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
     return v;
 }
+// Reciprocal square root of a pivot that is positive and normal (the hardware's, 2 ulp; no denormal path).
+NKB_DEV float rsqrt_normal(float v) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
+NKB_DEV bool pivot_valid(float v) { return v >= FLT_MIN && v <= FLT_MAX; }
+constexpr float kMassPivotFloor = 1.0e-6f;       // articulation_mass.cuh:269-335
+
+// Solves a symmetric positive 6 x 6 system held in registers: `a` is the lower triangle by rows (21), then the right-hand side
+// (6); the triangle is replaced by the Cholesky factor's, its diagonal's reciprocals are in `inv`.  kFloor holds the pivots to
+// the mass matrix's floor.  False when a pivot is not positive and finite.
+template <bool kFloor>
+NKB_DEV bool solve6(float (&a)[28], float (&inv)[6], float (&x)[6]) {
+    bool valid = true;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        float pivot = a[k * (k + 1) / 2 + k];
+        if (kFloor) pivot = fmaxf(pivot, kMassPivotFloor);
+        valid &= pivot_valid(pivot);
+        inv[k] = rsqrt_normal(pivot);
+        a[21 + k] *= inv[k];
+#pragma unroll
+        for (int i = k + 1; i < 6; ++i) a[i * (i + 1) / 2 + k] *= inv[k];
+#pragma unroll
+        for (int i = k + 1; i < 6; ++i) {
+            a[21 + i] = fmaf(-a[i * (i + 1) / 2 + k], a[21 + k], a[21 + i]);
+#pragma unroll
+            for (int j = k + 1; j <= i; ++j) a[i * (i + 1) / 2 + j] = fmaf(-a[i * (i + 1) / 2 + k], a[j * (j + 1) / 2 + k], a[i * (i + 1) / 2 + j]);
+        }
+    }
+#pragma unroll
+    for (int k = 5; k >= 0; --k) {
+        float s = a[21 + k];
+#pragma unroll
+        for (int i = k + 1; i < 6; ++i) s = fmaf(-a[i * (i + 1) / 2 + k], x[i], s);
+        x[k] = s * inv[k];
+    }
+    return valid;
+}
+
 // Two sums over the warp at the price of one and two broadcasts: the halves of the warp carry one each after the first exchange.
 NKB_DEV void warp_sum2(float& a, float& b, uint32_t lane) {
     const bool upper = (lane & 16u) != 0u;

@@ -86,15 +86,6 @@ NKB_DEV float head_row_dot(const Env& e, uint32_t h, uint32_t side, uint32_t ax,
     return s;
 }
 
-// Mass entry (i, k) of a block.
-NKB_DEV float block_mass(const Env& e, uint32_t block, uint32_t i, uint32_t k) {
-    if (block == e.t->B) return sm_mass(e)[i * e.lay->ld + k];
-    const float* bm = sm_bmass(e, block);
-    if (i < 3u || k < 3u) return (i == k) ? bm[0] : 0.f;
-    const uint32_t a = i - 3u, b = k - 3u;
-    const uint32_t idx = a == b ? a : (a + b == 1u ? 3u : a + b == 2u ? 4u : 5u);
-    return bm[1u + idx];
-}
 NKB_DEV float* block_vel(const Env& e, uint32_t block, bool position) {
     if (block == e.t->B) return sm_vec(e, position ? kVecPseudo : kVecU);
     return position ? sm_bpseudo(e, block) : sm_bvel(e, block);
@@ -406,13 +397,11 @@ NKB_DEV void respond(const HeadRegs& r, V3 move, V3& f, float& cxx, float& cyy, 
 
 // Row steps J d of a block's incident heads (block_descent_tile.cuh:2019-2044); lane = head, d staged in shared
 // memory with zeros past the block's dimension.
-template <bool kArtic>
 NKB_DEV void row_steps(Env& e, const Tile& tile, uint32_t b, const float* dvec) {
-    const uint32_t nb = tile.nblocks, dim = kArtic ? blk_dim(e, b) : 6u;
-    constexpr bool artic = kArtic;
+    const uint32_t nb = tile.nblocks, dim = blk_dim(e, b);
     const uint32_t* inc = blk_inc(e, nb);
     const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
-    const uint32_t chunks = (dim + 3u) >> 2, n4 = chunks << 2;
+    const uint32_t chunks = (dim + 3u) >> 2;
     const float4* d4 = reinterpret_cast<const float4*>(dvec);
 #pragma unroll 1
     for (uint32_t k = ib + e.lane; k < ie; k += 32u) {
@@ -420,48 +409,24 @@ NKB_DEV void row_steps(Env& e, const Tile& tile, uint32_t b, const float* dvec) 
         const bool cone = head_axes(e, h) == 3u;
         V3 step = mk3(0.f, 0.f, 0.f);
         const uint32_t jo = hu(e, HF_JOFF, h);
-        if (artic) {
-            if (jo & kUnitRow) step.x = hf(e, HF_UNITV, h) * dvec[jo & 0xffffu];
-            else {
-                const float4* j4 = reinterpret_cast<const float4*>(sm_jpool(e) + jo);
-                float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        if (jo & kUnitRow) step.x = hf(e, HF_UNITV, h) * dvec[jo & 0xffffu];
+        else {
+            const float4* j4 = reinterpret_cast<const float4*>(sm_jpool(e) + jo);
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll 1
-                for (uint32_t c = 0u; c < chunks; ++c) {
-                    const float4 d = d4[c], r0 = j4[c];
-                    s0 = fmaf(r0.x, d.x, s0); s0 = fmaf(r0.y, d.y, s0); s0 = fmaf(r0.z, d.z, s0); s0 = fmaf(r0.w, d.w, s0);
-                    if (cone) {
-                        const float4 r1 = j4[chunks + c], r2 = j4[2u * chunks + c];
-                        s1 = fmaf(r1.x, d.x, s1); s1 = fmaf(r1.y, d.y, s1); s1 = fmaf(r1.z, d.z, s1); s1 = fmaf(r1.w, d.w, s1);
-                        s2 = fmaf(r2.x, d.x, s2); s2 = fmaf(r2.y, d.y, s2); s2 = fmaf(r2.z, d.z, s2); s2 = fmaf(r2.w, d.w, s2);
-                    }
+            for (uint32_t c = 0u; c < chunks; ++c) {
+                const float4 d = d4[c], r0 = j4[c];
+                s0 = fmaf(r0.x, d.x, s0); s0 = fmaf(r0.y, d.y, s0); s0 = fmaf(r0.z, d.z, s0); s0 = fmaf(r0.w, d.w, s0);
+                if (cone) {
+                    const float4 r1 = j4[chunks + c], r2 = j4[2u * chunks + c];
+                    s1 = fmaf(r1.x, d.x, s1); s1 = fmaf(r1.y, d.y, s1); s1 = fmaf(r1.z, d.z, s1); s1 = fmaf(r1.w, d.w, s1);
+                    s2 = fmaf(r2.x, d.x, s2); s2 = fmaf(r2.y, d.y, s2); s2 = fmaf(r2.z, d.z, s2); s2 = fmaf(r2.w, d.w, s2);
                 }
-                step = mk3(s0, s1, s2);
             }
-        } else if (k - ib < e.lay->rjac_heads) {
-            // rigid block whose head rows were staged at the start of the descent: 3 rows of 8 floats per head
-            const float4* j4 = reinterpret_cast<const float4*>(e.sm + e.lay->rjac + e.newton_shift + (k - ib) * 24u);
-            const float4 d0 = d4[0], d1 = d4[1];
-            const float4 a0 = j4[0], a1 = j4[1];
-            step.x = a0.x * d0.x + a0.y * d0.y + a0.z * d0.z + a0.w * d0.w + a1.x * d1.x + a1.y * d1.y;
-            if (cone) {
-                const float4 b0 = j4[2], b1 = j4[3], c0 = j4[4], c1 = j4[5];
-                step.y = b0.x * d0.x + b0.y * d0.y + b0.z * d0.z + b0.w * d0.w + b1.x * d1.x + b1.y * d1.y;
-                step.z = c0.x * d0.x + c0.y * d0.y + c0.z * d0.z + c0.w * d0.w + c1.x * d1.x + c1.y * d1.y;
-            }
-        } else {
-            const uint32_t side = head_owner(e, h, 0u) == b ? 0u : 1u;
-            const uint32_t axes = cone ? 3u : 1u;
-#pragma unroll 1
-            for (uint32_t ax = 0u; ax < axes; ++ax) {
-                float s = 0.f;
-#pragma unroll 1
-                for (uint32_t i = 0u; i < dim; ++i) s += head_jac(e, h, side, ax, i, b) * dvec[i];
-                setc(step, (int)ax, s);
-            }
+            step = mk3(s0, s1, s2);
         }
         hst3(e, HF_STEP, h, step);
     }
-    (void)n4;
     __syncwarp();
 }
 
@@ -535,14 +500,9 @@ NKB_DEV void apply_moves(Env& e, const Tile& tile, uint32_t b, float alpha) {
 // Newton steps with exact line search on one block.  A lane owns coordinates lane + 32 r (r < NR) and the same rows of
 // the Newton matrix, which lives in the env's shared-memory slice in float4-readable rows; lane k also owns the k-th
 // incident head in the row evaluations and publishes its response through the head's shared-memory fields.
-// kRigid = false compiles the descent for worlds without free bodies: the articulation is the only block and the
-// rigid-block code (dense 6 x 6 mass, staged 3 x 8 Jacobian rows) drops out.
-// kDim = 0: the articulation's block, dimension read at run time.  kDim = 6: a free rigid body; the loops over its
-// coordinates have constant bounds and unroll.  Each instance carries only its own kind's code.
-template <int NR, bool kRigid, int kDim>
+template <int NR>
 NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
-    const uint32_t l = e.lane, nb = tile.nblocks, dim = kDim != 0 ? (uint32_t)kDim : blk_dim(e, b);
-    constexpr bool artic = kDim == 0;
+    const uint32_t l = e.lane, nb = tile.nblocks, dim = blk_dim(e, b);
     const uint32_t* inc = blk_inc(e, nb);
     const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
     // A block without a push-out row keeps its zero position correction: its descent would minimise u^T M u from u = 0.
@@ -554,47 +514,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     float* hi_v = sm_vec(e, kVecS0);
     float* lo_v = sm_vec(e, kVecS1);
     float* u_v = sm_vec(e, kVecS2);
-    float* H = e.sm + e.lay->chol + e.newton_shift;
-    float* m6 = e.sm + e.lay->bm6 + e.newton_shift;      // 6 x 12 dense mass of a rigid block, then 3 x 8 Jacobian rows of one head
-    float* jscr = m6 + 72u;
-    // rigid block: dense mass, and the Jacobian rows of its incident heads staged once for the whole descent
-    // (3 rows of 8 floats per head, as many heads as the staging area holds)
-    if (!artic) {
-        if (l < 6u) {
-            const float* bm = sm_bmass(e, b);
-            float* row = m6 + l * 12u;
-#pragma unroll
-            for (uint32_t k = 0u; k < 8u; ++k) row[k] = 0.f;
-            if (l < 3u) row[l] = bm[0];
-            else {
-                const uint32_t a = l - 3u;
-                row[3u] = a == 0u ? bm[1] : a == 1u ? bm[4] : bm[5];
-                row[4u] = a == 0u ? bm[4] : a == 1u ? bm[2] : bm[6];
-                row[5u] = a == 0u ? bm[5] : a == 1u ? bm[6] : bm[3];
-            }
-        }
-        if (l < 24u) jscr[l] = 0.f;
-        // lane = incident head: its three rows [direction, arm x direction, 0, 0], signed by the side it sits on
-        const uint32_t staged_count = min(ie - ib, e.lay->rjac_heads);      // at most 32: one pass
-        if (l < staged_count) {
-            const uint32_t h = inc[ib + l];
-            const float sgn = head_owner(e, h, 0u) == b ? 1.f : -1.f;
-            const uint32_t as = head_axes(e, h);
-            const V3 arm = hf3(e, sgn > 0.f ? HF_RA : HF_RB, h);
-            float4* out = reinterpret_cast<float4*>(e.sm + e.lay->rjac + e.newton_shift + l * 24u);
-#pragma unroll
-            for (uint32_t ax = 0u; ax < 3u; ++ax) {
-                float4 lo4 = make_float4(0.f, 0.f, 0.f, 0.f), hi4 = lo4;
-                if (ax < as) {
-                    const V3 dir = hf3(e, ax == 0u ? HF_N : ax == 1u ? HF_T1 : HF_T2, h);
-                    const V3 ang = cross(arm, dir);
-                    lo4 = make_float4(sgn * dir.x, sgn * dir.y, sgn * dir.z, sgn * ang.x);
-                    hi4 = make_float4(sgn * ang.y, sgn * ang.z, 0.f, 0.f);
-                }
-                out[2u * ax] = lo4; out[2u * ax + 1u] = hi4;
-            }
-        }
-    }
+    float* H = e.sm + e.lay->chol;
     bool coord[NR];
     float* Hr[NR];
     const float* Mr[NR];                // this lane's rows of the block mass, zero past the block's dimension
@@ -603,7 +523,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         const uint32_t c = l + 32u * r;
         coord[r] = c < dim;
         Hr[r] = H + (coord[r] ? c : 0u) * ldh;
-        Mr[r] = artic ? sm_mass(e) + (coord[r] ? c : 0u) * e.lay->ld : m6 + (coord[r] ? c : 0u) * 12u;
+        Mr[r] = sm_mass(e) + (coord[r] ? c : 0u) * e.lay->ld;
     }
     bool coupled = false;
 #pragma unroll 1
@@ -649,7 +569,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 hf(e, HF_C, h) = cxx; hf(e, HF_C + 1u, h) = cyy; hf(e, HF_C + 2u, h) = czz; hf(e, HF_C + 3u, h) = cyz;
                 const bool contributes = f.x != 0.f || f.y != 0.f || f.z != 0.f || cxx != 0.f || cyy != 0.f || czz != 0.f || cyz != 0.f ||
                                          noise.x != 0.f || noise.y != 0.f || noise.z != 0.f;
-                const bool unit = artic && (hu(e, HF_JOFF, h) & kUnitRow) != 0u;
+                const bool unit = (hu(e, HF_JOFF, h) & kUnitRow) != 0u;
                 dense_any |= (contributes && !unit) ? 1u : 0u;
             }
             // ---- lane = coordinate: inertial part of H (rows of this lane) and g ----
@@ -670,7 +590,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 if (coord[r]) {
                     const float4* Mr4 = reinterpret_cast<const float4*>(Mr[r]);
                     float4* Hr4 = reinterpret_cast<float4*>(Hr[r]);
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
                     for (uint32_t c = 0u; c < chunks; ++c) {
                         const float4 m = Mr4[c], hi = reinterpret_cast<const float4*>(hi_v)[c], lo = reinterpret_cast<const float4*>(lo_v)[c];
                         Hr4[c] = m;
@@ -685,7 +605,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             }
             tick(e, 16);
             // rows on a single coordinate only touch that coordinate (block_descent_tile.cuh:1555-1568)
-            if (artic) {
+            {
                 const uint16_t* utab = unit_table(e, nb);
                 const uint32_t vs = e.vstride;
 #pragma unroll
@@ -707,20 +627,12 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 for (uint32_t k = ib; k < ie; ++k) {
                     const uint32_t hs = inc[k];
                     const uint32_t jo = hu(e, HF_JOFF, hs);
-                    if (artic && (jo & kUnitRow)) continue;
+                    if (jo & kUnitRow) continue;
                     const V3 f = hf3(e, HF_F, hs), nz = mk3(hf(e, HF_NZ, hs), hf(e, HF_NZ + 1u, hs), hf(e, HF_NZ + 2u, hs));
                     const float c0 = hf(e, HF_C, hs), c1 = hf(e, HF_C + 1u, hs), c2 = hf(e, HF_C + 2u, hs), c12 = hf(e, HF_C + 3u, hs);
                     if (!(f.x != 0.f || f.y != 0.f || f.z != 0.f || c0 != 0.f || c1 != 0.f || c2 != 0.f || c12 != 0.f || nz.x != 0.f || nz.y != 0.f || nz.z != 0.f)) continue;
-                    const float* jr; uint32_t js;
-                    if (artic) { jr = sm_jpool(e) + jo; js = chunks << 2; }
-                    else if (k - ib < e.lay->rjac_heads) { jr = e.sm + e.lay->rjac + e.newton_shift + (k - ib) * 24u; js = 8u; }
-                    else {
-                        const uint32_t ss = head_owner(e, hs, 0u) == b ? 0u : 1u, as = head_axes(e, hs);
-                        __syncwarp();
-                        if (l < 6u) for (uint32_t ax = 0u; ax < 3u; ++ax) jscr[ax * 8u + l] = ax < as ? head_jac(e, hs, ss, ax, l, b) : 0.f;
-                        __syncwarp();
-                        jr = jscr; js = 8u;
-                    }
+                    const float* jr = sm_jpool(e) + jo;
+                    const uint32_t js = chunks << 2;
                     const float4* r0 = reinterpret_cast<const float4*>(jr);
                     const float4* r1 = reinterpret_cast<const float4*>(jr + js);
                     const float4* r2 = reinterpret_cast<const float4*>(jr + 2u * js);
@@ -733,7 +645,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                         const float a0 = j0 * c0, a1 = j1 * c1 + j2 * c12, a2 = j2 * c2 + j1 * c12;
                         if (coord[r]) {
                             float4* Hr4 = reinterpret_cast<float4*>(Hr[r]);
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
                             for (uint32_t cc = 0u; cc < chunks; ++cc) {
                                 float4 h4 = Hr4[cc];
                                 const float4 x = r0[cc], y = r1[cc], z = r2[cc];
@@ -754,7 +666,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 if (coord[r]) {
                     float4* Hr4 = reinterpret_cast<float4*>(Hr[r]);
                     Hr[r][l + 32u * r] += diag[r];
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
                     for (uint32_t c = 0u; c < chunks; ++c) {
                         const float4 v = Hr4[c], uu = reinterpret_cast<const float4*>(u_v)[c];
                         finite &= isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
@@ -782,7 +694,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) inverse[r] = 0.f;
             __syncwarp();
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
             for (uint32_t k = 0u; k < dim; ++k) {
                 float value[NR];
                 const float4* Hk4 = reinterpret_cast<const float4*>(H + k * ldh);
@@ -793,7 +705,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                     if (coord[r] && l + 32u * r >= k) {
                         const float4* Hr4 = reinterpret_cast<const float4*>(Hr[r]);
                         float s0 = 0.f, s1 = 0.f;
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
                         for (uint32_t c = 0u; c < full; ++c) {
                             const float4 a = Hr4[c], bb = Hk4[c];
                             s0 = fmaf(a.x, bb.x, s0); s1 = fmaf(a.y, bb.y, s1); s0 = fmaf(a.z, bb.z, s0); s1 = fmaf(a.w, bb.w, s1);
@@ -822,7 +734,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             float rr[NR], scaled[NR];
 #pragma unroll
             for (int r = 0; r < NR; ++r) rr[r] = force[r];
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
             for (uint32_t j = 0u; j < dim; ++j) {
 #pragma unroll
                 for (int r = 0; r < NR; ++r) scaled[r] = rr[r] * inverse[r];
@@ -833,7 +745,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                     rr[r] = c == j ? y : ((coord[r] && c > j) ? fmaf(-Hr[r][j], y, rr[r]) : rr[r]);
                 }
             }
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
             for (uint32_t jj = dim; jj > 0u; --jj) {
                 const uint32_t j = jj - 1u;
 #pragma unroll
@@ -859,7 +771,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             float ms = 0.f;
             if (coord[r]) {
                 const float4* Mr4 = reinterpret_cast<const float4*>(Mr[r]);
-#pragma unroll (kDim != 0 ? 8 : 1)
+#pragma unroll 1
                 for (uint32_t c = 0u; c < chunks; ++c) {
                     const float4 m = Mr4[c], dd = reinterpret_cast<const float4*>(dvec)[c];
                     ms = fmaf(m.x, dd.x, ms); ms = fmaf(m.y, dd.y, ms); ms = fmaf(m.z, dd.z, ms); ms = fmaf(m.w, dd.w, ms);
@@ -879,7 +791,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             if (!(total_dec > 0.f)) break;
         }
         tick(e, 20);
-        row_steps<artic>(e, tile, b, dvec);
+        row_steps(e, tile, b, dvec);
         tick(e, 21);
         const float alpha = search_line(e, tile, b, islope, icurv);
         tick(e, 22);
@@ -931,35 +843,37 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     __syncwarp();
 }
 
-// One evaluation of a block's constraint rows at step length alpha (lane = head, as many passes as the block has heads):
-// sums the line's slope, curvature and rounding magnitude, and leaves every head's impulse, curvature and noise scale at the
-// trial point in its record, where the assembly of the next Newton system finds them.
+// One constraint row's share of an evaluation at step length alpha: adds to the line's slope, curvature and rounding magnitude,
+// and leaves the head's impulse, curvature and noise scale at the trial point in its record, where the assembly of the next
+// Newton system finds them.
+NKB_DEV void evaluate_head(const Env& e, uint32_t h, float alpha, double& slope, float& curvature, float& magnitude) {
+    const float4 dual = hq(e, HF_DUAL, h), res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h), step = hq(e, HF_STEP, h);
+    const float rho = dual.w, lower = move.w, upper = step.w;
+    const V3 trial = mk3(fmaf(alpha, step.x, move.x), fmaf(alpha, step.y, move.y), fmaf(alpha, step.z, move.z));
+    const STerm n = scalar_impulse(dual.x, rho, res.x - trial.x, lower, upper);
+    V3 f = mk3(n.impulse, 0.f, 0.f), noise = mk3(fmaf(n.curvature, fabsf(res.x) + fabsf(trial.x), fabsf(n.impulse)), 0.f, 0.f);
+    float cyy = 0.f, czz = 0.f, cyz = 0.f;
+    slope = fma((double)f.x, (double)step.x, slope);
+    curvature = fmaf(n.curvature * step.x, step.x, curvature);
+    magnitude = fmaf(fmaf(kImpulseRounding, noise.x - fabsf(f.x), fabsf(f.x)), fabsf(step.x), magnitude);
+    if (res.w > 0.f) {
+        cone_impulse(mk3(dual.x, dual.y, dual.z), rho, res.y - trial.y, res.z - trial.z, dual.x, res.w, f.y, f.z, cyy, czz, cyz);
+        noise.y = fmaf(cyy, fabsf(res.y) + fabsf(trial.y), fabsf(f.y));
+        noise.z = fmaf(czz, fabsf(res.z) + fabsf(trial.z), fabsf(f.z));
+        slope = fma((double)f.y, (double)step.y, slope); slope = fma((double)f.z, (double)step.z, slope);
+        curvature = fmaf(fmaf(cyy, step.y, cyz * step.z), step.y, fmaf(fmaf(czz, step.z, cyz * step.y), step.z, curvature));
+        magnitude = fmaf(fmaf(kImpulseRounding, noise.y - fabsf(f.y), fabsf(f.y)), fabsf(step.y), magnitude);
+        magnitude = fmaf(fmaf(kImpulseRounding, noise.z - fabsf(f.z), fabsf(f.z)), fabsf(step.z), magnitude);
+    }
+    hq(e, HF_F, h) = make_float4(f.x, f.y, f.z, n.curvature);
+    hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
+    *reinterpret_cast<float2*>(&hf(e, HF_NZ + 1u, h)) = make_float2(noise.y, noise.z);
+}
+// The rows of a block, lane = head, as many passes as the block has heads.
 NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint32_t ie, float alpha, double& slope, float& curvature, float& magnitude) {
     slope = 0.0; curvature = 0.f; magnitude = 0.f;
 #pragma unroll 1
-    for (uint32_t k = ib + e.lane; k < ie; k += 32u) {
-        const uint32_t h = inc[k];
-        const float4 dual = hq(e, HF_DUAL, h), res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h), step = hq(e, HF_STEP, h);
-        const float rho = dual.w, lower = move.w, upper = step.w;
-        const V3 trial = mk3(fmaf(alpha, step.x, move.x), fmaf(alpha, step.y, move.y), fmaf(alpha, step.z, move.z));
-        const STerm n = scalar_impulse(dual.x, rho, res.x - trial.x, lower, upper);
-        V3 f = mk3(n.impulse, 0.f, 0.f), noise = mk3(fabsf(n.impulse) + n.curvature * (fabsf(res.x) + fabsf(trial.x)), 0.f, 0.f);
-        float cyy = 0.f, czz = 0.f, cyz = 0.f;
-        slope = fma((double)f.x, (double)step.x, slope);
-        curvature = fmaf(n.curvature * step.x, step.x, curvature);
-        magnitude += (fabsf(f.x) + kImpulseRounding * (noise.x - fabsf(f.x))) * fabsf(step.x);
-        if (res.w > 0.f) {
-            cone_impulse(mk3(dual.x, dual.y, dual.z), rho, res.y - trial.y, res.z - trial.z, dual.x, res.w, f.y, f.z, cyy, czz, cyz);
-            noise.y = fabsf(f.y) + cyy * (fabsf(res.y) + fabsf(trial.y));
-            noise.z = fabsf(f.z) + czz * (fabsf(res.z) + fabsf(trial.z));
-            slope = fma((double)f.y, (double)step.y, slope); slope = fma((double)f.z, (double)step.z, slope);
-            curvature += cyy * step.y * step.y + czz * step.z * step.z + 2.0f * cyz * step.y * step.z;
-            magnitude += (fabsf(f.y) + kImpulseRounding * (noise.y - fabsf(f.y))) * fabsf(step.y) + (fabsf(f.z) + kImpulseRounding * (noise.z - fabsf(f.z))) * fabsf(step.z);
-        }
-        hq(e, HF_F, h) = make_float4(f.x, f.y, f.z, n.curvature);
-        hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
-        *reinterpret_cast<float2*>(&hf(e, HF_NZ + 1u, h)) = make_float2(noise.y, noise.z);
-    }
+    for (uint32_t k = ib + e.lane; k < ie; k += 32u) evaluate_head(e, inc[k], alpha, slope, curvature, magnitude);
     slope = warp_sum(slope);
     warp_sum2(curvature, magnitude, e.lane);
 }
@@ -1066,7 +980,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
                 alpha = 1.f;
             }
             tick(e, 20);
-            row_steps<true>(e, tile, b, flat);
+            row_steps(e, tile, b, flat);
             tick(e, 21);
         } else {
 #pragma unroll
@@ -1114,7 +1028,11 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             fin &= fabs(after) <= FLT_MAX;
             rounded &= (float)after == (float)u[r];
             longest = fmaxf(longest, fabsf(alpha * (float)dir[r]));
-            u[r] = after;
+        }
+        if (step >= 0 && !__all_sync(NKB_FULL, fin)) { failure = true; break; }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            u[r] = fma((double)alpha, step == -2 ? 0.0 : dir[r], u[r]);
             inertial[r] = fma((double)alpha, step == -2 ? 0.0 : md[r], inertial[r]);
             force[r] = 0.f;
         }
@@ -1126,7 +1044,6 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
                 hq(e, HF_MOVE, h) = make_float4(fmaf(alpha, s.x, m.x), fmaf(alpha, s.y, m.y), fmaf(alpha, s.z, m.z), m.w);
             }
         if (step >= 0) {
-            if (!__all_sync(NKB_FULL, fin)) { failure = true; break; }
             rounded = __all_sync(NKB_FULL, rounded);
             primal = rounded ? 0.f : warp_max_positive(longest);
             if (!(alpha > 0.f) || rounded || step + 1 == (int)kNewtonSteps) break;
@@ -1359,43 +1276,331 @@ NKB_DEV Env bare_env(float* sm, const SmemLayout* lay, const TemplateView* t, co
     e.axis = mk3(0.f, 0.f, 0.f);
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
     e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink; e.vel0[0] = e.vel0[1] = 0.f;
-    e.status = 0u; e.branching = false; e.vstride = vstride; e.newton_shift = 0u; e.vec_shift = 0u;
+    e.status = 0u; e.branching = false; e.vstride = vstride;
 #ifdef NKB_STAGE_TAPS
     e.cyc = nullptr; e.t0 = 0;
 #endif
     return e;
 }
 
-// What a warp needs to descend rigid blocks, passed by value so that the function below can stay out of line without
-// forcing the caller's env record into local memory.
+// What a warp needs to descend rigid blocks.
 struct RigidRun {
     float* sm;
     const SmemLayout* lay;
     const TemplateView* t;
-    uint32_t lane, vstride, newton_shift, vec_shift;
+    uint32_t lane, vstride;
     uint32_t nheads, nblocks, iteration;
     float tol;
 };
 struct RigidResult { float momentum, residual; uint32_t status; };
 
-// Descends the rigid blocks order[k_begin + first], order[k_begin + first + stride], ... < k_end of one colour.
-// Inlined at both call sites (the lead's and the helpers'): out of line, the layout offsets would be read through a
-// pointer instead of the kernel's constant bank, which measured 30 % slower on a 48-box pile.
-#ifndef NKB_RIGID_RUN_QUALIFIER
-#define NKB_RIGID_RUN_QUALIFIER __forceinline__
-#endif
-template <bool kRigid>
-__device__ NKB_RIGID_RUN_QUALIFIER RigidResult descend_rigid_run(RigidRun run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
+// A warp works on several free bodies at once, `lay->body_lanes` lanes (8 or 16) on each: blocks of one colour share no
+// constraint row.  Inside a group a lane is a constraint row in the line search (rows j, j + width, ...) and a row of the 6 x 6
+// Newton system in its assembly (lanes 8..15 of a 16-lane group take the odd heads); everything of the block's own size (its
+// velocity, its mass, the factorisation) is replicated over the group's lanes in registers, so that neither shared memory nor
+// an exchange sits inside those chains.  Loops run until the last group of the warp is done; a group that is done leaves its
+// state alone.
+struct BodyLanes {
+    uint32_t width, j, mask, first;      // lanes per body, lane within the group, the group's lanes, its first lane
+    NKB_DEV bool any(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) != 0u; }
+    NKB_DEV bool all(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) == mask; }
+    template <typename T> NKB_DEV T sum(T v) const {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
+        if (width > 8u) v += __shfl_xor_sync(NKB_FULL, v, 8);
+        return v;
+    }
+};
+NKB_DEV BodyLanes body_lanes(const Env& e) {
+    BodyLanes g;
+    g.width = e.lay->body_lanes; g.j = e.lane & (g.width - 1u); g.first = e.lane & ~(g.width - 1u);
+    g.mask = ((1u << g.width) - 1u) << g.first;
+    return g;
+}
+// M v of a free body: mass, and the world inertia xx yy zz xy xz yz
+struct BodyMass { float m, i[6]; };
+NKB_DEV void body_mass_mul(const BodyMass& b, const double (&v)[6], double (&out)[6]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k] = (double)b.m * v[k];
+    out[3] = fma((double)b.i[0], v[3], fma((double)b.i[3], v[4], (double)b.i[4] * v[5]));
+    out[4] = fma((double)b.i[3], v[3], fma((double)b.i[1], v[4], (double)b.i[5] * v[5]));
+    out[5] = fma((double)b.i[4], v[3], fma((double)b.i[5], v[4], (double)b.i[2] * v[5]));
+}
+// Row j < 6 of a contact's Jacobian is J_ax[j] = dir_ax . w_j with w_j the unit vector for the linear rows and unit x arm for
+// the angular ones (dir . (unit x arm) = (arm x dir) . unit); rows 6 and 7 of a group of eight get zeros.
+NKB_DEV V3 body_row_axis(uint32_t row, V3 arm) {
+    return row == 0u ? mk3(1.f, 0.f, 0.f) : row == 1u ? mk3(0.f, 1.f, 0.f) : row == 2u ? mk3(0.f, 0.f, 1.f)
+         : row == 3u ? mk3(0.f, -arm.z, arm.y) : row == 4u ? mk3(arm.z, 0.f, -arm.x) : row == 5u ? mk3(-arm.y, arm.x, 0.f) : mk3(0.f, 0.f, 0.f);
+}
+template <typename T> NKB_DEV T pick6(const T (&v)[6], uint32_t k) { return k == 0u ? v[0] : k == 1u ? v[1] : k == 2u ? v[2] : k == 3u ? v[3] : k == 4u ? v[4] : v[5]; }
+
+// products with their fused multiply-adds spelled out
+NKB_DEV float dot_fma(V3 a, V3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+NKB_DEV V3 cross_fma(V3 a, V3 b) { return mk3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x))); }
+
+// Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: `32 / body_lanes` blocks at a
+// time, warp `first` of `stride`.  Same model, stopping rules and exact line search as descend_block; the sums that one
+// compensates in float run in double, the inertial force is carried as in descend_tree.
+// What bounds it is the length of the chain of one block (assembly, factorisation, line search).  One block per warp with six
+// busy lanes and its matrix in shared memory took about 16 k cycles per block; see the team and box figures at World::BuildLayout.
+// Inlined for the lead and for its helpers (out of line it spilled the callers' registers and ran 5 % slower), so every fused
+// multiply-add is written as one: left to the compiler, the two copies contracted some products differently, and a block's
+// result depended on who ran it.
+NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     Env e = bare_env(run.sm, run.lay, run.t, nullptr, 0u, run.lane, run.vstride);
-    e.newton_shift = run.newton_shift; e.vec_shift = run.vec_shift;
-    Tile tile;
-    tile.nheads = run.nheads; tile.nblocks = run.nblocks; tile.iteration = run.iteration;
-    tile.momentum = 0.f; tile.residual = 0.f; tile.tol = run.tol;
-    const uint32_t* order = block_order(e, run.nblocks);
+    const TemplateView& t = *e.t;
+    const BodyLanes g = body_lanes(e);
+    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
+    const uint32_t* order = block_order(e, nb);
+    float most_moved = 0.f, worst = 0.f;
+    bool failed = false;
 #pragma unroll 1
-    for (uint32_t k = k_begin + first; k < k_end; k += stride) descend_block<1, kRigid, 6>(e, tile, order[k], position);
+    for (uint32_t base = k_begin + first * groups; base < k_end; base += stride * groups) {
+        const uint32_t turn = base + e.lane / g.width;
+        const bool have = turn < k_end;
+        const uint32_t b = order[have ? turn : base];
+        const uint32_t* inc = blk_inc(e, nb) + blk_inc_begin(e, nb, b);
+        const uint32_t count = have ? blk_inc_begin(e, nb, b + 1u) - blk_inc_begin(e, nb, b) : 0u;
+        // a block without a push-out row keeps its zero position correction; in the velocity phase an unconstrained block
+        // still has to reach its free velocity
+        const bool began = have && !(position && count == 0u);
+        bool active = began, coupled = false, failure = false;
+#pragma unroll 1
+        for (uint32_t k = g.j; k < count; k += g.width) {
+            const uint32_t h = inc[k], o = hu(e, HF_OWNER, h);
+            coupled |= (o & 0xffffu) != kNoBlock16 && (o >> 16) != kNoBlock16;
+            hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_STEP, h, mk3(0.f, 0.f, 0.f));
+        }
+        coupled = g.any(coupled);
+        BodyMass mass;
+        {
+            const float* bm = sm_bmass(e, b);
+            mass.m = bm[0];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) mass.i[k] = bm[1 + k];
+        }
+        float* velocity = block_vel(e, b, position);
+        // how the directions of a descent start: toward the free velocity in the first velocity sweep (-1), else only M (u - u_free)
+        // and the rows where the block stands (-2); Newton steps from 0 on.  Every group is at the same step.
+        int step = run.iteration == 0u && !position ? -1 : -2;
+        double u[6], dir[6], inertial[6];
+        float force[6], primal = FLT_MAX;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const double fr = position ? 0.0 : (double)sm_bfree(e, b)[k];
+            u[k] = velocity[k];
+            dir[k] = step == -1 ? fr - u[k] : u[k] - fr;
+            inertial[k] = 0.0; force[k] = 0.f;
+        }
+#pragma unroll 1
+        for (;;) {
+            double md[6];
+            body_mass_mul(mass, dir, md);
+            bool search = active && step > -2;
+            double icurv = 0.0, islope = 0.0;
+            float initial = 0.f, alpha = 0.f;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) icurv = fma(dir[k], md[k], icurv);
+            if (step < 0) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) inertial[k] = step == -1 ? -md[k] : md[k];
+                islope = -icurv;
+                search = search && icurv > 0.0 && icurv <= FLT_MAX;
+            } else {
+                double along = 0.0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) { islope = fma(inertial[k], dir[k], islope); along = fma((double)force[k], dir[k], along); }
+                initial = -(float)along;                     // d solves H d = force
+                const bool sane = isfinite(initial) && fabs(islope) <= FLT_MAX && icurv <= FLT_MAX;
+                failure |= active && !sane;
+                active = active && sane && initial < 0.f;
+                search = active; alpha = 1.f;
+            }
+            // rows' steps along d: dir . (d_lin + d_ang x arm), signed by the side the block is on
+            if (search)
+#pragma unroll 1
+                for (uint32_t k = g.j; k < count; k += g.width) {
+                    const uint32_t h = inc[k];
+                    const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                    const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h);
+                    const V3 ang = mk3((float)dir[3], (float)dir[4], (float)dir[5]);
+                    V3 v = mk3((float)dir[0], (float)dir[1], (float)dir[2]) + cross_fma(ang, arm);
+                    if (!first_side) v = -v;
+                    V3 s = mk3(dot_fma(hf3(e, HF_N, h), v), 0.f, 0.f);
+                    if (!position) { s.y = dot_fma(hf3(e, HF_T1, h), v); s.z = dot_fma(hf3(e, HF_T2, h), v); }
+                    hst3(e, HF_STEP, h, s);
+                }
+            // exact line search (block_descent_tile.cuh:2048-2125); groups without a search take one evaluation at the start
+            {
+                float low = 0.f, high = 0.f;
+                bool bounded = false, trying = active;
+                int trials = 0;
+#pragma unroll 1
+                while (__any_sync(NKB_FULL, trying)) {
+                    double rows = 0.0;
+                    float curvature = 0.f, magnitude = 0.f;
+                    if (trying)
+#pragma unroll 1
+                        for (uint32_t k = g.j; k < count; k += g.width) evaluate_head(e, inc[k], alpha, rows, curvature, magnitude);
+                    __syncwarp();
+                    rows = g.sum(rows); curvature = g.sum(curvature); magnitude = g.sum(magnitude);
+                    if (!trying) continue;
+                    if (!search) { trying = false; continue; }
+                    const float slope = (float)(fma((double)alpha, icurv, islope) - rows);
+                    curvature += (float)icurv;
+                    if (initial == 0.f) {                      // the first sweep's search starts by measuring its initial slope
+                        initial = slope;
+                        if (initial < 0.f) alpha = 1.f; else trying = false;
+                        continue;
+                    }
+                    magnitude += fmaf(alpha, (float)icurv, fabsf((float)islope));
+                    bool give_up = ++trials >= (int)kLineSteps;
+                    if (isfinite(slope) && isfinite(curvature)) {
+                        if (fabsf(slope) <= fmaxf(kLineTol * -initial, kRoundings * FLT_EPSILON * magnitude)) { trying = false; continue; }
+                        if (slope < 0.f) low = alpha; else { high = alpha; bounded = true; }
+                        give_up |= bounded && high - low <= FLT_EPSILON * high;
+                        const float next = alpha - __fdividef(slope, curvature);
+                        alpha = next > low && (!bounded || next < high) ? next : bounded ? 0.5f * (low + high) : 2.0f * alpha;
+                    } else { high = alpha; bounded = true; alpha = 0.5f * (low + high); }
+                    if (give_up) { alpha = low; search = false; }       // one more evaluation, at the point returned
+                }
+            }
+            // take the step
+            {
+                bool finite = true, rounded = true;
+                float longest = 0.f;
+                double after[6];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    after[k] = fma((double)alpha, dir[k], u[k]);
+                    finite &= fabs(after[k]) <= FLT_MAX;
+                    rounded &= (float)after[k] == (float)u[k];
+                    longest = fmaxf(longest, fabsf(alpha * (float)dir[k]));
+                }
+                if (step >= 0) { failure |= active && !finite; active = active && finite; }
+                if (active) {
+                    if (alpha != 0.f) {
+#pragma unroll
+                        for (int k = 0; k < 6; ++k) { u[k] = after[k]; inertial[k] = fma((double)alpha, md[k], inertial[k]); }
+#pragma unroll 1
+                        for (uint32_t k = g.j; k < count; k += g.width) {
+                            const uint32_t h = inc[k];
+                            const float4 s = hq(e, HF_STEP, h), m = hq(e, HF_MOVE, h);
+                            hq(e, HF_MOVE, h) = make_float4(fmaf(alpha, s.x, m.x), fmaf(alpha, s.y, m.y), fmaf(alpha, s.z, m.z), m.w);
+                        }
+                    }
+                    if (step >= 0) {
+                        primal = rounded ? 0.f : longest;
+                        active = alpha > 0.f && !rounded && step + 1 < (int)kNewtonSteps;
+                    }
+                }
+            }
+            if (!__any_sync(NKB_FULL, active)) break;
+            step = step < 0 ? 0 : step + 1;
+            __syncwarp();
+            // the next Newton system: this lane's row of H, its entry of the force balance and its rounding scale
+            float hr[6], scale = 0.f;
+            double gsum = 0.0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) hr[k] = 0.f;
+            if (part == 0u && row < 6u) {
+                if (row < 3u) { hr[0] = row == 0u ? mass.m : 0.f; hr[1] = row == 1u ? mass.m : 0.f; hr[2] = row == 2u ? mass.m : 0.f; }
+                else {
+                    hr[3] = row == 3u ? mass.i[0] : row == 4u ? mass.i[3] : mass.i[4];
+                    hr[4] = row == 3u ? mass.i[3] : row == 4u ? mass.i[1] : mass.i[5];
+                    hr[5] = row == 3u ? mass.i[4] : row == 4u ? mass.i[5] : mass.i[2];
+                }
+                gsum = -pick6(inertial, row);
+                scale = fabsf((float)gsum);
+            }
+            if (active)
+#pragma unroll 1
+                for (uint32_t k = part; k < count; k += parts) {
+                    const uint32_t h = inc[k];
+                    const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                    const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), w = body_row_axis(row, arm);
+                    const float4 f = hq(e, HF_F, h);
+                    const float j0 = dot_fma(n, w), sgn = first_side ? 1.f : -1.f;
+                    V3 a;
+                    if (position) {                                    // push-out rows have a normal axis only
+                        gsum = fma((double)(sgn * j0), (double)f.x, gsum);
+                        scale = fmaf(fabsf(j0), hf(e, HF_NZ, h), scale);
+                        a = n * (j0 * f.w);
+                    } else {
+                        const float4 c = hq(e, HF_C + 1u, h);
+                        const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
+                        const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h);
+                        const float j1 = dot_fma(t1, w), j2 = dot_fma(t2, w);
+                        gsum = fma((double)(sgn * j0), (double)f.x, gsum); gsum = fma((double)(sgn * j1), (double)f.y, gsum); gsum = fma((double)(sgn * j2), (double)f.z, gsum);
+                        scale = fmaf(fabsf(j0), c.w, fmaf(fabsf(j1), nz.x, fmaf(fabsf(j2), nz.y, scale)));
+                        const float p0 = j0 * f.w, p1 = fmaf(j1, c.x, j2 * c.z), p2 = fmaf(j2, c.y, j1 * c.z);
+                        a = mk3(fmaf(n.x, p0, fmaf(t1.x, p1, t2.x * p2)), fmaf(n.y, p0, fmaf(t1.y, p1, t2.y * p2)), fmaf(n.z, p0, fmaf(t1.z, p1, t2.z * p2)));
+                    }
+                    const V3 m = cross_fma(arm, a);
+                    hr[0] = __fadd_rn(hr[0], a.x); hr[1] = __fadd_rn(hr[1], a.y); hr[2] = __fadd_rn(hr[2], a.z); hr[3] = __fadd_rn(hr[3], m.x); hr[4] = __fadd_rn(hr[4], m.y); hr[5] = __fadd_rn(hr[5], m.z);
+                }
+            __syncwarp();
+            if (parts > 1u) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) hr[k] += __shfl_xor_sync(NKB_FULL, hr[k], 8);
+                gsum += __shfl_xor_sync(NKB_FULL, gsum, 8); scale += __shfl_xor_sync(NKB_FULL, scale, 8);
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) scale = fmaf(fabsf(hr[k]), fabsf((float)u[k]), scale);
+            const float own = (float)gsum;
+            const bool finite = g.all(isfinite(own)), small = g.all(row >= 6u || fabsf(own) <= kRoundings * FLT_EPSILON * scale);
+            failure |= active && !finite;
+            active = active && finite;
+            // the group's rows to every lane of it
+            float a[28], inv[6], x[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
+                a[21 + i] = force[i];
+#pragma unroll
+                for (int k = 0; k <= i; ++k) a[i * (i + 1) / 2 + k] = __shfl_sync(NKB_FULL, hr[k], g.first + i);
+            }
+            if (active && small) {
+                bool still = true;
+                if (run.tol > 0.f) {
+                    const float im = __ldg(t.inv_mass + b);
+                    const float* w = sm_bwinv(e, b);
+                    const V3 ang = mk3(dot_fma(mk3(w[0], w[3], w[4]), mk3(force[3], force[4], force[5])), dot_fma(mk3(w[3], w[1], w[5]), mk3(force[3], force[4], force[5])),
+                                       dot_fma(mk3(w[4], w[5], w[2]), mk3(force[3], force[4], force[5])));
+                    still = fabsf(force[0] * im) < run.tol && fabsf(force[1] * im) < run.tol && fabsf(force[2] * im) < run.tol &&
+                            fabsf(ang.x) < run.tol && fabsf(ang.y) < run.tol && fabsf(ang.z) < run.tol;
+                }
+                if (still) { primal = 0.f; active = false; }
+            }
+            if (!__any_sync(NKB_FULL, active)) break;
+            const bool definite = solve6<false>(a, inv, x);
+            failure |= active && !definite;
+            active = active && definite;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) dir[k] = x[k];
+        }
+        // the block's rows and velocity go back
+        if (began) {
+#pragma unroll 1
+            for (uint32_t k = g.j; k < count; k += g.width) {
+                const uint32_t h = inc[k];
+                const float4 res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h);
+                hq(e, HF_RES, h) = make_float4(__fsub_rn(res.x, move.x), __fsub_rn(res.y, move.y), __fsub_rn(res.z, move.z), res.w);
+            }
+            float moved = failure ? FLT_MAX : 0.f;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) moved = fmaxf(moved, residual_abs((float)u[k] - velocity[k]));
+            failed |= failure;
+            most_moved = fmaxf(most_moved, moved);
+            worst = fmaxf(worst, fmaxf(failure ? FLT_MAX : primal, coupled ? moved : 0.f));
+        }
+        __syncwarp();
+        if (began && g.j < 6u) velocity[g.j] = (float)pick6(u, g.j);
+        __syncwarp();
+    }
     RigidResult out;
-    out.momentum = tile.momentum; out.residual = tile.residual; out.status = e.status;
+    out.momentum = warp_max_positive(most_moved); out.residual = warp_max_positive(worst);
+    out.status = __any_sync(NKB_FULL, failed) ? (uint32_t)kStatusSolverFailure : 0u;
     return out;
 }
 
@@ -1436,7 +1641,7 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
 template <int NR, bool kRigid>
 NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
     if (e.t->tree_depth != 0u && !e.branching) descend_tree<NR>(e, tile, position);
-    else descend_block<NR, kRigid, 0>(e, tile, e.t->B, position);
+    else descend_block<NR>(e, tile, e.t->B, position);
 }
 
 // Blocks descend colour by colour, blocks of one colour in index order (block_descent_tile.cuh:2749-2820).
@@ -1451,7 +1656,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
     } else {
         const uint32_t team = e.lay->team;
         RigidRun run;
-        run.sm = e.sm; run.lay = e.lay; run.t = e.t; run.lane = e.lane; run.vstride = e.vstride; run.newton_shift = 0u; run.vec_shift = 0u;
+        run.sm = e.sm; run.lay = e.lay; run.t = e.t; run.lane = e.lane; run.vstride = e.vstride;
         run.nheads = tile.nheads; run.nblocks = nb; run.iteration = tile.iteration; run.tol = tile.tol;
 #pragma unroll 1
         for (uint32_t k = 0u; k < count;) {
@@ -1461,10 +1666,10 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
             const uint32_t colour = blk_color(e, nb, b);
             uint32_t k_end = k + 1u;
 #pragma unroll 1
-            while (k_end < count && order[k_end] != e.t->B && blk_color(e, nb, order[k_end]) == colour) ++k_end;
             // colour 31 is the overflow colour (index_blocks hands it to every block past the 31st colour): not a set of
-            // independent blocks, so it stays with the lead
-            const bool shared_out = team > 1u && k_end - k > 1u && colour < 31u && team_command(e.sm, *e.lay)->dead == 0u;
+            // independent blocks, so they descend one by one
+            while (colour < 31u && k_end < count && order[k_end] != e.t->B && blk_color(e, nb, order[k_end]) == colour) ++k_end;
+            const bool shared_out = team > 1u && k_end - k > 32u / e.lay->body_lanes && team_command(e.sm, *e.lay)->dead == 0u;
             const uint32_t stride = shared_out ? team : 1u;
             uint32_t seq = 0u;
             if (shared_out) {
@@ -1480,7 +1685,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
             // helper failed to answer, and take the helpers' shares
 #pragma unroll 1
             do {
-                const RigidResult part = descend_rigid_run<kRigid>(run, k, k_end, share, stride, position);
+                const RigidResult part = descend_bodies(run, k, k_end, share, stride, position);
                 mine.momentum = fmaxf(mine.momentum, part.momentum); mine.residual = fmaxf(mine.residual, part.residual);
                 mine.status |= part.status;
                 if (shared_out && share == 0u) {
@@ -1576,93 +1781,141 @@ NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velo
     }
 }
 
+// Momentum balance of the free bodies, a group of lanes on each (BodyLanes): lane = row, the rows' Jacobian entries from the
+// contact frames.
+NKB_DEV void measure_bodies(Env& e, Tile& tile, bool reconstruct) {
+    const TemplateView& t = *e.t;
+    const BodyLanes g = body_lanes(e);
+    const uint32_t nb = tile.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
+    const uint32_t* order = block_order(e, nb);
+    const uint32_t blocks = order[nb];
+    float worst = 0.f;
+#pragma unroll 1
+    for (uint32_t base = 0u; base < blocks; base += groups) {
+        const uint32_t turn = base + e.lane / g.width;
+        const uint32_t b = turn < blocks ? order[turn] : t.B;
+        const bool have = b != t.B;                                // the articulation's block has its own measure
+        const uint32_t* inc = blk_inc(e, nb) + blk_inc_begin(e, nb, b);
+        const uint32_t count = have ? blk_inc_begin(e, nb, b + 1u) - blk_inc_begin(e, nb, b) : 0u;
+        double balance = 0.0;
+        if (have) {
+            const float* vel = block_vel(e, b, false);
+            const float* fr = sm_bfree(e, b);
+            if (part == 0u && row < 6u) {
+                const float* bm = sm_bmass(e, b);
+                if (row < 3u) balance = -(double)bm[0] * ((double)vel[row] - fr[row]);
+                else {
+                    const float m3 = row == 3u ? bm[1] : row == 4u ? bm[4] : bm[5], m4 = row == 3u ? bm[4] : row == 4u ? bm[2] : bm[6], m5 = row == 3u ? bm[5] : row == 4u ? bm[6] : bm[3];
+                    balance = -((double)m3 * ((double)vel[3] - fr[3]) + (double)m4 * ((double)vel[4] - fr[4]) + (double)m5 * ((double)vel[5] - fr[5]));
+                }
+            }
+#pragma unroll 1
+            for (uint32_t k = part; k < count; k += parts) {
+                const uint32_t h = inc[k];
+                const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                const V3 w = body_row_axis(row, hf3(e, first_side ? HF_RA : HF_RB, h)), lam = head_lambda(e, h);
+                const float sgn = first_side ? 1.f : -1.f;
+                balance = fma((double)(sgn * dot(hf3(e, HF_N, h), w)), (double)lam.x, balance);
+                balance = fma((double)(sgn * dot(hf3(e, HF_T1, h), w)), (double)lam.y, balance);
+                balance = fma((double)(sgn * dot(hf3(e, HF_T2, h), w)), (double)lam.z, balance);
+            }
+        }
+        __syncwarp();
+        if (parts > 1u) balance += __shfl_xor_sync(NKB_FULL, balance, 8);
+        const bool finite = g.all(fabs(balance) <= FLT_MAX);
+        float force[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) force[k] = __shfl_sync(NKB_FULL, (float)balance, g.first + k);
+        if (have) {
+            float residual = FLT_MAX;
+            if (finite) {
+                const float im = __ldg(t.inv_mass + b);
+                const V3 ang = sym_mulv(sm_bwinv(e, b), mk3(force[3], force[4], force[5]));
+                const float dir[6] = {force[0] * im, force[1] * im, force[2] * im, ang.x, ang.y, ang.z};
+                residual = 0.f;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) residual = fmaxf(residual, isfinite(dir[k]) ? fabsf(dir[k]) : FLT_MAX);
+                if (reconstruct) {
+                    if (g.j < 6u) block_vel(e, b, false)[g.j] += pick6(dir, g.j);
+                    tile.momentum = fmaxf(tile.momentum, residual);
+                }
+            }
+            worst = fmaxf(worst, residual);
+        }
+        __syncwarp();
+    }
+    tile.residual = fmaxf(tile.residual, warp_max_positive(worst));
+    tile.momentum = warp_max(tile.momentum);
+}
+
 // Momentum balance of every moving block against the physical multipliers (block_descent_tile.cuh:2379-2489).
 template <int NR, bool kRigid>
 NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
     const uint32_t nb = tile.nblocks, l = e.lane;
     const uint32_t* inc = blk_inc(e, nb);
-    const uint32_t* order = block_order(e, nb);
-    const uint32_t count = order[nb];
-#pragma unroll 1
-    for (uint32_t turn = 0u; turn < count; ++turn) {
-        const uint32_t b = kRigid ? order[turn] : e.t->B;
-        const uint32_t dim = blk_dim(e, b);
-        const bool artic = !kRigid || b == e.t->B;
-        float* vel = block_vel(e, b, false);
-        const float* fr = block_free(e, b);
-        const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
-        double balance[NR];
-        bool coord[NR];
+    if constexpr (kRigid) measure_bodies(e, tile, reconstruct);
+    const uint32_t b = e.t->B, dim = e.t->ndof;
+    if (dim == 0u) return;
+    float* vel = block_vel(e, b, false);
+    const float* fr = block_free(e, b);
+    const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
+    double balance[NR];
+    bool coord[NR];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) { balance[r] = 0.0; coord[r] = l + 32u * r < dim; }
-        if (artic) {
-            const uint32_t n4 = (dim + 3u) & ~3u;
-            const uint16_t* utab = unit_table(e, nb);
-            const uint32_t vs = e.vstride;
+    for (int r = 0; r < NR; ++r) { balance[r] = 0.0; coord[r] = l + 32u * r < dim; }
+    {
+        const uint32_t n4 = (dim + 3u) & ~3u;
+        const uint16_t* utab = unit_table(e, nb);
+        const uint32_t vs = e.vstride;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint32_t c = l + 32u * r;
+            if (!coord[r]) continue;
+            const float* Mr = sm_mass(e) + c * e.lay->ld;
+#pragma unroll 1
+            for (uint32_t j = 0u; j < dim; ++j) balance[r] -= (double)Mr[j] * ((double)vel[j] - fr[j]);
+#pragma unroll 1
+            for (uint32_t slot = 0u; slot < 4u; ++slot) {
+                const uint32_t h = utab[slot * vs + c];
+                if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAMX, h);
+            }
+        }
+#pragma unroll 1
+        for (uint32_t k = ib; k < ie; ++k) {
+            const uint32_t h = inc[k];
+            const uint32_t jo = hu(e, HF_JOFF, h);
+            if (jo & kUnitRow) continue;
+            const V3 lam = head_lambda(e, h);
+            const float* jr = sm_jpool(e) + jo;
+            const bool cone = head_axes(e, h) == 3u;
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
                 const uint32_t c = l + 32u * r;
                 if (!coord[r]) continue;
-                const float* Mr = sm_mass(e) + c * e.lay->ld;
-#pragma unroll 1
-                for (uint32_t j = 0u; j < dim; ++j) balance[r] -= (double)Mr[j] * ((double)vel[j] - fr[j]);
-#pragma unroll 1
-                for (uint32_t slot = 0u; slot < 4u; ++slot) {
-                    const uint32_t h = utab[slot * vs + c];
-                    if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAMX, h);
-                }
-            }
-#pragma unroll 1
-            for (uint32_t k = ib; k < ie; ++k) {
-                const uint32_t h = inc[k];
-                const uint32_t jo = hu(e, HF_JOFF, h);
-                if (jo & kUnitRow) continue;
-                const V3 lam = head_lambda(e, h);
-                const float* jr = sm_jpool(e) + jo;
-                const bool cone = head_axes(e, h) == 3u;
-#pragma unroll
-                for (int r = 0; r < NR; ++r) {
-                    const uint32_t c = l + 32u * r;
-                    if (!coord[r]) continue;
-                    balance[r] += (double)jr[c] * lam.x;
-                    if (cone) balance[r] += (double)jr[n4 + c] * lam.y + (double)jr[2u * n4 + c] * lam.z;
-                }
-            }
-        } else {
-            if (coord[0]) for (uint32_t j = 0u; j < dim; ++j) balance[0] -= (double)block_mass(e, b, l, j) * ((double)vel[j] - fr[j]);
-#pragma unroll 1
-            for (uint32_t k = ib; k < ie; ++k) {
-                const uint32_t h = inc[k];
-                const uint32_t side = head_owner(e, h, 0u) == b ? 0u : 1u, axes = head_axes(e, h);
-                const V3 lam = head_lambda(e, h);
-#pragma unroll 1
-                for (uint32_t ax = 0u; ax < axes; ++ax) {
-                    const float imp = comp(lam, (int)ax);
-                    if (imp == 0.f) continue;
-                    if (coord[0]) balance[0] += (double)head_jac(e, h, side, ax, l, b) * imp;
-                }
+                balance[r] += (double)jr[c] * lam.x;
+                if (cone) balance[r] += (double)jr[n4 + c] * lam.y + (double)jr[2u * n4 + c] * lam.z;
             }
         }
-        float force[NR], dir[NR];
-        bool ok = true;
+    }
+    float force[NR], dir[NR];
+    bool ok = true;
 #pragma unroll
-        for (int r = 0; r < NR; ++r) { force[r] = coord[r] ? (float)balance[r] : 0.f; dir[r] = 0.f; ok &= !coord[r] || fabs(balance[r]) <= FLT_MAX; }
-        const bool finite = __all_sync(NKB_FULL, ok);
-        float residual = FLT_MAX;
-        if (finite) {
-            solve_block_mass<NR>(e, b, force, dir);
-            float worst = 0.f;
+    for (int r = 0; r < NR; ++r) { force[r] = coord[r] ? (float)balance[r] : 0.f; dir[r] = 0.f; ok &= !coord[r] || fabs(balance[r]) <= FLT_MAX; }
+    const bool finite = __all_sync(NKB_FULL, ok);
+    float residual = FLT_MAX;
+    if (finite) {
+        solve_block_mass<NR>(e, b, force, dir);
+        float worst = 0.f;
 #pragma unroll
-            for (int r = 0; r < NR; ++r) if (coord[r]) worst = fmaxf(worst, isfinite(dir[r]) ? fabsf(dir[r]) : FLT_MAX);
-            residual = warp_max(worst);
-        }
-        tile.residual = fmaxf(tile.residual, residual);
-        if (reconstruct && finite) {
+        for (int r = 0; r < NR; ++r) if (coord[r]) worst = fmaxf(worst, isfinite(dir[r]) ? fabsf(dir[r]) : FLT_MAX);
+        residual = warp_max(worst);
+    }
+    tile.residual = fmaxf(tile.residual, residual);
+    if (reconstruct && finite) {
 #pragma unroll
-            for (int r = 0; r < NR; ++r) if (coord[r]) vel[l + 32u * r] += dir[r];
-            tile.momentum = fmaxf(tile.momentum, residual);
-            __syncwarp();
-        }
+        for (int r = 0; r < NR; ++r) if (coord[r]) vel[l + 32u * r] += dir[r];
+        tile.momentum = fmaxf(tile.momentum, residual);
+        __syncwarp();
     }
 }
 

@@ -291,16 +291,11 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     }
 }
 
-// A helper warp's life: wait for a command, do its share (rigid blocks of a colour on private Newton scratch, or a slice of
+// A helper warp's life: wait for a command, do its share (rigid blocks of a colour, or a slice of
 // a stage's outer loop), answer, until told to leave (or until a wait runs out).
 template <bool kRigid>
 NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const TemplateView& t, const StateView& state, uint32_t env,
                          uint32_t member, uint32_t lane, uint32_t vstride) {
-    // private copies of the regions a block descent scratches in (same arrangement as the env's own: Newton matrix, block
-    // mass, staged rows; then the solver vectors); everything else is the env's own
-    const uint32_t newton_span = shared_layout.rjac + 24u * shared_layout.rjac_heads - shared_layout.chol;
-    const uint32_t base = shared_layout.team_area + kTeamCommandWords + ((4u * shared_layout.team + 3u) & ~3u) + (member - 1u) * shared_layout.helper_words;
-    const uint32_t newton_shift = base - shared_layout.chol, vec_shift = base + newton_span - shared_layout.vecs;
     const TeamCommand* cmd = team_command(sm, shared_layout);
     uint32_t* answer = reinterpret_cast<uint32_t*>(team_result(sm, shared_layout, member));
     uint32_t last = 0u;
@@ -332,12 +327,11 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
         if (op == kTeamDescend && k_begin < k_end && k_end <= nblocks && nblocks <= t.B + 1u) {
             RigidRun run;
             run.sm = sm; run.lay = &shared_layout; run.t = &t; run.lane = lane; run.vstride = vstride;
-            run.newton_shift = newton_shift; run.vec_shift = vec_shift;
             run.nheads = cmd->nheads; run.nblocks = nblocks; run.iteration = cmd->iteration; run.tol = cmd->tol;
 #ifdef NKB_STAGE_TAPS
             const long long tap0 = clock64();
 #endif
-            r = descend_rigid_run<kRigid>(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
+            r = descend_bodies(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
 #ifdef NKB_STAGE_TAPS
             if (state.dbg_cycles != nullptr && lane == 0u && member == 1u) {
                 uint32_t* cyc = state.dbg_cycles + (size_t)env * 32u;

@@ -66,11 +66,6 @@ NKB_DEV void tree_load_row(const Env& e, const TreeLane& t, const float* matrix,
     row.diag = src[t.coord];
 }
 
-// Reciprocal square root of a pivot that is positive and normal (the hardware's, 2 ulp; no denormal path).
-NKB_DEV float rsqrt_normal(float v) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
-NKB_DEV bool pivot_valid(float v) { return v >= FLT_MIN && v <= FLT_MAX; }
-constexpr float kMassPivotFloor = 1.0e-6f;       // articulation_mass.cuh:269-335
-
 // Rows of the tree in shared memory: joint lanes first .. first + rows.  With one coordinate per lane the base's lanes hold no
 // joint and get no row.
 template <int NR> NKB_DEV uint32_t tree_first(const Env& e) { return NR == 1 && e.t->floating_root ? 6u : 0u; }
@@ -177,35 +172,13 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
         for (int k = 0; k < 7; ++k) { const float4 v = reinterpret_cast<const float4*>(entries)[k]; a[4 * k] = v.x; a[4 * k + 1] = v.y; a[4 * k + 2] = v.z; a[4 * k + 3] = v.w; }
         if (kKeep) __syncwarp();
         float inv[kTreeBase];
-#pragma unroll
-        for (int k = 0; k < kTreeBase; ++k) {
-            float pivot = a[k * (k + 1) / 2 + k];
-            if (kKeep) pivot = fmaxf(pivot, kMassPivotFloor);
-            valid &= pivot_valid(pivot);
-            inv[k] = rsqrt_normal(pivot);
-            a[21 + k] *= inv[k];
-#pragma unroll
-            for (int i = k + 1; i < kTreeBase; ++i) a[i * (i + 1) / 2 + k] *= inv[k];
-#pragma unroll
-            for (int i = k + 1; i < kTreeBase; ++i) {
-                a[21 + i] = fmaf(-a[i * (i + 1) / 2 + k], a[21 + k], a[21 + i]);
-#pragma unroll
-                for (int j = k + 1; j <= i; ++j) a[i * (i + 1) / 2 + j] = fmaf(-a[i * (i + 1) / 2 + k], a[j * (j + 1) / 2 + k], a[i * (i + 1) / 2 + j]);
-            }
-        }
+        valid &= solve6<kKeep>(a, inv, base_x);
         if (kKeep && lane == 0u) {          // every lane holds the block; nobody reads the entries any more
             float4* out = reinterpret_cast<float4*>(entries);
 #pragma unroll
             for (int k = 0; k < 5; ++k) out[k] = make_float4(a[4 * k], a[4 * k + 1], a[4 * k + 2], a[4 * k + 3]);
             out[5] = make_float4(a[20], inv[0], inv[1], inv[2]);
             out[6] = make_float4(inv[3], inv[4], inv[5], 0.f);
-        }
-#pragma unroll
-        for (int k = kTreeBase - 1; k >= 0; --k) {
-            float s = a[21 + k];
-#pragma unroll
-            for (int i = k + 1; i < kTreeBase; ++i) s = fmaf(-a[i * (i + 1) / 2 + k], base_x[i], s);
-            base_x[k] = s * inv[k];
         }
 #pragma unroll
         for (int k = 0; k < kTreeBase; ++k) acc = fmaf(-row.base[k], base_x[k], acc);

@@ -135,11 +135,11 @@ struct SmemLayout {
     uint32_t bpose, bvel, bwinv, aabb, bmass, bfree, bpseudo;   // bodies
     uint32_t pairs, ccount, cpoint, cnormal, cdepth, cfeat;     // contacts
     uint32_t cstage;                                            // cache rebuild staging (shares the Jacobian pool, dead by then)
-    uint32_t heads, jpool, binfo, chol, bm6;                    // solver (chol: Newton matrix; bm6: rigid block mass + head rows)
-    uint32_t rjac, rjac_heads;                                  // staged Jacobian rows of one rigid block's heads (24 words each)
+    uint32_t heads, jpool, binfo, chol;                         // solver (chol: the articulation's Newton matrix)
+    uint32_t body_lanes;                                        // lanes that work on one free body: 8 or 16
     // Team mode: `team` warps advance one env; warp 0 leads, the others wait for work (rigid blocks of one colour).
-    // team_area: 12 command words, 4 result words per member, then helper_words of private Newton scratch per helper.
-    uint32_t team, team_area, helper_words;
+    // team_area: 12 command words, then 4 result words per member.
+    uint32_t team, team_area;
     // Fault drills for the team's bounded waits (tests only): bit 0 = the lead leaves without dismissing its helpers,
     // bit 1 = helpers never answer a command.  Either way every wait runs out, a status bit is set and the kernel ends.
     uint32_t team_drill;

@@ -358,7 +358,6 @@ void World::BuildLayout() {
     s.ld = pad_ld(n);
     s.pose = take(7 * L); s.vel = take(6 * L);
     // the dynamics stage's link scratch and the solver's Newton scratch are live at different times and share one region
-    const uint32_t hn = std::max(n, 6u);
     const uint32_t overlay = at;
     s.xrot = take(9 * L); s.xtr = take(3 * L); s.vbias = 0; s.acc = take(6 * L); s.pbias = take(6 * L); s.ic = take(10 * L);
     const uint32_t dynamics_end = at;
@@ -369,9 +368,7 @@ void World::BuildLayout() {
     // controllers of modes 3 and 4 work on the dense factor.
     tv.mass_tree = t.tree_depth != 0u && 2u * t.tree_depth <= n && t.cfg.control_mode != 3u && t.cfg.control_mode != 4u ? 1u : 0u;
     const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
-    s.chol = take(std::max(hn * pad_ld(hn), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u)); s.bm6 = take(72 + 24);
-    s.rjac_heads = t.n_free ? std::min(tv.head_cap, 32u) : 0u;
-    s.rjac = take(24 * s.rjac_heads);
+    s.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
     at = std::max(at, dynamics_end);
     s.mass = take(n * s.ld); s.factor = take(tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld); s.vstride = n > 32u ? 64u : 32u;
     s.vecs = take(6 * s.vstride);
@@ -396,23 +393,26 @@ void World::BuildLayout() {
     // leave the SM with one or two resident warps; instead several warps share the env and descend the rigid blocks
     // of one colour side by side (blocks of a colour share no constraint row).  Registers allow about 11 resident
     // warps per SM, so teams only pay where shared memory already holds residency below that.
-    s.team = 1u; s.team_area = at; s.helper_words = 0u; s.team_drill = 0u;
+    s.team = 1u; s.team_area = at; s.team_drill = 0u;
     if (const char* drill = std::getenv("NUKA_B200_TEAM_DRILL")) s.team_drill = static_cast<uint32_t>(std::atoi(drill)) & 3u;
     {
-        const uint32_t helper = (s.rjac + 24u * s.rjac_heads - s.chol) + 6u * s.vstride;     // Newton matrix, block mass, staged rows as the env lays them out; vectors
+        auto area = [](uint32_t w) { return 12u + ((4u * w + 3u) & ~3u); };
         uint32_t team = 1u;
         if (t.n_free >= 8u) {
             const uint32_t envs_alone = std::max<uint32_t>(1u, (227u * 1024u) / (at * 4u + 1024u));      // resident envs, one warp each
-            while (team * 2u <= kWarpsPerBlockMax && envs_alone * team * 2u <= 11u &&
-                   (at + 12u + 4u * (team * 2u) + helper * (team * 2u - 1u)) * 4u <= 220u * 1024u) team *= 2u;
+            while (team * 2u <= kWarpsPerBlockMax && envs_alone * team * 2u <= 11u && (at + area(team * 2u)) * 4u <= 220u * 1024u) team *= 2u;
         }
+        // Lanes per free body in a block descent.  A body alone on its env's one warp leaves most lanes idle: 8 lanes each,
+        // four bodies at a time.  A team has warps for two bodies each (a colour of a 48-box pile holds about 13).  The choice
+        // follows the template, not a forced team size: sums over rows depend on it, and team sizes give bit-identical states.
+        s.body_lanes = team > 1u ? 16u : 8u;
         if (const char* forced = std::getenv("NUKA_B200_TEAM")) {                        // team-size experiments
             const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
-            if (w >= 1u && w <= kWarpsPerBlockMax && t.n_free != 0u && (at + 12u + 4u * w + helper * (w - 1u)) * 4u <= 220u * 1024u) team = w;
+            if (w >= 1u && w <= kWarpsPerBlockMax && t.n_free != 0u && (at + area(w)) * 4u <= 220u * 1024u) team = w;
         }
         if (team > 1u) {
-            s.team = team; s.helper_words = (helper + 3u) & ~3u;
-            s.team_area = take(12u + ((4u * team + 3u) & ~3u) + s.helper_words * (team - 1u));
+            s.team = team;
+            s.team_area = take(area(team));
         }
     }
     s.words = at;
