@@ -35,16 +35,14 @@ NKB_DEV void world_inv_inertia(Q4 pose_q, Q4 inertial_q, V3 inv_i, float* out) {
     }
 }
 
-// Poses and velocities of every collidable row into shared memory; free bodies take their gravity kick.
-NKB_DEV void stage_bodies(Env& e, bool kick) {
+// Poses of every collidable row into shared memory: link mirrors follow the link poses; free bodies come from global memory,
+// with their velocities, when `load` is set and keep their integrated state otherwise.
+NKB_DEV void stage_body_poses(Env& e, bool load) {
     const TemplateView& t = *e.t;
-    const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
 #pragma unroll 1
     for (uint32_t b = e.lane; b < t.B; b += 32u) {
         const uint32_t link = __ldg(t.body_to_link + b);
         float* bp = sm_bpose(e, b);
-        float* bv = sm_bvel(e, b);
-        const size_t gb = (size_t)e.env * t.B + b;
         if (link != kNoLink) {
             const float* lp = sm_pose(e, link);
             if (__ldg(t.body_geom_kind + b) != 0u) {
@@ -55,26 +53,33 @@ NKB_DEV void stage_bodies(Env& e, bool kick) {
 #pragma unroll
                 for (int k = 0; k < 7; ++k) bp[k] = lp[k];
             }
-#pragma unroll
-            for (int k = 0; k < 6; ++k) bv[k] = 0.f;
-        } else {
+        } else if (load) {
+            const size_t gb = (size_t)e.env * t.B + b;
             const float* gp = e.s->body_pose + gb * 7u;
 #pragma unroll
             for (int k = 0; k < 7; ++k) bp[k] = gp[k];
-            V3 lv = ld3(e.s->body_linvel + gb * 3u);
-            const V3 av = ld3(e.s->body_angvel + gb * 3u);
-            const bool dynamic = __ldg(t.inv_mass + b) > 0.f;
-            if (kick && dynamic) lv = lv + g * t.cfg.dt;
-            if (dynamic) { st3(bv, lv); st3(bv + 3, av); }
-            else { st3(bv, mk3(0.f, 0.f, 0.f)); st3(bv + 3, mk3(0.f, 0.f, 0.f)); }      // static rows share the zero slot
-        }
-        float* w = sm_bwinv(e, b);
-        if (__ldg(t.inv_mass + b) > 0.f) world_inv_inertia(ldq(bp + 3), ldq(t.inertial_quat + 4u * b), ld3(t.inv_inertia + 3u * b), w);
-        else {
-#pragma unroll
-            for (int k = 0; k < 6; ++k) w[k] = 0.f;
+            if (__ldg(t.inv_mass + b) > 0.f) {
+                float* bv = sm_bvel(e, b);
+                st3(bv, ld3(e.s->body_linvel + gb * 3u)); st3(bv + 3, ld3(e.s->body_angvel + gb * 3u));
+            }
         }
     }
+    __syncwarp();
+}
+
+// Free bodies take their gravity kick and their world inverse inertia; every other row shares the zero slot.
+NKB_DEV void stage_body_kick(Env& e) {
+    const TemplateView& t = *e.t;
+    const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
+    if (e.lane < 6u) { e.sm[e.lay->bvel + 6u * t.n_free + e.lane] = 0.f; e.sm[e.lay->bwinv + 6u * t.n_free + e.lane] = 0.f; }
+    if (t.n_free != 0u)
+#pragma unroll 1
+        for (uint32_t b = e.lane; b < t.B; b += 32u) {
+            if (!(__ldg(t.inv_mass + b) > 0.f)) continue;
+            float* bv = sm_bvel(e, b);
+            if (__ldg(t.body_to_link + b) == kNoLink) st3(bv, ld3(bv) + g * t.cfg.dt);
+            world_inv_inertia(ldq(sm_bpose(e, b) + 3), ldq(t.inertial_quat + 4u * b), ld3(t.inv_inertia + 3u * b), sm_bwinv(e, b));
+        }
     __syncwarp();
 }
 
@@ -165,6 +170,7 @@ NKB_DEV void stage_store_contacts(Env& e, uint32_t pair_count) {
         e.s->pairs[gs * 2u] = ab >> 16; e.s->pairs[gs * 2u + 1u] = ab & 0xffffu;
         const uint32_t n = s < t.slot_cap ? sm_ccount(e)[s] : 0u;
         e.s->contact_count[gs] = n;
+#pragma unroll 1
         for (uint32_t i = 0; i < 4u; ++i) {
             const bool live = i < n;
             const uint32_t at = s * 4u + i;

@@ -114,19 +114,17 @@ NKB_DEV void stage_drives(Env& e) {
     e.tau = inverse_dynamics ? 0.f : ff;
 }
 
-// Bias forces, mass matrix, factor and unconstrained acceleration; optionally the semi-implicit velocity
-// update.  Leaves M and its L D L^T factor in shared memory for the constraint solve.
+// Bias forces and mass matrix at the current kinematics; E, r is the joint transform of this lane's link.  Leaves M in shared
+// memory and this lane's entries of the generalised bias in `bias`.
 template <int NR>
-NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
+NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, L = t.L, n = t.ndof, ld = e.lay->ld;
     const bool link = l < L;
     const bool froot = link && e.parent == kNoLink && e.jtype == kFloating;
     const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
     const float dt = t.cfg.dt;
-    float E[9]; V3 r = mk3(0.f, 0.f, 0.f);
     if (link) {
-        joint_xform(e, E, r);
         float* xe = sm_xrot(e, l);
 #pragma unroll
         for (int k = 0; k < 9; ++k) xe[k] = E[k];
@@ -209,37 +207,19 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
         }
         __syncwarp();
     }
-    // generalized bias and right-hand side, lane = coordinate
-    float rhs[NR];
-    bool dof[NR];
+    // generalised bias, lane = coordinate
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        const uint32_t c = l + 32u * r;
-        const float diss_of_link = __shfl_sync(NKB_FULL, e.drive_dissipation, e.dof_link[r]);
-        const float tau_of_link = __shfl_sync(NKB_FULL, e.tau, e.dof_link[r]);
-        const float qd_of_link = __shfl_sync(NKB_FULL, e.qd, e.dof_link[r]);
-        const float q_of_link = __shfl_sync(NKB_FULL, e.q, e.dof_link[r]);
-        rhs[r] = 0.f;
-        dof[r] = c < n;
-        if (dof[r]) {
+        bias[r] = 0.f;
+        if (l + 32u * r < n) {
             const uint32_t dl = e.dof_link[r];
             const float* pb = sm_pbias(e, dl);
-            float bias;
             if (e.dof_comp[r] == kNoLink) {
                 V3 a = ld3(t.axis + 3u * dl);
                 const float ls = dot(a, a);
                 if (ls > 1.0e-12f) a = a * rsqrtf(ls);
-                const uint32_t jt = __ldg(t.jtype + dl);
-                bias = jt == kRevolute ? dot(a, ld3(pb)) : dot(a, ld3(pb + 3));
-                e.vel0[r] = qd_of_link;
-                const float damping = __ldg(t.damping + dl) + diss_of_link;
-                const float spring = __ldg(t.stiffness + dl) * (q_of_link - __ldg(t.spring_ref + dl));
-                rhs[r] = tau_of_link - bias - damping * e.vel0[r] - spring;
-            } else {
-                bias = pb[e.dof_comp[r]];
-                e.vel0[r] = sm_vel(e, dl)[e.dof_comp[r]];
-                rhs[r] = -bias;
-            }
+                bias[r] = __ldg(t.jtype + dl) == kRevolute ? dot(a, ld3(pb)) : dot(a, ld3(pb + 3));
+            } else bias[r] = pb[e.dof_comp[r]];
         }
     }
     // mass matrix, ops/articulation_mass.cuh:124-253
@@ -301,6 +281,40 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
 #pragma unroll 1
         for (uint32_t k = l; k < n * n; k += 32u) out[k] = M[(k / n) * ld + k % n];
     }
+}
+
+// Accelerations under the lanes' efforts (e.tau), the bias and the passive terms; `factor` factors M first (it stays in shared
+// memory for the constraint solve and for further calls); optionally the semi-implicit velocity update.
+template <int NR>
+NKB_DEV void stage_accelerations(Env& e, const float (&bias)[NR], bool factor, bool integrate_velocity) {
+    const TemplateView& t = *e.t;
+    const uint32_t l = e.lane, n = t.ndof, ld = e.lay->ld;
+    const bool link = l < t.L;
+    const float dt = t.cfg.dt;
+    const float* M = sm_mass(e);
+    float rhs[NR], vel0[NR];
+    bool dof[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const float diss_of_link = __shfl_sync(NKB_FULL, e.drive_dissipation, e.dof_link[r]);
+        const float tau_of_link = __shfl_sync(NKB_FULL, e.tau, e.dof_link[r]);
+        const float qd_of_link = __shfl_sync(NKB_FULL, e.qd, e.dof_link[r]);
+        const float q_of_link = __shfl_sync(NKB_FULL, e.q, e.dof_link[r]);
+        rhs[r] = 0.f; vel0[r] = 0.f;
+        dof[r] = l + 32u * r < n;
+        if (dof[r]) {
+            const uint32_t dl = e.dof_link[r];
+            if (e.dof_comp[r] == kNoLink) {
+                vel0[r] = qd_of_link;
+                const float damping = __ldg(t.damping + dl) + diss_of_link;
+                const float spring = __ldg(t.stiffness + dl) * (q_of_link - __ldg(t.spring_ref + dl));
+                rhs[r] = tau_of_link - bias[r] - damping * vel0[r] - spring;
+            } else {
+                vel0[r] = sm_vel(e, dl)[e.dof_comp[r]];
+                rhs[r] = -bias[r];
+            }
+        }
+    }
     float x[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) x[r] = dof[r] ? rhs[r] : 0.f;
@@ -316,49 +330,51 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
         tree_solve<NR, true>(e, tl, row, high ? x[NR - 1] : x[0], base_row, x[0], sm_factor(e), joint, base_x);
         tree_scatter<NR>(e, joint, base_x, x);
     } else {
-        // L D L^T, unit lower triangle with D on the diagonal and pivot floor 1e-6 (articulation_mass.cuh:269-335).
-        // Column by column, lane = row: entry (row, k) = (M[row][k] - sum_{j<k} L[row][j] L[k][j] d_j) / d_k, the terms
-        // subtracted in ascending j exactly as the reference's in-place elimination subtracts them, but with both rows
-        // and the pivots read ahead of one short dependent chain instead of a read-modify-write per term.
         float* F = sm_factor(e);
-        float* piv = sm_vec(e, kVecTmp);
+        if (factor) {
+            // L D L^T, unit lower triangle with D on the diagonal and pivot floor 1e-6 (articulation_mass.cuh:269-335).
+            // Column by column, lane = row: entry (row, k) = (M[row][k] - sum_{j<k} L[row][j] L[k][j] d_j) / d_k, the terms
+            // subtracted in ascending j exactly as the reference's in-place elimination subtracts them, but with both rows
+            // and the pivots read ahead of one short dependent chain instead of a read-modify-write per term.
+            float* piv = sm_vec(e, kVecTmp);
 #pragma unroll 1
-        for (uint32_t k = l; k < n * ld; k += 32u) F[k] = M[k];
-        __syncwarp();
+            for (uint32_t k = l; k < n * ld; k += 32u) F[k] = M[k];
+            __syncwarp();
 #pragma unroll 1
-        for (uint32_t k = 0; k < n; ++k) {
-            const float* Fk = F + k * ld;
-            float v[NR];
+            for (uint32_t k = 0; k < n; ++k) {
+                const float* Fk = F + k * ld;
+                float v[NR];
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const uint32_t row = l + 32u * r;
-                v[r] = 0.f;
-                if (row >= k && row < n) {
-                    const float* Fr = F + row * ld;
-                    const float4* Fr4 = reinterpret_cast<const float4*>(Fr);
-                    const float4* Fk4 = reinterpret_cast<const float4*>(Fk);
-                    const float4* piv4 = reinterpret_cast<const float4*>(piv);
-                    float acc = Fr[k];
-                    const uint32_t full = k >> 2;
+                for (int r = 0; r < NR; ++r) {
+                    const uint32_t row = l + 32u * r;
+                    v[r] = 0.f;
+                    if (row >= k && row < n) {
+                        const float* Fr = F + row * ld;
+                        const float4* Fr4 = reinterpret_cast<const float4*>(Fr);
+                        const float4* Fk4 = reinterpret_cast<const float4*>(Fk);
+                        const float4* piv4 = reinterpret_cast<const float4*>(piv);
+                        float acc = Fr[k];
+                        const uint32_t full = k >> 2;
 #pragma unroll 1
-                    for (uint32_t c = 0u; c < full; ++c) {
-                        const float4 a = Fr4[c], b4 = Fk4[c], p = piv4[c];
-                        acc -= a.x * b4.x * p.x; acc -= a.y * b4.y * p.y; acc -= a.z * b4.z * p.z; acc -= a.w * b4.w * p.w;
+                        for (uint32_t c = 0u; c < full; ++c) {
+                            const float4 a = Fr4[c], b4 = Fk4[c], p = piv4[c];
+                            acc -= a.x * b4.x * p.x; acc -= a.y * b4.y * p.y; acc -= a.z * b4.z * p.z; acc -= a.w * b4.w * p.w;
+                        }
+#pragma unroll 1
+                        for (uint32_t j = full << 2; j < k; ++j) acc -= Fr[j] * Fk[j] * piv[j];
+                        v[r] = acc;
                     }
-#pragma unroll 1
-                    for (uint32_t j = full << 2; j < k; ++j) acc -= Fr[j] * Fk[j] * piv[j];
-                    v[r] = acc;
                 }
-            }
-            const float dk = fmaxf(coord_bcast<NR>(v, k), 1.0e-6f);
-            __syncwarp();
+                const float dk = fmaxf(coord_bcast<NR>(v, k), 1.0e-6f);
+                __syncwarp();
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const uint32_t row = l + 32u * r;
-                if (row == k) { F[row * ld + k] = dk; piv[k] = dk; }
-                else if (row > k && row < n) F[row * ld + k] = v[r] / dk;
+                for (int r = 0; r < NR; ++r) {
+                    const uint32_t row = l + 32u * r;
+                    if (row == k) { F[row * ld + k] = dk; piv[k] = dk; }
+                    else if (row > k && row < n) F[row * ld + k] = v[r] / dk;
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
         // the strict upper triangle keeps M's entries; only the lower triangle and the diagonal are read below
         // solve L D L^T x = rhs, lane = coordinate (articulation_mass.cuh:357-396)
@@ -393,7 +409,7 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
             const uint32_t c = e.dof_comp[0], i = c % 3u, j = (i + 1u) % 3u, k = (i + 2u) % 3u;
             const float* rv = sm_vel(e, e.dof_link[0]);
             const float transport = c < 3u ? 0.f : rv[j] * rv[3u + k] - rv[k] * rv[3u + j];
-            nv = e.vel0[0] + dt * (x[0] + transport);
+            nv = vel0[0] + dt * (x[0] + transport);
         }
         __syncwarp();
         if (base_coord) sm_vel(e, e.dof_link[0])[e.dof_comp[0]] = nv;
@@ -402,14 +418,12 @@ NKB_DEV void stage_dynamics(Env& e, bool integrate_velocity) {
 }
 
 // Computed-torque control (control mode 3), the quantities of the reference's ApplyDynamicsDriveKernel
-// (ops/articulation.cu:1315-1418).  Runs between a force-free dynamics pass (which leaves M's factor in shared memory and
-// the free accelerations in the lanes) and the step's dynamics pass.  With S the selector of the scalar joints,
+// (ops/articulation.cu:1315-1418).  Runs between a force-free solve for the accelerations (which leaves M's factor in shared
+// memory and the accelerations in the lanes) and the step's own.  With S the selector of the scalar joints,
 // H = (S M^-1 S^T)^-1 is the inertia the actuators see, a floating base's reaction included; the command is
 // H (a* + kp (q* - q) + kd (qd* - qd)) - H qdd_free - d qd (bias compensation without the passive joint damping).
-// Lane c owns column c of each small matrix and runs the reference's serial column loops (same operation order, double
-// accumulators where the reference has them); the matrices live in regions that are idle between the two dynamics passes:
-// the Newton matrix holds S M^-1 S^T and its factors, the head records' region holds H, the solver vectors the small
-// tables.
+// Lane = actuated joint in the products (double accumulators where the reference has them).  H lives in the head records'
+// region, idle between the two calls for accelerations, the small tables in the solver vectors.
 // Out of line, with its inputs by value: the controller runs in one control mode only and must not weigh on the register
 // allocation of the step kernel's common path.
 struct TorqueIn {
@@ -435,8 +449,9 @@ static __device__ __noinline__ void task_metric_pseudoinverse(float* a, float* v
             const float app = a[p * 6u + p], aqq = a[q * 6u + q], apq = a[p * 6u + q];
             if (fabsf(apq) <= FLT_EPSILON * (fabsf(app) + fabsf(aqq))) continue;       // the same words in every lane: a uniform branch
             changed = true;
-            const double theta = ((double)aqq - app) / (2.0 * apq);
-            const float tangent = (float)(copysign(1.0, theta) / (fabs(theta) + sqrt(1.0 + theta * theta)));
+            // tangent = sign(theta) / (|theta| + sqrt(1 + theta^2)) with theta = d / s, multiplied through by |s|
+            const double d = (double)aqq - app, s = 2.0 * (double)apq;
+            const float tangent = (float)((d < 0.0 ? -s : s) / (fabs(d) + sqrt(d * d + s * s)));
             const float cosine = rsqrtf(1.0f + tangent * tangent), sine = tangent * cosine;
             __syncwarp();
             if (lane < n) {
@@ -478,11 +493,11 @@ static __device__ __noinline__ void task_metric_pseudoinverse(float* a, float* v
 }
 
 // The task frame's velocity and acceleration in the world from the task link's twist and force-free acceleration (link
-// frame, angular first) plus J q'', the pose error, and from them kp x_err - kd v - a (ops/articulation.cu:1490-1513).
-static __device__ __noinline__ void task_right_hand_side(TorqueIn e, const float* acc0, const float* J, const float* qdd, float* trhs, uint32_t rows,
-                                                         V3 task_pos, Q4 task_q, Q4 link_q, V3 offset, Q4 desired) {
+// frame, angular first) plus J q'' (`jq`), the pose error, and from them kp x_err - kd v - a (ops/articulation.cu:1490-1513).
+static __device__ __noinline__ void task_right_hand_side(TorqueIn e, const float* acc0, float* trhs, uint32_t rows,
+                                                         V3 task_pos, Q4 task_q, Q4 link_q, V3 offset, Q4 desired, const float* jq) {
     const TemplateView& t = *e.t;
-    const uint32_t n = t.ndof, L = t.L, tl = t.cfg.task_link;
+    const uint32_t L = t.L, tl = t.cfg.task_link;
     const float* vel = e.sm + e.lay->vel + 6u * tl;
     const V3 omega = ld3(vel), linear = ld3(vel + 3);
     const V3 alpha = mk3(acc0[0], acc0[1], acc0[2]), linear_accel = mk3(acc0[3], acc0[4], acc0[5]);
@@ -491,13 +506,6 @@ static __device__ __noinline__ void task_right_hand_side(TorqueIn e, const float
     const V3 task_angular = qrot(link_q, omega);
     V3 task_accel = qrot(link_q, (linear_accel + cross(omega, linear)) + (cross(alpha, offset) + cross(omega, cross(omega, offset)))) + g;
     V3 task_angular_accel = qrot(link_q, alpha);
-    float jq[6];
-    for (uint32_t r = 0u; r < 6u; ++r) {
-        float sum = 0.f;
-#pragma unroll 1
-        for (uint32_t i = 0u; i < n; ++i) sum += J[r * n + i] * qdd[i];
-        jq[r] = sum;
-    }
     task_accel = task_accel + mk3(jq[0], jq[1], jq[2]);
     task_angular_accel = task_angular_accel + mk3(jq[3], jq[4], jq[5]);
     const V3 position_error = ld3(e.s->task_target + (size_t)e.env * 3u) - task_pos;
@@ -605,38 +613,65 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     __syncwarp();
     const Q4 desired = ldq(e.s->task_rotation + (size_t)e.env * 4u);
     const uint32_t rows = desired.w * desired.w + desired.x * desired.x + desired.y * desired.y + desired.z * desired.z > 1.0e-12f ? 6u : 3u;
-    // B: M x = J_r^T through the L D L^T factor, lane = task row
-    if (l < rows) {
-        float x[32 * NR];
-#pragma unroll 1
-        for (uint32_t i = 0u; i < n; ++i) x[i] = J[l * n + i];
-#pragma unroll 1
-        for (uint32_t j = 0u; j < n; ++j)
-#pragma unroll 1
-            for (uint32_t i = j + 1u; i < n; ++i) x[i] -= F[i * ld + j] * x[j];
-#pragma unroll 1
-        for (uint32_t i = 0u; i < n; ++i) x[i] /= F[i * ld + i];
-#pragma unroll 1
-        for (uint32_t end = n; end > 0u; --end) {
-            const uint32_t i = end - 1u;
-            float sum = x[i];
-#pragma unroll 1
-            for (uint32_t j = i + 1u; j < n; ++j) sum -= F[j * ld + i] * x[j];
-            x[i] = sum;
+    // B: M x = J_r^T through the L D L^T factor, lane = coordinate, all task rows side by side in registers
+    {
+        float x[NR][6], own[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const uint32_t c = l + 32u * q;
+            own[q] = c < n ? F[c * ld + c] : 1.f;
+#pragma unroll
+            for (uint32_t r = 0u; r < 6u; ++r) x[q][r] = c < n && r < rows ? J[r * n + c] : 0.f;
         }
+        for (int half = 0; half < 2; ++half) {
 #pragma unroll 1
-        for (uint32_t c = 0u; c < active; ++c) resp[l * active + c] = x[dofs[c]];
+            for (uint32_t step = 0u; step < n; ++step) {
+                const uint32_t j = half == 0 ? step : n - 1u - step;
+                float xj[6];
+#pragma unroll
+                for (uint32_t r = 0u; r < 6u; ++r) if (r < rows) xj[r] = __shfl_sync(NKB_FULL, NR == 1 || j < 32u ? x[0][r] : x[NR - 1][r], j & 31u); else xj[r] = 0.f;
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    const uint32_t c = l + 32u * q;
+                    if (c >= n || (half == 0 ? c <= j : c >= j)) continue;
+                    const float f = half == 0 ? F[c * ld + j] : F[j * ld + c];
+#pragma unroll
+                    for (uint32_t r = 0u; r < 6u; ++r) x[q][r] -= f * xj[r];
+                }
+            }
+            if (half == 0)
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+#pragma unroll
+                    for (uint32_t r = 0u; r < 6u; ++r) x[q][r] /= own[q];
+        }
+        const uint32_t first = n - active;                   // the actuated joints are the last coordinates
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const uint32_t c = l + 32u * q;
+            if (c < first || c >= n) continue;
+#pragma unroll
+            for (uint32_t r = 0u; r < 6u; ++r) if (r < rows) resp[r * active + c - first] = x[q][r];
+        }
     }
     __syncwarp();
-    if (column)
+    if (column) {
+        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
-        for (uint32_t r = 0u; r < rows; ++r) {
-            double v = 0.0;
-#pragma unroll 1
-            for (uint32_t a = 0u; a < active; ++a) v += (double)H[l * active + a] * resp[r * active + a];
-            tmap[r * active + l] = (float)v;
+        for (uint32_t a = 0u; a < active; ++a) {
+            const double h = H[l * active + a];
+#pragma unroll
+            for (uint32_t r = 0u; r < 6u; ++r) if (r < rows) v[r] += h * resp[r * active + a];
         }
+#pragma unroll
+        for (uint32_t r = 0u; r < 6u; ++r) if (r < rows) tmap[r * active + l] = (float)v[r];
+    }
+    if (l < 6u) {                                            // J q'' of the force-free pass, lane = task row
+        float sum = 0.f;
 #pragma unroll 1
+        for (uint32_t i = 0u; i < n; ++i) sum += J[l * n + i] * qdd[i];
+        force[l] = sum;
+    }
     for (uint32_t i = l; i < 72u; i += 32u) metric[i] = 0.f;      // metric and inverse
     __syncwarp();
 #pragma unroll 1
@@ -650,7 +685,7 @@ static __device__ __noinline__ float osc_command(TorqueIn e, OscIn o, uint32_t* 
     __syncwarp();
     task_metric_pseudoinverse(metric, eigenvectors, rows, inverse, l);
     // the task frame's velocity and force-free acceleration in the world, the task-space right-hand side: lane 0
-    if (l == 0u) task_right_hand_side(e, o.acc0, J, qdd, trhs, rows, task_pos, task_q, link_q, offset, desired);
+    if (l == 0u) task_right_hand_side(e, o.acc0, trhs, rows, task_pos, task_q, link_q, offset, desired, force);
     // posture: nullspace gains on the chain's joints (as accelerations through H), own gains elsewhere
     if (scalar) {
         const float pd_error = e.s->drive_target[at] - e.q, rate_error = e.s->vel_target[at] - e.qd;
@@ -728,13 +763,11 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     const size_t at = (size_t)e.env * L + l;
     float* vecs = e.sm + e.lay->vecs;
     constexpr uint32_t vs = 32u * NR;
-    float* diag = vecs + vs * kVecAcc;
     float* free_acc = vecs + vs * kVecFree;
     float* passive = vecs + vs * kVecU;
     float* rhs = vecs + vs * kVecPseudo;
     uint32_t* dofs = reinterpret_cast<uint32_t*>(vecs + vs * kVecTmp);
     float* command = vecs + vs * kVecTmp2;
-    float* A = e.sm + e.lay->chol;                         // active x active, row stride `active`
     float* H = e.sm + e.lay->heads;
     const float* F = e.sm + e.lay->factor;
     out.applied = 1u;
@@ -760,76 +793,20 @@ __device__ __noinline__ TorqueOut computed_torque(TorqueIn e) {
     }
     __syncwarp();
     const bool column = l < active;
-    float x[32 * NR];
-    // S M^-1 S^T, column by column: M x = e_dof(c) through the L D L^T factor (articulation_mass.cuh:357-411)
-    if (column) {
+    // H = (S M^-1 S^T)^-1 is the Schur complement of M on the actuated joints.  They are the last coordinates (a floating base's
+    // six come first), so with M = L D L^T it is L_jj D_jj L_jj^T of the factor at hand; the sums run in double.
+    const uint32_t head = n - active;
 #pragma unroll 1
-        for (uint32_t i = 0u; i < n; ++i) x[i] = i == dofs[l] ? 1.0f : 0.0f;
+    for (uint32_t i = l; i < active * active; i += 32u) {
+        const uint32_t r = i / active, c = i - r * active, last = min(r, c);
+        const float* Fr = F + (head + r) * ld + head;
+        const float* Fc = F + (head + c) * ld + head;
+        double v = 0.0;
 #pragma unroll 1
-        for (uint32_t j = 0u; j < n; ++j)
-#pragma unroll 1
-            for (uint32_t i = j + 1u; i < n; ++i) x[i] -= F[i * ld + j] * x[j];
-#pragma unroll 1
-        for (uint32_t i = 0u; i < n; ++i) x[i] /= F[i * ld + i];
-#pragma unroll 1
-        for (uint32_t end = n; end > 0u; --end) {
-            const uint32_t i = end - 1u;
-            float s = x[i];
-#pragma unroll 1
-            for (uint32_t j = i + 1u; j < n; ++j) s -= F[j * ld + i] * x[j];
-            x[i] = s;
-        }
-#pragma unroll 1
-        for (uint32_t r = 0u; r < active; ++r) A[r * active + l] = x[dofs[r]];
-    }
-    __syncwarp();
-    if (column)
-#pragma unroll 1
-        for (uint32_t c = 0u; c < l; ++c) {
-            const float v = 0.5f * (A[l * active + c] + A[c * active + l]);
-            A[l * active + c] = v; A[c * active + l] = v;
-        }
-    __syncwarp();
-    // L D L^T of the actuated block (FactorControlMass): every lane follows the pivots, lane i owns row i
-    bool definite = true;
-#pragma unroll 1
-    for (uint32_t j = 0u; j < active; ++j) {
-        double pivot = A[j * active + j];
-#pragma unroll 1
-        for (uint32_t k = 0u; k < j; ++k) { const double v = A[j * active + k]; pivot -= v * v * diag[k]; }
-        if (!(pivot > 0.0) || !isfinite(pivot)) { definite = false; break; }
-        __syncwarp();
-        if (l == 0u) diag[j] = (float)pivot;
-        if (column && l > j) {
-            double v = A[l * active + j];
-#pragma unroll 1
-            for (uint32_t k = 0u; k < j; ++k) v -= (double)A[l * active + k] * A[j * active + k] * diag[k];
-            A[l * active + j] = (float)(v / pivot);
-        }
-        __syncwarp();
-    }
-    if (!definite) { out.status = kStatusControlFailure; return out; }
-    // H = inverse, column by column (SolveControlMass on unit vectors)
-    if (column) {
-#pragma unroll 1
-        for (uint32_t i = 0u; i < active; ++i) {
-            double v = i == l ? 1.0 : 0.0;
-#pragma unroll 1
-            for (uint32_t j = 0u; j < i; ++j) v -= (double)A[i * active + j] * x[j];
-            x[i] = (float)v;
-        }
-#pragma unroll 1
-        for (uint32_t i = 0u; i < active; ++i) x[i] /= diag[i];
-#pragma unroll 1
-        for (uint32_t ii = active; ii > 0u; --ii) {
-            const uint32_t i = ii - 1u;
-            double v = x[i];
-#pragma unroll 1
-            for (uint32_t j = i + 1u; j < active; ++j) v -= (double)A[j * active + i] * x[j];
-            x[i] = (float)v;
-        }
-#pragma unroll 1
-        for (uint32_t r = 0u; r < active; ++r) H[r * active + l] = x[r];
+        for (uint32_t k = 0u; k < last; ++k) v += (double)Fr[k] * Fc[k] * F[(head + k) * ld + head + k];
+        const float d = F[(head + last) * ld + head + last];
+        v += r == c ? (double)d : (double)(r > c ? Fr[last] : Fc[last]) * d;
+        H[i] = (float)v;
     }
     __syncwarp();
     if (osc) {
@@ -898,13 +875,11 @@ NKB_DEV void stage_integrate_links(Env& e, bool use_pseudo) {
 }
 
 // Link spatial velocities after the solve, ops/articulation.cu:647-689.
-NKB_DEV void stage_link_velocities(Env& e) {
+NKB_DEV void stage_link_velocities(Env& e, const float (&E)[9], V3 r) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane;
     const bool link = l < t.L;
     const bool froot = link && e.parent == kNoLink && e.jtype == kFloating;
-    float E[9]; V3 r = mk3(0.f, 0.f, 0.f);
-    if (link) joint_xform(e, E, r);
     V3 jw = mk3(0.f, 0.f, 0.f), jv = jw;
     if (e.jtype == kRevolute) jw = e.axis * e.qd; else if (e.jtype == kPrismatic) jv = e.axis * e.qd;
 #pragma unroll 1

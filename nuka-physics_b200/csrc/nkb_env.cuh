@@ -19,7 +19,6 @@ struct Env {
     float drive_command, drive_dissipation, drive_lower, drive_upper;
     // lane = dof: a lane owns coordinates lane and lane + 32 (the second only when the articulation has more than 32)
     uint32_t dof_link[2], dof_comp[2];   // comp == kNoLink for scalar joints
-    float vel0[2];           // step-start coordinate velocity
     uint32_t status;
     bool branching;          // a contact of this step acts on two branches of the articulation's tree
     uint32_t vstride;        // words per shared-memory vector: 32 x coordinates per lane
@@ -90,7 +89,7 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
     e.qdd = 0.f; e.tau = 0.f;
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
     e.vstride = 32u * NR;
-    e.dof_link[1] = 0u; e.dof_comp[1] = kNoLink; e.vel0[1] = 0.f;
+    e.dof_link[1] = 0u; e.dof_comp[1] = kNoLink;
 #pragma unroll
     for (uint32_t r = 0u; r < (uint32_t)NR; ++r) {
         const uint32_t c = lane + 32u * r;
@@ -98,7 +97,6 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
         e.dof_link[r] = dof ? __ldg(t.dof_link + c) : 0u;
         e.dof_comp[r] = kNoLink;
         if (dof && __ldg(t.jtype + e.dof_link[r]) == kFloating) e.dof_comp[r] = c - __ldg(t.link_dof + e.dof_link[r]);
-        e.vel0[r] = 0.f;
     }
     e.status = 0u; e.branching = false;
 #ifdef NKB_STAGE_TAPS

@@ -5,7 +5,7 @@
 
 namespace nkb {
 
-constexpr uint32_t kWarpsPerBlockMax = 8u;
+constexpr uint32_t kWarpsPerBlockMax = 16u, kTeamMax = 8u;
 
 struct ResetField {
     void* dst;            // E x words

@@ -162,24 +162,13 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             for (int r = 0; r < NR; ++r) {
                 const uint32_t c = lane + 32u * r;
                 if (dof[r]) {
-                    float ent[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        const uint32_t cl = side == 0 ? la : lb;
-                        if (cl == 0xffffu) continue;
-                        if (!((__ldg(t.anc_mask + cl) >> e.dof_link[r]) & 1u)) continue;
-                        const float sgn = side == 0 ? 1.f : -1.f;
-#pragma unroll
-                        for (int ax = 0; ax < 3; ++ax) {
-                            const V3 f = dirs[ax] * sgn;
-                            float v;
-                            if (jt[r] == kFloating) v = e.dof_comp[r] < 3u ? dot(cross(axis_w[r], point - origin[r]), f) + 0.0f : dot(axis_w[r], f);
-                            else if (jt[r] == kPrismatic) v = dot(axis_w[r], f);
-                            else v = dot(cross(axis_w[r], point - origin[r]), f) + 0.0f;
-                            ent[ax] += v;
-                        }
-                    }
-                    pool[joff + c] = ent[0]; pool[joff + n4 + c] = ent[1]; pool[joff + 2u * n4 + c] = ent[2];
+                    // the side signs of this coordinate: it moves side a's link, side b's, both (no relative motion) or neither
+                    float sgn = 0.f;
+                    if (la != 0xffffu && ((__ldg(t.anc_mask + la) >> e.dof_link[r]) & 1u)) sgn += 1.f;
+                    if (lb != 0xffffu && ((__ldg(t.anc_mask + lb) >> e.dof_link[r]) & 1u)) sgn -= 1.f;
+                    const bool turns = jt[r] == kFloating ? e.dof_comp[r] < 3u : jt[r] != kPrismatic;
+                    const V3 w = (turns ? cross(axis_w[r], point - origin[r]) : axis_w[r]) * sgn;
+                    pool[joff + c] = dot(w, dirs[0]) + 0.0f; pool[joff + n4 + c] = dot(w, dirs[1]) + 0.0f; pool[joff + 2u * n4 + c] = dot(w, dirs[2]) + 0.0f;
                 } else if (c < n4) { pool[joff + c] = 0.f; pool[joff + n4 + c] = 0.f; pool[joff + 2u * n4 + c] = 0.f; }
             }
             if (lane == 0u) {

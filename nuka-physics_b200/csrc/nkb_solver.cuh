@@ -1275,7 +1275,7 @@ NKB_DEV Env bare_env(float* sm, const SmemLayout* lay, const TemplateView* t, co
     e.q = e.qd = e.qdd = e.tau = 0.f;
     e.axis = mk3(0.f, 0.f, 0.f);
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
-    e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink; e.vel0[0] = e.vel0[1] = 0.f;
+    e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink;
     e.status = 0u; e.branching = false; e.vstride = vstride;
 #ifdef NKB_STAGE_TAPS
     e.cyc = nullptr; e.t0 = 0;

@@ -166,29 +166,86 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 #ifndef NKB_MAXNREG_SLIM
 #define NKB_MAXNREG_SLIM 128
 #endif
-// Lines the block's warps up (one env each) at the start of a step and around its solve, so that they run the straight-line
-// stages side by side and share the fetches of their instructions: about 200 KB of code per step against the 128 KB an SM
-// keeps at hand, and 15 warps at 15 different places of it were stalled on instruction fetch more than half of the time
-// (ncu: no_instruction 6.6 of 12.4 cycles per issue).  16 384 quadrupeds, 4 steps: 25.4 ms without the three barriers,
-// 15.5 ms with them; a barrier before every sweep as well (which adds waiting for the env with the most sweeps) 15.6 ms.
-// Every warp of the block passes the same barriers (warps without an env have left); a team's helpers wait for their lead
-// elsewhere, so worlds in team mode do without.
-NKB_DEV void align_block(const StepParams& p) { if (p.sm.team <= 1u) __syncthreads(); }
+// Warps that wait for one another after their solves and then go through the straight-line stages (the end of a step, the
+// start of the next) side by side, so that they share the fetches of their instructions: about 200 KB of code per step against
+// the 128 KB an SM keeps at hand.  Warps at 15 different places of it are stalled on instruction fetch more than half of the
+// time (ncu: no_instruction 6.6 of 12.4 cycles per issue; 16 384 quadrupeds, 4 steps: 20.9 ms without any meeting).
+// Solves differ by a factor of three between envs, so a fixed group (a block-wide barrier) waits for its slowest member: 40 %
+// of the solve time (11.7 ms).  Here the next `group` warps of the block to finish their solves go on together, whoever they
+// are, and a warp whose env is done takes the next env of the launch's queue.
+// One shared word carries the number of waiting warps (low byte) and a generation; a warp goes on when the generation moves.
+// Whoever completes a group moves it, and so does a warp that leaves for good when those that wait are all that are left.  A
+// wait that outlasts its cycle budget just ends: who walks with whom changes no result.
+struct Rally { uint32_t word, alive; };
+constexpr long long kRallyPatience = 100000000ll;        // cycles: about 50 ms
+NKB_DEV uint32_t rally_peek(const uint32_t* w) { return *reinterpret_cast<const volatile uint32_t*>(w); }
+NKB_DEV void rally_wait(Rally* r, uint32_t group, uint32_t lane) {
+    if (group <= 1u) return;
+    __syncwarp();
+    uint32_t generation = 0u;
+    if (lane == 0u) {
+        const uint32_t before = atomicAdd(&r->word, 1u);
+        generation = before >> 8;
+        __threadfence_block();
+        if ((before & 0xffu) + 1u >= min(group, rally_peek(&r->alive)))
+            for (uint32_t seen = rally_peek(&r->word), found; (seen >> 8) == generation; seen = found)
+                if ((found = atomicCAS(&r->word, seen, (generation + 1u) << 8)) == seen) break;
+    }
+    generation = __shfl_sync(NKB_FULL, generation, 0);
+    const long long begin = clock64();
+    while ((rally_peek(&r->word) >> 8) == generation) {            // every lane polls the same word: the warp stays together
+        if (clock64() - begin > kRallyPatience) break;
+        __nanosleep(64);
+    }
+    __syncwarp();
+}
+NKB_DEV void rally_leave(Rally* r, uint32_t group, uint32_t lane) {
+    if (group <= 1u || lane != 0u) return;
+    const uint32_t left = atomicSub(&r->alive, 1u) - 1u;
+    __threadfence_block();
+    for (uint32_t seen = rally_peek(&r->word), found; (seen & 0xffu) != 0u && (seen & 0xffu) >= min(group, left); seen = found)
+        if ((found = atomicCAS(&r->word, seen, ((seen >> 8) + 1u) << 8)) == seen) break;
+}
 
 template <int NR, bool kRigid, bool kControl>
-NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t lane) {
+NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t lane, Rally* rally) {
     const TemplateView& t = p.t;
     const bool has_artic = t.L != 0u, has_bodies = t.B != 0u;
     const bool has_collidables = has_bodies && t.cfg.max_contacts != 0u;
     const bool use_pseudo = t.cfg.pos_iters != 0u && (t.cfg.max_contacts != 0u || t.L != 0u);
+    Env e;
+    env_begin<NR>(e, p, sm, env, lane);
+    // A step ends where the next begins, with the kinematics of the new coordinates: one pass over them serves both.
 #pragma unroll 1
-    for (uint32_t step = 0u; step < p.steps; ++step) {
-        Env e;
-        align_block(p);
-        env_begin<NR>(e, p, sm, env, lane);
+    for (uint32_t step = 0u;; ++step) {
+        float E[9];
+        V3 r = mk3(0.f, 0.f, 0.f);
+        if (has_artic) {
+            stage_fk(e);
+            if (lane < t.L) joint_xform(e, E, r);
+            tick(e, 1);
+            if (step != 0u) { stage_link_velocities(e, E, r); stage_store_links(e); }
+        }
+        if (has_bodies) {
+            stage_body_poses(e, step == 0u);
+            if (step != 0u) stage_store_bodies(e, true);
+        }
+        if (step != 0u) {
+            uint32_t st = __reduce_or_sync(NKB_FULL, e.status);
+            // The gyro bit describes the latest step only (the reference clears it before every body integration,
+            // ops/articulation.cu:1053-1056, 1810-1812); every other bit stays until the env is reset.
+            if (lane == 0u && (st != 0u || has_bodies)) {
+                const uint32_t before = p.s.status[env];
+                const uint32_t after = (has_bodies ? before & ~kStatusGyroFailure : before) | st;
+                if (after != before) p.s.status[env] = after;
+            }
+            __syncwarp();
+            tick(e, 13);
+            if (step == p.steps) return;
+        }
+        e.status = 0u; e.branching = false;
         if (p.mode == kModeRefresh) {
-            if (has_artic) { stage_fk(e); }
-            if (has_bodies) { stage_bodies(e, false); stage_store_bodies(e, false); }
+            if (has_bodies) stage_store_bodies(e, false);
             if (has_artic) {
                 float* gp = p.s.link_pose + (size_t)env * t.L * 7u;
 #pragma unroll 1
@@ -196,16 +253,18 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             }
             return;
         }
-        tick(e, 0);
         if (has_artic) {
-            stage_fk(e); tick(e, 1); stage_drives(e);
-            // computed torque and operational-space control (pipeline.cpp:406-426) take two passes: a force-free one on the current kinematics, the
-            // controller on its mass response and accelerations, then the step's own pass
-            // the controllers are compiled into the kControl builds of the kernel only (they would cost every other world registers)
+            stage_drives(e);
+            float bias[NR];
+            stage_dynamics<NR>(e, E, r, bias);
+            // Computed torque and operational-space control (pipeline.cpp:406-426) take the accelerations twice, force-free for
+            // the controller and then under its feedforward effort; the mass matrix and the bias are the same.  The controllers
+            // are compiled into the kControl builds of the kernel only (they would cost every other world registers).
             const bool two_passes = kControl && (t.cfg.control_mode == 3u || t.cfg.control_mode == 4u) && p.mode != kModeDynamicsOnly;
+            const int first = two_passes ? 0 : 1;
 #pragma unroll 1
-            for (int pass = two_passes ? 0 : 1; pass < 2; ++pass) {
-                stage_dynamics<NR>(e, pass == 1 && p.mode != kModeDynamicsOnly);
+            for (int pass = first; pass < 2; ++pass) {
+                stage_accelerations<NR>(e, bias, pass == first, pass == 1 && p.mode != kModeDynamicsOnly);
                 if constexpr (kControl) { if (pass == 0) stage_computed_torque<NR>(e); }
             }
             tick(e, 2);
@@ -215,7 +274,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
         uint32_t pair_count = 0u, nheads = 0u;
-        if (has_bodies) stage_bodies(e, true);
+        if (has_bodies) stage_body_kick(e);
         if (has_collidables) {
             stage_aabbs(e);
             pair_count = t.broadphase_tree != 0u ? stage_pairs_lbvh(e) : stage_pairs(e);
@@ -229,9 +288,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         }
         if (p.mode == kModeCollideOnly) {
             if (has_bodies) stage_store_bodies(e, false);
-            uint32_t st = e.status;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) st |= __shfl_xor_sync(NKB_FULL, st, o);
+            const uint32_t st = __reduce_or_sync(NKB_FULL, e.status);
             if (lane == 0u) p.s.status[env] |= st;
             return;
         }
@@ -241,9 +298,9 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         else warm_start_range(e, nheads, 0u, 1u);
         __syncwarp();
         tick(e, 7);
-        align_block(p);
         stage_solve<NR, kRigid>(e, nheads);
-        align_block(p);
+        rally_wait(rally, p.group, lane);
+        tick(e, 29);
         if (has_collidables) {
             stage_cache_commit(e, nheads, [&](uint32_t ncontact) {
                 if constexpr (kRigid) team_fork(e, kTeamCacheOwners, ncontact, [&](uint32_t first, uint32_t stride) { cache_owners_range(e, ncontact, first, stride); });
@@ -255,39 +312,6 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         if (has_artic) { stage_integrate_links(e, use_pseudo); }
         if (has_bodies) stage_integrate_bodies(e, use_pseudo);
         __syncwarp();
-        if (has_artic) { stage_fk(e); stage_link_velocities(e); stage_store_links(e); }
-        if (has_bodies) {
-            // link mirrors follow the new link poses; free bodies keep their integrated pose
-#pragma unroll 1
-            for (uint32_t b = lane; b < t.B; b += 32u) {
-                const uint32_t link = __ldg(t.body_to_link + b);
-                if (link == kNoLink) continue;
-                float* bp = sm_bpose(e, b);
-                const float* lp = sm_pose(e, link);
-                if (__ldg(t.body_geom_kind + b) != 0u) {
-                    const Q4 pq = ldq(lp + 3);
-                    st3(bp, ld3(lp) + qrot(pq, ld3(t.body_geom_pos + 3u * b)));
-                    stq(bp + 3, qmul(pq, ldq(t.body_geom_quat + 4u * b)));
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) bp[k] = lp[k];
-                }
-            }
-            __syncwarp();
-            stage_store_bodies(e, true);
-        }
-        uint32_t st = e.status;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) st |= __shfl_xor_sync(NKB_FULL, st, o);
-        // The gyro bit describes the latest step only (the reference clears it before every body integration,
-        // ops/articulation.cu:1053-1056, 1810-1812); every other bit stays until the env is reset.
-        if (lane == 0u && (st != 0u || has_bodies)) {
-            const uint32_t before = p.s.status[env];
-            const uint32_t after = (has_bodies ? before & ~kStatusGyroFailure : before) | st;
-            if (after != before) p.s.status[env] = after;
-        }
-        __syncwarp();
-        tick(e, 13);
     }
 }
 
@@ -368,20 +392,40 @@ __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SL
     uint32_t env = blockIdx.x * ((blockDim.x >> 5) / team) + slot;
     float* sm = smem + (size_t)slot * p.sm.words;
     if constexpr (kRigid) {
-        // team mode: every lead zeroes its team's sequence numbers before any helper looks (the one block-wide barrier of
-        // the kernel, passed by every thread before any leaves)
+        // team mode: every lead zeroes its team's sequence numbers before any helper looks (a block-wide barrier, passed by
+        // every thread before any leaves)
         if (team > 1u) {
             if (member == 0u) team_open(sm, p.sm, lane);
             __syncthreads();
         }
     }
     if (p.sel_ids != nullptr) env = env < p.sel_count ? p.sel_ids[env] : 0xffffffffu;
+    __shared__ Rally rally;
+    if (p.group > 1u) {
+        if (threadIdx.x == 0u) { rally.word = 0u; rally.alive = min(blockDim.x >> 5, p.s.env_count - min(p.s.env_count, env)); }
+        __syncthreads();
+    }
     if (env >= p.s.env_count) return;                       // the whole team leaves together
     if (p.sel_mask != nullptr && p.sel_mask[env] == 0u) return;
     if constexpr (kRigid) {
         if (member != 0u) { team_helper<kRigid>(sm, p.sm, p.t, p.s, env, member, lane, 32u * NR); return; }
     }
-    advance_env<NR, kRigid, kControl>(p, sm, env, lane);
+#pragma unroll 1
+    for (;;) {
+        advance_env<NR, kRigid, kControl>(p, sm, env, lane, &rally);
+        if (p.queue == nullptr) break;
+        uint32_t next = 0u;
+        if (lane == 0u) next = atomicAdd(p.queue, 1u);
+        env = gridDim.x * (blockDim.x >> 5) + __shfl_sync(NKB_FULL, next, 0);
+        if (env >= p.s.env_count) break;
+    }
+    rally_leave(&rally, p.group, lane);
+    if (p.queue != nullptr && lane == 0u) {
+        // the launch's last warp leaves the queue zeroed for the next launch
+        __threadfence();
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        if (atomicInc(p.queue + 1, warps - 1u) == warps - 1u) *reinterpret_cast<volatile uint32_t*>(p.queue) = 0u;
+    }
     if constexpr (kRigid) { if ((p.sm.team_drill & 1u) == 0u) team_dismiss(sm, p.sm, lane); }
 }
 
@@ -435,7 +479,8 @@ static cudaError_t variant_launch(const StepParams& p, uint32_t warps_per_block,
     if (err != cudaSuccess) return err;
     const uint32_t envs = p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
     if (envs == 0u) return cudaSuccess;
-    const uint32_t blocks = (envs + envs_per_block - 1u) / envs_per_block;
+    const uint32_t needed = (envs + envs_per_block - 1u) / envs_per_block;
+    const uint32_t blocks = p.queue != nullptr ? p.grid : needed;       // a persistent launch's grid is smaller than the batch
     step_kernel<NR, kRigid, kSlim, kControl><<<blocks, warps_per_block * 32u, bytes, stream>>>(p);
     return cudaGetLastError();
 }

@@ -185,11 +185,11 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float g, 
     }
     if (!kKeep && !__all_sync(NKB_FULL, valid)) return false;
     // joints root to leaf: a depth's solution reaches its descendants by shuffle
-#pragma unroll
-    for (int p = 0; p < kTreeLevels - 1; ++p) {
-        if (p >= depth - 1) break;
-        const float xp = __shfl_sync(NKB_FULL, acc * inverse, t.ancestor(p) & 31u);
-        if (t.level != kTreeNone && t.level > (uint32_t)p) acc = fmaf(-row.limb[p], xp, acc);
+#pragma unroll 1
+    for (int p = 0; p < depth - 1; ++p) {
+        const uint32_t word = p < 4 ? t.anc[0] : p < 8 ? t.anc[1] : t.anc[2];
+        const float xp = __shfl_sync(NKB_FULL, acc * inverse, (word >> (8 * (p & 3))) & 31u);
+        if (t.level != kTreeNone && t.level > (uint32_t)p) acc = fmaf(-mine[8 + p], xp, acc);
     }
     x = acc * inverse;
     return true;

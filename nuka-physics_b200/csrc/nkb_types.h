@@ -155,6 +155,11 @@ struct StepParams {
     SmemLayout sm;
     uint32_t mode;
     uint32_t steps;
+    // Step launches of worlds without teams: warps of a block that wait for one another after each solve (see Rally; 0 or 1:
+    // none), and the blocks of a persistent launch whose warps fetch further envs from `queue` (two zeroed words, left zeroed).
+    uint32_t group;
+    uint32_t grid;
+    uint32_t* queue;
     // Env selection of a refresh launch (null: every env).  sel_ids lists sel_count envs, one warp each; sel_mask is
     // an E-word device array whose non-zero entries pick the envs of a full-size launch.
     const uint32_t* sel_ids;

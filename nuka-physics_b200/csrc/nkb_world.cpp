@@ -380,7 +380,7 @@ void World::BuildLayout() {
     s.pairs = take(SC); s.ccount = take(SC); s.cpoint = take(12 * SC); s.cnormal = take(12 * SC); s.cdepth = take(4 * SC);
     s.cfeat = take(8 * SC);                       // contact identity words
     // before the heads exist the region serves the tree broadphase and then the narrowphase as scratch
-    s.heads = take(std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kWarpsPerBlockMax : 1u)) : 0u));
+    s.heads = take(std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kTeamMax : 1u)) : 0u));
     // the Jacobian pool also holds the AABBs (dead once the narrowphase is done) and, after the solve, the cache staging
     // entries + owner marks
     const uint32_t stage_cap = std::min(tv.point_cap, 4u * SC);
@@ -400,7 +400,7 @@ void World::BuildLayout() {
         uint32_t team = 1u;
         if (t.n_free >= 8u) {
             const uint32_t envs_alone = std::max<uint32_t>(1u, (227u * 1024u) / (at * 4u + 1024u));      // resident envs, one warp each
-            while (team * 2u <= kWarpsPerBlockMax && envs_alone * team * 2u <= 11u && (at + area(team * 2u)) * 4u <= 220u * 1024u) team *= 2u;
+            while (team * 2u <= kTeamMax && envs_alone * team * 2u <= 11u && (at + area(team * 2u)) * 4u <= 220u * 1024u) team *= 2u;
         }
         // Lanes per free body in a block descent.  A body alone on its env's one warp leaves most lanes idle: 8 lanes each,
         // four bodies at a time.  A team has warps for two bodies each (a colour of a 48-box pile holds about 13).  The choice
@@ -408,7 +408,7 @@ void World::BuildLayout() {
         s.body_lanes = team > 1u ? 16u : 8u;
         if (const char* forced = std::getenv("NUKA_B200_TEAM")) {                        // team-size experiments
             const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
-            if (w >= 1u && w <= kWarpsPerBlockMax && t.n_free != 0u && (at + area(w)) * 4u <= 220u * 1024u) team = w;
+            if (w >= 1u && w <= kTeamMax && t.n_free != 0u && (at + area(w)) * 4u <= 220u * 1024u) team = w;
         }
         if (team > 1u) {
             s.team = team;
@@ -437,27 +437,25 @@ void World::BuildLayout() {
     if (const char* forced = std::getenv("NUKA_B200_SLIM")) slim_ = has_slim && std::atoi(forced) != 0;     // variant experiments and tests
     const size_t* fits = resident[slim_ ? 1 : 0];
     const size_t most = best[slim_ ? 1 : 0];
-    // Block shape: the warps of a block go through the step side by side (align_block), so that they share instruction
-    // fetches; the largest block among those that keep the most warps resident (228 KB shared memory, 1 KB reserved per
-    // block) serves that best.  Two exceptions.  Where an SM holds four warps or fewer, fetches are no bottleneck and waiting
-    // for one another only costs (2048 humanoids, 3 per SM: 13.6 ms in blocks of 3, 10.7 ms in blocks of 1).  And a batch that
-    // does not fill the SMs is spread over all of them in blocks of about two fifths of an SM's share (1000 quadrupeds, 6.8
-    // per SM: 2.66 ms in blocks of 1, 2.39 of 3, 2.50 of 5 and 7; 300: 2.07 of 1, 2.30 of 5).
+    // Block shape and how its warps meet (Rally).
     warps_per_block_ = team;
     for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) if (fits[w] == most) warps_per_block_ = w;
+    group_ = 0u; grid_ = 0u;
     if (team == 1u) {
         int sms = 148;
         Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
         const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
         if (most <= 4u) warps_per_block_ = 1u;
-        else if (share < most) {            // the largest such block that still lets the whole batch in at once
-            const uint32_t cap = std::max(1u, (2u * share + 2u) / 5u);
-            for (uint32_t w = 1u; w <= cap; ++w) if (fits[w] >= share) warps_per_block_ = w;
+        else if (share < most)
+            for (uint32_t w = 1u; w <= std::min(share, kWarpsPerBlockMax); ++w) if (fits[w] >= share) warps_per_block_ = w;
+        if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // block-shape experiments
+            const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
+            if (w >= 1u && w <= kWarpsPerBlockMax && fits[w] != 0u) warps_per_block_ = w;
         }
-    }
-    if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // block-shape experiments
-        const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
-        if (w >= 1u && w <= kWarpsPerBlockMax && w % team == 0u && fits[w] != 0u) warps_per_block_ = w;
+        group_ = std::min(warps_per_block_, 5u);
+        if (const char* forced = std::getenv("NUKA_B200_GROUP")) group_ = static_cast<uint32_t>(std::atoi(forced));
+        const uint32_t grid = static_cast<uint32_t>(sms) * static_cast<uint32_t>(fits[warps_per_block_] / warps_per_block_);
+        if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
     if (std::getenv("NUKA_B200_DEBUG_LAYOUT") != nullptr) {
         std::fprintf(stderr, "[nuka_b200] %zu B of shared memory per env, %d registers per thread%s; resident warps per SM by block size:", bytes,
@@ -497,6 +495,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.free_slot = Upload(t.free_slot); v.n_free = t.n_free;
         v.n_adm = (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size());
         SetBroadphase(0u);
+        if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
         const size_t E = env_count_, L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
         StateView& s = params_.s;
         s.env_count = env_count_;
@@ -643,6 +642,7 @@ void World::Step(uint32_t n) {
     Check(cudaSetDevice(device_), "cudaSetDevice");
     StepParams p = params_;
     p.mode = kModeStep;
+    p.group = group_; p.grid = grid_; p.queue = queue_;
     if (!graph_mode_) {
         // the kernel advances several steps per launch (inputs are constant across them; state goes back to global
         // memory after every step, so the split changes no result); the cap keeps any one launch short

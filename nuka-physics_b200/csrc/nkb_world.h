@@ -107,6 +107,8 @@ private:
     StepParams params_{};
     StateView readout_{};               // contact read-out pointers while the read-out is switched off
     uint32_t warps_per_block_ = 1;
+    uint32_t group_ = 0, grid_ = 0;            // step launches: see StepParams
+    uint32_t* queue_ = nullptr;
     bool slim_ = false;        // the world runs the 128-register build of its kernel variant
     std::vector<void*> allocations_;
     ResetParams reset_{};
