@@ -23,6 +23,8 @@ __global__ void reset_kernel(ResetParams r) {
 extern const StepVariant kStepNarrow, kStepNarrowSlim, kStepNarrowRigid, kStepWide, kStepWideRigid;
 extern const StepVariant kStepNarrowControl, kStepNarrowRigidControl, kStepWideControl, kStepWideRigidControl;
 
+extern const StepVariant kStagesNarrow, kSolveNarrow, kStagesNarrowRigid, kSolveNarrowRigid, kStagesWide, kSolveWide;
+
 bool step_kernel_has_slim(uint32_t ndof, uint32_t n_free, bool control) { return ndof <= 32u && n_free == 0u && !control; }
 
 // up to 32 or up to 64 coordinates per articulation; with or without free rigid bodies; the slim (128-register) build
@@ -44,6 +46,13 @@ int step_kernel_resident_blocks(uint32_t ndof, uint32_t n_free, bool slim, bool 
 cudaError_t launch_step(const StepParams& p, uint32_t warps_per_block, bool slim, cudaStream_t stream) {
     const bool control = p.t.cfg.control_mode == 3u || p.t.cfg.control_mode == 4u;
     return step_variant(p.t.ndof, p.t.n_free, slim && !control, control).launch(p, warps_per_block, stream);
+}
+
+const StepVariant* split_variant(uint32_t ndof, uint32_t n_free, bool control, StepPart part) {
+    if (control || (ndof > 32u && n_free != 0u)) return nullptr;
+    if (ndof > 32u) return part == kPartStages ? &kStagesWide : &kSolveWide;
+    if (n_free != 0u) return part == kPartStages ? &kStagesNarrowRigid : &kSolveNarrowRigid;
+    return part == kPartStages ? &kStagesNarrow : &kSolveNarrow;
 }
 
 // One observation record per env, composed from the state arrays in one pass (the reference's gym layer builds the same

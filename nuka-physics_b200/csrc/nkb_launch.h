@@ -39,6 +39,8 @@ struct StepVariant {
     int (*registers)();
     cudaError_t (*launch)(const StepParams& p, uint32_t warps_per_block, cudaStream_t stream);
 };
+// The kernel of one part of a split step (kPartStages, kPartSolve) for such a world, or null where steps run in one kernel only.
+const StepVariant* split_variant(uint32_t ndof, uint32_t n_free, bool control, StepPart part);
 // Enqueues `p.steps` fused steps (or one parity-tap stage, see StepMode) for every env.
 cudaError_t launch_step(const StepParams& p, uint32_t warps_per_block, bool slim, cudaStream_t stream);
 // Restores `count` envs (all when r.env_ids is null) from their snapshots.

@@ -207,7 +207,51 @@ NKB_DEV void rally_leave(Rally* r, uint32_t group, uint32_t lane) {
         if ((found = atomicCAS(&r->word, seen, ((seen >> 8) + 1u) << 8)) == seen) break;
 }
 
-template <int NR, bool kRigid, bool kControl>
+// ---- a step split over launches -------------------------------------------------------------------------------------------
+// The straight-line stages of a step are about 170 KB of code that every env runs once, the solve about 60 KB that envs run a
+// different number of times.  In one kernel the two fight: warps that run the stages together share the instruction fetches
+// (an SM keeps 128 KB at hand; apart from one another they fetch everything again, one instruction in six cycles for the whole
+// SM), but then they wait for the longest solve among them.  Split, the stages run in blocks whose warps stay together, and
+// the solves run one warp to a block, each SM taking the next env as one finishes.  In between an env's slice of shared memory
+// waits in global memory (L2 for the usual batches): only what the other side reads, heads and rows up to the live count.
+template <bool kLoad>
+NKB_DEV void image_words(float* img, uint32_t at, float* sm, uint32_t to, uint32_t words, uint32_t lane) {
+    // regions start on 16-byte boundaries and are padded to them
+    float4* g = reinterpret_cast<float4*>(img + at);
+    float4* s = reinterpret_cast<float4*>(sm + to);
+#pragma unroll 4
+    for (uint32_t k = lane; k < (words + 3u) >> 2; k += 32u) { if (kLoad) s[k] = __ldcg(g + k); else __stcg(g + k, s[k]); }
+}
+// Keeps the warps of a stages block side by side (each passes the same barriers; warps without an env have left).
+template <int kPart> NKB_DEV void stay_together() { if constexpr (kPart == kPartStages) __syncthreads(); }
+// What crosses: kBefore from the stages to the solve, kAfter from the solve back to the stages, kAside past the solve.
+enum ImageSet : int { kBefore = 0, kAfter = 1, kAside = 2 };
+template <bool kLoad, int kSet>
+NKB_DEV void image_move(Env& e, const StepParams& p, float* img, uint32_t nheads) {
+    const TemplateView& t = p.t;
+    const SmemLayout &a = p.im, &b = p.sm;
+    const uint32_t l = e.lane, slots = t.B != 0u ? t.n_free + 1u : 0u, n4 = (t.ndof + 3u) & ~3u;
+    auto move = [&](uint32_t from, uint32_t to, uint32_t words) { if (words != 0u) image_words<kLoad>(img, from, e.sm, to, words, l); };
+    if (kSet == kAside) {
+        move(a.bpose, b.bpose, 7u * t.B);
+        move(a.pairs, b.pairs, t.slot_cap); move(a.cnormal, b.cnormal, 12u * t.slot_cap); move(a.cfeat, b.cfeat, 8u * t.slot_cap);
+        return;
+    }
+    move(a.vel, b.vel, t.L != 0u ? 6u : 0u);
+    move(a.bvel, b.bvel, 6u * slots);
+    move(a.heads, b.heads, kHeadStride * nheads);
+    if (kSet == kBefore) {
+        move(a.mass, b.mass, t.ndof * b.ld); move(a.factor, b.factor, b.factor_words);
+        move(a.bwinv, b.bwinv, 6u * slots);
+        move(a.cdepth, b.cdepth, 4u * t.slot_cap);
+        move(a.jpool, b.jpool, 3u * n4 * min(nheads, t.point_cap));
+    } else {
+        move(a.vecs + b.vstride * kVecPseudo, b.vecs + b.vstride * kVecPseudo, t.ndof);
+        move(a.bpseudo, b.bpseudo, 6u * slots);
+    }
+}
+
+template <int NR, bool kRigid, bool kControl, int kPart>
 NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t lane, Rally* rally) {
     const TemplateView& t = p.t;
     const bool has_artic = t.L != 0u, has_bodies = t.B != 0u;
@@ -215,9 +259,31 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     const bool use_pseudo = t.cfg.pos_iters != 0u && (t.cfg.max_contacts != 0u || t.L != 0u);
     Env e;
     env_begin<NR>(e, p, sm, env, lane);
+    uint32_t nheads = 0u;
+    float* img = nullptr;
+    float4* lanes = nullptr;
+    uint32_t* tail = nullptr;
+    bool resumed = kPart == kPartSolve;                 // the first trip starts behind the stages that lead to the solve
+    if constexpr (kPart != kPartWhole) {
+        resumed = resumed || p.resume != 0u;
+        img = p.image + (size_t)env * p.image_stride;
+        lanes = reinterpret_cast<float4*>(img + p.image_stride - kImageLaneWords);
+        tail = reinterpret_cast<uint32_t*>(lanes + 32);
+        if (resumed) {
+            const float4 mine = __ldcg(lanes + lane);
+            const uint4 words = __ldcg(reinterpret_cast<const uint4*>(tail));
+            e.qd = mine.x; e.qdd = mine.y; e.tau = mine.z; e.drive_dissipation = mine.w;
+            e.status = lane == 0u ? words.x : 0u; nheads = words.y; e.branching = words.z != 0u;
+            image_move<true, kPart == kPartSolve ? kBefore : kAfter>(e, p, img, nheads);
+            if (kPart == kPartStages) image_move<true, kAside>(e, p, img, nheads);
+            __syncwarp();
+        }
+    }
     // A step ends where the next begins, with the kinematics of the new coordinates: one pass over them serves both.
 #pragma unroll 1
-    for (uint32_t step = 0u;; ++step) {
+    for (uint32_t step = resumed ? 1u : 0u;; ++step) {
+      if (kPart != kPartSolve && !resumed) {
+        stay_together<kPart>();
         float E[9];
         V3 r = mk3(0.f, 0.f, 0.f);
         if (has_artic) {
@@ -241,7 +307,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             }
             __syncwarp();
             tick(e, 13);
-            if (step == p.steps) return;
+            if (kPart == kPartStages ? p.last != 0u : step == p.steps) return;
         }
         e.status = 0u; e.branching = false;
         if (p.mode == kModeRefresh) {
@@ -273,7 +339,8 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             if (lane < t.L) p.s.qddot[(size_t)env * t.L + lane] = e.qdd;
             return;
         }
-        uint32_t pair_count = 0u, nheads = 0u;
+        uint32_t pair_count = 0u;
+        stay_together<kPart>();
         if (has_bodies) stage_body_kick(e);
         if (has_collidables) {
             stage_aabbs(e);
@@ -292,15 +359,31 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             if (lane == 0u) p.s.status[env] |= st;
             return;
         }
+        stay_together<kPart>();
         nheads = stage_rows<NR>(e, pair_count);
         tick(e, 6);
         if constexpr (kRigid) team_fork(e, kTeamWarmStart, nheads, [&](uint32_t first, uint32_t stride) { warm_start_range(e, nheads, first, stride); });
         else warm_start_range(e, nheads, 0u, 1u);
         __syncwarp();
         tick(e, 7);
-        stage_solve<NR, kRigid>(e, nheads);
-        rally_wait(rally, p.group, lane);
-        tick(e, 29);
+        if constexpr (kPart == kPartStages) {
+            image_move<false, kBefore>(e, p, img, nheads); image_move<false, kAside>(e, p, img, nheads);
+            __stcg(lanes + lane, make_float4(e.qd, e.qdd, e.tau, e.drive_dissipation));
+            const uint32_t st = __reduce_or_sync(NKB_FULL, e.status);
+            if (lane == 0u) __stcg(reinterpret_cast<uint4*>(tail), make_uint4(st, nheads, e.branching ? 1u : 0u, 0u));
+            return;
+        }
+      }
+        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid>(e, nheads);
+        if constexpr (kPart == kPartSolve) {
+            image_move<false, kAfter>(e, p, img, nheads);
+            __stcg(reinterpret_cast<float*>(lanes + lane), e.qd);
+            const uint32_t st = __reduce_or_sync(NKB_FULL, e.status);
+            if (lane == 0u) tail[0] = st;
+            return;
+        }
+        resumed = false;
+        if constexpr (kPart == kPartWhole) { rally_wait(rally, p.group, lane); tick(e, 29); }
         if (has_collidables) {
             stage_cache_commit(e, nheads, [&](uint32_t ncontact) {
                 if constexpr (kRigid) team_fork(e, kTeamCacheOwners, ncontact, [&](uint32_t first, uint32_t stride) { cache_owners_range(e, ncontact, first, stride); });
@@ -383,7 +466,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
 
 // Block layout: blockDim.x / 32 warps, `team` consecutive warps per env (one unless the world runs in team mode); an
 // env's shared-memory slice is shared by its team.
-template <int NR, bool kRigid, bool kSlim, bool kControl>
+template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
 __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SLIM : NKB_MAXNREG)) step_kernel(const __grid_constant__ StepParams p) {
     extern __shared__ __align__(16) float smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -412,7 +495,7 @@ __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SL
     }
 #pragma unroll 1
     for (;;) {
-        advance_env<NR, kRigid, kControl>(p, sm, env, lane, &rally);
+        advance_env<NR, kRigid, kControl, kPart>(p, sm, env, lane, &rally);
         if (p.queue == nullptr) break;
         uint32_t next = 0u;
         if (lane == 0u) next = atomicAdd(p.queue, 1u);
@@ -432,7 +515,7 @@ __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SL
 // Raises the kernel's dynamic shared-memory limit to `bytes` if it is not there yet.  The limit is per function and
 // per device and only ever grows, so worlds of different sizes stepped from different threads cannot undo each other's
 // setting between the attribute call and the launch.
-template <int NR, bool kRigid, bool kSlim, bool kControl>
+template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
 static cudaError_t variant_reserve_shared(size_t bytes) {
     static std::mutex lock;
     static size_t reserved[64] = {0};
@@ -443,49 +526,50 @@ static cudaError_t variant_reserve_shared(size_t bytes) {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> hold(lock);
     if (bytes <= reserved[device]) return cudaSuccess;
-    err = cudaFuncSetAttribute(step_kernel<NR, kRigid, kSlim, kControl>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    err = cudaFuncSetAttribute(step_kernel<NR, kRigid, kSlim, kControl, kPart>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (err == cudaSuccess) reserved[device] = bytes;
     return err;
 }
 
-template <int NR, bool kRigid, bool kSlim, bool kControl>
+template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
 static int variant_resident_blocks(uint32_t warps_per_block, size_t shared_bytes) {
-    if (variant_reserve_shared<NR, kRigid, kSlim, kControl>(shared_bytes) != cudaSuccess) {
+    if (variant_reserve_shared<NR, kRigid, kSlim, kControl, kPart>(shared_bytes) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, step_kernel<NR, kRigid, kSlim, kControl>, (int)(warps_per_block * 32u), shared_bytes) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, step_kernel<NR, kRigid, kSlim, kControl, kPart>, (int)(warps_per_block * 32u), shared_bytes) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return blocks;
 }
 
-template <int NR, bool kRigid, bool kSlim, bool kControl>
+template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
 static int variant_registers() {
     cudaFuncAttributes attr{};
-    if (cudaFuncGetAttributes(&attr, step_kernel<NR, kRigid, kSlim, kControl>) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaFuncGetAttributes(&attr, step_kernel<NR, kRigid, kSlim, kControl, kPart>) != cudaSuccess) { cudaGetLastError(); return 0; }
     return attr.numRegs;
 }
 
-template <int NR, bool kRigid, bool kSlim, bool kControl>
+template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
 static cudaError_t variant_launch(const StepParams& p, uint32_t warps_per_block, cudaStream_t stream) {
     const uint32_t team = kRigid ? p.sm.team : 1u;
     const uint32_t envs_per_block = warps_per_block / team;
     if (envs_per_block == 0u || envs_per_block * team != warps_per_block || envs_per_block > kWarpsPerBlockMax) return cudaErrorInvalidConfiguration;
     const size_t bytes = (size_t)envs_per_block * p.sm.words * sizeof(float);
-    const cudaError_t err = variant_reserve_shared<NR, kRigid, kSlim, kControl>(bytes);
+    const cudaError_t err = variant_reserve_shared<NR, kRigid, kSlim, kControl, kPart>(bytes);
     if (err != cudaSuccess) return err;
     const uint32_t envs = p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
     if (envs == 0u) return cudaSuccess;
     const uint32_t needed = (envs + envs_per_block - 1u) / envs_per_block;
     const uint32_t blocks = p.queue != nullptr ? p.grid : needed;       // a persistent launch's grid is smaller than the batch
-    step_kernel<NR, kRigid, kSlim, kControl><<<blocks, warps_per_block * 32u, bytes, stream>>>(p);
+    step_kernel<NR, kRigid, kSlim, kControl, kPart><<<blocks, warps_per_block * 32u, bytes, stream>>>(p);
     return cudaGetLastError();
 }
 
-#define NKB_STEP_VARIANT(name, NR, RIGID, SLIM, CONTROL) \
-    extern const StepVariant name = {variant_resident_blocks<NR, RIGID, SLIM, CONTROL>, variant_registers<NR, RIGID, SLIM, CONTROL>, variant_launch<NR, RIGID, SLIM, CONTROL>};
+#define NKB_STEP_VARIANT(name, NR, RIGID, SLIM, CONTROL, PART) \
+    extern const StepVariant name = {variant_resident_blocks<NR, RIGID, SLIM, CONTROL, PART>, variant_registers<NR, RIGID, SLIM, CONTROL, PART>, \
+                                     variant_launch<NR, RIGID, SLIM, CONTROL, PART>};
 
 }  // namespace nkb

@@ -2,5 +2,5 @@
 #include "nkb_step.cuh"
 
 namespace nkb {
-NKB_STEP_VARIANT(kStepNarrowRigid, 1, true, false, false)
+NKB_STEP_VARIANT(kStepNarrowRigid, 1, true, false, false, kPartWhole)
 }  // namespace nkb

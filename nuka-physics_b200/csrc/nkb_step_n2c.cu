@@ -3,5 +3,5 @@
 #include "nkb_step.cuh"
 
 namespace nkb {
-NKB_STEP_VARIANT(kStepWideControl, 2, false, false, true)
+NKB_STEP_VARIANT(kStepWideControl, 2, false, false, true, kPartWhole)
 }  // namespace nkb

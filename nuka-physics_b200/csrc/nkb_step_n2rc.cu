@@ -3,5 +3,5 @@
 #include "nkb_step.cuh"
 
 namespace nkb {
-NKB_STEP_VARIANT(kStepWideRigidControl, 2, true, false, true)
+NKB_STEP_VARIANT(kStepWideRigidControl, 2, true, false, true, kPartWhole)
 }  // namespace nkb

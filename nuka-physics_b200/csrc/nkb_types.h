@@ -136,6 +136,7 @@ struct SmemLayout {
     uint32_t pairs, ccount, cpoint, cnormal, cdepth, cfeat;     // contacts
     uint32_t cstage;                                            // cache rebuild staging (shares the Jacobian pool, dead by then)
     uint32_t heads, jpool, binfo, chol;                         // solver (chol: the articulation's Newton matrix)
+    uint32_t factor_words;                                      // words of the mass matrix's factor
     uint32_t body_lanes;                                        // lanes that work on one free body: 8 or 16
     // Team mode: `team` warps advance one env; warp 0 leads, the others wait for work (rigid blocks of one colour).
     // team_area: 12 command words, then 4 result words per member.
@@ -146,6 +147,10 @@ struct SmemLayout {
     uint32_t words;                                             // total per env
     uint32_t ld;                                                // leading dimension of mass/factor (ndof | 1)
 };
+
+// A step in one launch, or split around its constraint solve: the straight-line stages of all envs, then the solves.
+enum StepPart : int { kPartWhole = 0, kPartStages = 1, kPartSolve = 2 };
+constexpr uint32_t kImageLaneWords = 4u * 32u + 4u;     // an image's tail: four words per lane, then status, heads, branching
 
 enum StepMode : uint32_t { kModeStep = 0, kModeDynamicsOnly = 1, kModeCollideOnly = 2, kModeRefresh = 3 };
 
@@ -160,6 +165,11 @@ struct StepParams {
     uint32_t group;
     uint32_t grid;
     uint32_t* queue;
+    // Split steps (kernel parts 1 and 2, see StepPart): where an env's slice waits between the launches, arranged as `im` says.
+    float* image;
+    uint32_t image_stride;
+    uint32_t resume, last;              // part 1: finish the step whose solve is done first; stop there
+    SmemLayout im;
     // Env selection of a refresh launch (null: every env).  sel_ids lists sel_count envs, one warp each; sel_mask is
     // an E-word device array whose non-zero entries pick the envs of a full-size launch.
     const uint32_t* sel_ids;

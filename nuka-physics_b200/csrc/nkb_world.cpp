@@ -370,7 +370,8 @@ void World::BuildLayout() {
     const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
     s.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
     at = std::max(at, dynamics_end);
-    s.mass = take(n * s.ld); s.factor = take(tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld); s.vstride = n > 32u ? 64u : 32u;
+    s.mass = take(n * s.ld); s.factor_words = tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld;
+    s.factor = take(s.factor_words); s.vstride = n > 32u ? 64u : 32u;
     s.vecs = take(6 * s.vstride);
     const uint32_t slots = B ? t.n_free + 1u : 0u;
     s.bpose = take(7 * B); s.bvel = take(6 * slots);
@@ -457,7 +458,37 @@ void World::BuildLayout() {
         const uint32_t grid = static_cast<uint32_t>(sms) * static_cast<uint32_t>(fits[warps_per_block_] / warps_per_block_);
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
+    // Split steps.
+    stages_ = solve_ = nullptr;
+    bool split = team == 1u && n != 0u && SC != 0u;
+    if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = split && std::atoi(forced) != 0;
+    if (split) {
+        stages_ = split_variant(n, t.n_free, control, kPartStages); solve_ = split_variant(n, t.n_free, control, kPartSolve);
+    }
+    if (stages_ != nullptr) {
+        // the solve's slice: what it reads and its own scratch, nothing of the kinematics and the contacts
+        SmemLayout& v = solve_sm_;
+        v = s;
+        at = 0;
+        v.vel = take(6);
+        v.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
+        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride);
+        v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
+        v.cdepth = take(4 * SC);
+        v.heads = take(kHeadStride * tv.head_cap);
+        v.jpool = take(tv.point_cap * 3u * ((n + 3u) & ~3u));
+        v.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);
+        v.words = at;
+        size_t top = 0;
+        for (uint32_t w = 1; w <= kWarpsPerBlockMax && w * bytes <= 227u * 1024u; ++w) {
+            const size_t r = static_cast<size_t>(stages_->resident_blocks(w, w * bytes)) * w;
+            if (r >= top) { top = r; stages_warps_ = w; }
+        }
+        if (const char* forced = std::getenv("NUKA_B200_STAGES_WARPS")) stages_warps_ = std::max(1u, static_cast<uint32_t>(std::atoi(forced)));
+    }
     if (std::getenv("NUKA_B200_DEBUG_LAYOUT") != nullptr) {
+        if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %d registers, %u warps per block; solve %u B, %d registers, %d resident\n", stages_->registers(), stages_warps_,
+                                             solve_sm_.words * 4u, solve_->registers(), solve_->resident_blocks(1, solve_sm_.words * 4u));
         std::fprintf(stderr, "[nuka_b200] %zu B of shared memory per env, %d registers per thread%s; resident warps per SM by block size:", bytes,
                      step_kernel_registers(n, t.n_free, slim_, control), slim_ ? " (slim build)" : "");
         for (uint32_t w = 1; w <= kWarpsPerBlockMax; ++w) std::fprintf(stderr, " %u:%zu", w, fits[w]);
@@ -496,6 +527,12 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.n_adm = (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size());
         SetBroadphase(0u);
         if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
+        if (stages_ != nullptr) {
+            params_.im = params_.sm;
+            params_.image_stride = ((params_.sm.words + 3u) & ~3u) + kImageLaneWords;
+            image_ = Alloc<float>(static_cast<size_t>(env_count_) * params_.image_stride, false);
+            params_.image = image_;
+        }
         const size_t E = env_count_, L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
         StateView& s = params_.s;
         s.env_count = env_count_;
@@ -640,37 +677,55 @@ void World::Step(uint32_t n) {
     if (n == 0u) return;
     step_count_ += n;
     Check(cudaSetDevice(device_), "cudaSetDevice");
-    StepParams p = params_;
-    p.mode = kModeStep;
-    p.group = group_; p.grid = grid_; p.queue = queue_;
-    if (!graph_mode_) {
-        // the kernel advances several steps per launch (inputs are constant across them; state goes back to global
-        // memory after every step, so the split changes no result); the cap keeps any one launch short
-        for (uint32_t done = 0u; done < n; done += kMaxStepsPerLaunch) {
-            p.steps = std::min(n - done, kMaxStepsPerLaunch);
-            Check(launch_step(p, warps_per_block_, slim_, stream_), "step launch");
-            ++launches_;
-        }
-        return;
-    }
+    if (!graph_mode_) { EnqueueSteps(n); return; }
     if (!graph_valid_) {
         if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
         if (graph_) { cudaGraphDestroy(graph_); graph_ = nullptr; }
-        p.steps = 1;
         // configure the kernel's shared-memory attribute outside the capture
         StepParams warm = params_;
         warm.mode = kModeRefresh; warm.steps = 1;
         Check(launch_step(warm, warps_per_block_, slim_, stream_), "graph warm-up launch");
         ++launches_;
         Check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
-        const cudaError_t launched = launch_step(p, warps_per_block_, slim_, stream_);
+        std::string failed;
+        const uint64_t before = launches_;
+        try { EnqueueSteps(1); } catch (const Error& err) { failed = err.what(); }
+        graph_launches_ = launches_ - before;
+        launches_ = before;
         const cudaError_t ended = cudaStreamEndCapture(stream_, &graph_);
-        Check(launched, "captured step launch");
+        if (!failed.empty()) throw Error(kCudaError, failed);
         Check(ended, "end capture");
         Check(cudaGraphInstantiate(&graph_exec_, graph_, 0), "graph instantiate");
         graph_valid_ = true;
     }
-    for (uint32_t k = 0; k < n; ++k) { Check(cudaGraphLaunch(graph_exec_, stream_), "graph launch"); ++launches_; }
+    for (uint32_t k = 0; k < n; ++k) { Check(cudaGraphLaunch(graph_exec_, stream_), "graph launch"); launches_ += graph_launches_; }
+}
+
+void World::EnqueueSteps(uint32_t n) {
+    StepParams p = params_;
+    p.mode = kModeStep;
+    if (stages_ != nullptr) {
+        StepParams v = p;
+        v.sm = solve_sm_;
+        p.steps = v.steps = 1;
+        for (uint32_t k = 0; k <= n; ++k) {
+            p.resume = k != 0u ? 1u : 0u; p.last = k == n ? 1u : 0u;
+            Check(stages_->launch(p, stages_warps_, stream_), "step stages launch");
+            ++launches_;
+            if (k == n) break;
+            Check(solve_->launch(v, 1u, stream_), "step solve launch");
+            ++launches_;
+        }
+        return;
+    }
+    p.group = group_; p.grid = grid_; p.queue = queue_;
+    // the kernel advances several steps per launch (inputs are constant across them; state goes back to global
+    // memory after every step, so the split changes no result); the cap keeps any one launch short
+    for (uint32_t done = 0u; done < n; done += kMaxStepsPerLaunch) {
+        p.steps = std::min(n - done, kMaxStepsPerLaunch);
+        Check(launch_step(p, warps_per_block_, slim_, stream_), "step launch");
+        ++launches_;
+    }
 }
 
 void World::Reset(const uint32_t* env_ids, uint32_t count) {

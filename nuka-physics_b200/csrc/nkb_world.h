@@ -109,6 +109,13 @@ private:
     uint32_t warps_per_block_ = 1;
     uint32_t group_ = 0, grid_ = 0;            // step launches: see StepParams
     uint32_t* queue_ = nullptr;
+    // split steps (null variants: steps run in one kernel): the kernels, the solve's own shared-memory layout, block size of the
+    // stages, the envs' images between launches
+    const StepVariant *stages_ = nullptr, *solve_ = nullptr;
+    SmemLayout solve_sm_{};
+    uint32_t stages_warps_ = 1;
+    float* image_ = nullptr;
+    void EnqueueSteps(uint32_t n);
     bool slim_ = false;        // the world runs the 128-register build of its kernel variant
     std::vector<void*> allocations_;
     ResetParams reset_{};
@@ -119,7 +126,7 @@ private:
     bool graph_mode_ = false, graph_valid_ = false;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;
-    uint64_t launches_ = 0;
+    uint64_t launches_ = 0, graph_launches_ = 1;
     uint64_t step_count_ = 0;
     struct PersistentField { void* ptr; uint32_t words; };
     std::vector<PersistentField> persistent_;
