@@ -266,7 +266,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     bool resumed = kPart == kPartSolve;                 // the first trip starts behind the stages that lead to the solve
     if constexpr (kPart != kPartWhole) {
         resumed = resumed || p.resume != 0u;
-        img = p.image + (size_t)env * p.image_stride;
+        img = p.image + (size_t)(env - p.image_first) * p.image_stride;
         lanes = reinterpret_cast<float4*>(img + p.image_stride - kImageLaneWords);
         tail = reinterpret_cast<uint32_t*>(lanes + 32);
         if (resumed) {
@@ -473,6 +473,7 @@ __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SL
     const uint32_t team = kRigid ? p.sm.team : 1u;
     const uint32_t slot = warp / team, member = warp - slot * team;
     uint32_t env = blockIdx.x * ((blockDim.x >> 5) / team) + slot;
+    if constexpr (kPart != kPartWhole) env = p.first + env < p.end ? p.first + env : 0xffffffffu;
     float* sm = smem + (size_t)slot * p.sm.words;
     if constexpr (kRigid) {
         // team mode: every lead zeroes its team's sequence numbers before any helper looks (a block-wide barrier, passed by
@@ -560,7 +561,7 @@ static cudaError_t variant_launch(const StepParams& p, uint32_t warps_per_block,
     const size_t bytes = (size_t)envs_per_block * p.sm.words * sizeof(float);
     const cudaError_t err = variant_reserve_shared<NR, kRigid, kSlim, kControl, kPart>(bytes);
     if (err != cudaSuccess) return err;
-    const uint32_t envs = p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
+    const uint32_t envs = kPart != kPartWhole ? p.end - p.first : p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
     if (envs == 0u) return cudaSuccess;
     const uint32_t needed = (envs + envs_per_block - 1u) / envs_per_block;
     const uint32_t blocks = p.queue != nullptr ? p.grid : needed;       // a persistent launch's grid is smaller than the batch

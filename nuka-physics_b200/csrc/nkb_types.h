@@ -168,6 +168,7 @@ struct StepParams {
     // Split steps (kernel parts 1 and 2, see StepPart): where an env's slice waits between the launches, arranged as `im` says.
     float* image;
     uint32_t image_stride;
+    uint32_t first, end, image_first;   // the envs of this launch, the env the images start with
     uint32_t resume, last;              // part 1: finish the step whose solve is done first; stop there
     SmemLayout im;
     // Env selection of a refresh launch (null: every env).  sel_ids lists sel_count envs, one warp each; sel_mask is

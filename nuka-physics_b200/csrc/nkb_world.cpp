@@ -438,30 +438,39 @@ void World::BuildLayout() {
     if (const char* forced = std::getenv("NUKA_B200_SLIM")) slim_ = has_slim && std::atoi(forced) != 0;     // variant experiments and tests
     const size_t* fits = resident[slim_ ? 1 : 0];
     const size_t most = best[slim_ ? 1 : 0];
-    // Block shape and how its warps meet (Rally).
+    // Block shape, and how its warps meet (Rally).  The largest block that keeps the most warps resident, or, for a batch that
+    // does not fill the SMs, the largest that spreads it over all of them.  The warps of a block meet after each solve, all of
+    // them, where their code outgrows the instruction cache: worlds with contacts, more than one env to a block (4 steps of 1000
+    // quadrupeds, blocks of 7: 2.01 ms apart, 1.80 in groups of 5, 1.47 all together).  Without contacts a step is short enough
+    // for the cache and the warps go their own ways (4096 arms, 32 steps: 3.30 ms apart, 3.49 together); where an SM holds four
+    // warps or fewer, fetches are no bottleneck either.
     warps_per_block_ = team;
     for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) if (fits[w] == most) warps_per_block_ = w;
     group_ = 0u; grid_ = 0u;
+    int sms = 148;
+    Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
+    const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
     if (team == 1u) {
-        int sms = 148;
-        Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
-        const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
         if (most <= 4u) warps_per_block_ = 1u;
+        else if (share >= most && SC == 0u && fits[4] == most) warps_per_block_ = 4u;      // no meetings: small blocks pack better (3.10 ms against 3.29)
         else if (share < most)
             for (uint32_t w = 1u; w <= std::min(share, kWarpsPerBlockMax); ++w) if (fits[w] >= share) warps_per_block_ = w;
         if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // block-shape experiments
             const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
             if (w >= 1u && w <= kWarpsPerBlockMax && fits[w] != 0u) warps_per_block_ = w;
         }
-        group_ = std::min(warps_per_block_, 5u);
+        group_ = SC != 0u ? warps_per_block_ : 0u;
         if (const char* forced = std::getenv("NUKA_B200_GROUP")) group_ = static_cast<uint32_t>(std::atoi(forced));
         const uint32_t grid = static_cast<uint32_t>(sms) * static_cast<uint32_t>(fits[warps_per_block_] / warps_per_block_);
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
-    // Split steps.
+    // Split steps (see image_move): for batches that go over the SMs more than once, 12 envs to an SM and up.  Below, one kernel
+    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.74 ms in one kernel, 1.88
+    // split; 3000: 2.91 and 2.26; 1200 quadrupeds with 4 boxes: 3.08 and 3.28; 2400: 4.65 and 4.35; 1000 humanoids: 6.69 and
+    // 6.99; 2048: 9.50 and 8.61).
     stages_ = solve_ = nullptr;
-    bool split = team == 1u && n != 0u && SC != 0u;
-    if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = split && std::atoi(forced) != 0;
+    bool split = team == 1u && n != 0u && SC != 0u && share > 12u && env_count_ > static_cast<uint32_t>(sms) * most;
+    if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && n != 0u && SC != 0u && std::atoi(forced) != 0;
     if (split) {
         stages_ = split_variant(n, t.n_free, control, kPartStages); solve_ = split_variant(n, t.n_free, control, kPartSolve);
     }
@@ -482,9 +491,9 @@ void World::BuildLayout() {
         size_t top = 0;
         for (uint32_t w = 1; w <= kWarpsPerBlockMax && w * bytes <= 227u * 1024u; ++w) {
             const size_t r = static_cast<size_t>(stages_->resident_blocks(w, w * bytes)) * w;
-            if (r >= top) { top = r; stages_warps_ = w; }
+            if (r > top || (r == top && w <= 8u)) { top = r; stages_warps_ = w; }       // 8 against 16 warps: 3 % at 2500 and 4096 quadrupeds, equal from 8000 on
         }
-        if (const char* forced = std::getenv("NUKA_B200_STAGES_WARPS")) stages_warps_ = std::max(1u, static_cast<uint32_t>(std::atoi(forced)));
+        if (const char* forced = std::getenv("NUKA_B200_STAGES_WARPS")) stages_warps_ = std::max(1u, std::min(stages_warps_, static_cast<uint32_t>(std::atoi(forced))));
     }
     if (std::getenv("NUKA_B200_DEBUG_LAYOUT") != nullptr) {
         if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %d registers, %u warps per block; solve %u B, %d registers, %d resident\n", stages_->registers(), stages_warps_,
@@ -528,10 +537,24 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         SetBroadphase(0u);
         if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
         if (stages_ != nullptr) {
+            // images of the whole batch up to 2 GB, at least of 8192 envs: a larger batch goes in rounds over the same buffer
             params_.im = params_.sm;
             params_.image_stride = ((params_.sm.words + 3u) & ~3u) + kImageLaneWords;
-            image_ = Alloc<float>(static_cast<size_t>(env_count_) * params_.image_stride, false);
-            params_.image = image_;
+            const size_t bytes = static_cast<size_t>(params_.image_stride) * sizeof(float);
+            image_envs_ = static_cast<uint32_t>(std::min<size_t>(env_count_, std::max<size_t>(8192u, (size_t{2} << 30) / bytes)));
+            void* image = nullptr;
+            if (cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess) {
+                allocations_.push_back(image);
+                params_.image = static_cast<float*>(image);
+                Check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
+                for (uint32_t c = 0; c + 1u < kChunks; ++c) {
+                    Check(cudaStreamCreateWithFlags(&side_[c], cudaStreamNonBlocking), "cudaStreamCreate");
+                    Check(cudaEventCreateWithFlags(&join_[c], cudaEventDisableTiming), "cudaEventCreate");
+                }
+            } else {
+                cudaGetLastError();                 // no room for the images: steps run in one kernel
+                stages_ = solve_ = nullptr;
+            }
         }
         const size_t E = env_count_, L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
         StateView& s = params_.s;
@@ -552,6 +575,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         s.dbg_mass = nullptr; s.dbg_qdot_pseudo = nullptr; s.dbg_cycles = nullptr;
         Seed();
     } catch (...) {
+        ReleaseStreams();
         for (void* p : allocations_) cudaFree(p);
         allocations_.clear();
         throw;
@@ -563,7 +587,16 @@ World::~World() {
     cudaStreamSynchronize(stream_);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (graph_) cudaGraphDestroy(graph_);
+    ReleaseStreams();
     for (void* p : allocations_) cudaFree(p);
+}
+
+void World::ReleaseStreams() {
+    if (fork_) cudaEventDestroy(fork_);
+    for (uint32_t c = 0; c + 1u < kChunks; ++c) {
+        if (join_[c]) cudaEventDestroy(join_[c]);
+        if (side_[c]) cudaStreamDestroy(side_[c]);
+    }
 }
 
 // Every env starts from the template (reference src/nk/pipeline/world.cpp:289-654); the same table drives
@@ -705,16 +738,31 @@ void World::EnqueueSteps(uint32_t n) {
     StepParams p = params_;
     p.mode = kModeStep;
     if (stages_ != nullptr) {
-        StepParams v = p;
-        v.sm = solve_sm_;
-        p.steps = v.steps = 1;
-        for (uint32_t k = 0; k <= n; ++k) {
-            p.resume = k != 0u ? 1u : 0u; p.last = k == n ? 1u : 0u;
-            Check(stages_->launch(p, stages_warps_, stream_), "step stages launch");
-            ++launches_;
-            if (k == n) break;
-            Check(solve_->launch(v, 1u, stream_), "step solve launch");
-            ++launches_;
+        // Parts of the batch on streams of their own, forked from the world's and joined to it: while one part's last solves run,
+        // the others fill the SMs (4096 quadrupeds, 4 steps: 2.93 ms in one part, 2.80 in three; 16 384: 9.55 and 9.16).
+        p.steps = 1;
+        for (uint32_t done = 0u; done < env_count_; done += image_envs_) {
+            const uint32_t round = std::min(image_envs_, env_count_ - done);
+            p.image_first = done;
+            Check(cudaEventRecord(fork_, stream_), "step fork");
+            for (uint32_t c = 0; c < kChunks; ++c) {
+                const cudaStream_t stream = c == 0u ? stream_ : side_[c - 1u];
+                if (c != 0u) Check(cudaStreamWaitEvent(stream, fork_, 0), "step fork");
+                p.first = done + static_cast<uint32_t>(static_cast<uint64_t>(round) * c / kChunks);
+                p.end = done + static_cast<uint32_t>(static_cast<uint64_t>(round) * (c + 1u) / kChunks);
+                StepParams v = p;
+                v.sm = solve_sm_;
+                for (uint32_t k = 0; k <= n; ++k) {
+                    p.resume = k != 0u ? 1u : 0u; p.last = k == n ? 1u : 0u;
+                    Check(stages_->launch(p, stages_warps_, stream), "step stages launch");
+                    ++launches_;
+                    if (k == n) break;
+                    Check(solve_->launch(v, 1u, stream), "step solve launch");
+                    ++launches_;
+                }
+                if (c != 0u) Check(cudaEventRecord(join_[c - 1u], stream), "step join");
+            }
+            for (uint32_t c = 1; c < kChunks; ++c) Check(cudaStreamWaitEvent(stream_, join_[c - 1u], 0), "step join");
         }
         return;
     }

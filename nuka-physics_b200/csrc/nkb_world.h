@@ -114,8 +114,12 @@ private:
     const StepVariant *stages_ = nullptr, *solve_ = nullptr;
     SmemLayout solve_sm_{};
     uint32_t stages_warps_ = 1;
-    float* image_ = nullptr;
+    uint32_t image_envs_ = 0;                  // envs the image buffer holds: larger batches go in rounds
+    static constexpr uint32_t kChunks = 3u;    // parts of a round, each on a stream of its own
+    cudaStream_t side_[kChunks - 1] = {};
+    cudaEvent_t fork_ = nullptr, join_[kChunks - 1] = {};
     void EnqueueSteps(uint32_t n);
+    void ReleaseStreams();
     bool slim_ = false;        // the world runs the 128-register build of its kernel variant
     std::vector<void*> allocations_;
     ResetParams reset_{};
