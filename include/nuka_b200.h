@@ -252,6 +252,13 @@ nuka_result_t nuka_b200_world_info(nuka_world_handle world, nuka_b200_world_info
  * velocity update (fills JOINT_ACCELERATION and MASS_MATRIX), 2 = collision only (fills the contact taps). */
 nuka_result_t nuka_b200_world_run_stage(nuka_world_handle world, uint32_t stage);
 
+/* nuka_world_download_field into page-locked memory of the library's own: the whole field, complete when the call returns;
+ * *bytes is released with nuka_b200_host_release, from any thread, before or after the world is destroyed.  The library keeps
+ * released blocks for later calls.  NUKA_ERR_NOT_SUPPORTED when the blocks in use would exceed 256 MB (download into memory of
+ * the caller's instead). */
+nuka_result_t nuka_b200_world_download_host(nuka_world_handle world, nuka_state_field_t field, void** bytes, size_t* nbytes);
+void nuka_b200_host_release(void* bytes);
+
 /* Kernel launches enqueued by this world since creation (for throughput reports). */
 nuka_result_t nuka_b200_world_launch_count(nuka_world_handle world, uint64_t* out);
 

@@ -566,6 +566,67 @@ nuka_result_t nuka_world_download_field(nuka_world_handle world, nuka_state_fiel
     return Transfer(world, field, bytes, nbytes, byte_offset, false);
 }
 
+// Page-locked blocks for downloads.  A copy into pageable memory goes through the driver's staging buffer at about 4 GB/s and
+// faults the destination's fresh pages (1.28 MB: 320 us); into page-locked memory it is one transfer at link speed (45 us).
+// Locking pages takes longer than either, so released blocks are kept, by power-of-two size; blocks handed out and kept
+// together stay within kHostPoolBytes.
+namespace {
+struct HostPool {
+    static constexpr size_t kHostPoolBytes = size_t{256} << 20, kSmallest = 4096;
+    std::mutex lock;
+    std::unordered_map<void*, size_t> sizes;                    // every block, handed out or kept
+    std::unordered_map<size_t, std::vector<void*>> kept;
+    size_t total = 0;
+    void* Take(size_t bytes) {
+        size_t size = kSmallest;
+        while (size < bytes) size <<= 1;
+        std::lock_guard<std::mutex> hold(lock);
+        auto& list = kept[size];
+        if (!list.empty()) { void* p = list.back(); list.pop_back(); return p; }
+        if (size > kHostPoolBytes) return nullptr;
+        for (auto it = kept.begin(); it != kept.end() && total + size > kHostPoolBytes; ++it)
+            while (!it->second.empty() && total + size > kHostPoolBytes) {
+                cudaFreeHost(it->second.back()); sizes.erase(it->second.back()); it->second.pop_back(); total -= it->first;
+            }
+        void* p = nullptr;
+        if (total + size > kHostPoolBytes) return nullptr;
+        if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        total += size; sizes[p] = size;
+        return p;
+    }
+    void Give(void* p) {
+        std::lock_guard<std::mutex> hold(lock);
+        const auto it = sizes.find(p);
+        if (it != sizes.end()) kept[it->second].push_back(p);
+    }
+};
+HostPool& Pool() { static HostPool* pool = new HostPool; return *pool; }     // outlives arrays released at exit
+}  // namespace
+
+nuka_result_t nuka_b200_world_download_host(nuka_world_handle world, nuka_state_field_t field, void** bytes, size_t* nbytes) {
+    if (bytes == nullptr || nbytes == nullptr) { SetError("out pointer is null"); return NUKA_RESULT_INVALID_ARG; }
+    *bytes = nullptr; *nbytes = 0;
+    NKB_WORLD(w)
+    return Guard([&]() {
+        nkb::FieldInfo info;
+        if (!w->Field(static_cast<uint32_t>(field), &info)) { SetError("field is not served by this path"); return NUKA_RESULT_NOT_SUPPORTED; }
+        const size_t total = info.per_env * w->env_count() * 4u;
+        if (total == 0u) { SetError("the field is empty"); return NUKA_RESULT_NOT_SUPPORTED; }
+        if (cudaSetDevice(w->device()) != cudaSuccess) { SetError("cudaSetDevice failed"); return NUKA_RESULT_CUDA_ERROR; }
+        void* block = Pool().Take(total);
+        if (block == nullptr) { SetError("no page-locked memory left for downloads"); return NUKA_RESULT_NOT_SUPPORTED; }
+        if (cudaMemcpyAsync(block, info.ptr, total, cudaMemcpyDeviceToHost, w->stream()) != cudaSuccess || cudaStreamSynchronize(w->stream()) != cudaSuccess) {
+            Pool().Give(block);
+            SetError("field download failed");
+            return NUKA_RESULT_CUDA_ERROR;
+        }
+        *bytes = block; *nbytes = total;
+        return NUKA_RESULT_OK;
+    });
+}
+
+void nuka_b200_host_release(void* bytes) { if (bytes != nullptr) Pool().Give(bytes); }
+
 nuka_result_t nuka_b200_world_info(nuka_world_handle world, nuka_b200_world_info_t* out) {
     NKB_WORLD(w)
     if (out == nullptr) { SetError("out pointer is null"); return NUKA_RESULT_INVALID_ARG; }

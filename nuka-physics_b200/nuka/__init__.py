@@ -111,6 +111,19 @@ class FieldView:
         return (2, self._world.device.gpu_index)   # kDLCUDA
 
 
+class _HostBlock:
+    """Page-locked memory of the library under a downloaded array; goes back when the last array over it does."""
+
+    __slots__ = ("_ptr", "_release", "__array_interface__")
+
+    def __init__(self, lib, ptr, shape, typestr):
+        self._ptr, self._release = ptr, lib.nuka_b200_host_release
+        self.__array_interface__ = {"shape": shape, "typestr": typestr, "data": (ptr, False), "version": 3}
+
+    def __del__(self):
+        self._release(self._ptr)
+
+
 class Checkpoint:
     """A captured world state (reference nuka.h:387-404)."""
 
@@ -323,7 +336,11 @@ class World:
 
     def download(self, field):
         v = self.view(field)
-        out = np.zeros(v.shape, dtype=v.dtype)
+        lib = _abi.lib()
+        block, size = ctypes.c_void_p(), ctypes.c_size_t()
+        if lib.nuka_b200_world_download_host(self._h, int(field), ctypes.byref(block), ctypes.byref(size)) == _abi.OK:
+            return np.asarray(_HostBlock(lib, block.value, v.shape, v.dtype.str))
+        out = np.zeros(v.shape, dtype=v.dtype)              # no page-locked block to be had
         _check(_abi.lib().nuka_world_download_field(self._h, int(field), out.ctypes.data, out.nbytes, 0))
         return out
 

@@ -62,7 +62,7 @@ EXPORTS = [
     "nuka_world_set_gravity_z", "nuka_world_set_velocity_iterations", "nuka_world_get_velocity_iterations", "nuka_world_synchronize",
     "nuka_world_reset", "nuka_world_reset_envs", "nuka_world_forward_kinematics", "nuka_world_get_stream", "nuka_world_record_event",
     "nuka_world_get_buffer_view", "nuka_world_upload_field", "nuka_world_download_field", "nuka_world_create_from_template",
-    "nuka_b200_world_info", "nuka_b200_world_run_stage", "nuka_b200_world_launch_count", "nuka_b200_world_reset_envs_static",
+    "nuka_b200_world_info", "nuka_b200_world_run_stage", "nuka_b200_world_launch_count", "nuka_b200_world_reset_envs_static", "nuka_b200_world_download_host", "nuka_b200_host_release",
     "nuka_b200_world_pack_observations", "nuka_b200_observation_desc_defaults", "nuka_b200_world_reset_envs_masked",
     "nuka_b200_world_set_contact_readout", "nuka_b200_world_set_broadphase", "nuka_b200_template_check", "nuka_b200_cook_options_defaults", "nuka_b200_scene_cook", "nuka_world_checkpoint_capture", "nuka_world_checkpoint_restore", "nuka_checkpoint_destroy",
     "nuka_checkpoint_write", "nuka_world_checkpoint_read", "nuka_checkpoint_byte_size", "nuka_checkpoint_equal", "nuka_world_state_hash",
@@ -118,6 +118,9 @@ def lib():
     L.nuka_world_get_dof_name.argtypes = [vp, ctypes.c_uint32, ctypes.c_char_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]
     L.nuka_world_upload_field.argtypes = [vp, ctypes.c_int, vp, sz, sz]
     L.nuka_world_download_field.argtypes = [vp, ctypes.c_int, vp, sz, sz]
+    L.nuka_b200_world_download_host.argtypes = [vp, ctypes.c_int, ctypes.POINTER(vp), ctypes.POINTER(sz)]
+    L.nuka_b200_host_release.argtypes = [vp]
+    L.nuka_b200_host_release.restype = None
     L.nuka_b200_world_info.argtypes = [vp, ctypes.POINTER(WorldInfo)]
     L.nuka_b200_world_run_stage.argtypes = [vp, u32]
     L.nuka_b200_world_launch_count.argtypes = [vp, ctypes.POINTER(ctypes.c_uint64)]
