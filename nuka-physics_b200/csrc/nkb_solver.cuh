@@ -1304,6 +1304,23 @@ struct BodyLanes {
     uint32_t width, j, mask, first;      // lanes per body, lane within the group, the group's lanes, its first lane
     NKB_DEV bool any(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) != 0u; }
     NKB_DEV bool all(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) == mask; }
+    // v[k] summed over the group's lanes, dealt out: lane j gets the sums of v[(j & 7) N / 8 ...] in v[0 .. N / 8).  Each
+    // exchange halves what a lane still holds (28 shuffles for 32 values over 8 lanes; a sum per value would take 96)
+    template <typename T, int N> NKB_DEV void deal(T (&v)[N]) const {
+        int held = N / 2;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1, held >>= 1) {
+            const bool upper = (j & o) != 0u;
+#pragma unroll
+            for (int k = 0; k < held; ++k) {
+                const T give = upper ? v[k] : v[k + held], keep = upper ? v[k + held] : v[k];
+                v[k] = keep + __shfl_xor_sync(NKB_FULL, give, o);
+            }
+        }
+        if (width > 8u)
+#pragma unroll
+            for (int k = 0; k < N / 8; ++k) v[k] += __shfl_xor_sync(NKB_FULL, v[k], 8);
+    }
     template <typename T> NKB_DEV T sum(T v) const {
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
@@ -1338,6 +1355,30 @@ template <typename T> NKB_DEV T pick6(const T (&v)[6], uint32_t k) { return k ==
 NKB_DEV float dot_fma(V3 a, V3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
 NKB_DEV V3 cross_fma(V3 a, V3 b) { return mk3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x))); }
 
+NKB_DEV V3 mix_fma(V3 a, float p, V3 b, float q) { return mk3(fmaf(a.x, p, b.x * q), fmaf(a.y, p, b.y * q), fmaf(a.z, p, b.z * q)); }
+// One constraint row J = (n, m), m = arm x n, in a lane's share of a body's Newton system: its impulse's part of the force
+// balance and its part of the rounding scale (entry i of which sits in share[4 i + 3], entry k of the lower triangle in
+// share[4 (k / 3) + k % 3]: dealt out over eight lanes, lane i gets row i's scale and three entries of the matrix).
+NKB_DEV void body_row_share(V3 n, V3 m, float impulse, float size, float (&share)[32], double (&balance)[8]) {
+    const float j[6] = {n.x, n.y, n.z, m.x, m.y, m.z};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        balance[i] = fma((double)j[i], (double)impulse, balance[i]);
+        share[4 * i + 3] = fmaf(fabsf(j[i]), size, share[4 * i + 3]);
+    }
+}
+// J (K J)^T of one row: J = (n, m), its row of K J = (p, q)
+NKB_DEV void body_block_share(V3 n, V3 m, V3 p, V3 q, float (&share)[32]) {
+    const float j[6] = {n.x, n.y, n.z, m.x, m.y, m.z}, c[6] = {p.x, p.y, p.z, q.x, q.y, q.z};
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int k = 0; k <= i; ++k) {
+            const int at = i * (i + 1) / 2 + k;
+            share[4 * (at / 3) + at % 3] = fmaf(j[i], c[k], share[4 * (at / 3) + at % 3]);
+        }
+}
+
 // Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: `32 / body_lanes` blocks at a
 // time, warp `first` of `stride`.  Same model, stopping rules and exact line search as descend_block; the sums that one
 // compensates in float run in double, the inertial force is carried as in descend_tree.
@@ -1350,7 +1391,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
     Env e = bare_env(run.sm, run.lay, run.t, nullptr, 0u, run.lane, run.vstride);
     const TemplateView& t = *e.t;
     const BodyLanes g = body_lanes(e);
-    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
+    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u;
     const uint32_t* order = block_order(e, nb);
     float most_moved = 0.f, worst = 0.f;
     bool failed = false;
@@ -1498,68 +1539,61 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             if (!__any_sync(NKB_FULL, active)) break;
             step = step < 0 ? 0 : step + 1;
             __syncwarp();
-            // the next Newton system: this lane's row of H, its entry of the force balance and its rounding scale
-            float hr[6], scale = 0.f;
-            double gsum = 0.0;
+            // the next Newton system.  A lane takes the heads j, j + width, ...: its share of H (lower triangle), of the force
+            // balance and of the rounding scale; the lanes then add their shares
+            float a[28], own, scale;
+            {
+                float share[32];
+                double balance[8];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) hr[k] = 0.f;
-            if (part == 0u && row < 6u) {
-                if (row < 3u) { hr[0] = row == 0u ? mass.m : 0.f; hr[1] = row == 1u ? mass.m : 0.f; hr[2] = row == 2u ? mass.m : 0.f; }
-                else {
-                    hr[3] = row == 3u ? mass.i[0] : row == 4u ? mass.i[3] : mass.i[4];
-                    hr[4] = row == 3u ? mass.i[3] : row == 4u ? mass.i[1] : mass.i[5];
-                    hr[5] = row == 3u ? mass.i[4] : row == 4u ? mass.i[5] : mass.i[2];
-                }
-                gsum = -pick6(inertial, row);
-                scale = fabsf((float)gsum);
-            }
-            if (active)
+                for (int k = 0; k < 32; ++k) share[k] = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) balance[k] = 0.0;
+                if (active)
 #pragma unroll 1
-                for (uint32_t k = part; k < count; k += parts) {
-                    const uint32_t h = inc[k];
-                    const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
-                    const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), w = body_row_axis(row, arm);
-                    const float4 f = hq(e, HF_F, h);
-                    const float j0 = dot_fma(n, w), sgn = first_side ? 1.f : -1.f;
-                    V3 a;
-                    if (position) {                                    // push-out rows have a normal axis only
-                        gsum = fma((double)(sgn * j0), (double)f.x, gsum);
-                        scale = fmaf(fabsf(j0), hf(e, HF_NZ, h), scale);
-                        a = n * (j0 * f.w);
-                    } else {
-                        const float4 c = hq(e, HF_C + 1u, h);
-                        const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
-                        const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h);
-                        const float j1 = dot_fma(t1, w), j2 = dot_fma(t2, w);
-                        gsum = fma((double)(sgn * j0), (double)f.x, gsum); gsum = fma((double)(sgn * j1), (double)f.y, gsum); gsum = fma((double)(sgn * j2), (double)f.z, gsum);
-                        scale = fmaf(fabsf(j0), c.w, fmaf(fabsf(j1), nz.x, fmaf(fabsf(j2), nz.y, scale)));
-                        const float p0 = j0 * f.w, p1 = fmaf(j1, c.x, j2 * c.z), p2 = fmaf(j2, c.y, j1 * c.z);
-                        a = mk3(fmaf(n.x, p0, fmaf(t1.x, p1, t2.x * p2)), fmaf(n.y, p0, fmaf(t1.y, p1, t2.y * p2)), fmaf(n.z, p0, fmaf(t1.z, p1, t2.z * p2)));
+                    for (uint32_t k = g.j; k < count; k += g.width) {
+                        const uint32_t h = inc[k];
+                        const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                        const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), m0 = cross_fma(arm, n);
+                        const float4 f = hq(e, HF_F, h);
+                        body_row_share(n, m0, first_side ? f.x : -f.x, hf(e, HF_NZ, h), share, balance);
+                        body_block_share(n, m0, n * f.w, m0 * f.w, share);
+                        if (!position) {                               // push-out rows have a normal axis only
+                            const float4 c = hq(e, HF_C + 1u, h);
+                            const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
+                            const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h), m1 = cross_fma(arm, t1), m2 = cross_fma(arm, t2);
+                            body_row_share(t1, m1, first_side ? f.y : -f.y, nz.x, share, balance);
+                            body_row_share(t2, m2, first_side ? f.z : -f.z, nz.y, share, balance);
+                            body_block_share(t1, m1, mix_fma(t1, c.x, t2, c.z), mix_fma(m1, c.x, m2, c.z), share);
+                            body_block_share(t2, m2, mix_fma(t2, c.y, t1, c.z), mix_fma(m2, c.y, m1, c.z), share);
+                        }
                     }
-                    const V3 m = cross_fma(arm, a);
-                    hr[0] = __fadd_rn(hr[0], a.x); hr[1] = __fadd_rn(hr[1], a.y); hr[2] = __fadd_rn(hr[2], a.z); hr[3] = __fadd_rn(hr[3], m.x); hr[4] = __fadd_rn(hr[4], m.y); hr[5] = __fadd_rn(hr[5], m.z);
+                __syncwarp();
+                g.deal(share); g.deal(balance);
+                scale = share[3];
+                const double inner = pick6(inertial, row);
+                own = (float)(balance[0] - (row < 6u ? inner : 0.0));
+                scale += row < 6u ? fabsf((float)inner) : 0.f;
+#pragma unroll
+                for (int k = 0; k < 21; ++k) a[k] = __shfl_sync(NKB_FULL, share[k % 3], g.first + k / 3);
+                a[0] = __fadd_rn(a[0], mass.m); a[2] = __fadd_rn(a[2], mass.m); a[5] = __fadd_rn(a[5], mass.m);
+                a[9] = __fadd_rn(a[9], mass.i[0]); a[13] = __fadd_rn(a[13], mass.i[3]); a[14] = __fadd_rn(a[14], mass.i[1]);
+                a[18] = __fadd_rn(a[18], mass.i[4]); a[19] = __fadd_rn(a[19], mass.i[5]); a[20] = __fadd_rn(a[20], mass.i[2]);
+                float reach[6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    reach[i] = 0.f;
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) reach[i] = fmaf(fabsf(i >= k ? a[i * (i + 1) / 2 + k] : a[k * (k + 1) / 2 + i]), fabsf((float)u[k]), reach[i]);
                 }
-            __syncwarp();
-            if (parts > 1u) {
-#pragma unroll
-                for (int k = 0; k < 6; ++k) hr[k] += __shfl_xor_sync(NKB_FULL, hr[k], 8);
-                gsum += __shfl_xor_sync(NKB_FULL, gsum, 8); scale += __shfl_xor_sync(NKB_FULL, scale, 8);
+                scale += pick6(reach, row);
             }
-#pragma unroll
-            for (int k = 0; k < 6; ++k) scale = fmaf(fabsf(hr[k]), fabsf((float)u[k]), scale);
-            const float own = (float)gsum;
             const bool finite = g.all(isfinite(own)), small = g.all(row >= 6u || fabsf(own) <= kRoundings * FLT_EPSILON * scale);
             failure |= active && !finite;
             active = active && finite;
-            // the group's rows to every lane of it
-            float a[28], inv[6], x[6];
+            float inv[6], x[6];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
-                a[21 + i] = force[i];
-#pragma unroll
-                for (int k = 0; k <= i; ++k) a[i * (i + 1) / 2 + k] = __shfl_sync(NKB_FULL, hr[k], g.first + i);
-            }
+            for (int i = 0; i < 6; ++i) a[21 + i] = force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
             if (active && small) {
                 bool still = true;
                 if (run.tol > 0.f) {
