@@ -88,7 +88,7 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
     e.qd = link ? p.s.qdot[at] : 0.f;
     e.qdd = 0.f; e.tau = 0.f;
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
-    e.vstride = 32u * NR;
+    e.vstride = 32u * (NR > 0 ? NR : 1);
     e.dof_link[1] = 0u; e.dof_comp[1] = kNoLink;
 #pragma unroll
     for (uint32_t r = 0u; r < (uint32_t)NR; ++r) {

@@ -20,32 +20,33 @@ __global__ void reset_kernel(ResetParams r) {
     }
 }
 
-extern const StepVariant kStepNarrow, kStepNarrowSlim, kStepNarrowRigid, kStepWide, kStepWideRigid;
+extern const StepVariant kStepBodies, kStepNarrow, kStepNarrowSlim, kStepNarrowRigid, kStepWide, kStepWideRigid;
 extern const StepVariant kStepNarrowControl, kStepNarrowRigidControl, kStepWideControl, kStepWideRigidControl;
 
 extern const StepVariant kStagesNarrow, kSolveNarrow, kStagesNarrowRigid, kSolveNarrowRigid, kStagesWide, kSolveWide;
 
 bool step_kernel_has_slim(uint32_t ndof, uint32_t n_free, bool control) { return ndof <= 32u && n_free == 0u && !control; }
 
-// up to 32 or up to 64 coordinates per articulation; with or without free rigid bodies; the slim (128-register) build
-// exists for the first kind only
-static const StepVariant& step_variant(uint32_t ndof, uint32_t n_free, bool slim, bool control) {
+// no articulation, up to 32 or up to 64 coordinates per articulation; with or without free rigid bodies; the slim
+// (128-register) build exists for articulations of up to 32 without bodies only
+static const StepVariant& step_variant(const TemplateView& t, bool slim) {
     // control modes 3 and 4 run the builds that hold the controllers
-    if (control) return ndof > 32u ? (n_free != 0u ? kStepWideRigidControl : kStepWideControl) : (n_free != 0u ? kStepNarrowRigidControl : kStepNarrowControl);
-    if (ndof > 32u) return n_free != 0u ? kStepWideRigid : kStepWide;
-    if (n_free != 0u) return kStepNarrowRigid;
+    const bool control = t.cfg.control_mode == 3u || t.cfg.control_mode == 4u;
+    if (t.L == 0u && t.n_free != 0u) return kStepBodies;
+    if (control) return t.ndof > 32u ? (t.n_free != 0u ? kStepWideRigidControl : kStepWideControl) : (t.n_free != 0u ? kStepNarrowRigidControl : kStepNarrowControl);
+    if (t.ndof > 32u) return t.n_free != 0u ? kStepWideRigid : kStepWide;
+    if (t.n_free != 0u) return kStepNarrowRigid;
     return slim ? kStepNarrowSlim : kStepNarrow;
 }
 
-int step_kernel_registers(uint32_t ndof, uint32_t n_free, bool slim, bool control) { return step_variant(ndof, n_free, slim, control).registers(); }
+int step_kernel_registers(const TemplateView& t, bool slim) { return step_variant(t, slim).registers(); }
 
-int step_kernel_resident_blocks(uint32_t ndof, uint32_t n_free, bool slim, bool control, uint32_t warps_per_block, size_t shared_bytes) {
-    return step_variant(ndof, n_free, slim, control).resident_blocks(warps_per_block, shared_bytes);
+int step_kernel_resident_blocks(const TemplateView& t, bool slim, uint32_t warps_per_block, size_t shared_bytes) {
+    return step_variant(t, slim).resident_blocks(warps_per_block, shared_bytes);
 }
 
 cudaError_t launch_step(const StepParams& p, uint32_t warps_per_block, bool slim, cudaStream_t stream) {
-    const bool control = p.t.cfg.control_mode == 3u || p.t.cfg.control_mode == 4u;
-    return step_variant(p.t.ndof, p.t.n_free, slim && !control, control).launch(p, warps_per_block, stream);
+    return step_variant(p.t, slim).launch(p, warps_per_block, stream);
 }
 
 const StepVariant* split_variant(uint32_t ndof, uint32_t n_free, bool control, StepPart part) {

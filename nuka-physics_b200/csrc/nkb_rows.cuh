@@ -63,7 +63,8 @@ NKB_DEV uint32_t side_block(const Env& e, uint32_t body, uint32_t& link) {
 template <int NR>
 NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
     const TemplateView& t = *e.t;
-    const uint32_t S = t.cfg.max_contacts, n = t.ndof, L = t.L, lane = e.lane;
+    constexpr int K = NR > 0 ? NR : 1;
+    const uint32_t S = t.cfg.max_contacts, n = NR > 0 ? t.ndof : 0u, L = NR > 0 ? t.L : 0u, lane = e.lane;
     const float dt = t.cfg.dt;
     const bool position_pass = t.cfg.pos_iters > 0u;
     uint32_t nheads = 0u, npoints = 0u;
@@ -122,11 +123,11 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
     __syncwarp();
     // chain Jacobians of articulated sides, lane = coordinate (ops/articulation_types.cuh:193-238)
     if (n != 0u && ncontact != 0u) {
-        V3 axis_w[NR], origin[NR];
-        uint32_t jt[NR];
-        bool dof[NR];
+        V3 axis_w[K], origin[K];
+        uint32_t jt[K];
+        bool dof[K];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
+        for (int r = 0; r < K; ++r) {
             axis_w[r] = mk3(0.f, 0.f, 0.f); origin[r] = axis_w[r];
             jt[r] = kFixed;
             dof[r] = lane + 32u * r < n;
@@ -159,7 +160,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             const V3 point = ld3(sm_cpoint(e, ref & 0xffffu));
             const V3 dirs[3] = {hf3(e, HF_N, h), hf3(e, HF_T1, h), hf3(e, HF_T2, h)};
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
+            for (int r = 0; r < K; ++r) {
                 const uint32_t c = lane + 32u * r;
                 if (dof[r]) {
                     // the side signs of this coordinate: it moves side a's link, side b's, both (no relative motion) or neither

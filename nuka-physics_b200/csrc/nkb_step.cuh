@@ -150,7 +150,7 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 
 // Register cap: measured on the 4096-env quadruped, the kernel runs fastest with about 150 registers and 12 warps per
 // SM; tighter caps (144 or 128 registers, 14 warps per SM) slow every warp by more than the extra residency returns.
-// NR = coordinates per lane: 1 for articulations of up to 32 coordinates, 2 for up to 64.
+// NR = coordinates per lane: 1 for articulations of up to 32 coordinates, 2 for up to 64, 0 for worlds without one.
 // kRigid = the world has free rigid bodies; without them the rigid-block solver code is compiled out.
 // Worlds with free bodies are held to fewer resident warps by shared memory than by registers (38 KB per env and more),
 // so their variants take a wider cap: no spills, and a team of 8 warps still fits the register file.
@@ -163,6 +163,11 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 // The slim build of the same kernel: at 128 registers a fourth warp fits each scheduler partition, so small envs (15 KB
 // of shared memory) reach 15 resident warps per SM instead of 12 and 4096 envs need two rounds instead of 2.3.  It
 // spills about 200 bytes; a world takes it only where the extra residency is really there (World::BuildLayout).
+// Worlds of bodies only run in teams of up to 8 warps, two piles to an SM: 128 registers for 16 warps, with 400 bytes of spills
+// (1024 piles of 48 boxes, 2 steps: 20.5 ms; 168 registers and teams of 6, 21.0; one pile to an SM, no spills, 26.6).
+#ifndef NKB_MAXNREG_BODIES
+#define NKB_MAXNREG_BODIES 128
+#endif
 #ifndef NKB_MAXNREG_SLIM
 #define NKB_MAXNREG_SLIM 128
 #endif
@@ -254,7 +259,8 @@ NKB_DEV void image_move(Env& e, const StepParams& p, float* img, uint32_t nheads
 template <int NR, bool kRigid, bool kControl, int kPart>
 NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t lane, Rally* rally) {
     const TemplateView& t = p.t;
-    const bool has_artic = t.L != 0u, has_bodies = t.B != 0u;
+    constexpr int K = NR > 0 ? NR : 1;
+    const bool has_artic = NR > 0 && t.L != 0u, has_bodies = t.B != 0u;
     const bool has_collidables = has_bodies && t.cfg.max_contacts != 0u;
     const bool use_pseudo = t.cfg.pos_iters != 0u && (t.cfg.max_contacts != 0u || t.L != 0u);
     Env e;
@@ -321,8 +327,8 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         }
         if (has_artic) {
             stage_drives(e);
-            float bias[NR];
-            stage_dynamics<NR>(e, E, r, bias);
+            float bias[K];
+            stage_dynamics<K>(e, E, r, bias);
             // Computed torque and operational-space control (pipeline.cpp:406-426) take the accelerations twice, force-free for
             // the controller and then under its feedforward effort; the mass matrix and the bias are the same.  The controllers
             // are compiled into the kControl builds of the kernel only (they would cost every other world registers).
@@ -330,8 +336,8 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             const int first = two_passes ? 0 : 1;
 #pragma unroll 1
             for (int pass = first; pass < 2; ++pass) {
-                stage_accelerations<NR>(e, bias, pass == first, pass == 1 && p.mode != kModeDynamicsOnly);
-                if constexpr (kControl) { if (pass == 0) stage_computed_torque<NR>(e); }
+                stage_accelerations<K>(e, bias, pass == first, pass == 1 && p.mode != kModeDynamicsOnly);
+                if constexpr (kControl) { if (pass == 0) stage_computed_torque<K>(e); }
             }
             tick(e, 2);
         }
@@ -400,7 +406,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
 
 // A helper warp's life: wait for a command, do its share (rigid blocks of a colour, or a slice of
 // a stage's outer loop), answer, until told to leave (or until a wait runs out).
-template <bool kRigid>
+template <int NR>
 NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const TemplateView& t, const StateView& state, uint32_t env,
                          uint32_t member, uint32_t lane, uint32_t vstride) {
     const TeamCommand* cmd = team_command(sm, shared_layout);
@@ -438,7 +444,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
 #ifdef NKB_STAGE_TAPS
             const long long tap0 = clock64();
 #endif
-            r = descend_bodies(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
+            r = descend_share<NR>(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
 #ifdef NKB_STAGE_TAPS
             if (state.dbg_cycles != nullptr && lane == 0u && member == 1u) {
                 uint32_t* cyc = state.dbg_cycles + (size_t)env * 32u;
@@ -467,7 +473,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
 // Block layout: blockDim.x / 32 warps, `team` consecutive warps per env (one unless the world runs in team mode); an
 // env's shared-memory slice is shared by its team.
 template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
-__global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SLIM : NKB_MAXNREG)) step_kernel(const __grid_constant__ StepParams p) {
+__global__ void __maxnreg__(NR == 0 ? NKB_MAXNREG_BODIES : kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SLIM : NKB_MAXNREG)) step_kernel(const __grid_constant__ StepParams p) {
     extern __shared__ __align__(16) float smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t team = kRigid ? p.sm.team : 1u;
@@ -492,7 +498,7 @@ __global__ void __maxnreg__(kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SL
     if (env >= p.s.env_count) return;                       // the whole team leaves together
     if (p.sel_mask != nullptr && p.sel_mask[env] == 0u) return;
     if constexpr (kRigid) {
-        if (member != 0u) { team_helper<kRigid>(sm, p.sm, p.t, p.s, env, member, lane, 32u * NR); return; }
+        if (member != 0u) { team_helper<NR>(sm, p.sm, p.t, p.s, env, member, lane, 32u * (NR > 0 ? NR : 1)); return; }
     }
 #pragma unroll 1
     for (;;) {

@@ -134,6 +134,7 @@ struct SmemLayout {
     uint32_t mass, factor, vecs, vstride;                       // articulation (vstride: words per vector, 32 or 64)
     uint32_t bpose, bvel, bwinv, aabb, bmass, bfree, bpseudo;   // bodies
     uint32_t pairs, ccount, cpoint, cnormal, cdepth, cfeat;     // contacts
+    uint32_t contacts_far;                                      // contact points and normals live in their read-out arrays
     uint32_t cstage;                                            // cache rebuild staging (shares the Jacobian pool, dead by then)
     uint32_t heads, jpool, binfo, chol;                         // solver (chol: the articulation's Newton matrix)
     uint32_t factor_words;                                      // words of the mass matrix's factor

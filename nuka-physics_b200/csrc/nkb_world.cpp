@@ -378,8 +378,7 @@ void World::BuildLayout() {
     s.bwinv = take(6 * slots); s.bmass = take(7 * slots); s.bfree = take(6 * slots); s.bpseudo = take(6 * slots);
     tv.slot_cap = std::min<uint32_t>(S, (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size()));
     const uint32_t SC = tv.slot_cap;
-    s.pairs = take(SC); s.ccount = take(SC); s.cpoint = take(12 * SC); s.cnormal = take(12 * SC); s.cdepth = take(4 * SC);
-    s.cfeat = take(8 * SC);                       // contact identity words
+    s.pairs = take(SC); s.ccount = take(SC); s.cdepth = take(4 * SC); s.cfeat = take(8 * SC);                       // cfeat: contact identity words
     // before the heads exist the region serves the tree broadphase and then the narrowphase as scratch
     s.heads = take(std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kTeamMax : 1u)) : 0u));
     // the Jacobian pool also holds the AABBs (dead once the narrowphase is done) and, after the solve, the cache staging
@@ -389,19 +388,38 @@ void World::BuildLayout() {
     s.cstage = s.jpool; s.aabb = s.jpool;
     const uint32_t nb = B + (n ? 1u : 0u);
     s.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);      // the unit-row table holds 16-bit head indices
+    const uint32_t without_points = at;
+    s.cpoint = take(12 * SC); s.cnormal = take(12 * SC); s.contacts_far = 0u;      // last: a team's env may leave them out
     if (const char* pad = std::getenv("NUKA_B200_SMEM_PAD_WORDS")) at += (static_cast<uint32_t>(std::atoi(pad)) + 3u) & ~3u;   // occupancy experiments
     // Team mode.  An env of many free bodies fills most of an SM's shared memory by itself, so one warp per env would
     // leave the SM with one or two resident warps; instead several warps share the env and descend the rigid blocks
-    // of one colour side by side (blocks of a colour share no constraint row).  Registers allow about 11 resident
-    // warps per SM, so teams only pay where shared memory already holds residency below that.
+    // of one colour side by side (blocks of a colour share no constraint row).
     s.team = 1u; s.team_area = at; s.team_drill = 0u;
     if (const char* drill = std::getenv("NUKA_B200_TEAM_DRILL")) s.team_drill = static_cast<uint32_t>(std::atoi(drill)) & 3u;
     {
         auto area = [](uint32_t w) { return 12u + ((4u * w + 3u) & ~3u); };
         uint32_t team = 1u;
         if (t.n_free >= 8u) {
-            const uint32_t envs_alone = std::max<uint32_t>(1u, (227u * 1024u) / (at * 4u + 1024u));      // resident envs, one warp each
-            while (team * 2u <= kTeamMax && envs_alone * team * 2u <= 11u && (at + area(team * 2u)) * 4u <= 220u * 1024u) team *= 2u;
+            // The team size that serves an SM best: envs resident at once (by shared memory, and by the registers that the team's
+            // warps need) times what a team of that size makes of one env.  The lead's share of a step does not shrink: a pile of
+            // 48 boxes takes 1, 1/1.6, 1/2.6 and 1/3.8 of the time with 1, 2, 4 and 8 warps.
+            const uint32_t warps = 65536u / (32u * std::max(1u, static_cast<uint32_t>(step_kernel_registers(tv, false))));
+            auto serve = [&](uint32_t words, uint32_t& size) {
+                double top = 0.0;
+                for (uint32_t w = 1u; w <= kTeamMax; ++w) {
+                    const uint32_t envs = std::min((228u * 1024u) / ((words + area(w)) * 4u + 1024u), warps / w);
+                    const double rate = envs / (0.14 + 0.86 / w);
+                    if (rate > top) { top = rate; size = w; }
+                }
+                return top;
+            };
+            // The points and normals of contacts, a fifth of a 48-box pile's slice, are touched a few times a step only.  Where
+            // leaving them in their read-out arrays lets another env in, they stay there (the pile: 113 kB, two envs to an SM).
+            uint32_t near = 1u, far = 1u;
+            const double here = serve(at, near), there = serve(without_points, far);
+            team = near;
+            if (there > here && far > 1u && std::getenv("NUKA_B200_NEAR") == nullptr) { s.contacts_far = 1u; at = s.team_area = without_points; team = far; }
+            while (team > 1u && (at + area(team)) * 4u > 220u * 1024u) --team;
         }
         // Lanes per free body in a block descent.  A body alone on its env's one warp leaves most lanes idle: 8 lanes each,
         // four bodies at a time.  A team has warps for two bodies each (a colour of a 48-box pile holds about 13).  The choice
@@ -428,7 +446,7 @@ void World::BuildLayout() {
     for (int slim = 0; slim < (has_slim ? 2 : 1); ++slim)
         for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) {
             if ((w / team) * bytes > 227u * 1024u) break;
-            resident[slim][w] = static_cast<size_t>(step_kernel_resident_blocks(n, t.n_free, slim != 0, control, w, (w / team) * bytes)) * w;      // asks the runtime
+            resident[slim][w] = static_cast<size_t>(step_kernel_resident_blocks(tv, slim != 0, w, (w / team) * bytes)) * w;      // asks the runtime
             best[slim] = std::max(best[slim], resident[slim][w]);
         }
     // The slim build pays about 200 bytes of spills for a fourth warp per scheduler partition: worth it where shared
@@ -445,7 +463,8 @@ void World::BuildLayout() {
     // for the cache and the warps go their own ways (4096 arms, 32 steps: 3.30 ms apart, 3.49 together); where an SM holds four
     // warps or fewer, fetches are no bottleneck either.
     warps_per_block_ = team;
-    for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) if (fits[w] == most) warps_per_block_ = w;
+    // A block holds one team (two piles in a block: 2 % slower, the first to finish waits for the other's slice).
+    for (uint32_t w = team; w <= (team > 1u ? team : kWarpsPerBlockMax); w += team) if (fits[w] == most) warps_per_block_ = w;
     group_ = 0u; grid_ = 0u;
     int sms = 148;
     Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
@@ -499,7 +518,7 @@ void World::BuildLayout() {
         if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %d registers, %u warps per block; solve %u B, %d registers, %d resident\n", stages_->registers(), stages_warps_,
                                              solve_sm_.words * 4u, solve_->registers(), solve_->resident_blocks(1, solve_sm_.words * 4u));
         std::fprintf(stderr, "[nuka_b200] %zu B of shared memory per env, %d registers per thread%s; resident warps per SM by block size:", bytes,
-                     step_kernel_registers(n, t.n_free, slim_, control), slim_ ? " (slim build)" : "");
+                     step_kernel_registers(tv, slim_), slim_ ? " (slim build)" : "");
         for (uint32_t w = 1; w <= kWarpsPerBlockMax; ++w) std::fprintf(stderr, " %u:%zu", w, fits[w]);
         std::fprintf(stderr, " -> %u warps per block, %u per env\n", warps_per_block_, team);
         std::fprintf(stderr, "[nuka_b200] word offsets: overlay %u mass %u vecs %u bodies %u contacts %u heads %u pool %u blocks %u end %u\n",
@@ -514,7 +533,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         const HostTemplate& t = tpl_;
         TemplateView& v = params_.t;
         v.L = t.L; v.B = t.B; v.ndof = t.ndof; v.max_depth = t.max_depth; v.floating_root = t.floating_root;
-        v.n_excluded = static_cast<uint32_t>(t.excluded.size());
+        v.n_excluded = static_cast<uint32_t>(t.excluded.size()); v.n_free = t.n_free;
         v.cfg = t.cfg;
         BuildLayout();
         v.parent = Upload(t.parent); v.jtype = Upload(t.jtype); v.depth = Upload(t.depth); v.child_begin = Upload(t.child_begin);
@@ -532,7 +551,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.inertial_quat = Upload(t.inertial_quat); v.excluded = Upload(t.excluded);
         v.adm_pairs = Upload(t.adm_pairs);
         v.adm_mask = Upload(t.adm_mask);
-        v.free_slot = Upload(t.free_slot); v.n_free = t.n_free;
+        v.free_slot = Upload(t.free_slot);
         v.n_adm = (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size());
         SetBroadphase(0u);
         if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
