@@ -16,9 +16,15 @@ NKB_DEV float* sm_bwinv(const Env& e, uint32_t b) { return e.sm + e.lay->bwinv +
 NKB_DEV float* sm_aabb(const Env& e, uint32_t b) { return e.sm + e.lay->aabb + 6u * b; }
 NKB_DEV uint32_t* sm_pairs(const Env& e) { return reinterpret_cast<uint32_t*>(e.sm + e.lay->pairs); }
 NKB_DEV uint32_t* sm_ccount(const Env& e) { return reinterpret_cast<uint32_t*>(e.sm + e.lay->ccount); }
-// Contact points and normals: in the slice, or in global memory where their read-out arrays are (see World::BuildLayout).
-NKB_DEV float* contact_points(const Env& e) { return e.lay->contacts_far != 0u ? e.s->contact_point + (size_t)e.env * e.t->cfg.max_contacts * 12u : e.sm + e.lay->cpoint; }
-NKB_DEV float* contact_normals(const Env& e) { return e.lay->contacts_far != 0u ? e.s->contact_normal + (size_t)e.env * e.t->cfg.max_contacts * 12u : e.sm + e.lay->cnormal; }
+// Contact points and normals: in the slice, or in global memory where their read-out arrays are (see World::BuildLayout).  Only
+// kernels that run in teams know the second place (the choice costs a kernel without contacts 2 %, by its registers).
+#ifdef NKB_TEAM_BUILD
+NKB_DEV bool contacts_far(const Env& e) { return e.lay->contacts_far != 0u; }
+#else
+NKB_DEV bool contacts_far(const Env&) { return false; }
+#endif
+NKB_DEV float* contact_points(const Env& e) { return contacts_far(e) ? e.s->contact_point + (size_t)e.env * e.t->cfg.max_contacts * 12u : e.sm + e.lay->cpoint; }
+NKB_DEV float* contact_normals(const Env& e) { return contacts_far(e) ? e.s->contact_normal + (size_t)e.env * e.t->cfg.max_contacts * 12u : e.sm + e.lay->cnormal; }
 NKB_DEV float* sm_cpoint(const Env& e, uint32_t pt) { return contact_points(e) + 3u * pt; }
 NKB_DEV float* sm_cnormal(const Env& e, uint32_t pt) { return contact_normals(e) + 3u * pt; }
 NKB_DEV float* sm_cdepth(const Env& e) { return e.sm + e.lay->cdepth; }
@@ -178,7 +184,7 @@ NKB_DEV void stage_store_contacts(Env& e, uint32_t pair_count) {
             const bool live = i < n;
             const uint32_t at = s * 4u + i;
             const V3 p = live ? ld3(sm_cpoint(e, at)) : mk3(0.f, 0.f, 0.f), nn = live ? ld3(sm_cnormal(e, at)) : mk3(0.f, 0.f, 0.f);
-            if (!live || e.lay->contacts_far == 0u) {
+            if (!live || !contacts_far(e)) {
                 st3(e.s->contact_point + (gs * 4u + i) * 3u, p);
                 st3(e.s->contact_normal + (gs * 4u + i) * 3u, nn);
             }

@@ -29,13 +29,17 @@ struct PairCtx {
     const TemplateView* t;
     uint32_t lane;
     float separation;
+#ifdef NKB_TEAM_BUILD
     float *points, *normals;
+#endif
     uint32_t stage_shift;       // words from the first warp's polygon staging areas to this warp's (team mode)
 };
 NKB_DEV PairCtx pair_ctx(const Env& e, float separation) {
     PairCtx c;
     c.sm = e.sm; c.lay = e.lay; c.t = e.t; c.lane = e.lane; c.separation = separation; c.stage_shift = 0u;
+#ifdef NKB_TEAM_BUILD
     c.points = contact_points(e); c.normals = contact_normals(e);
+#endif
     return c;
 }
 NKB_DEV float* ctx_frames(const PairCtx& c) { return c.sm + c.lay->heads; }                 // 12 B words
@@ -89,8 +93,13 @@ NKB_DEV unsigned long long side_token(uint32_t feature, const float* pose, V3 wo
 // the kernel (it is reached from every pair class).
 static __device__ __noinline__ void write_point(PairCtx c, uint32_t slot, uint32_t index, uint32_t a, uint32_t b, V3 pos, V3 normal, float pen, uint32_t key) {
     const uint32_t at = slot * 4u + index;
+#ifdef NKB_TEAM_BUILD
     st3(c.points + 3u * at, pos);
     st3(c.normals + 3u * at, normal);
+#else
+    st3(c.sm + c.lay->cpoint + 3u * at, pos);
+    st3(c.sm + c.lay->cnormal + 3u * at, normal);
+#endif
     c.sm[c.lay->cdepth + at] = pen + c.separation;
     const uint32_t feature = key == 0u ? 0xffffffffu : key;
     unsigned long long h = 1469598103934665603ull;

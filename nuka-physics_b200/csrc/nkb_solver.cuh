@@ -1386,16 +1386,21 @@ NKB_DEV void body_block_share(V3 n, V3 m, V3 p, V3 q, float (&share)[32]) {
 // Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: `32 / body_lanes` blocks at a
 // time, warp `first` of `stride`.  Same model, stopping rules and exact line search as descend_block; the sums that one
 // compensates in float run in double, the inertial force is carried as in descend_tree.
+// The 6 x 6 systems are assembled in one of two ways.  Summing heads per lane and dealing the sums out is the shorter chain (48-box
+// piles, 1024 envs: 28.7 to 26.9 ms; 1371 quadrupeds with 4 boxes: 3.53 to 3.41; 2 of them: 1.40 to 1.30); a row per lane is less
+// code, which counts where many warps run a solve apart from one another and wait for instructions (kRows, the solve of split
+// steps; 4096 quadrupeds with 4 boxes: 7.13 against 7.39).
 // What bounds it is the length of the chain of one block (assembly, factorisation, line search).  One block per warp with six
 // busy lanes and its matrix in shared memory took about 16 k cycles per block; see the team and box figures at World::BuildLayout.
 // Inlined for the lead and for its helpers (out of line it spilled the callers' registers and ran 5 % slower), so every fused
 // multiply-add is written as one: left to the compiler, the two copies contracted some products differently, and a block's
 // result depended on who ran it.
+template <bool kRows>
 NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     Env e = bare_env(run.sm, run.lay, run.t, nullptr, 0u, run.lane, run.vstride);
     const TemplateView& t = *e.t;
     const BodyLanes g = body_lanes(e);
-    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u;
+    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
     const uint32_t* order = block_order(e, nb);
     float most_moved = 0.f, worst = 0.f;
     bool failed = false;
@@ -1543,10 +1548,67 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             if (!__any_sync(NKB_FULL, active)) break;
             step = step < 0 ? 0 : step + 1;
             __syncwarp();
-            // the next Newton system.  A lane takes the heads j, j + width, ...: its share of H (lower triangle), of the force
-            // balance and of the rounding scale; the lanes then add their shares
+            // the next Newton system: the lower triangle of H, this lane's entry of the force balance and its rounding scale
             float a[28], own, scale;
-            {
+            if constexpr (kRows) {
+                // a lane builds one row, walking all of the body's heads (lanes 8..15 of 16 take the odd ones)
+                float hr[6];
+                scale = 0.f;
+                double gsum = 0.0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) hr[k] = 0.f;
+                if (part == 0u && row < 6u) {
+                    if (row < 3u) { hr[0] = row == 0u ? mass.m : 0.f; hr[1] = row == 1u ? mass.m : 0.f; hr[2] = row == 2u ? mass.m : 0.f; }
+                    else {
+                        hr[3] = row == 3u ? mass.i[0] : row == 4u ? mass.i[3] : mass.i[4];
+                        hr[4] = row == 3u ? mass.i[3] : row == 4u ? mass.i[1] : mass.i[5];
+                        hr[5] = row == 3u ? mass.i[4] : row == 4u ? mass.i[5] : mass.i[2];
+                    }
+                    gsum = -pick6(inertial, row);
+                    scale = fabsf((float)gsum);
+                }
+                if (active)
+#pragma unroll 1
+                    for (uint32_t k = part; k < count; k += parts) {
+                        const uint32_t h = inc[k];
+                        const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                        const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), w = body_row_axis(row, arm);
+                        const float4 f = hq(e, HF_F, h);
+                        const float j0 = dot_fma(n, w), sgn = first_side ? 1.f : -1.f;
+                        V3 a;
+                        if (position) {                                    // push-out rows have a normal axis only
+                            gsum = fma((double)(sgn * j0), (double)f.x, gsum);
+                            scale = fmaf(fabsf(j0), hf(e, HF_NZ, h), scale);
+                            a = n * (j0 * f.w);
+                        } else {
+                            const float4 c = hq(e, HF_C + 1u, h);
+                            const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
+                            const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h);
+                            const float j1 = dot_fma(t1, w), j2 = dot_fma(t2, w);
+                            gsum = fma((double)(sgn * j0), (double)f.x, gsum); gsum = fma((double)(sgn * j1), (double)f.y, gsum); gsum = fma((double)(sgn * j2), (double)f.z, gsum);
+                            scale = fmaf(fabsf(j0), c.w, fmaf(fabsf(j1), nz.x, fmaf(fabsf(j2), nz.y, scale)));
+                            const float p0 = j0 * f.w, p1 = fmaf(j1, c.x, j2 * c.z), p2 = fmaf(j2, c.y, j1 * c.z);
+                            a = mk3(fmaf(n.x, p0, fmaf(t1.x, p1, t2.x * p2)), fmaf(n.y, p0, fmaf(t1.y, p1, t2.y * p2)), fmaf(n.z, p0, fmaf(t1.z, p1, t2.z * p2)));
+                        }
+                        const V3 m = cross_fma(arm, a);
+                        hr[0] = __fadd_rn(hr[0], a.x); hr[1] = __fadd_rn(hr[1], a.y); hr[2] = __fadd_rn(hr[2], a.z); hr[3] = __fadd_rn(hr[3], m.x); hr[4] = __fadd_rn(hr[4], m.y); hr[5] = __fadd_rn(hr[5], m.z);
+                    }
+                __syncwarp();
+                if (parts > 1u) {
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) hr[k] += __shfl_xor_sync(NKB_FULL, hr[k], 8);
+                    gsum += __shfl_xor_sync(NKB_FULL, gsum, 8); scale += __shfl_xor_sync(NKB_FULL, scale, 8);
+                }
+#pragma unroll
+                for (int k = 0; k < 6; ++k) scale = fmaf(fabsf(hr[k]), fabsf((float)u[k]), scale);
+                own = (float)gsum;
+                // the group's rows to every lane of it
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+#pragma unroll
+                    for (int k = 0; k <= i; ++k) a[i * (i + 1) / 2 + k] = __shfl_sync(NKB_FULL, hr[k], g.first + i);
+            } else {
+                // a lane takes the heads j, j + width, ... and sums its share of everything; the lanes then add their shares
                 float share[32];
                 double balance[8];
 #pragma unroll
@@ -1647,12 +1709,12 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
 static __device__ __noinline__ RigidResult descend_bodies_call(float* sm, const SmemLayout* lay, const TemplateView* t, uint32_t lane, uint32_t vstride, uint32_t nheads, uint32_t nblocks,
                                                                uint32_t iteration, float tol, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     const RigidRun run = {sm, lay, t, lane, vstride, nheads, nblocks, iteration, tol};        // a struct argument would go through memory
-    return descend_bodies(run, k_begin, k_end, first, stride, position);
+    return descend_bodies<false>(run, k_begin, k_end, first, stride, position);
 }
-template <int NR>
+template <int NR, bool kRows>
 NKB_DEV RigidResult descend_share(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     if constexpr (NR == 0) return descend_bodies_call(run.sm, run.lay, run.t, run.lane, run.vstride, run.nheads, run.nblocks, run.iteration, run.tol, k_begin, k_end, first, stride, position);
-    else return descend_bodies(run, k_begin, k_end, first, stride, position);
+    else return descend_bodies<kRows>(run, k_begin, k_end, first, stride, position);
 }
 
 // Lead warp: releases the helpers for good (they need not answer).
@@ -1696,7 +1758,7 @@ NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
 }
 
 // Blocks descend colour by colour, blocks of one colour in index order (block_descent_tile.cuh:2749-2820).
-template <int NR, bool kRigid>
+template <int NR, bool kRigid, bool kRows>
 NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
     const uint32_t nb = tile.nblocks;
     const uint32_t* order = block_order(e, nb);
@@ -1736,7 +1798,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
             // helper failed to answer, and take the helpers' shares
 #pragma unroll 1
             do {
-                const RigidResult part = descend_share<NR>(run, k, k_end, share, stride, position);
+                const RigidResult part = descend_share<NR, kRows>(run, k, k_end, share, stride, position);
                 mine.momentum = fmaxf(mine.momentum, part.momentum); mine.residual = fmaxf(mine.residual, part.residual);
                 mine.status |= part.status;
                 if (shared_out && share == 0u) {
@@ -1977,7 +2039,7 @@ NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
 
 // The whole constraint solve of one env.  On entry the heads are built, the articulation's post-dynamics
 // velocity is in (e.qd, sm_vel(root)) and free-body velocities are in sm_bvel.
-template <int NR, bool kRigid>
+template <int NR, bool kRigid, bool kRows>
 NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, B = t.B, n = NR > 0 ? t.ndof : 0u;
@@ -2129,7 +2191,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         }
         if (phase == kPhaseVelocity) { tile.iteration = sweeps++; tile.momentum = 0.f; tile.residual = 0.f; }
         else tile.iteration = sweeps + pushes;
-        descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
+        descend_blocks<NR, kRigid, kRows>(e, tile, phase == kPhasePosition);
         if (phase == kPhasePosition) {
             if (++pushes >= positions) { phase = kPhaseDone; continue; }
         } else tick(e, 10);

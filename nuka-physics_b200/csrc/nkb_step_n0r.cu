@@ -1,4 +1,5 @@
 // step_kernel<0, true>: free rigid bodies, no articulation.
+#define NKB_TEAM_BUILD
 #include "nkb_step.cuh"
 
 namespace nkb {

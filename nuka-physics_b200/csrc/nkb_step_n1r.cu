@@ -1,4 +1,5 @@
 // step_kernel<1, true>: one coordinate per lane, with free rigid bodies.
+#define NKB_TEAM_BUILD
 #include "nkb_step.cuh"
 
 namespace nkb {

@@ -1,5 +1,6 @@
 // step_kernel<1, true, false, control>: one coordinate per lane, with free rigid bodies, with the computed-torque and
 // operational-space controllers between two dynamics passes (control modes 3 and 4).
+#define NKB_TEAM_BUILD
 #include "nkb_step.cuh"
 
 namespace nkb {

@@ -488,8 +488,8 @@ void World::BuildLayout() {
     // split; 3000: 2.91 and 2.26; 1200 quadrupeds with 4 boxes: 3.08 and 3.28; 2400: 4.65 and 4.35; 1000 humanoids: 6.69 and
     // 6.99; 2048: 9.50 and 8.61).
     stages_ = solve_ = nullptr;
-    bool split = team == 1u && n != 0u && SC != 0u && share > 12u && env_count_ > static_cast<uint32_t>(sms) * most;
-    if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && n != 0u && SC != 0u && std::atoi(forced) != 0;
+    bool split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && share > 12u && env_count_ > static_cast<uint32_t>(sms) * most;
+    if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && std::atoi(forced) != 0;
     if (split) {
         stages_ = split_variant(n, t.n_free, control, kPartStages); solve_ = split_variant(n, t.n_free, control, kPartSolve);
     }
@@ -877,7 +877,14 @@ void World::SetContactReadout(bool on) {
     if (on == (s.pair_count != nullptr)) return;
     if (on) { s.pair_count = readout_.pair_count; s.pairs = readout_.pairs; s.contact_count = readout_.contact_count;
               s.contact_point = readout_.contact_point; s.contact_normal = readout_.contact_normal; s.contact_depth = readout_.contact_depth; }
-    else { readout_ = s; s.pair_count = nullptr; }
+    else {
+        readout_ = s; s.pair_count = nullptr;
+        if (params_.sm.contacts_far != 0u) {           // the steps still need the place
+            const size_t words = static_cast<size_t>(env_count_) * params_.t.cfg.max_contacts * 12u;
+            if (far_point_ == nullptr) { far_point_ = Alloc<float>(words); far_normal_ = Alloc<float>(words); }
+            s.contact_point = far_point_; s.contact_normal = far_normal_;
+        }
+    }
     graph_valid_ = false;
 }
 
@@ -927,8 +934,8 @@ bool World::Field(uint32_t id, FieldInfo* out) {
         case 0x10002: return set(s.pair_count != nullptr ? s.pair_count : readout_.pair_count, 1, 1, false);
         case 0x10003: return set(s.pairs, S * 2, 1, false);
         case 0x10004: return set(s.contact_count, S, 1, false);
-        case 0x10005: return set(s.contact_point, S * 12, 0, false);
-        case 0x10006: return set(s.contact_normal, S * 12, 0, false);
+        case 0x10005: return set(s.pair_count != nullptr ? s.contact_point : readout_.contact_point, S * 12, 0, false);
+        case 0x10006: return set(s.pair_count != nullptr ? s.contact_normal : readout_.contact_normal, S * 12, 0, false);
         case 0x10007: return set(s.contact_depth, S * 4, 0, false);
         case 0x10008: return set(s.solver_sweeps, 1, 1, false);
         case 0x10009:

@@ -106,6 +106,7 @@ private:
     uint32_t env_count_;
     StepParams params_{};
     StateView readout_{};               // contact read-out pointers while the read-out is switched off
+    float *far_point_ = nullptr, *far_normal_ = nullptr;      // meanwhile, where contacts_far keeps its points and normals
     uint32_t warps_per_block_ = 1;
     uint32_t group_ = 0, grid_ = 0;            // step launches: see StepParams
     uint32_t* queue_ = nullptr;
