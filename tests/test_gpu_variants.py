@@ -1,0 +1,131 @@
+"""One env's step in the shapes a launch can take: one kernel or split around the solve, persistent blocks whose warps take the
+next env, contact points in the slice or in their read-out arrays.  Who runs a step and where its data waits changes no result,
+so the comparisons are bit-exact unless the line says why not."""
+import contextlib
+import os
+
+import numpy as np
+import pytest
+
+import nuka
+from nuka import Field as F, templates as T
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def layout(**forced):
+    """Layout choices forced through the environment; read while a world is created."""
+    before = {k: os.environ.get("NUKA_B200_" + k) for k in forced}
+    os.environ.update({"NUKA_B200_" + k: str(v) for k, v in forced.items()})
+    try:
+        yield
+    finally:
+        for k, v in before.items():
+            os.environ.pop("NUKA_B200_" + k) if v is None else os.environ.update({"NUKA_B200_" + k: v})
+
+
+def create(device, tb, state, E, **forced):
+    with layout(**forced):
+        w = nuka.World.create_from_template(device, tb.blob(), E)
+    names = {"q": F.JOINT_POSITION, "base_pose": F.BASE_POSE, "body_pose": F.RIGID_BODY_TRANSFORM}
+    for k, v in state.items():
+        w.upload(names[k], v[:E])
+    w.forward_kinematics()
+    return w
+
+
+def outputs(w, steps, graph=False):
+    w.set_execution_mode(graph)
+    for n in steps:
+        w.step_n(n)
+    fields = [F.RIGID_BODY_TRANSFORM, F.BODY_LINEAR_VELOCITY, F.ENV_STATUS, F.SOLVER_SWEEPS, F.SOLVER_RESIDUAL, F.CONTACT_COUNT, F.CONTACT_POINT, F.CONTACT_NORMAL]
+    if w.info.links_per_env:
+        fields += [F.JOINT_POSITION, F.JOINT_VELOCITY, F.BASE_POSE, F.LINK_VELOCITY, F.ACTUATOR_EFFORT]
+    out = {f.name: w.download(f) for f in fields}
+    w.destroy()
+    return out
+
+
+def assert_same(a, b, envs=slice(None)):
+    for k in a:
+        assert np.array_equal(a[k][envs], b[k][envs]), k
+
+
+# fewer envs than one part of a split step, one more than an SM's worth, a part that is not full; one step to a call and several
+@pytest.mark.parametrize("name,E,steps,graph", [("quadruped", 1, (1, 2), False), ("quadruped", 149, (30,), False), ("quadruped", 601, (25, 1), True),
+                                                ("humanoid", 7, (20,), False)])
+def test_split_steps_equal_whole_ones(device, name, E, steps, graph):
+    tb, st = getattr(T, name)(0), getattr(T, name + "_state")(E, 2)
+    whole = outputs(create(device, tb, st, E, SPLIT=0), steps)
+    split = outputs(create(device, tb, st, E, SPLIT=1), steps, graph)
+    assert whole["CONTACT_COUNT"].sum() > 0 or sum(steps) < 10
+    assert_same(whole, split)
+
+
+@pytest.mark.parametrize("E", [5, 150])
+def test_split_steps_with_free_boxes(device, E):
+    """Body systems are summed in another order in split steps.  Both forms are held to 1e-4 of the oracle over 30 steps of this
+    scene, so they are within 2e-4 of one another; counts are whole numbers."""
+    tb, st = T.quadruped(0, boxes=4), T.quadruped_state(E, 4)
+    whole = outputs(create(device, tb, st, E, SPLIT=0), (30,))
+    split = outputs(create(device, tb, st, E, SPLIT=1), (30,))
+    assert np.array_equal(whole["CONTACT_COUNT"], split["CONTACT_COUNT"]) and not split["ENV_STATUS"].any()
+    for k in ("JOINT_POSITION", "BASE_POSE", "RIGID_BODY_TRANSFORM"):
+        assert np.abs(whole[k] - split[k]).max() <= 2e-4 * max(1.0, np.abs(whole[k]).max()), k
+
+
+@pytest.mark.parametrize("E", [149, 1500, 4100])
+def test_an_env_does_not_depend_on_its_batch(device, E):
+    """Block shapes, meetings, the queue of a persistent launch and split steps follow the batch size."""
+    tb, st = T.quadruped(0), T.quadruped_state(E, 3)
+    few = {k: np.concatenate([v[:3], v[-3:]]) for k, v in st.items()}
+    a = outputs(create(device, tb, few, 6), (20, 3))
+    b = outputs(create(device, tb, st, E), (20, 3))
+    assert_same(a, {k: np.concatenate([v[:3], v[-3:]]) for k, v in b.items()})
+
+
+@pytest.mark.parametrize("count,team", [(48, 8), (48, 1), (40, 3)])
+def test_contact_points_in_their_read_out_arrays(device, count, team):
+    """A pile's contact points and normals stay in global memory where that makes room for another env."""
+    E = 3
+    tb, st = T.box_pile(0, count=count), T.box_pile_state(E, 0, count=count)
+    near = outputs(create(device, tb, st, E, NEAR=1, TEAM=team), (25,))
+    far = outputs(create(device, tb, st, E, TEAM=team), (25,))
+    assert near["CONTACT_COUNT"].sum() > count
+    assert_same(near, far)
+
+
+def test_read_out_keeps_its_last_values_while_off(device):
+    """The steps then keep their contact points elsewhere: the arrays stay as they were, and the states do not change."""
+    E = 2
+    tb, st = T.box_pile(0, count=48), T.box_pile_state(E, 0, count=48)
+    on = outputs(create(device, tb, st, E), (20, 5))
+    w = create(device, tb, st, E)
+    w.step_n(20)
+    before = w.download(F.CONTACT_POINT)
+    w.set_contact_readout(False)
+    w.step_n(5)
+    assert np.array_equal(w.download(F.CONTACT_POINT), before)
+    assert np.array_equal(w.download(F.RIGID_BODY_TRANSFORM), on["RIGID_BODY_TRANSFORM"])
+    w.set_contact_readout(True)
+    w.step_n(1)
+    assert not np.array_equal(w.download(F.CONTACT_POINT), before)
+    w.destroy()
+
+
+def test_downloads_outlive_the_world_and_one_another(device):
+    E = 64
+    w = create(device, T.quadruped(0), T.quadruped_state(E, 1), E)
+    first = w.download(F.JOINT_POSITION)
+    kept = first.copy()
+    w.step_n(3)
+    second = w.download(F.JOINT_POSITION)
+    assert np.array_equal(first, kept) and not np.array_equal(first, second)
+    kept2 = second.copy()
+    w.destroy()
+    v = create(device, T.quadruped(0), T.quadruped_state(E, 5), E)
+    again = [v.download(F.JOINT_POSITION) for _ in range(4)]
+    assert np.array_equal(first, kept) and np.array_equal(second, kept2)
+    assert all(np.array_equal(again[0], a) for a in again)
+    v.destroy()
