@@ -20,12 +20,16 @@ __global__ void reset_kernel(ResetParams r) {
     }
 }
 
-extern const StepVariant kStepBodies, kStepNarrow, kStepNarrowSlim, kStepNarrowRigid, kStepWide, kStepWideRigid;
+extern const StepVariant kStepBodies, kStepBare, kStepBareSlim, kStepBareControl, kStepNarrow, kStepNarrowSlim, kStepNarrowRigid, kStepWide, kStepWideRigid;
 extern const StepVariant kStepNarrowControl, kStepNarrowRigidControl, kStepWideControl, kStepWideRigidControl;
 
 extern const StepVariant kStagesNarrow, kSolveNarrow, kStagesNarrowRigid, kSolveNarrowRigid, kStagesWide, kSolveWide;
 
-bool step_kernel_has_slim(uint32_t ndof, uint32_t n_free, bool control) { return ndof <= 32u && n_free == 0u && !control; }
+bool step_kernel_has_slim(const TemplateView& t) {
+    return t.ndof <= 32u && t.n_free == 0u && t.cfg.control_mode != 3u && t.cfg.control_mode != 4u;
+}
+
+static bool has_contacts(const TemplateView& t) { return t.B != 0u && t.cfg.max_contacts != 0u; }
 
 // no articulation, up to 32 or up to 64 coordinates per articulation; with or without free rigid bodies; the slim
 // (128-register) build exists for articulations of up to 32 without bodies only
@@ -33,6 +37,7 @@ static const StepVariant& step_variant(const TemplateView& t, bool slim) {
     // control modes 3 and 4 run the builds that hold the controllers
     const bool control = t.cfg.control_mode == 3u || t.cfg.control_mode == 4u;
     if (t.L == 0u && t.n_free != 0u) return kStepBodies;
+    if (!has_contacts(t) && t.n_free == 0u && t.ndof <= 32u) return control ? kStepBareControl : slim ? kStepBareSlim : kStepBare;
     if (control) return t.ndof > 32u ? (t.n_free != 0u ? kStepWideRigidControl : kStepWideControl) : (t.n_free != 0u ? kStepNarrowRigidControl : kStepNarrowControl);
     if (t.ndof > 32u) return t.n_free != 0u ? kStepWideRigid : kStepWide;
     if (t.n_free != 0u) return kStepNarrowRigid;

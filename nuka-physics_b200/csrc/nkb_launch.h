@@ -29,7 +29,7 @@ struct ResetParams {
 // (up to 32 / up to 64 coordinates) and `n_free` (free dynamic bodies per env).
 int step_kernel_resident_blocks(const TemplateView& t, bool slim, uint32_t warps_per_block, size_t shared_bytes);
 // Whether a slim (128-register) build of the world's kernel variant exists.
-bool step_kernel_has_slim(uint32_t ndof, uint32_t n_free, bool control);
+bool step_kernel_has_slim(const TemplateView& t);
 // Registers per thread of the step kernel variant that serves the world.
 int step_kernel_registers(const TemplateView& t, bool slim);
 // Host-side handle of one compiled step-kernel variant.

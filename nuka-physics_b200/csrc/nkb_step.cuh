@@ -261,7 +261,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     const TemplateView& t = p.t;
     constexpr int K = NR > 0 ? NR : 1;
     const bool has_artic = NR > 0 && t.L != 0u, has_bodies = t.B != 0u;
-    const bool has_collidables = has_bodies && t.cfg.max_contacts != 0u;
+    const bool has_collidables = kPart != kPartBare && has_bodies && t.cfg.max_contacts != 0u;
     const bool use_pseudo = t.cfg.pos_iters != 0u && (t.cfg.max_contacts != 0u || t.L != 0u);
     Env e;
     env_begin<NR>(e, p, sm, env, lane);
@@ -270,7 +270,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
     float4* lanes = nullptr;
     uint32_t* tail = nullptr;
     bool resumed = kPart == kPartSolve;                 // the first trip starts behind the stages that lead to the solve
-    if constexpr (kPart != kPartWhole) {
+    if constexpr (kSplitPart<kPart>) {
         resumed = resumed || p.resume != 0u;
         img = p.image + (size_t)(env - p.image_first) * p.image_stride;
         lanes = reinterpret_cast<float4*>(img + p.image_stride - kImageLaneWords);
@@ -366,10 +366,10 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
         stay_together<kPart>();
-        nheads = stage_rows<NR>(e, pair_count);
+        nheads = stage_rows<NR, kPart != kPartBare>(e, pair_count);
         tick(e, 6);
         if constexpr (kRigid) team_fork(e, kTeamWarmStart, nheads, [&](uint32_t first, uint32_t stride) { warm_start_range(e, nheads, first, stride); });
-        else warm_start_range(e, nheads, 0u, 1u);
+        else if constexpr (kPart != kPartBare) warm_start_range(e, nheads, 0u, 1u);
         __syncwarp();
         tick(e, 7);
         if constexpr (kPart == kPartStages) {
@@ -389,7 +389,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
         resumed = false;
-        if constexpr (kPart == kPartWhole) { rally_wait(rally, p.group, lane); tick(e, 29); }
+        if constexpr (!kSplitPart<kPart>) { rally_wait(rally, p.group, lane); tick(e, 29); }
         if (has_collidables) {
             stage_cache_commit(e, nheads, [&](uint32_t ncontact) {
                 if constexpr (kRigid) team_fork(e, kTeamCacheOwners, ncontact, [&](uint32_t first, uint32_t stride) { cache_owners_range(e, ncontact, first, stride); });
@@ -479,7 +479,7 @@ __global__ void __maxnreg__(NR == 0 ? NKB_MAXNREG_BODIES : kRigid ? NKB_MAXNREG_
     const uint32_t team = kRigid ? p.sm.team : 1u;
     const uint32_t slot = warp / team, member = warp - slot * team;
     uint32_t env = blockIdx.x * ((blockDim.x >> 5) / team) + slot;
-    if constexpr (kPart != kPartWhole) env = p.first + env < p.end ? p.first + env : 0xffffffffu;
+    if constexpr (kSplitPart<kPart>) env = p.first + env < p.end ? p.first + env : 0xffffffffu;
     float* sm = smem + (size_t)slot * p.sm.words;
     if constexpr (kRigid) {
         // team mode: every lead zeroes its team's sequence numbers before any helper looks (a block-wide barrier, passed by
@@ -567,7 +567,7 @@ static cudaError_t variant_launch(const StepParams& p, uint32_t warps_per_block,
     const size_t bytes = (size_t)envs_per_block * p.sm.words * sizeof(float);
     const cudaError_t err = variant_reserve_shared<NR, kRigid, kSlim, kControl, kPart>(bytes);
     if (err != cudaSuccess) return err;
-    const uint32_t envs = kPart != kPartWhole ? p.end - p.first : p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
+    const uint32_t envs = kSplitPart<kPart> ? p.end - p.first : p.sel_ids != nullptr ? p.sel_count : p.s.env_count;
     if (envs == 0u) return cudaSuccess;
     const uint32_t needed = (envs + envs_per_block - 1u) / envs_per_block;
     const uint32_t blocks = p.queue != nullptr ? p.grid : needed;       // a persistent launch's grid is smaller than the batch

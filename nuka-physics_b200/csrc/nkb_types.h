@@ -149,8 +149,10 @@ struct SmemLayout {
     uint32_t ld;                                                // leading dimension of mass/factor (ndof | 1)
 };
 
-// A step in one launch, or split around its constraint solve: the straight-line stages of all envs, then the solves.
-enum StepPart : int { kPartWhole = 0, kPartStages = 1, kPartSolve = 2 };
+// A step in one launch, or split around its constraint solve: the straight-line stages of all envs, then the solves.  kPartBare is
+// a step in one launch of a world without contacts.
+enum StepPart : int { kPartWhole = 0, kPartStages = 1, kPartSolve = 2, kPartBare = 3 };
+template <int kPart> constexpr bool kSplitPart = kPart == kPartStages || kPart == kPartSolve;
 constexpr uint32_t kImageLaneWords = 4u * 32u + 4u;     // an image's tail: four words per lane, then status, heads, branching
 
 enum StepMode : uint32_t { kModeStep = 0, kModeDynamicsOnly = 1, kModeCollideOnly = 2, kModeRefresh = 3 };

@@ -382,9 +382,9 @@ void World::BuildLayout() {
     // before the heads exist the region serves the tree broadphase and then the narrowphase as scratch
     s.heads = take(std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kTeamMax : 1u)) : 0u));
     // the Jacobian pool also holds the AABBs (dead once the narrowphase is done) and, after the solve, the cache staging
-    // entries + owner marks
+    // entries, owner marks and retained bits
     const uint32_t stage_cap = std::min(tv.point_cap, 4u * SC);
-    s.jpool = take(std::max(std::max(tv.point_cap * 3u * ((n + 3u) & ~3u), stage_cap * 10u + 4u * SC), 6u * B));
+    s.jpool = take(std::max(std::max(tv.point_cap * 3u * ((n + 3u) & ~3u), stage_cap * 10u + 4u * SC + (4u * S + 31u) / 32u), 6u * B));
     s.cstage = s.jpool; s.aabb = s.jpool;
     const uint32_t nb = B + (n ? 1u : 0u);
     s.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);      // the unit-row table holds 16-bit head indices
@@ -442,17 +442,20 @@ void World::BuildLayout() {
     size_t resident[2][kWarpsPerBlockMax + 1] = {{0}, {0}};
     size_t best[2] = {0, 0};
     const bool control = t.cfg.control_mode == 3u || t.cfg.control_mode == 4u;       // these modes run the kernel builds that hold the controllers
-    const bool has_slim = step_kernel_has_slim(n, t.n_free, control);
+    const bool has_slim = step_kernel_has_slim(tv);
     for (int slim = 0; slim < (has_slim ? 2 : 1); ++slim)
         for (uint32_t w = team; w <= kWarpsPerBlockMax; w += team) {
             if ((w / team) * bytes > 227u * 1024u) break;
             resident[slim][w] = static_cast<size_t>(step_kernel_resident_blocks(tv, slim != 0, w, (w / team) * bytes)) * w;      // asks the runtime
             best[slim] = std::max(best[slim], resident[slim][w]);
         }
-    // The slim build pays about 200 bytes of spills for a fourth warp per scheduler partition: worth it where shared
-    // memory lets the extra warps in (measured on the 4096-env quadruped: 15 instead of 12 resident envs per SM, 0.445 ms
-    // per step instead of 0.508), not where shared memory caps residency first.
-    slim_ = has_slim && best[1] * 10u >= best[0] * 12u;
+    int sms = 148;
+    Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
+    const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
+    // The slim build pays 100 to 200 bytes of spills for a fourth warp per scheduler partition: worth it where shared memory lets
+    // the extra warps in and the batch needs them, more envs to an SM than the regular build keeps (4 steps of 1000 quadrupeds, 7 to
+    // an SM: 1.31 ms regular, 1.47 slim; 41 of 150 arms: 1.52 and 1.59; 32 of 4096 arms, 28 to an SM: 3.9 and 3.1).
+    slim_ = has_slim && share > best[0] && best[1] * 10u >= best[0] * 12u;
     if (const char* forced = std::getenv("NUKA_B200_SLIM")) slim_ = has_slim && std::atoi(forced) != 0;     // variant experiments and tests
     const size_t* fits = resident[slim_ ? 1 : 0];
     const size_t most = best[slim_ ? 1 : 0];
@@ -466,9 +469,6 @@ void World::BuildLayout() {
     // A block holds one team (two piles in a block: 2 % slower, the first to finish waits for the other's slice).
     for (uint32_t w = team; w <= (team > 1u ? team : kWarpsPerBlockMax); w += team) if (fits[w] == most) warps_per_block_ = w;
     group_ = 0u; grid_ = 0u;
-    int sms = 148;
-    Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
-    const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
     if (team == 1u) {
         if (most <= 4u) warps_per_block_ = 1u;
         else if (share >= most && SC == 0u && fits[4] == most) warps_per_block_ = 4u;      // no meetings: small blocks pack better (3.10 ms against 3.29)
