@@ -1386,21 +1386,20 @@ NKB_DEV void body_block_share(V3 n, V3 m, V3 p, V3 q, float (&share)[32]) {
 // Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: `32 / body_lanes` blocks at a
 // time, warp `first` of `stride`.  Same model, stopping rules and exact line search as descend_block; the sums that one
 // compensates in float run in double, the inertial force is carried as in descend_tree.
-// The 6 x 6 systems are assembled in one of two ways.  Summing heads per lane and dealing the sums out is the shorter chain (48-box
-// piles, 1024 envs: 28.7 to 26.9 ms; 1371 quadrupeds with 4 boxes: 3.53 to 3.41; 2 of them: 1.40 to 1.30); a row per lane is less
-// code, which counts where many warps run a solve apart from one another and wait for instructions (kRows, the solve of split
-// steps; 4096 quadrupeds with 4 boxes: 7.13 against 7.39).
+// The 6 x 6 systems are assembled by summing heads per lane and dealing the sums out, in every launch form: a sum's order decides
+// its last bits, and an env's state must not depend on the batch that it is in.  A row per lane that walks all heads of its body is
+// less code and a longer chain (48-box piles, 1024 envs: 28.7 ms, dealt out 26.9; policy steps of 150 quadrupeds with 6 boxes: 5.29
+// and 3.92; 2400 of them, in split steps: 7.72 and 6.70; 4096 with 4 boxes: 7.65 and 7.73).
 // What bounds it is the length of the chain of one block (assembly, factorisation, line search).  One block per warp with six
 // busy lanes and its matrix in shared memory took about 16 k cycles per block; see the team and box figures at World::BuildLayout.
 // Inlined for the lead and for its helpers (out of line it spilled the callers' registers and ran 5 % slower), so every fused
 // multiply-add is written as one: left to the compiler, the two copies contracted some products differently, and a block's
 // result depended on who ran it.
-template <bool kRows>
 NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     Env e = bare_env(run.sm, run.lay, run.t, nullptr, 0u, run.lane, run.vstride);
     const TemplateView& t = *e.t;
     const BodyLanes g = body_lanes(e);
-    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
+    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u;
     const uint32_t* order = block_order(e, nb);
     float most_moved = 0.f, worst = 0.f;
     bool failed = false;
@@ -1550,110 +1549,51 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             __syncwarp();
             // the next Newton system: the lower triangle of H, this lane's entry of the force balance and its rounding scale
             float a[28], own, scale;
-            if constexpr (kRows) {
-                // a lane builds one row, walking all of the body's heads (lanes 8..15 of 16 take the odd ones)
-                float hr[6];
-                scale = 0.f;
-                double gsum = 0.0;
+            // a lane takes the heads j, j + width, ... and sums its share of everything; the lanes then add their shares
+            float share[32];
+            double balance[8];
 #pragma unroll
-                for (int k = 0; k < 6; ++k) hr[k] = 0.f;
-                if (part == 0u && row < 6u) {
-                    if (row < 3u) { hr[0] = row == 0u ? mass.m : 0.f; hr[1] = row == 1u ? mass.m : 0.f; hr[2] = row == 2u ? mass.m : 0.f; }
-                    else {
-                        hr[3] = row == 3u ? mass.i[0] : row == 4u ? mass.i[3] : mass.i[4];
-                        hr[4] = row == 3u ? mass.i[3] : row == 4u ? mass.i[1] : mass.i[5];
-                        hr[5] = row == 3u ? mass.i[4] : row == 4u ? mass.i[5] : mass.i[2];
-                    }
-                    gsum = -pick6(inertial, row);
-                    scale = fabsf((float)gsum);
-                }
-                if (active)
+            for (int k = 0; k < 32; ++k) share[k] = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) balance[k] = 0.0;
+            if (active)
 #pragma unroll 1
-                    for (uint32_t k = part; k < count; k += parts) {
-                        const uint32_t h = inc[k];
-                        const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
-                        const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), w = body_row_axis(row, arm);
-                        const float4 f = hq(e, HF_F, h);
-                        const float j0 = dot_fma(n, w), sgn = first_side ? 1.f : -1.f;
-                        V3 a;
-                        if (position) {                                    // push-out rows have a normal axis only
-                            gsum = fma((double)(sgn * j0), (double)f.x, gsum);
-                            scale = fmaf(fabsf(j0), hf(e, HF_NZ, h), scale);
-                            a = n * (j0 * f.w);
-                        } else {
-                            const float4 c = hq(e, HF_C + 1u, h);
-                            const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
-                            const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h);
-                            const float j1 = dot_fma(t1, w), j2 = dot_fma(t2, w);
-                            gsum = fma((double)(sgn * j0), (double)f.x, gsum); gsum = fma((double)(sgn * j1), (double)f.y, gsum); gsum = fma((double)(sgn * j2), (double)f.z, gsum);
-                            scale = fmaf(fabsf(j0), c.w, fmaf(fabsf(j1), nz.x, fmaf(fabsf(j2), nz.y, scale)));
-                            const float p0 = j0 * f.w, p1 = fmaf(j1, c.x, j2 * c.z), p2 = fmaf(j2, c.y, j1 * c.z);
-                            a = mk3(fmaf(n.x, p0, fmaf(t1.x, p1, t2.x * p2)), fmaf(n.y, p0, fmaf(t1.y, p1, t2.y * p2)), fmaf(n.z, p0, fmaf(t1.z, p1, t2.z * p2)));
-                        }
-                        const V3 m = cross_fma(arm, a);
-                        hr[0] = __fadd_rn(hr[0], a.x); hr[1] = __fadd_rn(hr[1], a.y); hr[2] = __fadd_rn(hr[2], a.z); hr[3] = __fadd_rn(hr[3], m.x); hr[4] = __fadd_rn(hr[4], m.y); hr[5] = __fadd_rn(hr[5], m.z);
+                for (uint32_t k = g.j; k < count; k += g.width) {
+                    const uint32_t h = inc[k];
+                    const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
+                    const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), m0 = cross_fma(arm, n);
+                    const float4 f = hq(e, HF_F, h);
+                    body_row_share(n, m0, first_side ? f.x : -f.x, hf(e, HF_NZ, h), share, balance);
+                    body_block_share(n, m0, n * f.w, m0 * f.w, share);
+                    if (!position) {                               // push-out rows have a normal axis only
+                        const float4 c = hq(e, HF_C + 1u, h);
+                        const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
+                        const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h), m1 = cross_fma(arm, t1), m2 = cross_fma(arm, t2);
+                        body_row_share(t1, m1, first_side ? f.y : -f.y, nz.x, share, balance);
+                        body_row_share(t2, m2, first_side ? f.z : -f.z, nz.y, share, balance);
+                        body_block_share(t1, m1, mix_fma(t1, c.x, t2, c.z), mix_fma(m1, c.x, m2, c.z), share);
+                        body_block_share(t2, m2, mix_fma(t2, c.y, t1, c.z), mix_fma(m2, c.y, m1, c.z), share);
                     }
-                __syncwarp();
-                if (parts > 1u) {
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) hr[k] += __shfl_xor_sync(NKB_FULL, hr[k], 8);
-                    gsum += __shfl_xor_sync(NKB_FULL, gsum, 8); scale += __shfl_xor_sync(NKB_FULL, scale, 8);
                 }
+            __syncwarp();
+            g.deal(share); g.deal(balance);
+            scale = share[3];
+            const double inner = pick6(inertial, row);
+            own = (float)(balance[0] - (row < 6u ? inner : 0.0));
+            scale += row < 6u ? fabsf((float)inner) : 0.f;
 #pragma unroll
-                for (int k = 0; k < 6; ++k) scale = fmaf(fabsf(hr[k]), fabsf((float)u[k]), scale);
-                own = (float)gsum;
-                // the group's rows to every lane of it
+            for (int k = 0; k < 21; ++k) a[k] = __shfl_sync(NKB_FULL, share[k % 3], g.first + k / 3);
+            a[0] = __fadd_rn(a[0], mass.m); a[2] = __fadd_rn(a[2], mass.m); a[5] = __fadd_rn(a[5], mass.m);
+            a[9] = __fadd_rn(a[9], mass.i[0]); a[13] = __fadd_rn(a[13], mass.i[3]); a[14] = __fadd_rn(a[14], mass.i[1]);
+            a[18] = __fadd_rn(a[18], mass.i[4]); a[19] = __fadd_rn(a[19], mass.i[5]); a[20] = __fadd_rn(a[20], mass.i[2]);
+            float reach[6];
 #pragma unroll
-                for (int i = 0; i < 6; ++i)
+            for (int i = 0; i < 6; ++i) {
+                reach[i] = 0.f;
 #pragma unroll
-                    for (int k = 0; k <= i; ++k) a[i * (i + 1) / 2 + k] = __shfl_sync(NKB_FULL, hr[k], g.first + i);
-            } else {
-                // a lane takes the heads j, j + width, ... and sums its share of everything; the lanes then add their shares
-                float share[32];
-                double balance[8];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) share[k] = 0.f;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) balance[k] = 0.0;
-                if (active)
-#pragma unroll 1
-                    for (uint32_t k = g.j; k < count; k += g.width) {
-                        const uint32_t h = inc[k];
-                        const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
-                        const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), m0 = cross_fma(arm, n);
-                        const float4 f = hq(e, HF_F, h);
-                        body_row_share(n, m0, first_side ? f.x : -f.x, hf(e, HF_NZ, h), share, balance);
-                        body_block_share(n, m0, n * f.w, m0 * f.w, share);
-                        if (!position) {                               // push-out rows have a normal axis only
-                            const float4 c = hq(e, HF_C + 1u, h);
-                            const float2 nz = *reinterpret_cast<const float2*>(&hf(e, HF_NZ + 1u, h));
-                            const V3 t1 = hf3(e, HF_T1, h), t2 = hf3(e, HF_T2, h), m1 = cross_fma(arm, t1), m2 = cross_fma(arm, t2);
-                            body_row_share(t1, m1, first_side ? f.y : -f.y, nz.x, share, balance);
-                            body_row_share(t2, m2, first_side ? f.z : -f.z, nz.y, share, balance);
-                            body_block_share(t1, m1, mix_fma(t1, c.x, t2, c.z), mix_fma(m1, c.x, m2, c.z), share);
-                            body_block_share(t2, m2, mix_fma(t2, c.y, t1, c.z), mix_fma(m2, c.y, m1, c.z), share);
-                        }
-                    }
-                __syncwarp();
-                g.deal(share); g.deal(balance);
-                scale = share[3];
-                const double inner = pick6(inertial, row);
-                own = (float)(balance[0] - (row < 6u ? inner : 0.0));
-                scale += row < 6u ? fabsf((float)inner) : 0.f;
-#pragma unroll
-                for (int k = 0; k < 21; ++k) a[k] = __shfl_sync(NKB_FULL, share[k % 3], g.first + k / 3);
-                a[0] = __fadd_rn(a[0], mass.m); a[2] = __fadd_rn(a[2], mass.m); a[5] = __fadd_rn(a[5], mass.m);
-                a[9] = __fadd_rn(a[9], mass.i[0]); a[13] = __fadd_rn(a[13], mass.i[3]); a[14] = __fadd_rn(a[14], mass.i[1]);
-                a[18] = __fadd_rn(a[18], mass.i[4]); a[19] = __fadd_rn(a[19], mass.i[5]); a[20] = __fadd_rn(a[20], mass.i[2]);
-                float reach[6];
-#pragma unroll
-                for (int i = 0; i < 6; ++i) {
-                    reach[i] = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) reach[i] = fmaf(fabsf(i >= k ? a[i * (i + 1) / 2 + k] : a[k * (k + 1) / 2 + i]), fabsf((float)u[k]), reach[i]);
-                }
-                scale += pick6(reach, row);
+                for (int k = 0; k < 6; ++k) reach[i] = fmaf(fabsf(i >= k ? a[i * (i + 1) / 2 + k] : a[k * (k + 1) / 2 + i]), fabsf((float)u[k]), reach[i]);
             }
+            scale += pick6(reach, row);
             const bool finite = g.all(isfinite(own)), small = g.all(row >= 6u || fabsf(own) <= kRoundings * FLT_EPSILON * scale);
             failure |= active && !finite;
             active = active && finite;
@@ -1709,12 +1649,12 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
 static __device__ __noinline__ RigidResult descend_bodies_call(float* sm, const SmemLayout* lay, const TemplateView* t, uint32_t lane, uint32_t vstride, uint32_t nheads, uint32_t nblocks,
                                                                uint32_t iteration, float tol, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     const RigidRun run = {sm, lay, t, lane, vstride, nheads, nblocks, iteration, tol};        // a struct argument would go through memory
-    return descend_bodies<false>(run, k_begin, k_end, first, stride, position);
+    return descend_bodies(run, k_begin, k_end, first, stride, position);
 }
-template <int NR, bool kRows>
+template <int NR>
 NKB_DEV RigidResult descend_share(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     if constexpr (NR == 0) return descend_bodies_call(run.sm, run.lay, run.t, run.lane, run.vstride, run.nheads, run.nblocks, run.iteration, run.tol, k_begin, k_end, first, stride, position);
-    else return descend_bodies<kRows>(run, k_begin, k_end, first, stride, position);
+    else return descend_bodies(run, k_begin, k_end, first, stride, position);
 }
 
 // Lead warp: releases the helpers for good (they need not answer).
@@ -1758,7 +1698,7 @@ NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
 }
 
 // Blocks descend colour by colour, blocks of one colour in index order (block_descent_tile.cuh:2749-2820).
-template <int NR, bool kRigid, bool kRows>
+template <int NR, bool kRigid>
 NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
     const uint32_t nb = tile.nblocks;
     const uint32_t* order = block_order(e, nb);
@@ -1798,7 +1738,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
             // helper failed to answer, and take the helpers' shares
 #pragma unroll 1
             do {
-                const RigidResult part = descend_share<NR, kRows>(run, k, k_end, share, stride, position);
+                const RigidResult part = descend_share<NR>(run, k, k_end, share, stride, position);
                 mine.momentum = fmaxf(mine.momentum, part.momentum); mine.residual = fmaxf(mine.residual, part.residual);
                 mine.status |= part.status;
                 if (shared_out && share == 0u) {
@@ -2039,7 +1979,7 @@ NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
 
 // The whole constraint solve of one env.  On entry the heads are built, the articulation's post-dynamics
 // velocity is in (e.qd, sm_vel(root)) and free-body velocities are in sm_bvel.
-template <int NR, bool kRigid, bool kRows>
+template <int NR, bool kRigid>
 NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, B = t.B, n = NR > 0 ? t.ndof : 0u;
@@ -2191,7 +2131,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         }
         if (phase == kPhaseVelocity) { tile.iteration = sweeps++; tile.momentum = 0.f; tile.residual = 0.f; }
         else tile.iteration = sweeps + pushes;
-        descend_blocks<NR, kRigid, kRows>(e, tile, phase == kPhasePosition);
+        descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
         if (phase == kPhasePosition) {
             if (++pushes >= positions) { phase = kPhaseDone; continue; }
         } else tick(e, 10);

@@ -380,7 +380,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
       }
-        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid, kPart == kPartSolve>(e, nheads);
+        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid>(e, nheads);
         if constexpr (kPart == kPartSolve) {
             image_move<false, kAfter>(e, p, img, nheads);
             __stcg(reinterpret_cast<float*>(lanes + lane), e.qd);
@@ -444,7 +444,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
 #ifdef NKB_STAGE_TAPS
             const long long tap0 = clock64();
 #endif
-            r = descend_share<NR, false>(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
+            r = descend_share<NR>(run, k_begin, k_end, member, shared_layout.team, cmd->position != 0u);
 #ifdef NKB_STAGE_TAPS
             if (state.dbg_cycles != nullptr && lane == 0u && member == 1u) {
                 uint32_t* cyc = state.dbg_cycles + (size_t)env * 32u;
