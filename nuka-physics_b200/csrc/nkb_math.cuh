@@ -217,34 +217,35 @@ NKB_DEV float rsqrt_normal(float v) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;
 NKB_DEV bool pivot_valid(float v) { return v >= FLT_MIN && v <= FLT_MAX; }
 constexpr float kMassPivotFloor = 1.0e-6f;       // articulation_mass.cuh:269-335
 
-// Solves a symmetric positive 6 x 6 system held in registers: `a` is the lower triangle by rows (21), then the right-hand side
-// (6); the triangle is replaced by the Cholesky factor's, its diagonal's reciprocals are in `inv`.  kFloor holds the pivots to
-// the mass matrix's floor.  False when a pivot is not positive and finite.
-template <bool kFloor>
-NKB_DEV bool solve6(float (&a)[28], float (&inv)[6], float (&x)[6]) {
+// Solves a symmetric positive 6 x 6 system held in registers: `a` is the lower triangle by rows (21), replaced by the Cholesky
+// factor's, `g` the right-hand side; the diagonal's reciprocals are in `inv`.  kMass is the mass matrix's form: pivots held to its
+// floor, correctly rounded reciprocal roots, sums of the right-hand side in 64 bits (see tree_solve).  False when a pivot is not
+// positive and finite.
+template <bool kMass, typename Sum>
+NKB_DEV bool solve6(float (&a)[21], Sum (&g)[6], float (&inv)[6], float (&x)[6]) {
     bool valid = true;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         float pivot = a[k * (k + 1) / 2 + k];
-        if (kFloor) pivot = fmaxf(pivot, kMassPivotFloor);
+        if (kMass) pivot = fmaxf(pivot, kMassPivotFloor);
         valid &= pivot_valid(pivot);
-        inv[k] = rsqrt_normal(pivot);
-        a[21 + k] *= inv[k];
+        inv[k] = kMass ? __frsqrt_rn(pivot) : rsqrt_normal(pivot);
+        g[k] = g[k] * inv[k];
 #pragma unroll
         for (int i = k + 1; i < 6; ++i) a[i * (i + 1) / 2 + k] *= inv[k];
 #pragma unroll
         for (int i = k + 1; i < 6; ++i) {
-            a[21 + i] = fmaf(-a[i * (i + 1) / 2 + k], a[21 + k], a[21 + i]);
+            g[i] = fma((Sum)-a[i * (i + 1) / 2 + k], g[k], g[i]);
 #pragma unroll
             for (int j = k + 1; j <= i; ++j) a[i * (i + 1) / 2 + j] = fmaf(-a[i * (i + 1) / 2 + k], a[j * (j + 1) / 2 + k], a[i * (i + 1) / 2 + j]);
         }
     }
 #pragma unroll
     for (int k = 5; k >= 0; --k) {
-        float s = a[21 + k];
+        Sum s = g[k];
 #pragma unroll
-        for (int i = k + 1; i < 6; ++i) s = fmaf(-a[i * (i + 1) / 2 + k], x[i], s);
-        x[k] = s * inv[k];
+        for (int i = k + 1; i < 6; ++i) s = fma((Sum)-a[i * (i + 1) / 2 + k], (Sum)x[i], s);
+        x[k] = (float)(s * inv[k]);
     }
     return valid;
 }

@@ -1548,7 +1548,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             step = step < 0 ? 0 : step + 1;
             __syncwarp();
             // the next Newton system: the lower triangle of H, this lane's entry of the force balance and its rounding scale
-            float a[28], own, scale;
+            float a[21], rhs[6], own, scale;
             // a lane takes the heads j, j + width, ... and sums its share of everything; the lanes then add their shares
             float share[32];
             double balance[8];
@@ -1599,7 +1599,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             active = active && finite;
             float inv[6], x[6];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) a[21 + i] = force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
+            for (int i = 0; i < 6; ++i) rhs[i] = force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
             if (active && small) {
                 bool still = true;
                 if (run.tol > 0.f) {
@@ -1613,7 +1613,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                 if (still) { primal = 0.f; active = false; }
             }
             if (!__any_sync(NKB_FULL, active)) break;
-            const bool definite = solve6<false>(a, inv, x);
+            const bool definite = solve6<false>(a, rhs, inv, x);
             failure |= active && !definite;
             active = active && definite;
 #pragma unroll

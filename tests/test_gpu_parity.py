@@ -89,6 +89,29 @@ def test_quadruped_stages(device, oracle):
     w.destroy()
 
 
+# the bar lies between the dense factorisation in float (humanoid 5.1e-7; the tree's order with 32-bit sums and approximate roots:
+# 8.0e-7, quadruped 1.35e-7) and what the tree's factor gives with correctly rounded roots and 64-bit sums (5.0e-7, 0.86e-7)
+@pytest.mark.parametrize("name,bar", [("quadruped", 1.1e-7), ("humanoid", 6.0e-7)])
+def test_joint_accelerations_against_a_64_bit_solve(device, name, bar):
+    """Without gravity and velocities q'' = M^-1 tau exactly: the kernel's accelerations against a solve of its own M in 64 bits."""
+    E = 512
+    w = nuka.World.create_from_template(device, getattr(T, name)(0).blob(), E)
+    assert nuka._abi.lib().nuka_world_set_gravity_z(w._h, 0.0) == 0
+    L, rng = w.info.links_per_env, np.random.default_rng(0)
+    state = getattr(T, name + "_state")(E, 0)
+    w.upload(F.JOINT_POSITION, state["q"] + (0.3 * rng.normal(size=state["q"].shape)).astype(np.float32))
+    tau = (5.0 * rng.normal(size=(E, L))).astype(np.float32)
+    tau[:, 0] = 0.0
+    w.upload(F.JOINT_FEEDFORWARD, tau)
+    w.forward_kinematics(); w.run_stage(1)
+    mass = w.download(F.MASS_MATRIX).reshape(E, L + 5, L + 5).astype(np.float64)
+    force = np.concatenate([np.zeros((E, 6)), tau[:, 1:]], 1)
+    want = np.linalg.solve(mass, force[..., None])[:, 6:, 0]
+    error = np.linalg.norm(w.download(F.JOINT_ACCELERATION).reshape(E, L)[:, 1:] - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert np.sqrt(np.mean(error ** 2)) < bar
+    w.destroy()
+
+
 def test_quadruped_single_step_post_solve(device, oracle):
     E = 256
     q, qdot, base, lv = quad_inputs(E)
