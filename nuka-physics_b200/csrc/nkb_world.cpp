@@ -555,26 +555,6 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.n_adm = (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size());
         SetBroadphase(0u);
         if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
-        if (stages_ != nullptr) {
-            // images of the whole batch up to 2 GB, at least of 8192 envs: a larger batch goes in rounds over the same buffer
-            params_.im = params_.sm;
-            params_.image_stride = ((params_.sm.words + 3u) & ~3u) + kImageLaneWords;
-            const size_t bytes = static_cast<size_t>(params_.image_stride) * sizeof(float);
-            image_envs_ = static_cast<uint32_t>(std::min<size_t>(env_count_, std::max<size_t>(8192u, (size_t{2} << 30) / bytes)));
-            void* image = nullptr;
-            if (cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess) {
-                allocations_.push_back(image);
-                params_.image = static_cast<float*>(image);
-                Check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
-                for (uint32_t c = 0; c + 1u < kChunks; ++c) {
-                    Check(cudaStreamCreateWithFlags(&side_[c], cudaStreamNonBlocking), "cudaStreamCreate");
-                    Check(cudaEventCreateWithFlags(&join_[c], cudaEventDisableTiming), "cudaEventCreate");
-                }
-            } else {
-                cudaGetLastError();                 // no room for the images: steps run in one kernel
-                stages_ = solve_ = nullptr;
-            }
-        }
         const size_t E = env_count_, L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
         StateView& s = params_.s;
         s.env_count = env_count_;
@@ -593,6 +573,7 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         s.contact_point = Alloc<float>(E * S * 12); s.contact_normal = Alloc<float>(E * S * 12); s.contact_depth = Alloc<float>(E * S * 4);
         s.dbg_mass = nullptr; s.dbg_qdot_pseudo = nullptr; s.dbg_cycles = nullptr;
         Seed();
+        OpenSplitSteps();
     } catch (...) {
         ReleaseStreams();
         for (void* p : allocations_) cudaFree(p);
@@ -610,11 +591,41 @@ World::~World() {
     for (void* p : allocations_) cudaFree(p);
 }
 
+// What split steps need beside the world's state.  It is taken last, and a world that gets none of it runs its steps in one kernel,
+// with the same results: the state of a batch that just fits the device is not refused for the sake of speed.
+void World::OpenSplitSteps() {
+    if (stages_ == nullptr) return;
+    // images of the whole batch up to 2 GB, at least of 8192 envs: a larger batch goes in rounds over the same buffer
+    const uint32_t stride = ((params_.sm.words + 3u) & ~3u) + kImageLaneWords;
+    const size_t bytes = static_cast<size_t>(stride) * sizeof(float);
+    image_envs_ = static_cast<uint32_t>(std::min<size_t>(env_count_, std::max<size_t>(8192u, (size_t{2} << 30) / bytes)));
+    void* image = nullptr;
+    bool open = cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess;
+    if (open) open = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming) == cudaSuccess;
+    for (uint32_t c = 0; c + 1u < kChunks && open; ++c)
+        open = cudaStreamCreateWithFlags(&side_[c], cudaStreamNonBlocking) == cudaSuccess &&
+               cudaEventCreateWithFlags(&join_[c], cudaEventDisableTiming) == cudaSuccess;
+    if (open) {
+        allocations_.push_back(image);
+        params_.im = params_.sm;
+        params_.image = static_cast<float*>(image);
+        params_.image_stride = stride;
+        return;
+    }
+    cudaGetLastError();
+    if (image != nullptr) cudaFree(image);
+    ReleaseStreams();
+    stages_ = solve_ = nullptr;
+}
+
 void World::ReleaseStreams() {
     if (fork_) cudaEventDestroy(fork_);
+    fork_ = nullptr;
     for (uint32_t c = 0; c + 1u < kChunks; ++c) {
         if (join_[c]) cudaEventDestroy(join_[c]);
         if (side_[c]) cudaStreamDestroy(side_[c]);
+        join_[c] = nullptr;
+        side_[c] = nullptr;
     }
 }
 

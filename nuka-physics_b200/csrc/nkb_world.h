@@ -120,6 +120,7 @@ private:
     cudaStream_t side_[kChunks - 1] = {};
     cudaEvent_t fork_ = nullptr, join_[kChunks - 1] = {};
     void EnqueueSteps(uint32_t n);
+    void OpenSplitSteps();
     void ReleaseStreams();
     bool slim_ = false;        // the world runs the 128-register build of its kernel variant
     std::vector<void*> allocations_;

@@ -80,6 +80,36 @@ def test_an_env_does_not_depend_on_its_batch(device, name, E):
     assert_same(a, {k: np.concatenate([v[:3], v[-3:]]) for k, v in b.items()})
 
 
+def test_a_world_is_created_where_its_images_find_no_room(device):
+    """The buffer of split steps (about 25 KB per env here) is taken after the state: with room for the buffer and half of the state the
+    world is created, steps in one kernel, and gives the same states."""
+    torch = pytest.importorskip("torch")
+    E = 8192
+    tb, st = scene("boxes", E, 0)
+    free = lambda: torch.cuda.mem_get_info(0)[0]
+    torch.cuda.empty_cache()
+    needs, worlds = [], []
+    for split in (0, 1, 0, 1):                    # the first two load their kernels
+        before = free()
+        w = create(device, tb, st, E, SPLIT=split)
+        w.step_n(2)
+        w.synchronize()
+        needs.append(before - free())
+        worlds.append((w.launch_count(), {f.name: w.download(f) for f in (F.RIGID_BODY_TRANSFORM, F.JOINT_POSITION)}))
+        w.destroy()
+    state, images = needs[2], needs[3] - needs[2]
+    assert images > state > 32 << 20
+    fill = torch.empty(free() - images - state // 2, dtype=torch.uint8, device="cuda:0")
+    w = create(device, tb, st, E, SPLIT=1)
+    w.step_n(2)
+    assert w.launch_count() == worlds[2][0] != worlds[3][0]
+    for k, v in worlds[3][1].items():
+        assert np.array_equal(v, w.download(F[k])), k
+    w.destroy()
+    del fill
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("count,team", [(48, 8), (48, 1), (40, 3)])
 def test_contact_points_in_their_read_out_arrays(device, count, team):
     """A pile's contact points and normals stay in global memory where that makes room for another env."""
