@@ -600,10 +600,11 @@ void World::OpenSplitSteps() {
     const size_t bytes = static_cast<size_t>(stride) * sizeof(float);
     image_envs_ = static_cast<uint32_t>(std::min<size_t>(env_count_, std::max<size_t>(8192u, (size_t{2} << 30) / bytes)));
     void* image = nullptr;
-    bool open = cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess;
+    int priority = 0;                                                  // the caller's, whose step this is
+    bool open = cudaStreamGetPriority(stream_, &priority) == cudaSuccess && cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess;
     if (open) open = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming) == cudaSuccess;
     for (uint32_t c = 0; c + 1u < kChunks && open; ++c)
-        open = cudaStreamCreateWithFlags(&side_[c], cudaStreamNonBlocking) == cudaSuccess &&
+        open = cudaStreamCreateWithPriority(&side_[c], cudaStreamNonBlocking, priority) == cudaSuccess &&
                cudaEventCreateWithFlags(&join_[c], cudaEventDisableTiming) == cudaSuccess;
     if (open) {
         allocations_.push_back(image);

@@ -110,6 +110,27 @@ def test_a_world_is_created_where_its_images_find_no_room(device):
     torch.cuda.empty_cache()
 
 
+def test_split_steps_keep_the_callers_stream_priority(device):
+    """Every kernel of a step, those on the world's side streams too: read from the nodes of a captured one."""
+    torch = pytest.importorskip("torch")
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    stream = torch.cuda.Stream(priority=-1)
+    borrowed = nuka.Device.create(0, cuda_stream=stream.cuda_stream)
+    w = create(borrowed, T.quadruped(0), T.quadruped_state(32, 0), 32, SPLIT=1)
+    w.step_n(1)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        w.step_n(2)
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    count = runtime.cudaGraphGetNodes(raw)[2]
+    kernels = [n for n in runtime.cudaGraphGetNodes(raw, count)[1] if runtime.cudaGraphNodeGetType(n)[1] == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel]
+    priorities = [runtime.cudaGraphKernelNodeGetAttribute(n, runtime.cudaLaunchAttributeID.cudaLaunchAttributePriority)[1].priority for n in kernels]
+    assert len(priorities) == 15 and set(priorities) == {-1}           # three parts of three stages and two solves
+    w.destroy()
+    borrowed.destroy()
+
+
 @pytest.mark.parametrize("count,team", [(48, 8), (48, 1), (40, 3)])
 def test_contact_points_in_their_read_out_arrays(device, count, team):
     """A pile's contact points and normals stay in global memory where that makes room for another env."""
