@@ -253,9 +253,10 @@ nuka_result_t nuka_b200_world_info(nuka_world_handle world, nuka_b200_world_info
 nuka_result_t nuka_b200_world_run_stage(nuka_world_handle world, uint32_t stage);
 
 /* nuka_world_download_field into page-locked memory of the library's own: the whole field, complete when the call returns;
- * *bytes is released with nuka_b200_host_release, from any thread, before or after the world is destroyed.  The library keeps
- * released blocks for later calls.  NUKA_ERR_NOT_SUPPORTED when the blocks in use would exceed 256 MB (download into memory of
- * the caller's instead). */
+ * *bytes is released with nuka_b200_host_release, from any thread, before or after the world is destroyed; releasing it again has
+ * no effect.  The library keeps released blocks for later calls until the last device handle is destroyed.
+ * NUKA_ERR_NOT_SUPPORTED for a field above 64 MB, and when the blocks in use and kept would exceed 256 MB (download into memory
+ * of the caller's instead). */
 nuka_result_t nuka_b200_world_download_host(nuka_world_handle world, nuka_state_field_t field, void** bytes, size_t* nbytes);
 void nuka_b200_host_release(void* bytes);
 

@@ -10,6 +10,7 @@
 #include <unordered_map>
 
 #include "../../include/nuka_b200.h"
+#include "nkb_host_pool.h"
 #include "nkb_scene.h"
 #include "nkb_world.h"
 
@@ -87,6 +88,15 @@ uint64_t Fnv1a(uint64_t h, const void* data, size_t bytes) {
 HandleTable<DeviceRecord>& Devices() { static auto* t = new HandleTable<DeviceRecord>; return *t; }
 HandleTable<WorldRecord>& Worlds() { static auto* t = new HandleTable<WorldRecord>; return *t; }
 HandleTable<CheckpointRecord>& Checkpoints() { static auto* t = new HandleTable<CheckpointRecord>; return *t; }
+void* LockPages(size_t bytes) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+void UnlockPages(void* p) { if (cudaFreeHost(p) != cudaSuccess) cudaGetLastError(); }
+// Its users are the device handles.  Never destroyed: arrays may be released after main.
+nkb::HostPool& Pool() { static auto* pool = new nkb::HostPool(LockPages, UnlockPages); return *pool; }
 std::atomic<uint64_t> g_world_serial{0};
 
 template <typename Fn>
@@ -211,6 +221,7 @@ nuka_result_t nuka_device_create(const nuka_device_desc_t* desc, nuka_device_han
             rec->owns_stream = true;
         }
         *out = reinterpret_cast<nuka_device_handle>(Devices().Insert(std::move(rec)));
+        Pool().Join();
         return NUKA_RESULT_OK;
     });
 }
@@ -219,6 +230,7 @@ void nuka_device_destroy(nuka_device_handle device) {
     auto rec = Devices().Remove(reinterpret_cast<uintptr_t>(device));
     if (!rec) return;
     if (rec->owns_stream) { cudaSetDevice(rec->gpu); cudaStreamDestroy(rec->stream); }
+    try { Pool().Leave(); } catch (...) {}
 }
 
 nuka_result_t nuka_world_create_from_template(nuka_device_handle device, const nuka_world_desc_t* desc,
@@ -566,43 +578,6 @@ nuka_result_t nuka_world_download_field(nuka_world_handle world, nuka_state_fiel
     return Transfer(world, field, bytes, nbytes, byte_offset, false);
 }
 
-// Page-locked blocks for downloads.  A copy into pageable memory goes through the driver's staging buffer at about 4 GB/s and
-// faults the destination's fresh pages (1.28 MB: 320 us); into page-locked memory it is one transfer at link speed (45 us).
-// Locking pages takes longer than either, so released blocks are kept, by power-of-two size; blocks handed out and kept
-// together stay within kHostPoolBytes.
-namespace {
-struct HostPool {
-    static constexpr size_t kHostPoolBytes = size_t{256} << 20, kSmallest = 4096;
-    std::mutex lock;
-    std::unordered_map<void*, size_t> sizes;                    // every block, handed out or kept
-    std::unordered_map<size_t, std::vector<void*>> kept;
-    size_t total = 0;
-    void* Take(size_t bytes) {
-        size_t size = kSmallest;
-        while (size < bytes) size <<= 1;
-        std::lock_guard<std::mutex> hold(lock);
-        auto& list = kept[size];
-        if (!list.empty()) { void* p = list.back(); list.pop_back(); return p; }
-        if (size > kHostPoolBytes) return nullptr;
-        for (auto it = kept.begin(); it != kept.end() && total + size > kHostPoolBytes; ++it)
-            while (!it->second.empty() && total + size > kHostPoolBytes) {
-                cudaFreeHost(it->second.back()); sizes.erase(it->second.back()); it->second.pop_back(); total -= it->first;
-            }
-        void* p = nullptr;
-        if (total + size > kHostPoolBytes) return nullptr;
-        if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        total += size; sizes[p] = size;
-        return p;
-    }
-    void Give(void* p) {
-        std::lock_guard<std::mutex> hold(lock);
-        const auto it = sizes.find(p);
-        if (it != sizes.end()) kept[it->second].push_back(p);
-    }
-};
-HostPool& Pool() { static HostPool* pool = new HostPool; return *pool; }     // outlives arrays released at exit
-}  // namespace
-
 nuka_result_t nuka_b200_world_download_host(nuka_world_handle world, nuka_state_field_t field, void** bytes, size_t* nbytes) {
     if (bytes == nullptr || nbytes == nullptr) { SetError("out pointer is null"); return NUKA_RESULT_INVALID_ARG; }
     *bytes = nullptr; *nbytes = 0;
@@ -625,7 +600,9 @@ nuka_result_t nuka_b200_world_download_host(nuka_world_handle world, nuka_state_
     });
 }
 
-void nuka_b200_host_release(void* bytes) { if (bytes != nullptr) Pool().Give(bytes); }
+void nuka_b200_host_release(void* bytes) {
+    try { Pool().Give(bytes); } catch (...) {}                  // out of memory: the block stays handed out
+}
 
 nuka_result_t nuka_b200_world_info(nuka_world_handle world, nuka_b200_world_info_t* out) {
     NKB_WORLD(w)

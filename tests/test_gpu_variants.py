@@ -2,6 +2,7 @@
 next env, contact points in the slice or in their read-out arrays.  Who runs a step and where its data waits changes no result,
 so the comparisons are bit-exact."""
 import contextlib
+import ctypes
 import os
 
 import numpy as np
@@ -175,3 +176,22 @@ def test_downloads_outlive_the_world_and_one_another(device):
     assert np.array_equal(first, kept) and np.array_equal(second, kept2)
     assert all(np.array_equal(again[0], a) for a in again)
     v.destroy()
+
+
+def test_a_download_released_twice_is_handed_out_once(device):
+    w = create(device, T.quadruped(0), T.quadruped_state(16, 1), 16)
+    lib = nuka._abi.lib()
+
+    def block():
+        ptr, size = ctypes.c_void_p(), ctypes.c_size_t()
+        assert lib.nuka_b200_world_download_host(w._h, int(F.JOINT_POSITION), ctypes.byref(ptr), ctypes.byref(size)) == 0
+        return ptr.value
+
+    first = block()
+    lib.nuka_b200_host_release(first)
+    lib.nuka_b200_host_release(first)
+    a, b = block(), block()
+    assert a != b
+    lib.nuka_b200_host_release(a)
+    lib.nuka_b200_host_release(b)
+    w.destroy()
