@@ -536,22 +536,35 @@ World::World(int device, cudaStream_t stream, const HostTemplate& tpl, uint32_t 
         v.n_excluded = static_cast<uint32_t>(t.excluded.size()); v.n_free = t.n_free;
         v.cfg = t.cfg;
         BuildLayout();
-        v.parent = Upload(t.parent); v.jtype = Upload(t.jtype); v.depth = Upload(t.depth); v.child_begin = Upload(t.child_begin);
-        v.children = Upload(t.children); v.link_dof = Upload(t.link_dof); v.link_body = Upload(t.link_body);
-        v.geom_kind = Upload(t.geom_kind); v.limit_flags = Upload(t.limit_flags); v.dof_link = Upload(t.dof_link); v.anc_mask = Upload(t.anc_mask);
-        v.tree_lanes = Upload(t.tree_lanes); v.link_leaf = Upload(t.link_leaf);
-        v.axis = Upload(t.axis); v.offset = Upload(t.offset); v.local_quat = Upload(t.local_quat); v.inertia10 = Upload(t.inertia10);
-        v.damping = Upload(t.damping); v.armature = Upload(t.armature); v.frictionloss = Upload(t.frictionloss);
-        v.stiffness = Upload(t.stiffness); v.spring_ref = Upload(t.spring_ref); v.limit_lower = Upload(t.limit_lower);
-        v.limit_upper = Upload(t.limit_upper); v.geom_pos = Upload(t.geom_pos); v.geom_quat = Upload(t.geom_quat);
-        v.body_geom_kind = Upload(t.body_geom_kind); v.body_geom_pos = Upload(t.body_geom_pos); v.body_geom_quat = Upload(t.body_geom_quat);
-        v.shape_kind = Upload(t.shape_kind); v.contype = Upload(t.contype); v.conaffinity = Upload(t.conaffinity); v.group = Upload(t.group);
-        v.body_to_link = Upload(t.body_to_link); v.body_id = Upload(t.body_id); v.shape_params = Upload(t.shape_params); v.mu = Upload(t.mu);
-        v.inv_mass = Upload(t.inv_mass); v.inv_inertia = Upload(t.inv_inertia); v.inertial_pos = Upload(t.inertial_pos);
-        v.inertial_quat = Upload(t.inertial_quat); v.excluded = Upload(t.excluded);
-        v.adm_pairs = Upload(t.adm_pairs);
-        v.adm_mask = Upload(t.adm_mask);
-        v.free_slot = Upload(t.free_slot);
+        // the template's tables, in one allocation and one copy
+        auto each = [&](auto put) {
+            put(v.parent, t.parent); put(v.jtype, t.jtype); put(v.depth, t.depth); put(v.child_begin, t.child_begin);
+            put(v.children, t.children); put(v.link_dof, t.link_dof); put(v.link_body, t.link_body);
+            put(v.geom_kind, t.geom_kind); put(v.limit_flags, t.limit_flags); put(v.dof_link, t.dof_link);
+            put(v.anc_mask, t.anc_mask); put(v.tree_lanes, t.tree_lanes); put(v.link_leaf, t.link_leaf); put(v.axis, t.axis);
+            put(v.offset, t.offset); put(v.local_quat, t.local_quat); put(v.inertia10, t.inertia10); put(v.damping, t.damping);
+            put(v.armature, t.armature); put(v.frictionloss, t.frictionloss); put(v.stiffness, t.stiffness);
+            put(v.spring_ref, t.spring_ref); put(v.limit_lower, t.limit_lower); put(v.limit_upper, t.limit_upper);
+            put(v.geom_pos, t.geom_pos); put(v.geom_quat, t.geom_quat); put(v.body_geom_kind, t.body_geom_kind);
+            put(v.body_geom_pos, t.body_geom_pos); put(v.body_geom_quat, t.body_geom_quat); put(v.shape_kind, t.shape_kind);
+            put(v.contype, t.contype); put(v.conaffinity, t.conaffinity); put(v.group, t.group);
+            put(v.body_to_link, t.body_to_link); put(v.body_id, t.body_id); put(v.shape_params, t.shape_params); put(v.mu, t.mu);
+            put(v.inv_mass, t.inv_mass); put(v.inv_inertia, t.inv_inertia); put(v.inertial_pos, t.inertial_pos);
+            put(v.inertial_quat, t.inertial_quat); put(v.excluded, t.excluded); put(v.adm_pairs, t.adm_pairs);
+            put(v.adm_mask, t.adm_mask); put(v.free_slot, t.free_slot);
+        };
+        auto place = [](size_t words) { return (std::max<size_t>(words, 1u) + 63u) & ~size_t{63}; };       // 256-byte aligned
+        size_t words = 0;
+        each([&](auto&, const auto& table) { words += place(table.size() * sizeof(table[0]) / 4u); });
+        std::vector<uint32_t> tables(words, 0u);
+        uint32_t* device_tables = Alloc<uint32_t>(words, false);
+        size_t at = 0;
+        each([&](auto& pointer, const auto& table) {
+            pointer = reinterpret_cast<std::remove_reference_t<decltype(pointer)>>(device_tables + at);
+            if (!table.empty()) std::memcpy(tables.data() + at, table.data(), table.size() * sizeof(table[0]));
+            at += place(table.size() * sizeof(table[0]) / 4u);
+        });
+        Check(cudaMemcpyAsync(device_tables, tables.data(), words * 4u, cudaMemcpyHostToDevice, stream_), "template upload");
         v.n_adm = (t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) ? 0u : static_cast<uint32_t>(t.adm_pairs.size());
         SetBroadphase(0u);
         if (grid_ != 0u) queue_ = Alloc<uint32_t>(2);
