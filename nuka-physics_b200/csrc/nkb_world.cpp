@@ -358,10 +358,10 @@ void World::BuildLayout() {
     s.ld = pad_ld(n);
     s.pose = take(7 * L); s.vel = take(6 * L);
     // the dynamics stage's link scratch and the solver's Newton scratch are live at different times and share one region
-    const uint32_t overlay = at;
+    const uint32_t shared = at;
     s.xrot = take(9 * L); s.xtr = take(3 * L); s.vbias = 0; s.acc = take(6 * L); s.pbias = take(6 * L); s.ic = take(10 * L);
     const uint32_t dynamics_end = at;
-    if (std::getenv("NUKA_B200_NO_OVERLAY") == nullptr) at = overlay;
+    at = shared;
     tv.tree_depth = t.tree_depth; tv.tree_stride = tree_row_stride(t.tree_depth);
     // The mass matrix's factor on the tree: where the tree branches.  On a single chain it is as long as the dense one and its
     // steps cost more (7-link arm, 32 steps: 3.98 ms against 3.56 ms; quadruped, depth 3 of 18: 3.26 against 3.76).  The
@@ -390,7 +390,6 @@ void World::BuildLayout() {
     s.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);      // the unit-row table holds 16-bit head indices
     const uint32_t without_points = at;
     s.cpoint = take(12 * SC); s.cnormal = take(12 * SC); s.contacts_far = 0u;      // last: a team's env may leave them out
-    if (const char* pad = std::getenv("NUKA_B200_SMEM_PAD_WORDS")) at += (static_cast<uint32_t>(std::atoi(pad)) + 3u) & ~3u;   // occupancy experiments
     // Team mode.  An env of many free bodies fills most of an SM's shared memory by itself, so one warp per env would
     // leave the SM with one or two resident warps; instead several warps share the env and descend the rigid blocks
     // of one colour side by side (blocks of a colour share no constraint row).
@@ -474,12 +473,11 @@ void World::BuildLayout() {
         else if (share >= most && SC == 0u && fits[4] == most) warps_per_block_ = 4u;      // no meetings: small blocks pack better (3.10 ms against 3.29)
         else if (share < most)
             for (uint32_t w = 1u; w <= std::min(share, kWarpsPerBlockMax); ++w) if (fits[w] >= share) warps_per_block_ = w;
-        if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // block-shape experiments
+        if (const char* forced = std::getenv("NUKA_B200_WARPS_PER_BLOCK")) {          // tests
             const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
             if (w >= 1u && w <= kWarpsPerBlockMax && fits[w] != 0u) warps_per_block_ = w;
         }
         group_ = SC != 0u ? warps_per_block_ : 0u;
-        if (const char* forced = std::getenv("NUKA_B200_GROUP")) group_ = static_cast<uint32_t>(std::atoi(forced));
         const uint32_t grid = static_cast<uint32_t>(sms) * static_cast<uint32_t>(fits[warps_per_block_] / warps_per_block_);
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
@@ -512,7 +510,6 @@ void World::BuildLayout() {
             const size_t r = static_cast<size_t>(stages_->resident_blocks(w, w * bytes)) * w;
             if (r > top || (r == top && w <= 8u)) { top = r; stages_warps_ = w; }       // 8 against 16 warps: 3 % at 2500 and 4096 quadrupeds, equal from 8000 on
         }
-        if (const char* forced = std::getenv("NUKA_B200_STAGES_WARPS")) stages_warps_ = std::max(1u, std::min(stages_warps_, static_cast<uint32_t>(std::atoi(forced))));
     }
     if (std::getenv("NUKA_B200_DEBUG_LAYOUT") != nullptr) {
         if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %d registers, %u warps per block; solve %u B, %d registers, %d resident\n", stages_->registers(), stages_warps_,
@@ -520,7 +517,8 @@ void World::BuildLayout() {
         std::fprintf(stderr, "[nuka_b200] %zu B of shared memory per env, %d registers per thread%s; resident warps per SM by block size:", bytes,
                      step_kernel_registers(tv, slim_), slim_ ? " (slim build)" : "");
         for (uint32_t w = 1; w <= kWarpsPerBlockMax; ++w) std::fprintf(stderr, " %u:%zu", w, fits[w]);
-        std::fprintf(stderr, " -> %u warps per block, %u per env\n", warps_per_block_, team);
+        std::fprintf(stderr, " -> %u warps per block, %u per env, meetings of %u, %u persistent blocks%s\n", warps_per_block_, team, group_, grid_,
+                     s.contacts_far != 0u ? ", contact points in their read-out arrays" : "");
         std::fprintf(stderr, "[nuka_b200] word offsets: overlay %u mass %u vecs %u bodies %u contacts %u heads %u pool %u blocks %u end %u\n",
                      s.xrot, s.mass, s.vecs, s.bpose, s.pairs, s.heads, s.jpool, s.binfo, s.words);
     }
@@ -612,6 +610,7 @@ void World::OpenSplitSteps() {
     const uint32_t stride = ((params_.sm.words + 3u) & ~3u) + kImageLaneWords;
     const size_t bytes = static_cast<size_t>(stride) * sizeof(float);
     image_envs_ = static_cast<uint32_t>(std::min<size_t>(env_count_, std::max<size_t>(8192u, (size_t{2} << 30) / bytes)));
+    if (const char* forced = std::getenv("NUKA_B200_IMAGE_ENVS")) image_envs_ = std::max(1u, std::min(image_envs_, static_cast<uint32_t>(std::atoi(forced))));   // tests
     void* image = nullptr;
     int priority = 0;                                                  // the caller's, whose step this is
     bool open = cudaStreamGetPriority(stream_, &priority) == cudaSuccess && cudaMalloc(&image, image_envs_ * bytes) == cudaSuccess;
