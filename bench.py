@@ -4,11 +4,11 @@
     python bench.py --gpus N --steps K --warmup W          (torchrun launches it for N > 1)
     python bench.py --impl reference ...                   (the CPU arm: the oracle port on all host cores)
 
-A "step" is one physics step of every env of the workload: 4096 quadrupeds per GPU (BASELINE.json configs[1]).
+A "step" is one physics step of every env of the workload: 4096 quadrupeds per GPU.
 N > 1 gives every rank its own 4096-env shard (weak scaling, no collective in the step); every `--exchange-every` steps (4,
 the decimation at which the reference's gym env composes observations) each rank packs observation + reward records
 straight into its slice of one of two gather buffers, and the in-place all-gather of that buffer runs on a side stream
-under the next step (configs[4]'s exchange, double-buffered; the last gather of a timed run is added as a tail).
+under the next step (double-buffered; the last gather of a timed run is added as a tail).
 
 State preparation.  The cost of a step depends on what the robots are doing: while they drop onto their feet the solver
 runs all its sweeps, once they stand it stops early.  So both arms first run `config.settle_steps` untimed steps from
@@ -38,7 +38,7 @@ sys.path.insert(0, os.path.join(ROOT, "nuka-physics_b200"))
 ENVS_PER_GPU = 4096
 SETTLE_STEPS = 1000
 METRIC = "env-steps/sec (whole box) 4096-env 12-DoF quadruped"
-WORKLOAD = "quadruped (13 links, 18 DoF, 4 foot spheres + trunk box on a plane), configs[1]"
+WORKLOAD = "quadruped (13 links, 18 DoF, 4 foot spheres + trunk box on a plane)"
 NJ, NF, NL = 12, 1, 13
 ACTIVE_NOISE = 0.15          # rad, standard deviation of the per-step target noise of the `active` figure
 ACTIVE_POOL = 16             # distinct target sets cycled through
@@ -200,7 +200,7 @@ def fp32_peak(device_index):
 
 
 def captured_counters():
-    """Per-launch counters of one ncu capture of the step kernel on the prepared state (profiles/), or {}."""
+    """Counters of one step of the headline batch on the prepared state, from an ncu capture of its launches (profiles/), or {}."""
     try:
         with open(os.path.join(ROOT, "profiles", "step_kernel_quadruped_counters.txt")) as f:
             return json.load(f)
@@ -210,18 +210,18 @@ def captured_counters():
 
 OTHER_WORKLOADS = {
     # name: (description, default envs per GPU, settle steps, template, state, upload fields, (nj, F, L, free bodies))
-    "c1": ("configs[0]: 7-link fixed-base arm, no contacts, dt 1/500", 4096, 200, lambda T: T.arm7(0), lambda T, E, s: T.arm7_state(E, s), (7, 0, 8, 0)),
-    "c3": ("configs[2]: 35-coordinate humanoid, capsules, ground + limb self-contact, dt 1/200, 8 iterations", 8192, 300,
+    "c1": ("7-link fixed-base arm, no contacts, dt 1/500", 4096, 200, lambda T: T.arm7(0), lambda T, E, s: T.arm7_state(E, s), (7, 0, 8, 0)),
+    "c3": ("35-coordinate humanoid, capsules, ground + limb self-contact, dt 1/200, 8 iterations", 8192, 300,
            lambda T: T.humanoid(0), lambda T, E, s: T.humanoid_state(E, s), (29, 1, 30, 0)),
-    "c4": ("configs[3]: 48 free boxes on a plane, dt 1/240, 8 iterations", 16384, 240,
+    "c4": ("48 free boxes on a plane, dt 1/240, 8 iterations", 16384, 240,
            lambda T: T.box_pile(0), lambda T, E, s: T.box_pile_state(E, s), (0, 0, 0, 48)),
-    "c5": ("configs[4]'s shard: quadruped + 4 free 0.1 m boxes, dt 1/200, 4 iterations", 8192, 300,
+    "c5": ("one GPU's shard of 65536 envs: quadruped + 4 free 0.1 m boxes, dt 1/200, 4 iterations", 8192, 300,
            lambda T: T.quadruped(0, boxes=4), lambda T, E, s: T.quadruped_state(E, s), (12, 1, 13, 4)),
 }
 
 
 def run_other_workload(args):
-    """`--workload c1|c3|c4|c5`: the other configurations of BASELINE.json on one GPU, device-timed on a prepared state.
+    """`--workload c1|c3|c4|c5`: the other configurations on one GPU, device-timed on a prepared state.
     They are parity-test configurations, not the headline; the line has the same keys minus the CPU and end-to-end legs."""
     import torch
     import nuka
@@ -299,12 +299,12 @@ def main():
     ap.add_argument("--exchange-every", type=int, default=4,
                     help="N > 1: physics steps per observation exchange; 4 is the decimation of the reference's gym env, which composes "
                          "observations once per step_n(decimation) (python/nuka/gym/env.py:98, 255-256)")
-    ap.add_argument("--no-extra", action="store_true", help="skip the configs[4] figure (65536 quadruped + 4-box envs split over the ranks)")
+    ap.add_argument("--no-extra", action="store_true", help="skip the figure of 65536 quadruped + 4-box envs split over the ranks")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--workload", default="c2", choices=["c2"] + sorted(OTHER_WORKLOADS),
-                    help="c2 is the headline (configs[1]); the others are single-GPU lines of the parity configurations")
+                    help="c2 is the headline; the others are single-GPU lines of the parity configurations")
     ap.add_argument("--boxes", type=int, default=0,
-                    help="free 0.1 m boxes beside each quadruped: 4 with --envs 8192 per GPU is configs[4]'s shard (not the headline workload)")
+                    help="free 0.1 m boxes beside each quadruped: 4 with --envs 8192 per GPU is one GPU's shard of 65536 envs (not the headline workload)")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.impl == "reference":
@@ -532,7 +532,7 @@ def main():
         torch.cuda.synchronize()
     w.destroy()
 
-    # ---- configs[4]: 65536 envs of quadruped + 4 free boxes split evenly over the ranks, same exchange ---------------------
+    # ---- 65536 envs of quadruped + 4 free boxes split evenly over the ranks, same exchange ---------------------
     extra = None
     if not args.no_extra and not args.boxes:
         total = 65536
@@ -548,7 +548,7 @@ def main():
         (x_total,) = max_over_ranks([sum(x_ms)])
         torch.cuda.synchronize()
         wx.destroy()
-        extra = {"workload": "configs[4]: 65536 envs of quadruped + 4 free 0.1 m boxes split evenly over the ranks, observation all-gather as in the headline run (double-buffered, under the next step)",
+        extra = {"workload": "65536 envs of quadruped + 4 free 0.1 m boxes split evenly over the ranks, observation all-gather as in the headline run (double-buffered, under the next step)",
                  "scaling": "strong", "total_envs": total, "envs_per_gpu": Ex, "steps": x_steps, "settle_steps": 200,
                  "ms_per_step": x_total / x_steps, "value": total * x_steps / (x_total * 1e-3), "unit": "env-steps/s"}
 
@@ -573,20 +573,20 @@ def main():
             flops = counters["fp32_flop_per_env_step"] * value / world_size
             fp32 = {"achieved": flops / 1e12, "peak": peak_tflops, "unit": "TFLOP/s", "frac": flops / 1e12 / peak_tflops,
                     "flop_per_env_step": counters["fp32_flop_per_env_step"],
-                    "note": "executed FADD + FMUL + 2 FFMA of the captured launch (ncu thread-instruction counters) against the FMA rate "
+                    "note": "executed FADD + FMUL + 2 FFMA of the captured step (ncu thread-instruction counters) against the FMA rate "
                             "measured by csrc/probe/fp32_peak.cu in this run"}
         line = {
             "metric": METRIC, "value": value, "unit": "env-steps/s", "n_gpus": world_size, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": kernel_ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic",
-            "config": {"workload": WORKLOAD if not args.boxes else WORKLOAD.replace("configs[1]", f"configs[4]'s env: + {args.boxes} free 0.1 m boxes"),
+            "config": {"workload": WORKLOAD if not args.boxes else WORKLOAD + f" + {args.boxes} free 0.1 m boxes",
                        "envs_per_gpu": E, "dt": 1.0 / 200.0, "velocity_iterations": 4, "settle_steps": args.settle,
                        "drives": "hold the standing pose", "l2_flush_between_steps": flush is not None,
                        "obs_allgather": f"every {args.exchange_every} steps (the gym env's decimation), double-buffered; issued on a side stream when the next step starts" if gather else False, "mean_contact_slots": slots, "mean_contact_points": points, "mean_solver_sweeps": sweeps},
             "active": {"value": active_value, "unit": "env-steps/s", "ms_per_step": active_total / active_steps, "steps": active_steps,
                        "drives": f"targets redrawn every step: standing pose + N(0, {ACTIVE_NOISE}) rad"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": counters.get("dram_bytes_per_launch"), "peak_source": peak_kind, "algorithmic_bytes_per_env_step": bytes_per,
+                         "traffic": counters.get("dram_bytes_per_step"), "peak_source": peak_kind, "algorithmic_bytes_per_env_step": bytes_per,
                          "kernel": "step_kernel", "kernel_ms": kernel_ms, "issue": issue, "fp32": fp32,
                          "counters": counters.get("source")},
             "e2e": {"value": e2e_value, "unit": "env-steps/s", "ms_per_step": e2e_total / e2e_steps, "steps": e2e_steps,

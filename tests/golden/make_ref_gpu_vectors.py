@@ -5,8 +5,8 @@ from the reference checkout).  Three phases, because the driver needs a GPU and 
                                                         per-env start states and run.sh into oracle/_ref/run/, and the
                                                         reference's cook of each scene (no GPU needed) into tests/golden/
   bash oracle/_ref/run/run.sh                           on a machine with a GPU: steps the scenes with the reference and
-                                                        writes OUT/ref_*.nkt and OUT/ref_timing.jsonl (OUT defaults to the
-                                                        repository's scratch output folder)
+                                                        writes OUT/ref_*.nkt and OUT/ref_timing.jsonl (OUT defaults to
+                                                        out/ beside the script)
   python tests/golden/make_ref_gpu_vectors.py collect   copies the results into tests/golden/
 
 Both sides of the later comparison read the same .nks scene: the reference through its loader and cooker, this
@@ -37,9 +37,9 @@ CASES = {
     "quadruped_moving": (lambda: T.quadruped(0), lambda E: ref_cases.quadruped_moving_state(E, 0), 1.0 / 200.0, 4, 40, 10),
     # free rigid boxes dropping onto the plane and each other: box-box and box-plane manifolds, rigid blocks in the solver
     "pile12": (lambda: T.box_pile(0, count=12), lambda E: T.box_pile_state(E, 0, count=12), 1.0 / 240.0, 8, 60, 20),
-    # configs[4]'s env: the quadruped with four free boxes around it
+    # the quadruped with four free boxes around it
     "quadbox": (lambda: T.quadruped(0, boxes=4), lambda E: T.quadruped_state(E, 0), 1.0 / 200.0, 4, 60, 20),
-    # configs[2]'s env: the 35-coordinate humanoid with ground and limb self-contact
+    # the 35-coordinate humanoid with ground and limb self-contact
     "humanoid": (lambda: T.humanoid(0), lambda E: T.humanoid_state(E, 0), 1.0 / 200.0, 8, 40, 10),
     # computed-torque control (control mode 3): the arm without contacts, the quadruped landing with saturating force limits
     "arm7_ct": (lambda: T.arm7(0), lambda E: ref_cases.arm_computed_torque_state(E, 0), 1.0 / 500.0, 4, 100, 20),
@@ -81,7 +81,7 @@ TIMINGS = [("humanoid", 8192, 1.0 / 200.0, 8, 300, 30, lambda E: T.humanoid_stat
 def prepare():
     os.makedirs(RUN, exist_ok=True)
     lines = ["#!/bin/bash", "# written by tests/golden/make_ref_gpu_vectors.py", 'cd "$(dirname "$0")"',
-             'OUT="${OUT:-../../../gpurun_out}"', 'mkdir -p "$OUT"', ': > "$OUT/ref_timing.jsonl"']
+             'OUT="${OUT:-out}"', 'mkdir -p "$OUT"', ': > "$OUT/ref_timing.jsonl"']
     for name, (make, state, dt, iters, steps, every) in CASES.items():
         tb = make()
         with open(os.path.join(RUN, f"{name}.nks"), "w") as f:
@@ -182,6 +182,6 @@ if __name__ == "__main__":
     if len(sys.argv) >= 2 and sys.argv[1] == "prepare":
         prepare()
     elif len(sys.argv) >= 2 and sys.argv[1] == "collect":
-        collect(sys.argv[2] if len(sys.argv) > 2 else os.path.join(ROOT, "gpurun_out"))
+        collect(sys.argv[2] if len(sys.argv) > 2 else os.path.join(RUN, "out"))
     else:
         raise SystemExit(__doc__)
