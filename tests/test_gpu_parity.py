@@ -197,12 +197,13 @@ def test_benchmark_size_runs_are_reproducible(device):
     assert ends[0] == ends[1]
 
 
-def test_env_shards_equal_the_whole_batch(device):
-    """The property multi-GPU runs rest on, at configs[4]'s per-GPU size: 8192 quadruped + 4 boxes envs stepped as one
-    world and as two 4096-env shards (contiguous env ranges, as nuka.shard.env_range hands them out) end in
-    byte-identical state, so a sharded run equals the single-world run env for env."""
+@pytest.mark.parametrize("parts", [2, 8])
+def test_env_shards_equal_the_whole_batch(device, parts):
+    """The property multi-GPU runs rest on, at one GPU's share of 65536 envs: 8192 quadruped + 4 boxes envs stepped as one
+    world and as 4096-env (split steps, like the whole) or 1024-env shards (steps in one kernel; contiguous env ranges, as
+    nuka.shard.env_range hands them out) end in byte-identical state, so a sharded run equals the single-world run env for env."""
     from nuka import shard
-    E, parts = 8192, 2
+    E = 8192
     blob = T.quadruped(0, boxes=4).blob()
     st = T.quadruped_state(E, 4)
     fields = (F.JOINT_POSITION, F.JOINT_VELOCITY, F.BASE_POSE, F.RIGID_BODY_TRANSFORM, F.BODY_LINEAR_VELOCITY, F.CONTACT_COUNT)
@@ -245,8 +246,8 @@ def test_free_boxes_land_like_the_oracle(device, oracle):
     w.destroy()
 
 
-def test_full_box_pile_of_configs_3(device, oracle):
-    """configs[3]'s env at full size: 48 free boxes over a plane, 288 candidate slots, a contact-point capacity of
+def test_full_box_pile(device, oracle):
+    """The pile at full size: 48 free boxes over a plane, 288 candidate slots, a contact-point capacity of
     288 carried by the template.  Pair lists and contact counts bit-exact and poses within 1e-4 through the first
     landings (after which a tumbling pile amplifies rounding differences)."""
     E, count = 16, 48
@@ -267,7 +268,7 @@ def test_full_box_pile_of_configs_3(device, oracle):
 
 
 def test_quadruped_with_free_boxes(device, oracle):
-    """configs[4]'s env: the quadruped plus four free boxes (articulated and rigid blocks in one solve)."""
+    """The quadruped plus four free boxes (articulated and rigid blocks in one solve)."""
     E = 64
     st = T.quadruped_state(E, 4)
     w, o = make_pair(device, oracle, T.quadruped(0, boxes=4), E, {"q": st["q"], "base_pose": st["base_pose"]})
@@ -408,7 +409,7 @@ def test_torque_and_velocity_control_modes(device, oracle, mode):
 
 
 def test_humanoid_35_coordinates(device, oracle):
-    """configs[2]'s articulation: 30 links, 35 coordinates (two per warp lane), capsules on a plane and limb-limb
+    """The humanoid: 30 links, 35 coordinates (two per warp lane), capsules on a plane and limb-limb
     self-contact: mass matrix, accelerations, a single step and a short trajectory against the oracle.  Envs whose
     solve stops at the sweep limit (crossed legs pressing into each other) carry an unconverged state forward, which
     amplifies rounding differences, so the 2e-4 trajectory bound applies to the envs that converged in every step
