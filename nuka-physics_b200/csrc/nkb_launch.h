@@ -25,8 +25,8 @@ struct ResetParams {
 
 // Blocks of `warps_per_block` warps with `shared_bytes` of dynamic shared memory that one SM keeps resident (registers,
 // shared memory and block slots considered); 0 when the shape cannot launch.  The device must be current.
-// The step kernel has one variant per (coordinates per lane, free rigid bodies present) pair, chosen from `ndof`
-// (up to 32 / up to 64 coordinates) and `n_free` (free dynamic bodies per env).
+// The step kernel's variants follow the template: no articulation, up to 32 or up to 64 coordinates, with or without free bodies,
+// the controllers of modes 3 and 4 or not, no contacts at all; `slim` picks the 128-register build where there is one.
 int step_kernel_resident_blocks(const TemplateView& t, bool slim, uint32_t warps_per_block, size_t shared_bytes);
 // Whether a slim (128-register) build of the world's kernel variant exists.
 bool step_kernel_has_slim(const TemplateView& t);

@@ -1206,8 +1206,8 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
 // Blocks of one colour share no constraint row (index_blocks colours the graph whose edges are the two-sided heads), so
 // their descents touch disjoint head records and disjoint body velocities and may run side by side.  The env's lead warp
 // walks the descent order; for a run of rigid blocks of one colour it publishes a command in shared memory, and every
-// warp of the team (the lead included) takes the blocks member, member + team, ... of the run, each on Newton scratch of
-// its own.  A result does not depend on which warp ran a block, so team sizes give bit-identical states.
+// warp of the team (the lead included) takes its share of the run, 32 / body_lanes blocks at a time, in registers
+// (descend_bodies).  A result does not depend on which warp ran a block, so team sizes give bit-identical states.
 //
 // The warps meet through sequence numbers in shared memory, never through a hardware barrier: the lead bumps the
 // command's sequence number, a helper answers by copying it into its result record.  Every wait is bounded by a cycle

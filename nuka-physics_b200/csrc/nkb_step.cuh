@@ -148,8 +148,8 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
     }
 }
 
-// Register cap: measured on the 4096-env quadruped, the kernel runs fastest with about 150 registers and 12 warps per
-// SM; tighter caps (144 or 128 registers, 14 warps per SM) slow every warp by more than the extra residency returns.
+// Register cap of the regular builds: they settle at 160 registers without spills, three warps to a scheduler partition.  Which
+// worlds are worth a build of 128 registers and four warps is the slim build's question below.
 // NR = coordinates per lane: 1 for articulations of up to 32 coordinates, 2 for up to 64, 0 for worlds without one.
 // kRigid = the world has free rigid bodies; without them the rigid-block solver code is compiled out.
 // Worlds with free bodies are held to fewer resident warps by shared memory than by registers (38 KB per env and more),
@@ -160,9 +160,10 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 #ifndef NKB_MAXNREG_RIGID
 #define NKB_MAXNREG_RIGID 224
 #endif
-// The slim build of the same kernel: at 128 registers a fourth warp fits each scheduler partition, so small envs (15 KB
-// of shared memory) reach 15 resident warps per SM instead of 12 and 4096 envs need two rounds instead of 2.3.  It
-// spills about 200 bytes; a world takes it only where the extra residency is really there (World::BuildLayout).
+// The slim build of the same kernel: at 128 registers a fourth warp fits each scheduler partition, so small envs (14 KB
+// of shared memory) reach 16 resident warps per SM instead of 12.  It spills about 150 bytes; a world takes it only where the
+// extra residency is really there (World::BuildLayout).  The stages and the solve of split steps fit 128 registers without
+// spills (one coordinate per lane, no free bodies).
 // Worlds of bodies only run in teams of up to 8 warps, two piles to an SM: 128 registers for 16 warps, with 400 bytes of spills
 // (1024 piles of 48 boxes, 2 steps: 20.5 ms; 168 registers and teams of 6, 21.0; one pile to an SM, no spills, 26.6).
 #ifndef NKB_MAXNREG_BODIES
@@ -172,7 +173,7 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 #define NKB_MAXNREG_SLIM 128
 #endif
 // Warps that wait for one another after their solves and then go through the straight-line stages (the end of a step, the
-// start of the next) side by side, so that they share the fetches of their instructions: about 200 KB of code per step against
+// start of the next) side by side, so that they share the fetches of their instructions: about 230 KB of code per step against
 // the 128 KB an SM keeps at hand.  Warps at 15 different places of it are stalled on instruction fetch more than half of the
 // time (ncu: no_instruction 6.6 of 12.4 cycles per issue; 16 384 quadrupeds, 4 steps: 20.9 ms without any meeting).
 // Solves differ by a factor of three between envs, so a fixed group (a block-wide barrier) waits for its slowest member: 40 %

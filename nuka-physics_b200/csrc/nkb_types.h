@@ -146,7 +146,7 @@ struct SmemLayout {
     // bit 1 = helpers never answer a command.  Either way every wait runs out, a status bit is set and the kernel ends.
     uint32_t team_drill;
     uint32_t words;                                             // total per env
-    uint32_t ld;                                                // leading dimension of mass/factor (ndof | 1)
+    uint32_t ld;                // row stride of mass and factor: ndof padded to 4 mod 8 words; rows are read as float4 (tree_load_row)
 };
 
 // A step in one launch, or split around its constraint solve: the straight-line stages of all envs, then the solves.  kPartBare is

@@ -453,7 +453,7 @@ void World::BuildLayout() {
     const uint32_t share = (env_count_ + static_cast<uint32_t>(sms) - 1u) / static_cast<uint32_t>(sms);
     // The slim build pays 100 to 200 bytes of spills for a fourth warp per scheduler partition: worth it where shared memory lets
     // the extra warps in and the batch needs them, more envs to an SM than the regular build keeps (4 steps of 1000 quadrupeds, 7 to
-    // an SM: 1.31 ms regular, 1.47 slim; 41 of 150 arms: 1.52 and 1.59; 32 of 4096 arms, 28 to an SM: 3.9 and 3.1).
+    // an SM: 1.32 ms regular, 1.44 slim; 41 of 150 arms: 1.54 and 1.59; 32 of 4096 arms, 28 to an SM: 4.01 and 3.18).
     slim_ = has_slim && share > best[0] && best[1] * 10u >= best[0] * 12u;
     if (const char* forced = std::getenv("NUKA_B200_SLIM")) slim_ = has_slim && std::atoi(forced) != 0;     // variant experiments and tests
     const size_t* fits = resident[slim_ ? 1 : 0];
@@ -461,7 +461,7 @@ void World::BuildLayout() {
     // Block shape, and how its warps meet (Rally).  The largest block that keeps the most warps resident, or, for a batch that
     // does not fill the SMs, the largest that spreads it over all of them.  The warps of a block meet after each solve, all of
     // them, where their code outgrows the instruction cache: worlds with contacts, more than one env to a block (4 steps of 1000
-    // quadrupeds, blocks of 7: 2.01 ms apart, 1.80 in groups of 5, 1.47 all together).  Without contacts a step is short enough
+    // quadrupeds in the slim build, blocks of 7: 2.01 ms apart, 1.80 in groups of 5, 1.47 all together).  Without contacts a step is short enough
     // for the cache and the warps go their own ways (4096 arms, 32 steps: 3.30 ms apart, 3.49 together); where an SM holds four
     // warps or fewer, fetches are no bottleneck either.
     warps_per_block_ = team;
@@ -482,9 +482,9 @@ void World::BuildLayout() {
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
     // Split steps (see image_move): for batches that go over the SMs more than once, 12 envs to an SM and up.  Below, one kernel
-    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.74 ms in one kernel, 1.88
-    // split; 3000: 2.91 and 2.26; 1200 quadrupeds with 4 boxes: 3.08 and 3.28; 2400: 4.65 and 4.35; 1000 humanoids: 6.69 and
-    // 6.99; 2048: 9.50 and 8.61).
+    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.70 ms in one kernel, 1.90
+    // split; 3000: 2.86 and 2.24; 1000 humanoids: 6.30 and 6.85; 2048: 9.08 and 8.41).  With free bodies split steps pay earlier
+    // (1200 quadrupeds with 4 boxes: 4.05 and 3.68; 1776: 4.66 and 4.35; 2400: 5.83 and 5.11); one line serves both.
     stages_ = solve_ = nullptr;
     bool split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && share > 12u && env_count_ > static_cast<uint32_t>(sms) * most;
     if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && std::atoi(forced) != 0;
