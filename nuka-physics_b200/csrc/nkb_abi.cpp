@@ -99,10 +99,17 @@ void UnlockPages(void* p) { if (cudaFreeHost(p) != cudaSuccess) cudaGetLastError
 nkb::HostPool& Pool() { static auto* pool = new nkb::HostPool(LockPages, UnlockPages); return *pool; }
 std::atomic<uint64_t> g_world_serial{0};
 
+// A call that failed takes the runtime's record of its error along: a later launch of the thread, which reads that record, would
+// report it as its own.
+struct ClearsError { ~ClearsError() { if (failed) cudaGetLastError(); } bool failed = true; };
+
 template <typename Fn>
 nuka_result_t Guard(Fn&& fn) {
+    ClearsError record;
     try {
-        return fn();
+        const nuka_result_t result = fn();
+        record.failed = result != NUKA_RESULT_OK;
+        return result;
     } catch (const nkb::Error& e) {
         SetError(e.what());
         return static_cast<nuka_result_t>(e.code);

@@ -73,3 +73,21 @@ def test_templates_past_the_limits_are_rejected(device):
     assert lib.nuka_b200_template_check(blob, len(blob)) == nuka._abi.NOT_SUPPORTED
     with pytest.raises(nuka.NukaError):
         nuka.World.create_from_template(device, T.arm7(0).blob(), 0)       # an empty batch
+
+
+def test_a_world_that_does_not_fit_leaves_no_error_behind(device):
+    """A batch of two hundred million arms (6 GB for each array of joints) is refused for want of memory; the next world, a small
+    one, steps, and so does one that stood by."""
+    blob = T.arm7(0).blob()
+    by = nuka.World.create_from_template(device, blob, 2)
+    for _ in range(2):
+        with pytest.raises(nuka.NukaError) as err:
+            nuka.World.create_from_template(device, blob, 200_000_000)
+        assert err.value.code == nuka._abi.OUT_OF_MEMORY
+        by.step()
+        w = nuka.World.create_from_template(device, blob, 2)
+        w.step()
+        w.synchronize()
+        w.destroy()
+    by.synchronize()
+    by.destroy()
