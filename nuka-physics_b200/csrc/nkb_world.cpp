@@ -902,12 +902,12 @@ void World::SetContactReadout(bool on) {
     if (on) { s.pair_count = readout_.pair_count; s.pairs = readout_.pairs; s.contact_count = readout_.contact_count;
               s.contact_point = readout_.contact_point; s.contact_normal = readout_.contact_normal; s.contact_depth = readout_.contact_depth; }
     else {
+        const bool far = params_.sm.contacts_far != 0u;                   // the steps still need the place
+        const size_t words = static_cast<size_t>(env_count_) * params_.t.cfg.max_contacts * 12u;
+        if (far && far_point_ == nullptr) far_point_ = Alloc<float>(words);
+        if (far && far_normal_ == nullptr) far_normal_ = Alloc<float>(words);      // without room the read-out stays on
         readout_ = s; s.pair_count = nullptr;
-        if (params_.sm.contacts_far != 0u) {           // the steps still need the place
-            const size_t words = static_cast<size_t>(env_count_) * params_.t.cfg.max_contacts * 12u;
-            if (far_point_ == nullptr) { far_point_ = Alloc<float>(words); far_normal_ = Alloc<float>(words); }
-            s.contact_point = far_point_; s.contact_normal = far_normal_;
-        }
+        if (far) { s.contact_point = far_point_; s.contact_normal = far_normal_; }
     }
     graph_valid_ = false;
 }

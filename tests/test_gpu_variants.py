@@ -222,6 +222,38 @@ def test_read_out_keeps_its_last_values_while_off(device, shapes):
     w.destroy()
 
 
+@pytest.mark.parametrize("room", [0.5, 1.5])
+def test_read_out_stays_on_where_the_contacts_find_no_other_place(device, shapes, room):
+    """The points and the normals need an array each while the read-out is off; with room for neither or for one of them the call
+    fails and changes nothing, and succeeds later."""
+    torch = pytest.importorskip("torch")
+    E = 4096
+    tb, st = T.box_pile(0, count=48), T.box_pile_state(E, 0, count=48)
+    on = outputs(create(device, tb, st, E), (3, 2, 2))
+    w = create(device, tb, st, E)
+    assert all(x["far"] for x in shapes())
+    w.step_n(3)
+    w.synchronize()
+    size = on["CONTACT_POINT"].nbytes
+    assert size > 16 << 20
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info(0)[0] - int(room * size), dtype=torch.uint8, device="cuda:0")
+    before = w.download(F.CONTACT_POINT)
+    with pytest.raises(nuka.NukaError):
+        w.set_contact_readout(False)
+    w.step_n(2)
+    assert not np.array_equal(w.download(F.CONTACT_POINT), before)                # still written
+    del fill
+    torch.cuda.empty_cache()
+    w.set_contact_readout(False)
+    w.step_n(1)
+    w.set_contact_readout(True)
+    w.step_n(1)
+    for k, v in on.items():
+        assert np.array_equal(v, w.download(F[k])), k
+    w.destroy()
+
+
 def test_downloads_outlive_the_world_and_one_another(device):
     E = 64
     w = create(device, T.quadruped(0), T.quadruped_state(E, 1), E)
