@@ -250,13 +250,19 @@ NKB_DEV bool solve6(float (&a)[21], Sum (&g)[6], float (&inv)[6], float (&x)[6])
     return valid;
 }
 
-// Two sums over the warp at the price of one and two broadcasts: the halves of the warp carry one each after the first exchange.
-NKB_DEV void warp_sum2(float& a, float& b, uint32_t lane) {
+// The sums of a line evaluation, `rows` and the pair a, b, over the first 2 * half lanes (the others hold zeros), in every lane.  The
+// halves of the warp carry one of the pair each after the first exchange.
+NKB_DEV void line_sums(double& rows, float& a, float& b, uint32_t half, uint32_t lane) {
     const bool upper = (lane & 16u) != 0u;
     float keep = upper ? b : a;
     keep += __shfl_xor_sync(NKB_FULL, upper ? a : b, 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(NKB_FULL, keep, o);
+    if (half > 8u) rows += __shfl_xor_sync(NKB_FULL, rows, 16);
+#pragma unroll 1
+    for (uint32_t o = min(half, 8u); o > 0u; o >>= 1) {
+        keep += __shfl_xor_sync(NKB_FULL, keep, o);
+        rows += __shfl_xor_sync(NKB_FULL, rows, o);
+    }
+    rows = __shfl_sync(NKB_FULL, rows, 0);
     a = __shfl_sync(NKB_FULL, keep, 0);
     b = __shfl_sync(NKB_FULL, keep, 16);
 }

@@ -181,11 +181,20 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
         }
     }
     __syncwarp();
-    // joint rows, lane = link: limit lower/upper, dry friction, drive (ops/assemble_rows.cu:805-971)
+    // joint rows, lane = link: limit lower/upper, dry friction, drive (ops/assemble_rows.cu:805-971).  A drive's row has equal
+    // bounds: its impulse is that bound whatever the velocities do, and it adds no stiffness.  So it is no head of the solve: its impulse
+    // waits in a vector by coordinate.
+    if (NR > 0) {
+        float* fixed = sm_vec(e, kVecFixed);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) fixed[lane + 32u * r] = 0.f;
+        __syncwarp();
+        if (lane < L && joint_dofs(e.jtype) == 1u) fixed[e.link_dof] = fminf(fmaxf(e.drive_command, e.drive_lower), e.drive_upper) * dt;
+    }
 #pragma unroll 1
-    for (uint32_t kind = 0u; kind < 4u; ++kind) {
+    for (uint32_t kind = 0u; kind < 3u; ++kind) {
         bool emit = false;
-        float lower = 0.f, upper = 0.f, rhs = 0.f, pen = 0.f, unitv = 1.f, lambda = 0.f;
+        float lower = 0.f, upper = 0.f, rhs = 0.f, pen = 0.f, unitv = 1.f;
         uint32_t flags = 0u;
         if (lane < L && joint_dofs(e.jtype) == 1u) {
             const uint32_t lf = __ldg(t.limit_flags + lane);
@@ -199,9 +208,6 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             } else if (kind == 2u) {
                 const float fr = __ldg(t.frictionloss + lane);
                 if (fr > 0.f) { emit = true; flags = kHeadFriction | kHeadVelocityOnly; lower = -fr * dt; upper = fr * dt; }
-            } else if (kind == 3u) {
-                const float effort = fminf(fmaxf(e.drive_command, e.drive_lower), e.drive_upper);
-                if (effort != 0.f) { emit = true; flags = kHeadDrive | kHeadVelocityOnly; lower = upper = effort * dt; lambda = lower; }
             }
         }
         // limit rows interleave lower/upper per link: kinds 0 and 1 are placed together
@@ -253,7 +259,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
                 hf(e, HF_UNITV, h) = unitv;
                 hf(e, HF_LOWER, h) = lower; hf(e, HF_UPPER, h) = upper; hf(e, HF_MU, h) = 0.f;
                 hf(e, HF_PEN, h) = pen; hf(e, HF_RHS, h) = rhs;
-                hst3(e, HF_DUAL, h, mk3(lambda, 0.f, 0.f));
+                hst3(e, HF_DUAL, h, mk3(0.f, 0.f, 0.f));
             }
         }
         nheads = min(nheads + __popc(mask), t.head_cap);

@@ -26,17 +26,18 @@ constexpr float kImpulseRounding = 1.0f / kRoundings;
 
 struct Tile {
     uint32_t nheads, nblocks, iteration;
+    bool units;                         // there are rows on a single coordinate
     float momentum, residual, tol;
 };
 
 NKB_DEV uint32_t* sm_binfo(const Env& e) { return reinterpret_cast<uint32_t*>(e.sm + e.lay->binfo); }
-// binfo words: dim[nb], color[nb], inc_begin[nb + 1], inc[2 * head_cap], utab[4 * vstride], order[nb + 1]
+// binfo words: dim[nb], color[nb], inc_begin[nb + 1], inc[2 * head_cap], utab[3 * vstride, 16 bits each], order[nb + 1]
 NKB_DEV uint32_t& blk_dim(const Env& e, uint32_t b) { return sm_binfo(e)[b]; }
 NKB_DEV uint32_t& blk_color(const Env& e, uint32_t nb, uint32_t b) { return sm_binfo(e)[nb + b]; }
 NKB_DEV uint32_t& blk_inc_begin(const Env& e, uint32_t nb, uint32_t b) { return sm_binfo(e)[2u * nb + b]; }
 NKB_DEV uint32_t* blk_inc(const Env& e, uint32_t nb) { return sm_binfo(e) + 3u * nb + 1u; }
 // unit rows of the articulation by coordinate: utab[slot * vstride + coordinate] = head or 0xffff (slots: lower limit,
-// upper limit, dry friction, drive; vstride = 32 or 64 coordinates), 16-bit entries
+// upper limit, dry friction; vstride = 32 or 64 coordinates), 16-bit entries
 constexpr uint32_t kNoUnitHead = 0xffffu;
 NKB_DEV uint16_t* unit_table(const Env& e, uint32_t nb) { return reinterpret_cast<uint16_t*>(sm_binfo(e) + 3u * nb + 1u + 2u * e.t->head_cap); }
 // moving blocks in descent order, order[nb] = their count
@@ -279,14 +280,16 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
     __syncwarp();
 }
 
-// Incidence lists (heads of each block in head order) and greedy colours.
-NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
+// Incidence lists (heads of each block in head order) and greedy colours.  Without free bodies the articulation is the only block.
+template <bool kRigid>
+NKB_DEV void index_blocks(Env& e, Tile& tile, bool color) {
     const uint32_t nb = tile.nblocks;
     uint32_t* inc = blk_inc(e, nb);
     uint32_t at = 0u;
 #pragma unroll 1
-    for (uint32_t b = 0u; b < nb; ++b) {
+    for (uint32_t b = kRigid ? 0u : nb - 1u; b < nb; ++b) {
         if (e.lane == 0u) blk_inc_begin(e, nb, b) = at;
+        if (kRigid && blk_dim(e, b) == 0u) continue;                // no row acts on a block that does not move
 #pragma unroll 1
         for (uint32_t base = 0u; base < tile.nheads; base += 32u) {
             const uint32_t h = base + e.lane;
@@ -298,18 +301,28 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
         }
     }
     if (e.lane == 0u) blk_inc_begin(e, nb, nb) = at;
-    uint16_t* utab = unit_table(e, nb);
-#pragma unroll 1
-    for (uint32_t k = e.lane; k < 4u * e.vstride; k += 32u) utab[k] = (uint16_t)kNoUnitHead;
     __syncwarp();
+    // contact heads come first in an incidence list, rows on a single coordinate last
+    tile.units = at != 0u && (hu(e, HF_JOFF, inc[at - 1u]) & kUnitRow) != 0u && ((hu(e, HF_OWNER, inc[at - 1u]) & 0xffffu) == e.t->B);
+    if (tile.units) {
+        uint16_t* utab = unit_table(e, nb);
 #pragma unroll 1
-    for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
-        const uint32_t jo = hu(e, HF_JOFF, h), o = hu(e, HF_OWNER, h), fl = hu(e, HF_FLAGS, h);
-        if (!(jo & kUnitRow) || ((o & 0xffffu) != e.t->B && (o >> 16) != e.t->B)) continue;
-        const uint32_t slot = (fl & kHeadDrive) ? 3u : (fl & kHeadFriction) ? 2u : hf(e, HF_UNITV, h) < 0.f ? 1u : 0u;
-        utab[slot * e.vstride + (jo & 0xffffu)] = (uint16_t)h;
+        for (uint32_t k = e.lane; k < 3u * e.vstride; k += 32u) utab[k] = (uint16_t)kNoUnitHead;
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
+            const uint32_t jo = hu(e, HF_JOFF, h), o = hu(e, HF_OWNER, h), fl = hu(e, HF_FLAGS, h);
+            if (!(jo & kUnitRow) || ((o & 0xffffu) != e.t->B && (o >> 16) != e.t->B)) continue;
+            const uint32_t slot = (fl & kHeadFriction) ? 2u : hf(e, HF_UNITV, h) < 0.f ? 1u : 0u;
+            utab[slot * e.vstride + (jo & 0xffffu)] = (uint16_t)h;
+        }
+        __syncwarp();
     }
-    __syncwarp();
+    if constexpr (!kRigid) {
+        if (color && e.lane == 0u) { block_order(e, nb)[0] = nb - 1u; block_order(e, nb)[nb] = 1u; }
+        __syncwarp();
+        return;
+    }
     if (!color) return;
     uint32_t colours = 0u;       // 1 + the largest colour in use
 #pragma unroll 1
@@ -348,26 +361,23 @@ NKB_DEV void index_blocks(Env& e, const Tile& tile, bool color) {
     __syncwarp();
 }
 
-// residual = rhs dt - J u at the blocks' current velocities (block_descent_tile.cuh:891-930)
+// residual = rhs dt - J u at the blocks' current velocities (block_descent_tile.cuh:891-930); lane = axis of a head
 NKB_DEV void init_residuals(Env& e, const Tile& tile) {
     const TemplateView& t = *e.t;
     const float dt = t.cfg.dt;
 #pragma unroll 1
-    for (uint32_t h = e.lane; h < tile.nheads; h += 32u) {
-        const uint32_t axes = head_axes(e, h);
-        V3 res = mk3(0.f, 0.f, 0.f);
-#pragma unroll 1
-        for (uint32_t ax = 0u; ax < axes; ++ax) {
-            float along = 0.f;
+    for (uint32_t k = e.lane; k < 3u * tile.nheads; k += 32u) {
+        const uint32_t h = k / 3u, ax = k - 3u * h;
+        float along = 0.f;
+        const bool live = ax < head_axes(e, h);
+        if (live)
 #pragma unroll 1
             for (uint32_t side = 0u; side < 2u; ++side) {
                 const uint32_t b = head_owner(e, h, side);
                 if (b == kNoBlock16) continue;
                 along += head_row_dot(e, h, side, ax, b, block_vel(e, b, false));
             }
-            setc(res, (int)ax, (ax == 0u ? hf(e, HF_RHS, h) * dt : 0.f) - along);
-        }
-        hst3(e, HF_RES, h, res);
+        hf(e, HF_RES + ax, h) = live ? (ax == 0u ? hf(e, HF_RHS, h) * dt : 0.f) - along : 0.f;
     }
     __syncwarp();
 }
@@ -399,37 +409,28 @@ NKB_DEV void respond(const HeadRegs& r, V3 move, V3& f, float& cxx, float& cyy, 
     if (r.cone) cone_impulse(r.dual, r.rho, r.res.y - move.y, r.res.z - move.z, r.dual.x, r.mu, f.y, f.z, cyy, czz, cyz);
 }
 
-// Row steps J d of a block's incident heads (block_descent_tile.cuh:2019-2044); lane = head, d staged in shared
+// Row steps J d of the articulation's incident heads (block_descent_tile.cuh:2019-2044); lane = axis of a head, d staged in shared
 // memory with zeros past the block's dimension.
-NKB_DEV void row_steps(Env& e, const Tile& tile, uint32_t b, const float* dvec) {
-    const uint32_t nb = tile.nblocks, dim = blk_dim(e, b);
-    const uint32_t* inc = blk_inc(e, nb);
-    const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
+NKB_DEV void row_steps(Env& e, const uint32_t* inc, uint32_t ib, uint32_t ie, uint32_t dim, const float* dvec) {
     const uint32_t chunks = (dim + 3u) >> 2;
     const float4* d4 = reinterpret_cast<const float4*>(dvec);
 #pragma unroll 1
-    for (uint32_t k = ib + e.lane; k < ie; k += 32u) {
-        const uint32_t h = inc[k];
-        const bool cone = head_axes(e, h) == 3u;
-        V3 step = mk3(0.f, 0.f, 0.f);
+    for (uint32_t k = e.lane; k < 3u * (ie - ib); k += 32u) {
+        const uint32_t at = k / 3u, ax = k - 3u * at, h = inc[ib + at];
         const uint32_t jo = hu(e, HF_JOFF, h);
-        if (jo & kUnitRow) step.x = hf(e, HF_UNITV, h) * dvec[jo & 0xffffu];
-        else {
-            const float4* j4 = reinterpret_cast<const float4*>(sm_jpool(e) + jo);
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        float s = 0.f;
+        if (ax < head_axes(e, h)) {
+            if (jo & kUnitRow) s = hf(e, HF_UNITV, h) * dvec[jo & 0xffffu];
+            else {
+                const float4* j4 = reinterpret_cast<const float4*>(sm_jpool(e) + jo) + ax * chunks;
 #pragma unroll 1
-            for (uint32_t c = 0u; c < chunks; ++c) {
-                const float4 d = d4[c], r0 = j4[c];
-                s0 = fmaf(r0.x, d.x, s0); s0 = fmaf(r0.y, d.y, s0); s0 = fmaf(r0.z, d.z, s0); s0 = fmaf(r0.w, d.w, s0);
-                if (cone) {
-                    const float4 r1 = j4[chunks + c], r2 = j4[2u * chunks + c];
-                    s1 = fmaf(r1.x, d.x, s1); s1 = fmaf(r1.y, d.y, s1); s1 = fmaf(r1.z, d.z, s1); s1 = fmaf(r1.w, d.w, s1);
-                    s2 = fmaf(r2.x, d.x, s2); s2 = fmaf(r2.y, d.y, s2); s2 = fmaf(r2.z, d.z, s2); s2 = fmaf(r2.w, d.w, s2);
+                for (uint32_t c = 0u; c < chunks; ++c) {
+                    const float4 d = d4[c], r = j4[c];
+                    s = fmaf(r.x, d.x, s); s = fmaf(r.y, d.y, s); s = fmaf(r.z, d.z, s); s = fmaf(r.w, d.w, s);
                 }
             }
-            step = mk3(s0, s1, s2);
         }
-        hst3(e, HF_STEP, h, step);
+        hf(e, HF_STEP + ax, h) = s;
     }
     __syncwarp();
 }
@@ -448,8 +449,8 @@ NKB_DEV void line_terms(const HeadRegs& r, float alpha, CSum& rs, float& rc, flo
 
 // Exact line search on the block's one-dimensional model (block_descent_tile.cuh:2048-2125): the first
 // evaluation (alpha = 0) gives the initial slope, the following ones bracket and polish the root.  With at most
-// 32 incident heads each lane keeps its head in registers for the whole search.
-NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, float icurv) {
+// 32 incident heads each lane keeps its head in registers for the whole search.  `fixed` is the constant impulses' slope.
+NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, float icurv, float fixed, float fixed_size) {
     const uint32_t nb = tile.nblocks;
     const uint32_t* inc = blk_inc(e, nb);
     const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
@@ -467,10 +468,10 @@ NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, fl
 #pragma unroll 1
         for (uint32_t k = ib + e.lane; k < ie; k += 32u) { const HeadRegs r = load_head(e, inc[k]); line_terms(r, alpha, rs, rc, rm); }
         CSum total = {-rs.value, -rs.error};
-        if (e.lane == 0u) { csum_addp(total, alpha, icurv); csum_add(total, islope); }
+        if (e.lane == 0u) { csum_addp(total, alpha, icurv); csum_add(total, islope); csum_add(total, -fixed); }
         const float slope = warp_csum_total(total);
         const float curvature = icurv + warp_sum(rc);
-        const float magnitude = fabsf(islope) + alpha * icurv + warp_sum(rm);
+        const float magnitude = fabsf(islope) + alpha * icurv + fixed_size + warp_sum(rm);
         if (step < 0) {
             initial = slope;
             if (!(initial < 0.0f)) { have = true; result = 0.0f; break; }
@@ -539,9 +540,10 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     }
     coupled = __any_sync(NKB_FULL, coupled);
     __syncwarp();
-    float start[NR], fr[NR], u[NR];
+    float start[NR], fr[NR], u[NR], fixed[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
+        fixed[r] = position || !coord[r] ? 0.f : sm_vec(e, kVecFixed)[l + 32u * r];
         start[r] = coord[r] ? velocity[l + 32u * r] : 0.f;
         fr[r] = (coord[r] && !position) ? block_free(e, b)[l + 32u * r] : 0.f;
         u[r] = start[r];
@@ -609,13 +611,13 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             }
             tick(e, 16);
             // rows on a single coordinate only touch that coordinate (block_descent_tile.cuh:1555-1568)
-            {
+            if (tile.units) {
                 const uint16_t* utab = unit_table(e, nb);
                 const uint32_t vs = e.vstride;
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
 #pragma unroll 1
-                    for (uint32_t slot = 0u; slot < 4u; ++slot) {
+                    for (uint32_t slot = 0u; slot < 3u; ++slot) {
                         const uint32_t h = utab[slot * vs + l + 32u * r];
                         if (h == kNoUnitHead) continue;
                         const float v = hf(e, HF_UNITV, h);
@@ -625,6 +627,8 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                     }
                 }
             }
+#pragma unroll
+            for (int r = 0; r < NR; ++r) { csum_add(g[r], fixed[r]); scale[r] += fabsf(fixed[r]); }
             // dense rows: H += J^T C J, g += J^T f, one head at a time with its values broadcast from shared memory
             if (__any_sync(NKB_FULL, dense_any != 0u)) {
 #pragma unroll 1
@@ -769,7 +773,8 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) dvec[l + 32u * r] = d[r];
         __syncwarp();
-        CSum dec = {0.f, 0.f}, slo = {0.f, 0.f}, cur = {0.f, 0.f};
+        CSum dec = {0.f, 0.f}, slo = {0.f, 0.f}, cur = {0.f, 0.f}, fix = {0.f, 0.f};
+        float fix_size = 0.f;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             float ms = 0.f;
@@ -780,7 +785,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                     const float4 m = Mr4[c], dd = reinterpret_cast<const float4*>(dvec)[c];
                     ms = fmaf(m.x, dd.x, ms); ms = fmaf(m.y, dd.y, ms); ms = fmaf(m.z, dd.z, ms); ms = fmaf(m.w, dd.w, ms);
                 }
-                csum_addp(dec, force[r], d[r]); csum_addp(slo, inertia[r], d[r]); csum_addp(cur, d[r], ms);
+                csum_addp(dec, force[r], d[r]); csum_addp(slo, inertia[r], d[r]); csum_addp(cur, d[r], ms); csum_addp(fix, fixed[r], d[r]); fix_size += fabsf(fixed[r] * d[r]);
             }
         }
         const float icurv = warp_csum_total(cur);
@@ -795,9 +800,9 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             if (!(total_dec > 0.f)) break;
         }
         tick(e, 20);
-        row_steps(e, tile, b, dvec);
+        row_steps(e, inc, ib, ie, dim, dvec);
         tick(e, 21);
-        const float alpha = search_line(e, tile, b, islope, icurv);
+        const float alpha = search_line(e, tile, b, islope, icurv, warp_csum_total(fix), warp_sum(fix_size));
         tick(e, 22);
         tick_count(e, 23);
         if (step < 0) {
@@ -873,13 +878,26 @@ NKB_DEV void evaluate_head(const Env& e, uint32_t h, float alpha, double& slope,
     hq(e, HF_C + 1u, h) = make_float4(cyy, czz, cyz, noise.x);
     *reinterpret_cast<float2*>(&hf(e, HF_NZ + 1u, h)) = make_float2(noise.y, noise.z);
 }
-// The rows of a block, lane = head, as many passes as the block has heads.
-NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint32_t ie, float alpha, double& slope, float& curvature, float& magnitude) {
+// The rows of a block, lane = head, as many passes as the block has heads; 2 * half lanes take part.
+NKB_DEV void evaluate_line(const Env& e, const uint32_t* inc, uint32_t ib, uint32_t ie, uint32_t half, float alpha, double& slope, float& curvature, float& magnitude) {
     slope = 0.0; curvature = 0.f; magnitude = 0.f;
 #pragma unroll 1
     for (uint32_t k = ib + e.lane; k < ie; k += 32u) evaluate_head(e, inc[k], alpha, slope, curvature, magnitude);
-    slope = warp_sum(slope);
-    warp_sum2(curvature, magnitude, e.lane);
+    line_sums(slope, curvature, magnitude, half, e.lane);
+}
+
+// Row c of the mass matrix times a vector in shared memory (zeros past the last coordinate), in 64 bits.
+NKB_DEV double mass_row_times(const Env& e, uint32_t c, uint32_t chunks, const double* v) {
+    const float4* m4 = reinterpret_cast<const float4*>(sm_mass(e) + c * e.lay->ld);
+    const double2* v2 = reinterpret_cast<const double2*>(v);
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 1
+    for (uint32_t k = 0u; k < chunks; ++k) {
+        const float4 m = m4[k];
+        const double2 a = v2[2u * k], z = v2[2u * k + 1u];
+        s0 = fma((double)m.x, a.x, s0); s1 = fma((double)m.y, a.y, s1); s0 = fma((double)m.z, z.x, s0); s1 = fma((double)m.w, z.y, s1);
+    }
+    return s0 + s1;
 }
 
 // The articulation's descent with the Newton system kept in the sparsity of its tree (nkb_tree.cuh).  Same model, stopping
@@ -922,8 +940,8 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
     int step = tile.iteration == 0u && !position ? -1 : -2;
     bool coord[NR];
     double u[NR], dir[NR], inertial[NR];
-    float force[NR];
-    uint32_t units[NR][2];              // this coordinate's single-coordinate rows: heads by slot, two per word
+    float force[NR], fixed[NR];
+    const uint32_t half = ie - ib <= 1u ? 0u : min(16u, 1u << (31 - __clz(ie - ib - 1u)));        // of the lanes with a head
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
         const uint32_t c = l + 32u * r;
@@ -932,9 +950,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         const double fr = coord[r] && !position ? (double)block_free(e, b)[c] : 0.0;
         dir[r] = step == -1 ? fr - u[r] : u[r] - fr;
         inertial[r] = 0.0; force[r] = 0.f;
-        const uint16_t* utab = unit_table(e, nb) + c;
-        units[r][0] = utab[0] | ((uint32_t)utab[e.vstride] << 16);
-        units[r][1] = utab[2u * e.vstride] | ((uint32_t)utab[3u * e.vstride] << 16);
+        fixed[r] = position || !coord[r] ? 0.f : sm_vec(e, kVecFixed)[c];
     }
     bool failure = false;
     float primal = FLT_MAX;
@@ -946,30 +962,25 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) { wide[l + 32u * r] = dir[r]; flat[l + 32u * r] = (float)dir[r]; }
         __syncwarp();
-        double md[NR], along = 0.0, cur = 0.0, slo = 0.0;
+        double md[NR], sums[4] = {0.0, 0.0, 0.0, 0.0};             // along d: curvature, inertial slope, force, constant impulses
+        float fixed_size = 0.f;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            double s0 = 0.0, s1 = 0.0;
-            if (coord[r]) {
-                const float4* m4 = reinterpret_cast<const float4*>(sm_mass(e) + (l + 32u * r) * e.lay->ld);
-                const double2* d2 = reinterpret_cast<const double2*>(wide);
-#pragma unroll 1
-                for (uint32_t c = 0u; c < chunks; ++c) {
-                    const float4 m = m4[c];
-                    const double2 a = d2[2u * c], z = d2[2u * c + 1u];
-                    s0 = fma((double)m.x, a.x, s0); s1 = fma((double)m.y, a.y, s1); s0 = fma((double)m.z, z.x, s0); s1 = fma((double)m.w, z.y, s1);
-                }
-            }
-            md[r] = s0 + s1;
-            cur = fma(dir[r], md[r], cur);
-            slo = fma(inertial[r], dir[r], slo);
-            along = fma((double)force[r], dir[r], along);
+            md[r] = coord[r] ? mass_row_times(e, l + 32u * r, chunks, wide) : 0.0;
+            sums[0] = fma(dir[r], md[r], sums[0]);
+            sums[1] = fma(inertial[r], dir[r], sums[1]);
+            sums[2] = fma((double)force[r], dir[r], sums[2]);
+            sums[3] = fma((double)fixed[r], dir[r], sums[3]);
+            fixed_size = fmaf(fabsf(fixed[r]), fabsf((float)dir[r]), fixed_size);
         }
         bool search = step > -2;
         double icurv = 0.0, islope = 0.0;
         float initial = 0.f, alpha = 0.f;
         if (search) {
-            icurv = warp_sum(cur);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sums[k] = warp_sum(sums[k]);
+            fixed_size = warp_sum(fixed_size);
+            icurv = sums[0];
             if (step < 0) {
 #pragma unroll
                 for (int r = 0; r < NR; ++r) inertial[r] = -md[r];
@@ -977,14 +988,14 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
                 search = icurv > 0.0 && icurv <= FLT_MAX;
             } else {
                 // d solves H d = force, so the slope at alpha = 0 is -(force . d)
-                initial = -(float)warp_sum(along);
-                islope = warp_sum(slo);
+                initial = -(float)sums[2];
+                islope = sums[1];
                 if (!isfinite(initial) || !(fabs(islope) <= FLT_MAX) || !(icurv <= FLT_MAX)) { failure = true; break; }
                 if (!(initial < 0.f)) break;
                 alpha = 1.f;
             }
             tick(e, 20);
-            row_steps(e, tile, b, flat);
+            row_steps(e, inc, ib, ie, dim, flat);
             tick(e, 21);
         } else {
 #pragma unroll
@@ -998,10 +1009,10 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
 #pragma unroll 1
             for (;;) {
                 double rows; float curvature, magnitude;
-                evaluate_line(e, inc, ib, ie, alpha, rows, curvature, magnitude);
+                evaluate_line(e, inc, ib, ie, half, alpha, rows, curvature, magnitude);
                 tick_count(e, 28);
                 if (!search) break;
-                const float slope = (float)(islope + (double)alpha * icurv - rows);
+                const float slope = (float)(islope + (double)alpha * icurv - (rows + sums[3]));
                 curvature += (float)icurv;
                 if (initial == 0.f) {                      // the first sweep's search starts by measuring its initial slope
                     initial = slope;
@@ -1009,7 +1020,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
                     alpha = 1.f;
                     continue;
                 }
-                magnitude += fabsf((float)islope) + alpha * (float)icurv;
+                magnitude += fabsf((float)islope) + alpha * (float)icurv + fixed_size;
                 bool give_up = ++trials >= (int)kLineSteps;
                 if (isfinite(slope) && isfinite(curvature)) {
                     if (fabsf(slope) <= fmaxf(kLineTol * -initial, kRoundings * FLT_EPSILON * magnitude)) break;
@@ -1070,20 +1081,17 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         for (int r = 0; r < NR; ++r) {
             g[r] = -inertial[r]; scale[r] = fabsf((float)inertial[r]); diag[r] = 0.f;
             // rows on a single coordinate only touch that coordinate (block_descent_tile.cuh:1555-1568)
+            if (tile.units)
 #pragma unroll 1
-            for (uint32_t pair = 0u; pair < 2u; ++pair) {
-                uint32_t two = pair == 0u ? units[r][0] : units[r][1];
-#pragma unroll 1
-                while (two != (kNoUnitHead | (kNoUnitHead << 16))) {
-                    const bool first = (two & 0xffffu) != kNoUnitHead;
-                    const uint32_t h = first ? two & 0xffffu : two >> 16;
-                    two |= first ? kNoUnitHead : kNoUnitHead << 16;
+                for (uint32_t slot = 0u; slot < 3u; ++slot) {
+                    const uint32_t h = unit_table(e, nb)[slot * e.vstride + l + 32u * r];
+                    if (h == kNoUnitHead) continue;
                     const float v = hf(e, HF_UNITV, h);
                     diag[r] += v * hf(e, HF_C, h) * v;
                     g[r] = fma((double)v, (double)hf(e, HF_F, h), g[r]);
                     scale[r] += fabsf(v) * hf(e, HF_NZ, h);
                 }
-            }
+            g[r] += (double)fixed[r]; scale[r] += fabsf(fixed[r]);
         }
         const int depth = (int)t.tree_depth;
         __syncwarp();
@@ -1661,7 +1669,7 @@ NKB_DEV RigidResult descend_share(const RigidRun& run, uint32_t k_begin, uint32_
 NKB_DEV void team_dismiss(float* sm, const SmemLayout& lay, uint32_t lane) {
     if (lay.team <= 1u) return;
     Tile none;
-    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
+    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
     team_post(sm, lay, lane, kTeamExit, 0u, 0u, false, none);
 }
 
@@ -1673,7 +1681,7 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
     const uint32_t team = e.lay->team;
     if (team <= 1u || team_command(e.sm, *e.lay)->dead != 0u) { work(0u, 1u); return; }
     Tile none;
-    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
+    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
     const uint32_t seq = team_post(e.sm, *e.lay, e.lane, op, count, 0u, false, none);
     work(0u, team);
     if (team_collect(e.sm, *e.lay, e.lane, seq)) {
@@ -1914,22 +1922,23 @@ NKB_DEV void measure_articulation(Env& e, Tile& tile, bool reconstruct) {
     bool coord[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) { balance[r] = 0.0; coord[r] = l + 32u * r < dim; }
+    double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
+#pragma unroll
+    for (int r = 0; r < NR; ++r) wide[l + 32u * r] = coord[r] ? (double)vel[l + 32u * r] - fr[l + 32u * r] : 0.0;
+    __syncwarp();
     {
         const uint32_t n4 = (dim + 3u) & ~3u;
-        const uint16_t* utab = unit_table(e, nb);
-        const uint32_t vs = e.vstride;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const uint32_t c = l + 32u * r;
             if (!coord[r]) continue;
-            const float* Mr = sm_mass(e) + c * e.lay->ld;
+            balance[r] = (double)sm_vec(e, kVecFixed)[c] - mass_row_times(e, c, n4 >> 2, wide);
+            if (tile.units)
 #pragma unroll 1
-            for (uint32_t j = 0u; j < dim; ++j) balance[r] -= (double)Mr[j] * ((double)vel[j] - fr[j]);
-#pragma unroll 1
-            for (uint32_t slot = 0u; slot < 4u; ++slot) {
-                const uint32_t h = utab[slot * vs + c];
-                if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAMX, h);
-            }
+                for (uint32_t slot = 0u; slot < 3u; ++slot) {
+                    const uint32_t h = unit_table(e, nb)[slot * e.vstride + c];
+                    if (h != kNoUnitHead) balance[r] += (double)hf(e, HF_UNITV, h) * hf(e, HF_LAMX, h);
+                }
         }
 #pragma unroll 1
         for (uint32_t k = ib; k < ie; ++k) {
@@ -1984,9 +1993,10 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, B = t.B, n = NR > 0 ? t.ndof : 0u;
     Tile tile;
-    tile.nheads = nheads; tile.nblocks = B + (n != 0u ? 1u : 0u); tile.iteration = 0u;
+    tile.nheads = nheads; tile.nblocks = B + (n != 0u ? 1u : 0u); tile.iteration = 0u; tile.units = false;
     tile.momentum = tile.residual = 0.f; tile.tol = t.cfg.velocity_tolerance;
     // rigid blocks: free velocity, mass, carried constraint velocity (block_descent_rigid.cuh:4-48)
+    if constexpr (kRigid)
 #pragma unroll 1
     for (uint32_t b = l; b < B; b += 32u) {
         float* bv = sm_bvel(e, b);
@@ -2052,7 +2062,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
 #pragma unroll 1
     while (phase != kPhaseDone) {
         if (reindex) {
-            index_blocks(e, tile, phase == kPhaseVelocity);
+            index_blocks<kRigid>(e, tile, phase == kPhaseVelocity);
             reindex = false;
             if (phase == kPhaseVelocity) { init_residuals(e, tile); tick(e, 9); if (iterations == 0u) phase = kPhaseHandOver; }
         }
@@ -2072,6 +2082,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
                 }
                 if (l < t.L && joint_dofs(e.jtype) == 1u) e.qd = U[e.link_dof];
             }
+            if constexpr (kRigid)
 #pragma unroll 1
             for (uint32_t b = l; b < B; b += 32u) {
                 float* carry = e.s->carry_rigid + ((size_t)e.env * B + b) * 6u;

@@ -110,24 +110,19 @@ NKB_DEV void stage_integrate_bodies(Env& e, bool use_pseudo) {
     __syncwarp();
 }
 
-// Applied drive efforts from the solved drive multipliers (ops/articulation.cu:999-1016).
+// Applied drive efforts from the drives' impulses (ops/articulation.cu:999-1016).
 NKB_DEV void stage_readout_drives(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
-    float* tmp = sm_vec(e, kVecTmp);
-    tmp[e.lane] = 0.f;
-    uint32_t* has = reinterpret_cast<uint32_t*>(sm_vec(e, kVecTmp2));
-    has[e.lane] = 0u;
-    __syncwarp();
 #pragma unroll 1
     for (uint32_t h = e.lane; h < nheads; h += 32u) {
-        const uint32_t fl = hu(e, HF_FLAGS, h);
-        if (fl & kHeadDrive) { const uint32_t link = hu(e, HF_REF, h); tmp[link] = hf(e, HF_LAMX, h); has[link] = 1u; }
         // a limit row's slot keeps the multiplier of the velocity solve for the next step (block_descent_tile.cuh:2556)
-        if (fl & kHeadLimit) e.s->limit_lambda[((size_t)e.env * t.L + hu(e, HF_REF, h)) * 2u + (hf(e, HF_UNITV, h) < 0.f ? 1u : 0u)] = hf(e, HF_LAMX, h);
+        if (hu(e, HF_FLAGS, h) & kHeadLimit) e.s->limit_lambda[((size_t)e.env * t.L + hu(e, HF_REF, h)) * 2u + (hf(e, HF_UNITV, h) < 0.f ? 1u : 0u)] = hf(e, HF_LAMX, h);
     }
-    __syncwarp();
     float applied = 0.f;
-    if (e.lane < t.L && has[e.lane]) { applied = tmp[e.lane] / t.cfg.dt - e.drive_dissipation * e.qd; e.tau += applied; }
+    if (e.lane < t.L && joint_dofs(e.jtype) == 1u) {
+        const float impulse = sm_vec(e, kVecFixed)[e.link_dof];
+        if (impulse != 0.f) { applied = impulse / t.cfg.dt - e.drive_dissipation * e.qd; e.tau += applied; }
+    }
     if (e.lane < t.L) e.s->actuator[(size_t)e.env * t.L + e.lane] = applied;
     __syncwarp();
 }
@@ -243,6 +238,7 @@ NKB_DEV void image_move(Env& e, const StepParams& p, float* img, uint32_t nheads
         move(a.pairs, b.pairs, t.slot_cap); move(a.cnormal, b.cnormal, 12u * t.slot_cap); move(a.cfeat, b.cfeat, 8u * t.slot_cap);
         return;
     }
+    if (kLoad || kSet == kBefore) move(a.vecs + b.vstride * kVecFixed, b.vecs + b.vstride * kVecFixed, t.ndof);      // the stages' own
     move(a.vel, b.vel, t.L != 0u ? 6u : 0u);
     move(a.bvel, b.bvel, 6u * slots);
     move(a.heads, b.heads, kHeadStride * nheads);

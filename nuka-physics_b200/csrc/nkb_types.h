@@ -28,7 +28,7 @@ enum : uint32_t { kStatusPairOverflow = 1u << 0, kStatusDofOverflow = 1u << 2, k
                   kStatusTeamTimeout = 1u << 21 };     // a warp of an env's team gave up waiting for another (team mode)
 // head flags
 enum : uint32_t { kHeadContact = 1u << 0, kHeadContactNormal = 1u << 1, kHeadSpeculative = 1u << 2,
-                  kHeadVelocityOnly = 1u << 3, kHeadDrive = 1u << 4, kHeadLimit = 1u << 5, kHeadFriction = 1u << 6,
+                  kHeadVelocityOnly = 1u << 3, kHeadLimit = 1u << 5, kHeadFriction = 1u << 6,
                   kHeadScalar = 1u << 7 /* position pass: only the normal axis */ };
 constexpr uint32_t kHeadStride = 60u;   // words of shared memory per solver head: groups of four, 28 mod 32 for conflict-free vector access
 

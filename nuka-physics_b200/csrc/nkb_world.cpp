@@ -294,7 +294,7 @@ HostTemplate HostTemplate::Parse(const void* blob_in, size_t bytes) {
     t.joint_rows = 0;
     for (uint32_t l = 0; l < L; ++l) {
         if (JointDofs(t.jtype[l]) != 1u) continue;
-        t.joint_rows += ((t.limit_flags[l] & 1u) ? 1u : 0u) + ((t.limit_flags[l] & 2u) ? 1u : 0u) + (t.frictionloss[l] > 0.f ? 1u : 0u) + 1u;
+        t.joint_rows += ((t.limit_flags[l] & 1u) ? 1u : 0u) + ((t.limit_flags[l] & 2u) ? 1u : 0u) + (t.frictionloss[l] > 0.f ? 1u : 0u);
     }
     if (!(t.cfg.dt > 0.f) || !std::isfinite(t.cfg.dt)) throw Error(kInvalidArg, "template dt must be positive");
     return t;
@@ -372,7 +372,7 @@ void World::BuildLayout() {
     at = std::max(at, dynamics_end);
     s.mass = take(n * s.ld); s.factor_words = tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld;
     s.factor = take(s.factor_words); s.vstride = n > 32u ? 64u : 32u;
-    s.vecs = take(6 * s.vstride);
+    s.vecs = take(7 * s.vstride);
     const uint32_t slots = B ? t.n_free + 1u : 0u;
     s.bpose = take(7 * B); s.bvel = take(6 * slots);
     s.bwinv = take(6 * slots); s.bmass = take(7 * slots); s.bfree = take(6 * slots); s.bpseudo = take(6 * slots);
@@ -498,7 +498,7 @@ void World::BuildLayout() {
         at = 0;
         v.vel = take(6);
         v.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
-        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride);
+        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(7 * s.vstride);
         v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
         v.cdepth = take(4 * SC);
         v.heads = take(kHeadStride * tv.head_cap);

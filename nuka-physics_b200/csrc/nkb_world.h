@@ -40,7 +40,7 @@ struct HostTemplate {
     std::vector<float> body_geom_pos, body_geom_quat;
     std::vector<uint32_t> free_slot;
     uint32_t n_free = 0;
-    uint32_t joint_rows = 0;     // limit + friction + drive rows one env can emit
+    uint32_t joint_rows = 0;     // limit + friction rows one env can emit
     static HostTemplate Parse(const void* blob, size_t bytes);
 };
 
