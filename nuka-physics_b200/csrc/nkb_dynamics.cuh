@@ -10,45 +10,6 @@
 
 namespace nkb {
 
-// World poses of every link, ops/articulation.cu:1561-1596 with kinematics.cuh:25-42 joint frames.
-NKB_DEV void stage_fk(Env& e) {
-    const TemplateView& t = *e.t;
-    const uint32_t l = e.lane;
-    const bool link = l < t.L;
-    V3 rpos = mk3(0.f, 0.f, 0.f);
-    Q4 rrot = mkq(1.f, 0.f, 0.f, 0.f);
-    if (link) {
-        rpos = ld3(t.offset + 3u * l);
-        rrot = ldq(t.local_quat + 4u * l);
-        if (e.jtype == kRevolute) {
-            float s, c;
-            sincos_joint(0.5f * e.q, s, c);
-            rrot = qnorm_le(qmul(rrot, mkq(c, e.axis.x * s, e.axis.y * s, e.axis.z * s)), 1.0e-12f);
-        } else if (e.jtype == kPrismatic) {
-            rpos = rpos + qrot(rrot, e.axis * e.q);
-        }
-    }
-#pragma unroll 1
-    for (uint32_t d = 0; d <= t.max_depth; ++d) {
-        if (link && e.depth == d) {
-            float* out = sm_pose(e, l);
-            if (e.parent == kNoLink) {
-                if (e.jtype == kFloating) {
-                    const float* bp = e.s->base_pose + (size_t)e.env * 7u;
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) out[k] = bp[k];
-                } else { st3(out, rpos); stq(out + 3, rrot); }
-            } else {
-                const float* pp = sm_pose(e, e.parent);
-                const Q4 pq = ldq(pp + 3);
-                st3(out, ld3(pp) + qrot(pq, rpos));
-                stq(out + 3, qnorm_le(qmul(pq, rrot), 1.0e-12f));
-            }
-        }
-        __syncwarp();
-    }
-}
-
 // Joint transform (E, r) of this lane's link, ops/articulation.cu:259-277.
 NKB_DEV void joint_xform(const Env& e, float* E, V3& r) {
     const TemplateView& t = *e.t;
@@ -70,6 +31,69 @@ NKB_DEV void joint_xform(const Env& e, float* E, V3& r) {
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int b = 0; b < 3; ++b) E[a * 3 + b] = rot.m[b * 3 + a];
+}
+
+// One pass from the root to the leaves over everything that a link takes from its parent: world poses (ops/articulation.cu:1561-1596
+// with kinematics.cuh:25-42 joint frames), spatial velocities (:647-689) and the accelerations at zero joint acceleration, gravity
+// injected at the root (:505-645).  E, r is the joint transform of this lane's link; `first` takes the floating base's twist from
+// global memory, else it is in the slice.  A pass is as long as the tree is deep, a few hundred cycles to a level, and the three
+// chains share it (apart from one another, and with the velocities computed again for the accelerations, four passes).
+NKB_DEV void stage_kinematics(Env& e, const float (&E)[9], V3 r, bool first) {
+    const TemplateView& t = *e.t;
+    const uint32_t l = e.lane;
+    const bool link = l < t.L;
+    const bool froot = link && e.parent == kNoLink && e.jtype == kFloating;
+    V3 rpos = mk3(0.f, 0.f, 0.f), jw = rpos, jv = rpos;
+    Q4 rrot = mkq(1.f, 0.f, 0.f, 0.f);
+    if (link) {
+        rpos = ld3(t.offset + 3u * l);
+        rrot = ldq(t.local_quat + 4u * l);
+        if (e.jtype == kRevolute) {
+            float s, c;
+            sincos_joint(0.5f * e.q, s, c);
+            rrot = qnorm_le(qmul(rrot, mkq(c, e.axis.x * s, e.axis.y * s, e.axis.z * s)), 1.0e-12f);
+            jw = e.axis * e.qd;
+        } else if (e.jtype == kPrismatic) {
+            rpos = rpos + qrot(rrot, e.axis * e.q);
+            jv = e.axis * e.qd;
+        }
+    }
+    const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
+#pragma unroll 1
+    for (uint32_t d = 0; d <= t.max_depth; ++d) {
+        if (link && e.depth == d) {
+            float *pose = sm_pose(e, l), *vel = sm_vel(e, l), *acc = sm_acc(e, l);
+            if (froot) {
+                const float* bp = e.s->base_pose + (size_t)e.env * 7u;
+#pragma unroll
+                for (int k = 0; k < 7; ++k) pose[k] = bp[k];
+                if (first) {
+                    const float* lv = e.s->link_vel + ((size_t)e.env * t.L + l) * 6u;
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) vel[k] = lv[k];
+                }
+                st3(acc, mk3(0.f, 0.f, 0.f)); st3(acc + 3, -qrot_inv(ldq(bp + 3), g));
+            } else {
+                V3 pw = mk3(0.f, 0.f, 0.f), pv = pw, paw = pw, pav = -g;
+                if (e.parent == kNoLink) { st3(pose, rpos); stq(pose + 3, rrot); }
+                else {
+                    const float *pp = sm_pose(e, e.parent), *pvel = sm_vel(e, e.parent), *pacc = sm_acc(e, e.parent);
+                    const Q4 pq = ldq(pp + 3);
+                    pw = ld3(pvel); pv = ld3(pvel + 3); paw = ld3(pacc); pav = ld3(pacc + 3);
+                    st3(pose, ld3(pp) + qrot(pq, rpos));
+                    stq(pose + 3, qnorm_le(qmul(pq, rrot), 1.0e-12f));
+                }
+                V3 vw, vv, aw, av, cw, cv;
+                xf_motion(E, r, pw, pv, vw, vv);
+                vw = vw + jw; vv = vv + jv;
+                st3(vel, vw); st3(vel + 3, vv);
+                motion_cross(vw, vv, jw, jv, cw, cv);
+                xf_motion(E, r, paw, pav, aw, av);
+                st3(acc, aw + cw); st3(acc + 3, av + cv);
+            }
+        }
+        __syncwarp();
+    }
 }
 
 // Affine joint drives, ops/articulation.cu:836-940: implicit PD position (mode 0), direct torque (1), velocity (2),
@@ -114,7 +138,7 @@ NKB_DEV void stage_drives(Env& e) {
     e.tau = inverse_dynamics ? 0.f : ff;
 }
 
-// Bias forces and mass matrix at the current kinematics; E, r is the joint transform of this lane's link.  Leaves M in shared
+// Bias forces and mass matrix at the kinematics of stage_kinematics; E, r is the joint transform of this lane's link.  Leaves M in shared
 // memory and this lane's entries of the generalised bias in `bias`.
 template <int NR>
 NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]) {
@@ -122,7 +146,6 @@ NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]
     const uint32_t l = e.lane, L = t.L, n = t.ndof, ld = e.lay->ld;
     const bool link = l < L;
     const bool froot = link && e.parent == kNoLink && e.jtype == kFloating;
-    const V3 g = mk3(t.cfg.gravity[0], t.cfg.gravity[1], t.cfg.gravity[2]);
     const float dt = t.cfg.dt;
     if (link) {
         float* xe = sm_xrot(e, l);
@@ -130,29 +153,8 @@ NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]
         for (int k = 0; k < 9; ++k) xe[k] = E[k];
         st3(sm_xtr(e, l), r);
     }
-    // joint velocity S qd in the link frame
-    V3 jw = mk3(0.f, 0.f, 0.f), jv = mk3(0.f, 0.f, 0.f);
-    if (e.jtype == kRevolute) jw = e.axis * e.qd; else if (e.jtype == kPrismatic) jv = e.axis * e.qd;
-    V3 vw = mk3(0.f, 0.f, 0.f), vv = mk3(0.f, 0.f, 0.f), cw = vw, cv = vv;
-    if (froot) {
-        const float* lv = e.s->link_vel + ((size_t)e.env * L + l) * 6u;
-        vw = ld3(lv); vv = ld3(lv + 3);
-        st3(sm_vel(e, l), vw); st3(sm_vel(e, l) + 3, vv);
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (uint32_t d = 0; d <= t.max_depth; ++d) {
-        if (link && e.depth == d && !froot) {
-            V3 pw = mk3(0.f, 0.f, 0.f), pv = pw;
-            if (e.parent != kNoLink) { pw = ld3(sm_vel(e, e.parent)); pv = ld3(sm_vel(e, e.parent) + 3); }
-            V3 tw, tv;
-            xf_motion(E, r, pw, pv, tw, tv);
-            vw = tw + jw; vv = tv + jv;
-            st3(sm_vel(e, l), vw); st3(sm_vel(e, l) + 3, vv);
-            motion_cross(vw, vv, jw, jv, cw, cv);
-        }
-        __syncwarp();
-    }
+    V3 vw = mk3(0.f, 0.f, 0.f), vv = vw, aw = vw, av = vw;
+    if (link) { vw = ld3(sm_vel(e, l)); vv = ld3(sm_vel(e, l) + 3); aw = ld3(sm_acc(e, l)); av = ld3(sm_acc(e, l) + 3); }
     // p = v x* (I v)
     const float* I10 = t.inertia10 + 10u * (link ? l : 0u);
     V3 pn = mk3(0.f, 0.f, 0.f), pf = pn;
@@ -160,21 +162,6 @@ NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]
         V3 in_, if_;
         rbi_mulv(I10, vw, vv, in_, if_);
         force_cross(vw, vv, in_, if_, pn, pf);
-    }
-    // accelerations root to leaf with gravity injected at the root
-    V3 aw = mk3(0.f, 0.f, 0.f), av = aw;
-#pragma unroll 1
-    for (uint32_t d = 0; d <= t.max_depth; ++d) {
-        if (link && e.depth == d) {
-            if (e.parent != kNoLink) xf_motion(E, r, ld3(sm_acc(e, e.parent)), ld3(sm_acc(e, e.parent) + 3), aw, av);
-            else if (e.jtype == kFloating) {
-                const V3 gl = qrot_inv(ldq(e.s->base_pose + (size_t)e.env * 7u + 3), g);
-                aw = mk3(0.f, 0.f, 0.f); av = -gl;
-            } else xf_motion(E, r, mk3(0.f, 0.f, 0.f), -g, aw, av);
-            aw = aw + cw; av = av + cv;
-            st3(sm_acc(e, l), aw); st3(sm_acc(e, l) + 3, av);
-        }
-        __syncwarp();
     }
     if (link) {
         V3 in_, if_;
@@ -210,22 +197,20 @@ NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]
     // generalised bias, lane = coordinate
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
+        const uint32_t dl = e.dof_link[r];
+        const V3 a = mk3(__shfl_sync(NKB_FULL, e.axis.x, dl), __shfl_sync(NKB_FULL, e.axis.y, dl), __shfl_sync(NKB_FULL, e.axis.z, dl));
+        const bool turns = __shfl_sync(NKB_FULL, e.jtype, dl) == kRevolute;
         bias[r] = 0.f;
         if (l + 32u * r < n) {
-            const uint32_t dl = e.dof_link[r];
             const float* pb = sm_pbias(e, dl);
-            if (e.dof_comp[r] == kNoLink) {
-                V3 a = ld3(t.axis + 3u * dl);
-                const float ls = dot(a, a);
-                if (ls > 1.0e-12f) a = a * rsqrtf(ls);
-                bias[r] = __ldg(t.jtype + dl) == kRevolute ? dot(a, ld3(pb)) : dot(a, ld3(pb + 3));
-            } else bias[r] = pb[e.dof_comp[r]];
+            if (e.dof_comp[r] == kNoLink) bias[r] = dot(a, ld3(turns ? pb : pb + 3));
+            else bias[r] = pb[e.dof_comp[r]];
         }
     }
     // mass matrix, ops/articulation_mass.cuh:124-253
     float* M = sm_mass(e);
 #pragma unroll 1
-    for (uint32_t k = l; k < n * ld; k += 32u) M[k] = 0.f;
+    for (uint32_t k = l; k < (n * ld) >> 2; k += 32u) reinterpret_cast<float4*>(M)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
     if (t.floating_root && l < 6u) {
         const float* ic = sm_ic(e, 0u);
@@ -241,38 +226,41 @@ NKB_DEV void stage_dynamics(Env& e, const float (&E)[9], V3 r, float (&bias)[NR]
             for (int c = 0; c < 3; ++c) { row[c] = -hx[(l - 3) * 3 + c]; row[3 + c] = (int)(l - 3) == c ? m : 0.f; }
         }
     }
-    if (link && !froot && joint_dofs(e.jtype) == 1u) {
+    // every joint's unit force walks to the root, all lanes in step; what they pass comes from the links' lanes
+    {
+        const bool joint = link && !froot && joint_dofs(e.jtype) == 1u;
         const uint32_t di = e.link_dof;
-        const float* ic = sm_ic(e, l);
-        V3 fn, ff;
-        if (e.jtype == kRevolute) rbi_mulv(ic, e.axis, mk3(0.f, 0.f, 0.f), fn, ff); else rbi_mulv(ic, mk3(0.f, 0.f, 0.f), e.axis, fn, ff);
-        float diag = e.jtype == kRevolute ? dot(e.axis, fn) : dot(e.axis, ff);
-        diag += __ldg(t.armature + l);
-        diag += dt * e.drive_dissipation;
-        M[di * ld + di] = diag;
+        V3 fn = mk3(0.f, 0.f, 0.f), ff = fn;
+        if (joint) {
+            const float* ic = sm_ic(e, l);
+            if (e.jtype == kRevolute) rbi_mulv(ic, e.axis, mk3(0.f, 0.f, 0.f), fn, ff); else rbi_mulv(ic, mk3(0.f, 0.f, 0.f), e.axis, fn, ff);
+            float diag = e.jtype == kRevolute ? dot(e.axis, fn) : dot(e.axis, ff);
+            diag += __ldg(t.armature + l);
+            diag += dt * e.drive_dissipation;
+            M[di * ld + di] = diag;
+        }
         uint32_t walk = l;
 #pragma unroll 1
-        for (;;) {
-            const uint32_t p = __ldg(t.parent + walk);
-            if (p == kNoLink) break;
+        for (bool going = joint; ;) {
+            const uint32_t p = __shfl_sync(NKB_FULL, e.parent, walk);
+            going = going && p != kNoLink;
+            if (!__any_sync(NKB_FULL, going)) break;
+            const uint32_t from = going ? p : l;
+            const uint32_t wt = __shfl_sync(NKB_FULL, e.jtype, from), dj = __shfl_sync(NKB_FULL, e.link_dof, from);
+            const V3 a = mk3(__shfl_sync(NKB_FULL, e.axis.x, from), __shfl_sync(NKB_FULL, e.axis.y, from), __shfl_sync(NKB_FULL, e.axis.z, from));
+            if (!going) continue;
             V3 pn2, pf2;
             xf_force_t(sm_xrot(e, walk), ld3(sm_xtr(e, walk)), fn, ff, pn2, pf2);
             fn = pn2; ff = pf2;
             walk = p;
-            const uint32_t wt = __ldg(t.jtype + walk);
-            if (joint_dofs(wt) == 0u) continue;
-            const uint32_t dj = __ldg(t.link_dof + walk);
             if (wt == kFloating) {
                 const float f6[6] = {fn.x, fn.y, fn.z, ff.x, ff.y, ff.z};
 #pragma unroll
                 for (int b = 0; b < 6; ++b) { M[di * ld + b] = f6[b]; M[b * ld + di] = f6[b]; }
-                continue;
+            } else if (joint_dofs(wt) == 1u) {
+                const float entry = wt == kRevolute ? dot(a, fn) : dot(a, ff);
+                M[di * ld + dj] = entry; M[dj * ld + di] = entry;
             }
-            V3 a = ld3(t.axis + 3u * walk);
-            const float ls = dot(a, a);
-            if (ls > 1.0e-12f) a = a * rsqrtf(ls);
-            const float entry = wt == kRevolute ? dot(a, fn) : dot(a, ff);
-            M[di * ld + dj] = entry; M[dj * ld + di] = entry;
         }
     }
     __syncwarp();
@@ -871,27 +859,6 @@ NKB_DEV void stage_integrate_links(Env& e, bool use_pseudo) {
         stq(bp + 3, qnorm_lt(qmul(rot, dq), 1.0e-24f));
         const V3 turned = qrot_inv(qnorm_lt(dq, 1.0e-24f), mk3(rv[3], rv[4], rv[5]));
         rv[3] = turned.x; rv[4] = turned.y; rv[5] = turned.z;
-    }
-}
-
-// Link spatial velocities after the solve, ops/articulation.cu:647-689.
-NKB_DEV void stage_link_velocities(Env& e, const float (&E)[9], V3 r) {
-    const TemplateView& t = *e.t;
-    const uint32_t l = e.lane;
-    const bool link = l < t.L;
-    const bool froot = link && e.parent == kNoLink && e.jtype == kFloating;
-    V3 jw = mk3(0.f, 0.f, 0.f), jv = jw;
-    if (e.jtype == kRevolute) jw = e.axis * e.qd; else if (e.jtype == kPrismatic) jv = e.axis * e.qd;
-#pragma unroll 1
-    for (uint32_t d = 0; d <= t.max_depth; ++d) {
-        if (link && e.depth == d && !froot) {
-            V3 pw = mk3(0.f, 0.f, 0.f), pv = pw;
-            if (e.parent != kNoLink) { pw = ld3(sm_vel(e, e.parent)); pv = ld3(sm_vel(e, e.parent) + 3); }
-            V3 tw, tv;
-            xf_motion(E, r, pw, pv, tw, tv);
-            st3(sm_vel(e, l), tw + jw); st3(sm_vel(e, l) + 3, tv + jv);
-        }
-        __syncwarp();
     }
 }
 

@@ -290,10 +290,10 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         float E[9];
         V3 r = mk3(0.f, 0.f, 0.f);
         if (has_artic) {
-            stage_fk(e);
             if (lane < t.L) joint_xform(e, E, r);
+            stage_kinematics(e, E, r, step == 0u);
             tick(e, 1);
-            if (step != 0u) { stage_link_velocities(e, E, r); stage_store_links(e); }
+            if (step != 0u) stage_store_links(e);
         }
         if (has_bodies) {
             stage_body_poses(e, step == 0u);
