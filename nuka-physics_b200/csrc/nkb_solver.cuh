@@ -2056,6 +2056,13 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const uint32_t iterations = t.cfg.vel_iters;
     // One loop drives the velocity sweeps, the hand-over and the split-impulse position sweeps so that each of
     // the large pieces (block indexing, block descent, dual update, momentum balance) is instantiated once.
+    // Without a row the articulation's velocity is the free one plus M^-1 times the drives' impulses: the momentum balance finds it
+    // from the free velocity, and a second time from there, to make up for the factor's rounding.
+    const bool linear = NR > 0 && !kRigid && nheads == 0u && iterations != 0u;
+    if (linear)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) sm_vec(e, kVecU)[l + 32u * r] = sm_vec(e, kVecFree)[l + 32u * r];
+    __syncwarp();
     enum { kPhaseVelocity, kPhaseHandOver, kPhasePosition, kPhaseDone };
     int phase = kPhaseVelocity;
     bool reindex = true;
@@ -2142,7 +2149,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         }
         if (phase == kPhaseVelocity) { tile.iteration = sweeps++; tile.momentum = 0.f; tile.residual = 0.f; }
         else tile.iteration = sweeps + pushes;
-        descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
+        if (!linear) descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
         if (phase == kPhasePosition) {
             if (++pushes >= positions) { phase = kPhaseDone; continue; }
         } else tick(e, 10);
@@ -2154,11 +2161,14 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         for (int stage = 0; stage < 3; ++stage) {
             const float worst_row = fmaxf(fmaxf(rows[0], rows[1]), rows[2]);
             bool run = true;
-            if (stage == 0) run = sweeps == iterations || fmaxf(worst_row, tile.residual) < tile.tol;
+            if (linear) {}
+            else if (stage == 0) run = sweeps == iterations || fmaxf(worst_row, tile.residual) < tile.tol;
             else if (stage == 1) run = worst_row < tile.tol && tile.residual >= tile.tol && tile.residual < FLT_MAX;
             if (stage == 1 && !run) break;
-            if (run) { measure_primals<NR, kRigid>(e, tile, stage == 1); tick(e, 25); tick_count(e, 27); }
-            if (stage == 1) {
+            const bool reconstruct = stage == 1 || (linear && stage == 0);
+            if (run) { measure_primals<NR, kRigid>(e, tile, reconstruct); tick(e, 25); tick_count(e, 27); }
+            if (linear && !(tile.residual < FLT_MAX)) { e.status |= kStatusSolverFailure; break; }
+            if (reconstruct) {
                 if (!(tile.residual < FLT_MAX)) break;
                 init_residuals(e, tile);
                 update_duals(e, tile, nullptr, true, false, rows);
