@@ -298,6 +298,33 @@ void nuka_b200_observation_desc_defaults(nuka_b200_observation_desc_t* desc);
 nuka_result_t nuka_b200_world_pack_observations(nuka_world_handle world, const nuka_b200_observation_desc_t* desc,
                                                 float* device_out, size_t capacity_floats, uint32_t* out_width);
 
+/* One pass of an episode loop over a floating-base robot with nj = L - 1 actuated joints, on the world's stream:
+ *     a = actions clipped to [-action_clip, action_clip]; last_action = a; drive target = default_position + action_scale x a
+ *     `steps` physics steps; episode_steps += 1
+ *     reward = exp(-4 (forward velocity - command[0])^2) - 2 max(0.25 - base height, 0)
+ *     terminated: base below termination_height, the base's up axis below min_up, or a status bit; truncated: episode_steps at
+ *     max_episode_length and not terminated; done = either
+ *     the done envs are reset (as nuka_b200_world_reset_envs_masked) and their targets, last actions and step counts begin again
+ *     every env's observation record goes to device_out and to device_copy (E x width floats each), its last action from this desc
+ * All pointers are device memory; none may be NULL. */
+typedef struct nuka_b200_episode_desc_t {
+    const float* actions;            /* E x nj in the caller's joint order */
+    float* last_action;              /* E x nj */
+    const float* default_position;   /* nj in the caller's joint order */
+    const uint32_t* joint_order;     /* nj: library joint slot of the caller's joint i, as in the observation desc */
+    const float* default_targets;    /* E x L: drive targets of a fresh episode */
+    const float* command;            /* 3 */
+    int32_t* episode_steps;          /* E */
+    float* reward;                   /* E */
+    uint8_t *terminated, *truncated, *done;      /* E, 0 or 1 */
+    uint32_t* done_mask;             /* E */
+    float action_scale, action_clip, termination_height, min_up;
+    int32_t max_episode_length;
+} nuka_b200_episode_desc_t;
+nuka_result_t nuka_b200_world_episode_step(nuka_world_handle world, const nuka_b200_episode_desc_t* desc, const nuka_b200_observation_desc_t* observation,
+                                           uint32_t steps, float* device_out, float* device_copy);
+
+
 /* nuka_world_reset_envs (nuka.h:380-385) with the env set chosen on the device: resets every env whose word in
  * device_mask (E x u32 device memory, read on the world's stream) is non-zero and recomputes their derived poses.
  * Nothing crosses to the host and nothing synchronises, so an episode loop can chain step, termination test and

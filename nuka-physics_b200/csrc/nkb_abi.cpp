@@ -636,6 +636,19 @@ void nuka_b200_observation_desc_defaults(nuka_b200_observation_desc_t* d) {
     d->clip = 100.0f;
 }
 
+namespace {
+nkb::ObservationParams ObservationOf(const nuka_b200_observation_desc_t& desc, uint32_t stride) {
+    nkb::ObservationParams o{};
+    o.command = desc.command; o.command_stride = desc.command_stride; o.last_action = desc.last_action;
+    o.default_position = desc.default_position; o.joint_order = desc.joint_order; o.reward = desc.reward;
+    o.lin_vel_scale = desc.lin_vel_scale; o.ang_vel_scale = desc.ang_vel_scale; o.dof_pos_scale = desc.dof_pos_scale;
+    o.dof_vel_scale = desc.dof_vel_scale;
+    for (int k = 0; k < 3; ++k) o.command_scale[k] = desc.command_scale[k];
+    o.clip = desc.clip; o.row_stride = stride;
+    return o;
+}
+}  // namespace
+
 nuka_result_t nuka_b200_world_pack_observations(nuka_world_handle world, const nuka_b200_observation_desc_t* desc,
                                                 float* device_out, size_t capacity_floats, uint32_t* out_width) {
     NKB_WORLD(w)
@@ -651,14 +664,31 @@ nuka_result_t nuka_b200_world_pack_observations(nuka_world_handle world, const n
     const size_t need = static_cast<size_t>(stride) * (w->env_count() - 1u) + record;
     if (capacity_floats < need) { SetError("observation buffer is too small"); return NUKA_RESULT_INVALID_ARG; }
     if (!(desc->clip >= 0.f)) { SetError("clip must not be negative"); return NUKA_RESULT_INVALID_ARG; }
-    nkb::ObservationParams o{};
-    o.command = desc->command; o.command_stride = desc->command_stride; o.last_action = desc->last_action;
-    o.default_position = desc->default_position; o.joint_order = desc->joint_order; o.reward = desc->reward;
-    o.lin_vel_scale = desc->lin_vel_scale; o.ang_vel_scale = desc->ang_vel_scale; o.dof_pos_scale = desc->dof_pos_scale;
-    o.dof_vel_scale = desc->dof_vel_scale;
-    for (int k = 0; k < 3; ++k) o.command_scale[k] = desc->command_scale[k];
-    o.clip = desc->clip; o.row_stride = stride;
+    const nkb::ObservationParams o = ObservationOf(*desc, stride);
     return Guard([&]() { w->PackObservations(o, device_out); return NUKA_RESULT_OK; });
+}
+
+nuka_result_t nuka_b200_world_episode_step(nuka_world_handle world, const nuka_b200_episode_desc_t* desc, const nuka_b200_observation_desc_t* observation,
+                                           uint32_t steps, float* device_out, float* device_copy) {
+    NKB_WORLD(w)
+    const uint32_t width = w->ObservationWidth();
+    if (width == 0u) { SetError("the world has no actuated joints to observe"); return NUKA_RESULT_NOT_SUPPORTED; }
+    if (desc == nullptr || observation == nullptr || device_out == nullptr || device_copy == nullptr) { SetError("episode desc, observation desc or an output is null"); return NUKA_RESULT_INVALID_ARG; }
+    const nuka_b200_episode_desc_t& d = *desc;
+    if (d.actions == nullptr || d.last_action == nullptr || d.default_position == nullptr || d.joint_order == nullptr || d.default_targets == nullptr ||
+        d.command == nullptr || d.episode_steps == nullptr || d.reward == nullptr || d.terminated == nullptr || d.truncated == nullptr ||
+        d.done == nullptr || d.done_mask == nullptr) { SetError("an array of the episode desc is null"); return NUKA_RESULT_INVALID_ARG; }
+    if (observation->command == nullptr || (observation->command_stride != 0u && observation->command_stride < 3u)) { SetError("observation command is null or its stride below 3"); return NUKA_RESULT_INVALID_ARG; }
+    if (observation->reward != nullptr || (observation->row_stride != 0u && observation->row_stride != width)) { SetError("episode steps write records without a reward column, one behind the other"); return NUKA_RESULT_INVALID_ARG; }
+    if (!(observation->clip >= 0.f)) { SetError("clip must not be negative"); return NUKA_RESULT_INVALID_ARG; }
+    nkb::EpisodeParams p{};
+    p.actions = d.actions; p.last_action = d.last_action; p.default_position = d.default_position; p.joint_order = d.joint_order;
+    p.default_targets = d.default_targets; p.command = d.command; p.episode_steps = d.episode_steps; p.reward = d.reward;
+    p.terminated = d.terminated; p.truncated = d.truncated; p.done = d.done; p.done_mask = d.done_mask;
+    p.action_scale = d.action_scale; p.action_clip = d.action_clip; p.termination_height = d.termination_height; p.min_up = d.min_up;
+    p.max_episode_length = d.max_episode_length;
+    const nkb::ObservationParams o = ObservationOf(*observation, width);
+    return Guard([&]() { w->EpisodeStep(p, o, steps, device_out, device_copy); return NUKA_RESULT_OK; });
 }
 
 nuka_result_t nuka_b200_world_reset_envs_masked(nuka_world_handle world, const uint32_t* device_mask) {

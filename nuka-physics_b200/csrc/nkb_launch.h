@@ -62,6 +62,24 @@ struct ObservationParams {
     float clip;
     uint32_t row_stride;            // floats between consecutive records in the output (>= the record width)
 };
+// An episode loop's inputs and outputs around the step (see nuka_b200_episode_desc_t); all pointers are device memory.
+struct EpisodeParams {
+    const float* actions;           // E x nj, caller joint order
+    float* last_action;             // E x nj
+    const float* default_position;  // nj, caller joint order
+    const uint32_t* joint_order;    // nj
+    const float* default_targets;   // E x L
+    const float* command;           // 3
+    int32_t* episode_steps;         // E
+    float* reward;                  // E
+    uint8_t *terminated, *truncated, *done;      // E
+    uint32_t* done_mask;            // E
+    float action_scale, action_clip, termination_height, min_up;
+    int32_t max_episode_length;
+};
+cudaError_t launch_apply_actions(const StateView& s, uint32_t L, const EpisodeParams& p, cudaStream_t stream);
+cudaError_t launch_judge_episodes(const StateView& s, uint32_t L, const EpisodeParams& p, cudaStream_t stream);
+cudaError_t launch_observe_episodes(const StateView& s, uint32_t L, const ObservationParams& o, const EpisodeParams& p, float* out, float* copy, cudaStream_t stream);
 cudaError_t launch_pack_observations(const StateView& s, uint32_t L, const ObservationParams& o, float* out, cudaStream_t stream);
 // Partial reset without a device allocation: the ids travel through a fixed device array of kStaticResetMaxIds words
 // that every world on `device` shares.  `device` must be current; r.env_ids is ignored.

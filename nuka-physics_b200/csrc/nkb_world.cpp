@@ -885,6 +885,20 @@ void World::PackObservations(const ObservationParams& o, float* device_out) {
     ++launches_;
 }
 
+// One pass of an episode loop: actions to drive targets, the steps, reward and termination, the reset of the finished envs, the
+// observation records.  Everything stays on the stream.
+void World::EpisodeStep(const EpisodeParams& p, const ObservationParams& o, uint32_t steps, float* out, float* copy) {
+    if (tpl_.L < 2u || !tpl_.floating_root) throw Error(kNotSupported, "episode steps need a floating-base articulation");
+    Check(cudaSetDevice(device_), "cudaSetDevice");
+    Check(launch_apply_actions(params_.s, tpl_.L, p, stream_), "action launch");
+    Step(steps);
+    Check(launch_judge_episodes(params_.s, tpl_.L, p, stream_), "episode launch");
+    launches_ += 2;
+    ResetMasked(p.done_mask);
+    Check(launch_observe_episodes(params_.s, tpl_.L, o, p, out, copy, stream_), "observation launch");
+    ++launches_;
+}
+
 // Route of the candidate-pair stage.  The table route tests every admissible pair's boxes each step (B^2 / 2 tests at
 // worst); the tree route sorts, builds and walks a tree of the env's boxes.  Both give the same list, so the choice is
 // a matter of cost: by default the tree takes over once the table is longer than kTreeCrossoverPairs.

@@ -68,6 +68,7 @@ public:
     void SetBroadphase(uint32_t mode);                              // 0: by table size, 1: admissible-pair table, 2: per-env tree
     void Synchronize();
     uint32_t ObservationWidth() const { return tpl_.L >= 2u ? 3u * (tpl_.L - 1u) + 12u : 0u; }      // without the reward column
+    void EpisodeStep(const EpisodeParams& p, const ObservationParams& o, uint32_t steps, float* out, float* copy);
     void PackObservations(const ObservationParams& o, float* device_out);
     bool Field(uint32_t id, FieldInfo* out);
     void SetVelocityIterations(uint32_t n) { params_.t.cfg.vel_iters = n; graph_valid_ = false; }

@@ -231,6 +231,12 @@ class World:
         """Writes one record per env into `out` (CUDA float32 tensor, row stride desc.row_stride or the record width) on the world's stream."""
         _check(_abi.lib().nuka_b200_world_pack_observations(self._h, ctypes.byref(desc), ctypes.c_void_p(out.data_ptr()), out.numel(), None))
 
+    def episode_step(self, desc, observation, steps, out, copy):
+        """One pass of an episode loop (nuka_b200_world_episode_step): `desc` an _abi.EpisodeDesc, `observation` from observation_desc,
+        `out` and `copy` contiguous CUDA float32 tensors of E x record width."""
+        _check(_abi.lib().nuka_b200_world_episode_step(self._h, ctypes.byref(desc), ctypes.byref(observation), int(steps),
+                                                       ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(copy.data_ptr())))
+
     def reset_envs_masked(self, mask):
         """Resets the envs whose word in `mask` (CUDA tensor of E 32-bit words) is non-zero; stays on the world's stream, no host sync."""
         _check(_abi.lib().nuka_b200_world_reset_envs_masked(self._h, ctypes.c_void_p(mask.data_ptr())))

@@ -49,6 +49,12 @@ class ObservationDesc(ctypes.Structure):
                 ("row_stride", ctypes.c_uint32)]
 
 
+class EpisodeDesc(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("actions", "last_action", "default_position", "joint_order", "default_targets", "command",
+                                               "episode_steps", "reward", "terminated", "truncated", "done", "done_mask")] + \
+               [(n, ctypes.c_float) for n in ("action_scale", "action_clip", "termination_height", "min_up")] + [("max_episode_length", ctypes.c_int32)]
+
+
 class CookOptions(ctypes.Structure):
     _fields_ = [("dt", ctypes.c_float), ("velocity_iterations", ctypes.c_uint32), ("position_iterations", ctypes.c_uint32),
                 ("default_kp", ctypes.c_float), ("default_kd", ctypes.c_float), ("add_default_ground", ctypes.c_uint32),
@@ -63,7 +69,7 @@ EXPORTS = [
     "nuka_world_reset", "nuka_world_reset_envs", "nuka_world_forward_kinematics", "nuka_world_get_stream", "nuka_world_record_event",
     "nuka_world_get_buffer_view", "nuka_world_upload_field", "nuka_world_download_field", "nuka_world_create_from_template",
     "nuka_b200_world_info", "nuka_b200_world_run_stage", "nuka_b200_world_launch_count", "nuka_b200_world_reset_envs_static", "nuka_b200_world_download_host", "nuka_b200_host_release",
-    "nuka_b200_world_pack_observations", "nuka_b200_observation_desc_defaults", "nuka_b200_world_reset_envs_masked",
+    "nuka_b200_world_pack_observations", "nuka_b200_observation_desc_defaults", "nuka_b200_world_reset_envs_masked", "nuka_b200_world_episode_step",
     "nuka_b200_world_set_contact_readout", "nuka_b200_world_set_broadphase", "nuka_b200_template_check", "nuka_b200_cook_options_defaults", "nuka_b200_scene_cook", "nuka_world_checkpoint_capture", "nuka_world_checkpoint_restore", "nuka_checkpoint_destroy",
     "nuka_checkpoint_write", "nuka_world_checkpoint_read", "nuka_checkpoint_byte_size", "nuka_checkpoint_equal", "nuka_world_state_hash",
     "nuka_world_get_dof_name",
@@ -106,6 +112,7 @@ def lib():
     L.nuka_b200_observation_desc_defaults.argtypes = [ctypes.POINTER(ObservationDesc)]
     L.nuka_b200_observation_desc_defaults.restype = None
     L.nuka_b200_world_reset_envs_masked.argtypes = [vp, vp]
+    L.nuka_b200_world_episode_step.argtypes = [vp, ctypes.POINTER(EpisodeDesc), ctypes.POINTER(ObservationDesc), u32, vp, vp]
     L.nuka_b200_cook_options_defaults.argtypes = [ctypes.POINTER(CookOptions)]
     L.nuka_b200_cook_options_defaults.restype = None
     L.nuka_b200_scene_cook.argtypes = [ctypes.c_char_p, sz, ctypes.POINTER(CookOptions), vp, sz, ctypes.POINTER(sz)]

@@ -5,14 +5,15 @@
     -> the 48-float observation record of python/nuka/tasks/go2_obs.py:11-20, composed by one kernel
        (nuka_b200_world_pack_observations); finished envs report their fresh-episode observation.
 
-Everything between two calls of step() stays on the world's stream: the finished envs are reset through a device
+The loop around the steps is one call of the library (nuka_b200_world_episode_step); tensor operations do the same for a task with a
+reward of its own.  Everything between two calls of step() stays on the world's stream: the finished envs are reset through a device
 mask (nuka_b200_world_reset_envs_masked), so no id list travels to the host and nothing synchronises.  The reward
 is a plain forward-velocity / height term; tasks replace ``compute_reward``.  Needs torch with CUDA; no gymnasium
 dependency.
 """
 import math
 
-from . import Field, World
+from . import Field, World, _abi
 
 ACTION_SCALE = 0.25         # python/nuka/tasks/go2_obs.py:64
 ACTION_CLIP = 100.0         # python/nuka/tasks/go2_obs.py:66
@@ -33,7 +34,8 @@ class NukaVecEnv:
         self.control_dt = self.dt * self.decimation
         self.max_episode_length = max(1, int(round(float(episode_length_s) / self.control_dt)))
         self.obs_width = self.world.observation_width()
-        cuda = torch.device("cuda", device.gpu_index)
+        cuda = self._device = torch.device("cuda", device.gpu_index)
+        self._episode = _abi.EpisodeDesc()
         self._stream_obj = self._stream()
         self.command = torch.tensor(command, dtype=torch.float32, device=cuda)
         self.termination_height = float(termination_height)
@@ -98,6 +100,39 @@ class NukaVecEnv:
         obs.record_stream(torch.cuda.current_stream())
         return obs
 
+    def _plain(self, tensor, dtype, *shape):
+        return (type(tensor) is self._torch.Tensor and tensor.dtype is dtype and tensor.shape == shape and tensor.device == self._device
+                and tensor.is_contiguous() and not tensor.requires_grad)
+
+    def _episode_desc(self, actions):
+        """The loop's arrays for the library's episode pass (nuka_b200_world_episode_step), or None where the tensor operations
+        below have to do: a task with a reward or an observation of its own, arrays that are not plain ones of the expected type."""
+        torch, E, nj, own = self._torch, self.num_envs, self.num_joints, type(self)
+        if any(getattr(own, name) is not getattr(NukaVecEnv, name) or name in self.__dict__ for name in ("compute_reward", "_up_axis_z", "_compose")):
+            return None
+        if not (self._plain(actions, torch.float32, E, nj) and self._plain(self.last_action, torch.float32, E, nj)
+                and self._plain(self.default_position, torch.float32, nj) and self._plain(self.joint_order, torch.int32, nj)
+                and self._plain(self.default_targets, torch.float32, E, nj + 1) and self._plain(self.command, torch.float32, 3)
+                and self._plain(self.episode_steps, torch.int32, E) and self._plain(self._done_mask, torch.int32, E)
+                and self._plain(self.obs, torch.float32, E, self.obs_width) and self.last_action.data_ptr() == self._obs_desc.last_action
+                and self._obs_desc.row_stride == 0 and self.max_episode_length < 1 << 31):
+            return None
+        d = self._episode
+        d.actions, d.last_action, d.default_position = actions.data_ptr(), self.last_action.data_ptr(), self.default_position.data_ptr()
+        d.joint_order, d.default_targets, d.command = self.joint_order.data_ptr(), self.default_targets.data_ptr(), self.command.data_ptr()
+        d.episode_steps, d.done_mask = self.episode_steps.data_ptr(), self._done_mask.data_ptr()
+        d.action_scale, d.action_clip, d.termination_height = self.action_scale, ACTION_CLIP, self.termination_height
+        d.min_up, d.max_episode_length = self.min_up, self.max_episode_length
+        return d
+
+    def _episode_pass(self, desc):
+        torch, E, cuda = self._torch, self.num_envs, self._device
+        obs, reward = torch.empty((E, self.obs_width), dtype=torch.float32, device=cuda), torch.empty(E, dtype=torch.float32, device=cuda)
+        terminated, truncated, done = (torch.empty(E, dtype=torch.bool, device=cuda) for _ in range(3))
+        desc.reward, desc.terminated, desc.truncated, desc.done = reward.data_ptr(), terminated.data_ptr(), truncated.data_ptr(), done.data_ptr()
+        self.world.episode_step(desc, self._obs_desc, self.decimation, self.obs, obs)
+        return obs, reward, terminated, truncated, done
+
     def step(self, actions):
         """``actions``: E x num_joints CUDA float tensor in the caller's joint order.  Returns (obs, reward, terminated,
         truncated, info).  The work runs on the world's stream; the caller's current stream is ordered behind it on the
@@ -105,6 +140,14 @@ class NukaVecEnv:
         torch = self._torch
         caller = torch.cuda.current_stream()
         self._stream_obj.wait_stream(caller)           # the actions were produced on the caller's stream
+        desc = self._episode_desc(actions)
+        if desc is not None:
+            with torch.cuda.stream(self._stream_obj):
+                obs, reward, terminated, truncated, done = self._episode_pass(desc)
+            caller.wait_stream(self._stream_obj)
+            for tensor in (obs, reward, terminated, truncated, done):
+                tensor.record_stream(caller)
+            return obs, reward, terminated, truncated, {"done": done}
         with torch.cuda.stream(self._stream_obj):
             action = actions.clamp(-ACTION_CLIP, ACTION_CLIP)
             target = self.default_position + self.action_scale * action            # caller joint order

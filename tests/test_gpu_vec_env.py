@@ -65,3 +65,39 @@ def test_fallen_envs_terminate_and_restart(device):
     assert bool(terminated.all()) and int(info["done"].sum()) == E
     assert int(env.episode_steps.max()) == 0
     env.close()
+
+
+class OwnReward(NukaVecEnv):
+    """A task with a reward of its own: its loop runs as tensor operations."""
+
+    def compute_reward(self):
+        return super().compute_reward()
+
+
+# one env, an odd batch, more than one block of every kernel; actions beyond the clip and not a number, ends by fall and by length
+@pytest.mark.parametrize("E,order", [(1, None), (37, [3, 4, 5, 0, 1, 2, 9, 10, 11, 6, 7, 8]), (1031, None)])
+def test_episode_pass_equals_the_tensor_operations(device, E, order):
+    torch = pytest.importorskip("torch")
+    make = lambda kind: kind(device, T.quadruped(0).blob(), E, decimation=3, episode_length_s=0.12, joint_order=order)
+    envs = make(NukaVecEnv), make(OwnReward)
+    launches = []
+    for env in envs:
+        env.reset()
+        env.episode_steps.copy_(torch.arange(E, device="cuda") % 5)
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    for k in range(12):
+        actions = 0.5 * torch.randn((E, 12), generator=gen, device="cuda")
+        actions[::5, 3] = 150.0
+        actions[k % E, 7] = float("nan")
+        before = [env.world.launch_count() for env in envs]
+        (obs, reward, *flags, info), (obs1, reward1, *flags1, info1) = (env.step(actions) for env in envs)
+        launches.append([env.world.launch_count() - n for env, n in zip(envs, before)])
+        assert torch.equal(torch.nan_to_num(obs, 7.0), torch.nan_to_num(obs1, 7.0)) and obs is not envs[0].obs
+        assert torch.allclose(reward, reward1, rtol=1e-6, atol=1e-6, equal_nan=True)         # an ulp of exp
+        for a, b in zip(flags + [info["done"]], flags1 + [info1["done"]]):
+            assert a.dtype == torch.bool and torch.equal(a, b)
+        for name in ("obs", "last_action", "episode_steps", "_targets", "_base"):
+            assert torch.equal(torch.nan_to_num(getattr(envs[0], name), 7.0), torch.nan_to_num(getattr(envs[1], name), 7.0)), (k, name)
+    assert all(a == b + 2 for a, b in launches)               # both forms count the world's launches: actions and verdicts are two more
+    for env in envs:
+        env.close()
