@@ -1214,7 +1214,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
 // Blocks of one colour share no constraint row (index_blocks colours the graph whose edges are the two-sided heads), so
 // their descents touch disjoint head records and disjoint body velocities and may run side by side.  The env's lead warp
 // walks the descent order; for a run of rigid blocks of one colour it publishes a command in shared memory, and every
-// warp of the team (the lead included) takes its share of the run, 32 / body_lanes blocks at a time, in registers
+// warp of the team (the lead included) takes its share of the run, four blocks at a time, in registers
 // (descend_bodies).  A result does not depend on which warp ran a block, so team sizes give bit-identical states.
 //
 // The warps meet through sequence numbers in shared memory, never through a hardware barrier: the lead bumps the
@@ -1306,17 +1306,18 @@ struct RigidRun {
 };
 struct RigidResult { float momentum, residual; uint32_t status; };
 
-// A warp works on several free bodies at once, `lay->body_lanes` lanes (8 or 16) on each: blocks of one colour share no
-// constraint row.  Inside a group a lane is a constraint row in the line search (rows j, j + width, ...) and a row of the 6 x 6
-// Newton system in its assembly (lanes 8..15 of a 16-lane group take the odd heads); everything of the block's own size (its
-// velocity, its mass, the factorisation) is replicated over the group's lanes in registers, so that neither shared memory nor
-// an exchange sits inside those chains.  Loops run until the last group of the warp is done; a group that is done leaves its
-// state alone.
+// A warp works on four free bodies at once, eight lanes on each: blocks of one colour share no constraint row.  Inside a group a
+// lane is a constraint row in the line search (rows j, j + 8, ...) and a row of the 6 x 6 Newton system in its assembly; everything
+// of the block's own size (its velocity, its mass, the factorisation) is replicated over the group's lanes in registers, so that
+// neither shared memory nor an exchange sits inside those chains.  Loops run until the last group of the warp is done; a group that
+// is done leaves its state alone.  A body of a 48-box pile has 3.5 rows: sixteen lanes to a body, two bodies to a warp, kept twice the
+// warps busy with the same instructions (1024 such piles 20.1 ms, eight lanes 15.5; 700 of 24 boxes 8.07 and 5.85).
+constexpr uint32_t kBodyLanes = 8u, kBodyGroups = 32u / kBodyLanes;
 struct BodyLanes {
-    uint32_t width, j, mask, first;      // lanes per body, lane within the group, the group's lanes, its first lane
+    uint32_t j, mask, first;             // lane within the group, the group's lanes, its first lane
     NKB_DEV bool any(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) != 0u; }
     NKB_DEV bool all(bool p) const { return (__ballot_sync(NKB_FULL, p) & mask) == mask; }
-    // v[k] summed over the group's lanes, dealt out: lane j gets the sums of v[(j & 7) N / 8 ...] in v[0 .. N / 8).  Each
+    // v[k] summed over the group's lanes, dealt out: lane j gets the sums of v[j N / 8 ...] in v[0 .. N / 8).  Each
     // exchange halves what a lane still holds (28 shuffles for 32 values over 8 lanes; a sum per value would take 96)
     template <typename T, int N> NKB_DEV void deal(T (&v)[N]) const {
         int held = N / 2;
@@ -1329,21 +1330,17 @@ struct BodyLanes {
                 v[k] = keep + __shfl_xor_sync(NKB_FULL, give, o);
             }
         }
-        if (width > 8u)
-#pragma unroll
-            for (int k = 0; k < N / 8; ++k) v[k] += __shfl_xor_sync(NKB_FULL, v[k], 8);
     }
     template <typename T> NKB_DEV T sum(T v) const {
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(NKB_FULL, v, o);
-        if (width > 8u) v += __shfl_xor_sync(NKB_FULL, v, 8);
         return v;
     }
 };
-NKB_DEV BodyLanes body_lanes(const Env& e) {
+NKB_DEV BodyLanes body_lanes(uint32_t lane) {
     BodyLanes g;
-    g.width = e.lay->body_lanes; g.j = e.lane & (g.width - 1u); g.first = e.lane & ~(g.width - 1u);
-    g.mask = ((1u << g.width) - 1u) << g.first;
+    g.j = lane & (kBodyLanes - 1u); g.first = lane & ~(kBodyLanes - 1u);
+    g.mask = ((1u << kBodyLanes) - 1u) << g.first;
     return g;
 }
 // M v of a free body: mass, and the world inertia xx yy zz xy xz yz
@@ -1391,7 +1388,7 @@ NKB_DEV void body_block_share(V3 n, V3 m, V3 p, V3 q, float (&share)[32]) {
         }
 }
 
-// Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: `32 / body_lanes` blocks at a
+// Descends the rigid blocks order[k_begin ..  k_end) of one colour whose turn falls to this warp: four blocks at a
 // time, warp `first` of `stride`.  Same model, stopping rules and exact line search as descend_block; the sums that one
 // compensates in float run in double, the inertial force is carried as in descend_tree.
 // The 6 x 6 systems are assembled by summing heads per lane and dealing the sums out, in every launch form: a sum's order decides
@@ -1406,14 +1403,14 @@ NKB_DEV void body_block_share(V3 n, V3 m, V3 p, V3 q, float (&share)[32]) {
 NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
     Env e = bare_env(run.sm, run.lay, run.t, nullptr, 0u, run.lane, run.vstride);
     const TemplateView& t = *e.t;
-    const BodyLanes g = body_lanes(e);
-    const uint32_t nb = run.nblocks, groups = 32u / g.width, row = g.j & 7u;
+    const BodyLanes g = body_lanes(e.lane);
+    const uint32_t nb = run.nblocks, row = g.j;
     const uint32_t* order = block_order(e, nb);
     float most_moved = 0.f, worst = 0.f;
     bool failed = false;
 #pragma unroll 1
-    for (uint32_t base = k_begin + first * groups; base < k_end; base += stride * groups) {
-        const uint32_t turn = base + e.lane / g.width;
+    for (uint32_t base = k_begin + first * kBodyGroups; base < k_end; base += stride * kBodyGroups) {
+        const uint32_t turn = base + e.lane / kBodyLanes;
         const bool have = turn < k_end;
         const uint32_t b = order[have ? turn : base];
         const uint32_t* inc = blk_inc(e, nb) + blk_inc_begin(e, nb, b);
@@ -1423,7 +1420,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
         const bool began = have && !(position && count == 0u);
         bool active = began, coupled = false, failure = false;
 #pragma unroll 1
-        for (uint32_t k = g.j; k < count; k += g.width) {
+        for (uint32_t k = g.j; k < count; k += kBodyLanes) {
             const uint32_t h = inc[k], o = hu(e, HF_OWNER, h);
             coupled |= (o & 0xffffu) != kNoBlock16 && (o >> 16) != kNoBlock16;
             hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_STEP, h, mk3(0.f, 0.f, 0.f));
@@ -1476,7 +1473,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             // rows' steps along d: dir . (d_lin + d_ang x arm), signed by the side the block is on
             if (search)
 #pragma unroll 1
-                for (uint32_t k = g.j; k < count; k += g.width) {
+                for (uint32_t k = g.j; k < count; k += kBodyLanes) {
                     const uint32_t h = inc[k];
                     const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
                     const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h);
@@ -1498,7 +1495,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                     float curvature = 0.f, magnitude = 0.f;
                     if (trying)
 #pragma unroll 1
-                        for (uint32_t k = g.j; k < count; k += g.width) evaluate_head(e, inc[k], alpha, rows, curvature, magnitude);
+                        for (uint32_t k = g.j; k < count; k += kBodyLanes) evaluate_head(e, inc[k], alpha, rows, curvature, magnitude);
                     __syncwarp();
                     rows = g.sum(rows); curvature = g.sum(curvature); magnitude = g.sum(magnitude);
                     if (!trying) continue;
@@ -1540,7 +1537,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
 #pragma unroll
                         for (int k = 0; k < 6; ++k) { u[k] = after[k]; inertial[k] = fma((double)alpha, md[k], inertial[k]); }
 #pragma unroll 1
-                        for (uint32_t k = g.j; k < count; k += g.width) {
+                        for (uint32_t k = g.j; k < count; k += kBodyLanes) {
                             const uint32_t h = inc[k];
                             const float4 s = hq(e, HF_STEP, h), m = hq(e, HF_MOVE, h);
                             hq(e, HF_MOVE, h) = make_float4(fmaf(alpha, s.x, m.x), fmaf(alpha, s.y, m.y), fmaf(alpha, s.z, m.z), m.w);
@@ -1557,7 +1554,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             __syncwarp();
             // the next Newton system: the lower triangle of H, this lane's entry of the force balance and its rounding scale
             float a[21], rhs[6], own, scale;
-            // a lane takes the heads j, j + width, ... and sums its share of everything; the lanes then add their shares
+            // a lane takes the heads j, j + 8, ... and sums its share of everything; the lanes then add their shares
             float share[32];
             double balance[8];
 #pragma unroll
@@ -1566,7 +1563,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             for (int k = 0; k < 8; ++k) balance[k] = 0.0;
             if (active)
 #pragma unroll 1
-                for (uint32_t k = g.j; k < count; k += g.width) {
+                for (uint32_t k = g.j; k < count; k += kBodyLanes) {
                     const uint32_t h = inc[k];
                     const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
                     const V3 arm = hf3(e, first_side ? HF_RA : HF_RB, h), n = hf3(e, HF_N, h), m0 = cross_fma(arm, n);
@@ -1630,7 +1627,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
         // the block's rows and velocity go back
         if (began) {
 #pragma unroll 1
-            for (uint32_t k = g.j; k < count; k += g.width) {
+            for (uint32_t k = g.j; k < count; k += kBodyLanes) {
                 const uint32_t h = inc[k];
                 const float4 res = hq(e, HF_RES, h), move = hq(e, HF_MOVE, h);
                 hq(e, HF_RES, h) = make_float4(__fsub_rn(res.x, move.x), __fsub_rn(res.y, move.y), __fsub_rn(res.z, move.z), res.w);
@@ -1730,7 +1727,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
             // colour 31 is the overflow colour (index_blocks hands it to every block past the 31st colour): not a set of
             // independent blocks, so they descend one by one
             while (colour < 31u && k_end < count && order[k_end] != e.t->B && blk_color(e, nb, order[k_end]) == colour) ++k_end;
-            const bool shared_out = team > 1u && k_end - k > 32u / e.lay->body_lanes && team_command(e.sm, *e.lay)->dead == 0u;
+            const bool shared_out = team > 1u && k_end - k > kBodyGroups && team_command(e.sm, *e.lay)->dead == 0u;
             const uint32_t stride = shared_out ? team : 1u;
             uint32_t seq = 0u;
             if (shared_out) {
@@ -1846,14 +1843,14 @@ NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velo
 // contact frames.
 NKB_DEV void measure_bodies(Env& e, Tile& tile, bool reconstruct) {
     const TemplateView& t = *e.t;
-    const BodyLanes g = body_lanes(e);
-    const uint32_t nb = tile.nblocks, groups = 32u / g.width, row = g.j & 7u, part = g.j >> 3, parts = g.width >> 3;
+    const BodyLanes g = body_lanes(e.lane);
+    const uint32_t nb = tile.nblocks, row = g.j;
     const uint32_t* order = block_order(e, nb);
     const uint32_t blocks = order[nb];
     float worst = 0.f;
 #pragma unroll 1
-    for (uint32_t base = 0u; base < blocks; base += groups) {
-        const uint32_t turn = base + e.lane / g.width;
+    for (uint32_t base = 0u; base < blocks; base += kBodyGroups) {
+        const uint32_t turn = base + e.lane / kBodyLanes;
         const uint32_t b = turn < blocks ? order[turn] : t.B;
         const bool have = b != t.B;                                // the articulation's block has its own measure
         const uint32_t* inc = blk_inc(e, nb) + blk_inc_begin(e, nb, b);
@@ -1862,7 +1859,7 @@ NKB_DEV void measure_bodies(Env& e, Tile& tile, bool reconstruct) {
         if (have) {
             const float* vel = block_vel(e, b, false);
             const float* fr = sm_bfree(e, b);
-            if (part == 0u && row < 6u) {
+            if (row < 6u) {
                 const float* bm = sm_bmass(e, b);
                 if (row < 3u) balance = -(double)bm[0] * ((double)vel[row] - fr[row]);
                 else {
@@ -1871,7 +1868,7 @@ NKB_DEV void measure_bodies(Env& e, Tile& tile, bool reconstruct) {
                 }
             }
 #pragma unroll 1
-            for (uint32_t k = part; k < count; k += parts) {
+            for (uint32_t k = 0u; k < count; ++k) {
                 const uint32_t h = inc[k];
                 const bool first_side = (hu(e, HF_OWNER, h) & 0xffffu) == b;
                 const V3 w = body_row_axis(row, hf3(e, first_side ? HF_RA : HF_RB, h)), lam = head_lambda(e, h);
@@ -1882,7 +1879,6 @@ NKB_DEV void measure_bodies(Env& e, Tile& tile, bool reconstruct) {
             }
         }
         __syncwarp();
-        if (parts > 1u) balance += __shfl_xor_sync(NKB_FULL, balance, 8);
         const bool finite = g.all(fabs(balance) <= FLT_MAX);
         float force[6];
 #pragma unroll

@@ -138,7 +138,6 @@ struct SmemLayout {
     uint32_t cstage;                                            // cache rebuild staging (shares the Jacobian pool, dead by then)
     uint32_t heads, jpool, binfo, chol;                         // solver (chol: the articulation's Newton matrix)
     uint32_t factor_words;                                      // words of the mass matrix's factor
-    uint32_t body_lanes;                                        // lanes that work on one free body: 8 or 16
     // Team mode: `team` warps advance one env; warp 0 leads, the others wait for work (rigid blocks of one colour).
     // team_area: 12 command words, then 4 result words per member.
     uint32_t team, team_area;

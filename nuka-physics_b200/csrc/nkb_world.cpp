@@ -420,10 +420,6 @@ void World::BuildLayout() {
             if (there > here && far > 1u && std::getenv("NUKA_B200_NEAR") == nullptr) { s.contacts_far = 1u; at = s.team_area = without_points; team = far; }
             while (team > 1u && (at + area(team)) * 4u > 220u * 1024u) --team;
         }
-        // Lanes per free body in a block descent.  A body alone on its env's one warp leaves most lanes idle: 8 lanes each,
-        // four bodies at a time.  A team has warps for two bodies each (a colour of a 48-box pile holds about 13).  The choice
-        // follows the template, not a forced team size: sums over rows depend on it, and team sizes give bit-identical states.
-        s.body_lanes = team > 1u ? 16u : 8u;
         if (const char* forced = std::getenv("NUKA_B200_TEAM")) {                        // team-size experiments
             const uint32_t w = static_cast<uint32_t>(std::atoi(forced));
             if (w >= 1u && w <= kTeamMax && t.n_free != 0u && (at + area(w)) * 4u <= 220u * 1024u) team = w;
