@@ -159,10 +159,10 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 // of shared memory) reach 16 resident warps per SM instead of 12.  It spills about 150 bytes; a world takes it only where the
 // extra residency is really there (World::BuildLayout).  The stages and the solve of split steps fit 128 registers without
 // spills (one coordinate per lane, no free bodies).
-// Worlds of bodies only run in teams of up to 8 warps, two piles to an SM: 128 registers for 16 warps, with 400 bytes of spills
-// (1024 piles of 48 boxes, 2 steps: 20.5 ms; 168 registers and teams of 6, 21.0; one pile to an SM, no spills, 26.6).
+// Worlds of bodies only run in teams, two piles to an SM: 168 registers for 12 warps, teams of 6 (1024
+// piles of 48 boxes, 2 steps: 14.5 ms; 128 registers, teams of 8 and 400 bytes of spills, 15.5; 700 of 24 4.82 and 5.85).
 #ifndef NKB_MAXNREG_BODIES
-#define NKB_MAXNREG_BODIES 128
+#define NKB_MAXNREG_BODIES 168
 #endif
 #ifndef NKB_MAXNREG_SLIM
 #define NKB_MAXNREG_SLIM 128
