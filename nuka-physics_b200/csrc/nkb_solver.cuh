@@ -25,7 +25,7 @@ constexpr float kLineTol = 1.0e-6f, kRoundings = 8.0f;
 constexpr float kImpulseRounding = 1.0f / kRoundings;
 
 struct Tile {
-    uint32_t nheads, nblocks, iteration;
+    uint32_t nheads, nblocks;
     bool units;                         // there are rows on a single coordinate
     float momentum, residual, tol;
 };
@@ -502,7 +502,9 @@ NKB_DEV void apply_moves(Env& e, const Tile& tile, uint32_t b, float alpha) {
     __syncwarp();
 }
 
-// Newton steps with exact line search on one block.  A lane owns coordinates lane + 32 r (r < NR) and the same rows of
+// Newton steps with exact line search on one block, from where it stands.  A descent ends at the block's minimum wherever it begins, so
+// the reference's search toward the free velocity ahead of the first sweep's Newton steps (block_descent_tile.cuh:2196-2210) is left out:
+// with it a policy step of 1000 quadrupeds took 2 % more line evaluations and time, 4096 quadrupeds with 4 boxes 5 %.  A lane owns coordinates lane + 32 r (r < NR) and the same rows of
 // the Newton matrix, which lives in the env's shared-memory slice in float4-readable rows; lane k also owns the k-th
 // incident head in the row evaluations and publishes its response through the head's shared-memory fields.
 template <int NR>
@@ -551,16 +553,12 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     bool failure = false;
     float primal = FLT_MAX;
     tick(e, 15);
-    // step -1 (first velocity sweep only) is the line search toward the free velocity; steps >= 0 are Newton steps
 #pragma unroll 1
-    for (int step = (tile.iteration == 0u && !position) ? -1 : 0; step < (int)kNewtonSteps; ++step) {
+    for (int step = 0; step < (int)kNewtonSteps; ++step) {
         float d[NR], force[NR], inertia[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) { d[r] = 0.f; force[r] = 0.f; inertia[r] = 0.f; }
-        if (step < 0) {
-#pragma unroll
-            for (int r = 0; r < NR; ++r) d[r] = coord[r] ? fr[r] - u[r] : 0.f;
-        } else {
+        {
             // ---- lane = head: responses at the current moves, published to shared memory ----
             uint32_t dense_any = 0u;
 #pragma unroll 1
@@ -789,30 +787,15 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
             }
         }
         const float icurv = warp_csum_total(cur);
-        float islope;
-        if (step < 0) {
-            if (!(icurv > 0.f && isfinite(icurv))) continue;
-            islope = -icurv;
-        } else {
-            const float total_dec = warp_csum_total(dec);
-            islope = warp_csum_total(slo);
-            if (!isfinite(total_dec) || !isfinite(islope) || !isfinite(icurv)) { failure = true; break; }
-            if (!(total_dec > 0.f)) break;
-        }
+        const float total_dec = warp_csum_total(dec), islope = warp_csum_total(slo);
+        if (!isfinite(total_dec) || !isfinite(islope) || !isfinite(icurv)) { failure = true; break; }
+        if (!(total_dec > 0.f)) break;
         tick(e, 20);
         row_steps(e, inc, ib, ie, dim, dvec);
         tick(e, 21);
         const float alpha = search_line(e, tile, b, islope, icurv, warp_csum_total(fix), warp_sum(fix_size));
         tick(e, 22);
         tick_count(e, 23);
-        if (step < 0) {
-            if (alpha > 0.f) {
-#pragma unroll
-                for (int r = 0; r < NR; ++r) u[r] = fmaf(alpha, d[r], u[r]);
-                apply_moves(e, tile, b, alpha);
-            }
-            continue;
-        }
         float after[NR];
         bool fin_l = true, rounded_l = true;
         float step_l = 0.f;
@@ -935,9 +918,8 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         hst3(e, HF_MOVE, h, mk3(0.f, 0.f, 0.f)); hst3(e, HF_STEP, h, mk3(0.f, 0.f, 0.f));
     }
     coupled = __any_sync(NKB_FULL, coupled);
-    // a direction is either a Newton step (step >= 0) or one of the two ways to begin: the first velocity sweep searches
-    // toward the free velocity (-1), the others only need M (u - u_free) and the rows at the start (-2)
-    int step = tile.iteration == 0u && !position ? -1 : -2;
+    // the first trip (step -1) only finds M (u - u_free) and the rows where the block stands; Newton steps from 0 on
+    int step = -1;
     bool coord[NR];
     double u[NR], dir[NR], inertial[NR];
     float force[NR], fixed[NR];
@@ -948,7 +930,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         coord[r] = c < dim;
         u[r] = coord[r] ? velocity[c] : 0.0;
         const double fr = coord[r] && !position ? (double)block_free(e, b)[c] : 0.0;
-        dir[r] = step == -1 ? fr - u[r] : u[r] - fr;
+        dir[r] = u[r] - fr;
         inertial[r] = 0.0; force[r] = 0.f;
         fixed[r] = position || !coord[r] ? 0.f : sm_vec(e, kVecFixed)[c];
     }
@@ -973,7 +955,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             sums[3] = fma((double)fixed[r], dir[r], sums[3]);
             fixed_size = fmaf(fabsf(fixed[r]), fabsf((float)dir[r]), fixed_size);
         }
-        bool search = step > -2;
+        bool search = step >= 0;
         double icurv = 0.0, islope = 0.0;
         float initial = 0.f, alpha = 0.f;
         if (search) {
@@ -981,19 +963,12 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             for (int k = 0; k < 4; ++k) sums[k] = warp_sum(sums[k]);
             fixed_size = warp_sum(fixed_size);
             icurv = sums[0];
-            if (step < 0) {
-#pragma unroll
-                for (int r = 0; r < NR; ++r) inertial[r] = -md[r];
-                islope = -icurv;
-                search = icurv > 0.0 && icurv <= FLT_MAX;
-            } else {
-                // d solves H d = force, so the slope at alpha = 0 is -(force . d)
-                initial = -(float)sums[2];
-                islope = sums[1];
-                if (!isfinite(initial) || !(fabs(islope) <= FLT_MAX) || !(icurv <= FLT_MAX)) { failure = true; break; }
-                if (!(initial < 0.f)) break;
-                alpha = 1.f;
-            }
+            // d solves H d = force, so the slope at alpha = 0 is -(force . d)
+            initial = -(float)sums[2];
+            islope = sums[1];
+            if (!isfinite(initial) || !(fabs(islope) <= FLT_MAX) || !(icurv <= FLT_MAX)) { failure = true; break; }
+            if (!(initial < 0.f)) break;
+            alpha = 1.f;
             tick(e, 20);
             row_steps(e, inc, ib, ie, dim, flat);
             tick(e, 21);
@@ -1014,12 +989,6 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
                 if (!search) break;
                 const float slope = (float)(islope + (double)alpha * icurv - (rows + sums[3]));
                 curvature += (float)icurv;
-                if (initial == 0.f) {                      // the first sweep's search starts by measuring its initial slope
-                    initial = slope;
-                    if (!(initial < 0.f)) break;
-                    alpha = 1.f;
-                    continue;
-                }
                 magnitude += fabsf((float)islope) + alpha * (float)icurv + fixed_size;
                 bool give_up = ++trials >= (int)kLineSteps;
                 if (isfinite(slope) && isfinite(curvature)) {
@@ -1039,7 +1008,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         float longest = 0.f;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            const double after = fma((double)alpha, step == -2 ? 0.0 : dir[r], u[r]);
+            const double after = fma((double)alpha, step < 0 ? 0.0 : dir[r], u[r]);
             fin &= fabs(after) <= FLT_MAX;
             rounded &= (float)after == (float)u[r];
             longest = fmaxf(longest, fabsf(alpha * (float)dir[r]));
@@ -1047,8 +1016,8 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         if (step >= 0 && !__all_sync(NKB_FULL, fin)) { failure = true; break; }
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            u[r] = fma((double)alpha, step == -2 ? 0.0 : dir[r], u[r]);
-            inertial[r] = fma((double)alpha, step == -2 ? 0.0 : md[r], inertial[r]);
+            u[r] = fma((double)alpha, step < 0 ? 0.0 : dir[r], u[r]);
+            inertial[r] = fma((double)alpha, step < 0 ? 0.0 : md[r], inertial[r]);
             force[r] = 0.f;
         }
         if (alpha != 0.f)
@@ -1063,7 +1032,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             primal = rounded ? 0.f : warp_max_positive(longest);
             if (!(alpha > 0.f) || rounded || step + 1 == (int)kNewtonSteps) break;
         }
-        step = step < 0 ? 0 : step + 1;
+        ++step;
         // ---- the next Newton system at the new velocity: this lane's row of H, its entry of the force balance ----
         __syncwarp();
 #pragma unroll
@@ -1226,7 +1195,7 @@ enum : uint32_t { kTeamDescend = 0x44455343u, kTeamExit = 0x45584954u,
                   kTeamNarrowphase = 0x4e415252u, kTeamWarmStart = 0x5741524du, kTeamCacheOwners = 0x4f574e52u };
 constexpr uint32_t kTeamCommandWords = 12u;                   // the team area: command, then 4 result words per member
 constexpr long long kTeamPatience = 4000000000ll;           // cycles a warp waits for another: about two seconds
-struct TeamCommand { uint32_t seq, op, k_begin, k_end, position, iteration, nblocks, nheads; float tol; uint32_t dead, pad0, pad1; };
+struct TeamCommand { uint32_t seq, op, k_begin, k_end, position, nblocks, nheads; float tol; uint32_t dead, pad0, pad1, pad2; };
 static_assert(sizeof(TeamCommand) == 4u * kTeamCommandWords, "the command occupies the first words of the team area");
 
 NKB_DEV TeamCommand* team_command(float* sm, const SmemLayout& lay) { return reinterpret_cast<TeamCommand*>(sm + lay.team_area); }
@@ -1251,7 +1220,7 @@ NKB_DEV uint32_t team_post(float* sm, const SmemLayout& lay, uint32_t lane, uint
     __syncwarp();
     if (lane == 0u) {
         cmd->op = op; cmd->k_begin = k_begin; cmd->k_end = k_end; cmd->position = position ? 1u : 0u;
-        cmd->iteration = tile.iteration; cmd->nblocks = tile.nblocks; cmd->nheads = tile.nheads; cmd->tol = tile.tol;
+        cmd->nblocks = tile.nblocks; cmd->nheads = tile.nheads; cmd->tol = tile.tol;
         __threadfence_block();
         team_poke(&cmd->seq, seq);
     }
@@ -1301,7 +1270,7 @@ struct RigidRun {
     const SmemLayout* lay;
     const TemplateView* t;
     uint32_t lane, vstride;
-    uint32_t nheads, nblocks, iteration;
+    uint32_t nheads, nblocks;
     float tol;
 };
 struct RigidResult { float momentum, residual; uint32_t status; };
@@ -1311,7 +1280,7 @@ struct RigidResult { float momentum, residual; uint32_t status; };
 // of the block's own size (its velocity, its mass, the factorisation) is replicated over the group's lanes in registers, so that
 // neither shared memory nor an exchange sits inside those chains.  Loops run until the last group of the warp is done; a group that
 // is done leaves its state alone.  A body of a 48-box pile has 3.5 rows: sixteen lanes to a body, two bodies to a warp, kept twice the
-// warps busy with the same instructions (1024 such piles 20.1 ms, eight lanes 15.5; 700 of 24 boxes 8.07 and 5.85).
+// warps busy with the same instructions (1024 such piles 20.1 ms, eight lanes 16.3; 700 of 24 boxes 8.07 and 6.20).
 constexpr uint32_t kBodyLanes = 8u, kBodyGroups = 32u / kBodyLanes;
 struct BodyLanes {
     uint32_t j, mask, first;             // lane within the group, the group's lanes, its first lane
@@ -1434,32 +1403,30 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             for (int k = 0; k < 6; ++k) mass.i[k] = bm[1 + k];
         }
         float* velocity = block_vel(e, b, position);
-        // how the directions of a descent start: toward the free velocity in the first velocity sweep (-1), else only M (u - u_free)
-        // and the rows where the block stands (-2); Newton steps from 0 on.  Every group is at the same step.
-        int step = run.iteration == 0u && !position ? -1 : -2;
+        // the first trip (step -1) only finds M (u - u_free) and the rows where the block stands; Newton steps from 0 on.  Every group
+        // is at the same step.
+        int step = -1;
         double u[6], dir[6], inertial[6];
         float force[6], primal = FLT_MAX;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             const double fr = position ? 0.0 : (double)sm_bfree(e, b)[k];
             u[k] = velocity[k];
-            dir[k] = step == -1 ? fr - u[k] : u[k] - fr;
+            dir[k] = u[k] - fr;
             inertial[k] = 0.0; force[k] = 0.f;
         }
 #pragma unroll 1
         for (;;) {
             double md[6];
             body_mass_mul(mass, dir, md);
-            bool search = active && step > -2;
+            bool search = active && step >= 0;
             double icurv = 0.0, islope = 0.0;
             float initial = 0.f, alpha = 0.f;
 #pragma unroll
             for (int k = 0; k < 6; ++k) icurv = fma(dir[k], md[k], icurv);
             if (step < 0) {
 #pragma unroll
-                for (int k = 0; k < 6; ++k) inertial[k] = step == -1 ? -md[k] : md[k];
-                islope = -icurv;
-                search = search && icurv > 0.0 && icurv <= FLT_MAX;
+                for (int k = 0; k < 6; ++k) inertial[k] = md[k];
             } else {
                 double along = 0.0;
 #pragma unroll
@@ -1502,11 +1469,6 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                     if (!search) { trying = false; continue; }
                     const float slope = (float)(fma((double)alpha, icurv, islope) - rows);
                     curvature += (float)icurv;
-                    if (initial == 0.f) {                      // the first sweep's search starts by measuring its initial slope
-                        initial = slope;
-                        if (initial < 0.f) alpha = 1.f; else trying = false;
-                        continue;
-                    }
                     magnitude += fmaf(alpha, (float)icurv, fabsf((float)islope));
                     bool give_up = ++trials >= (int)kLineSteps;
                     if (isfinite(slope) && isfinite(curvature)) {
@@ -1550,7 +1512,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                 }
             }
             if (!__any_sync(NKB_FULL, active)) break;
-            step = step < 0 ? 0 : step + 1;
+            ++step;
             __syncwarp();
             // the next Newton system: the lower triangle of H, this lane's entry of the force balance and its rounding scale
             float a[21], rhs[6], own, scale;
@@ -1652,13 +1614,13 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
 // One copy for the lead and its helpers, where nothing of an articulation sits in the caller's registers (worlds of bodies only):
 // their warps fetch the same instructions then (48-box piles: 22.2 ms against 20.4, see World::BuildLayout).
 static __device__ __noinline__ RigidResult descend_bodies_call(float* sm, const SmemLayout* lay, const TemplateView* t, uint32_t lane, uint32_t vstride, uint32_t nheads, uint32_t nblocks,
-                                                               uint32_t iteration, float tol, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
-    const RigidRun run = {sm, lay, t, lane, vstride, nheads, nblocks, iteration, tol};        // a struct argument would go through memory
+                                                               float tol, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
+    const RigidRun run = {sm, lay, t, lane, vstride, nheads, nblocks, tol};        // a struct argument would go through memory
     return descend_bodies(run, k_begin, k_end, first, stride, position);
 }
 template <int NR>
 NKB_DEV RigidResult descend_share(const RigidRun& run, uint32_t k_begin, uint32_t k_end, uint32_t first, uint32_t stride, bool position) {
-    if constexpr (NR == 0) return descend_bodies_call(run.sm, run.lay, run.t, run.lane, run.vstride, run.nheads, run.nblocks, run.iteration, run.tol, k_begin, k_end, first, stride, position);
+    if constexpr (NR == 0) return descend_bodies_call(run.sm, run.lay, run.t, run.lane, run.vstride, run.nheads, run.nblocks, run.tol, k_begin, k_end, first, stride, position);
     else return descend_bodies(run, k_begin, k_end, first, stride, position);
 }
 
@@ -1666,7 +1628,7 @@ NKB_DEV RigidResult descend_share(const RigidRun& run, uint32_t k_begin, uint32_
 NKB_DEV void team_dismiss(float* sm, const SmemLayout& lay, uint32_t lane) {
     if (lay.team <= 1u) return;
     Tile none;
-    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
+    none.nheads = 0u; none.nblocks = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
     team_post(sm, lay, lane, kTeamExit, 0u, 0u, false, none);
 }
 
@@ -1678,7 +1640,7 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
     const uint32_t team = e.lay->team;
     if (team <= 1u || team_command(e.sm, *e.lay)->dead != 0u) { work(0u, 1u); return; }
     Tile none;
-    none.nheads = 0u; none.nblocks = 0u; none.iteration = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
+    none.nheads = 0u; none.nblocks = 0u; none.units = false; none.momentum = 0.f; none.residual = 0.f; none.tol = 0.f;
     const uint32_t seq = team_post(e.sm, *e.lay, e.lane, op, count, 0u, false, none);
     work(0u, team);
     if (team_collect(e.sm, *e.lay, e.lane, seq)) {
@@ -1715,7 +1677,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
         const uint32_t team = e.lay->team;
         RigidRun run;
         run.sm = e.sm; run.lay = e.lay; run.t = e.t; run.lane = e.lane; run.vstride = e.vstride;
-        run.nheads = tile.nheads; run.nblocks = nb; run.iteration = tile.iteration; run.tol = tile.tol;
+        run.nheads = tile.nheads; run.nblocks = nb; run.tol = tile.tol;
 #pragma unroll 1
         for (uint32_t k = 0u; k < count;) {
             const uint32_t b = order[k];
@@ -1989,7 +1951,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, B = t.B, n = NR > 0 ? t.ndof : 0u;
     Tile tile;
-    tile.nheads = nheads; tile.nblocks = B + (n != 0u ? 1u : 0u); tile.iteration = 0u; tile.units = false;
+    tile.nheads = nheads; tile.nblocks = B + (n != 0u ? 1u : 0u); tile.units = false;
     tile.momentum = tile.residual = 0.f; tile.tol = t.cfg.velocity_tolerance;
     // rigid blocks: free velocity, mass, carried constraint velocity (block_descent_rigid.cuh:4-48)
     if constexpr (kRigid)
@@ -2143,8 +2105,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
             }
             continue;
         }
-        if (phase == kPhaseVelocity) { tile.iteration = sweeps++; tile.momentum = 0.f; tile.residual = 0.f; }
-        else tile.iteration = sweeps + pushes;
+        if (phase == kPhaseVelocity) { ++sweeps; tile.momentum = 0.f; tile.residual = 0.f; }
         if (!linear) descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
         if (phase == kPhasePosition) {
             if (++pushes >= positions) { phase = kPhaseDone; continue; }

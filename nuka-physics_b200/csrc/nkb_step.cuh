@@ -437,7 +437,7 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
         if (op == kTeamDescend && k_begin < k_end && k_end <= nblocks && nblocks <= t.B + 1u) {
             RigidRun run;
             run.sm = sm; run.lay = &shared_layout; run.t = &t; run.lane = lane; run.vstride = vstride;
-            run.nheads = cmd->nheads; run.nblocks = nblocks; run.iteration = cmd->iteration; run.tol = cmd->tol;
+            run.nheads = cmd->nheads; run.nblocks = nblocks; run.tol = cmd->tol;
 #ifdef NKB_STAGE_TAPS
             const long long tap0 = clock64();
 #endif

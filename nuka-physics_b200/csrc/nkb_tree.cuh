@@ -162,17 +162,17 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float rhs
             uint32_t i, j;
             if (lane >= 21u) { i = lane - 21u; j = 6u; }
             else { i = lane >= 15u ? 5u : lane >= 10u ? 4u : lane >= 6u ? 3u : lane >= 3u ? 2u : lane >= 1u ? 1u : 0u; j = lane - (i * (i + 1u)) / 2u; }
-            Sum s0 = block[8u * i + j], s1 = 0.f;
+            Sum s0 = block[8u * i + j];
             const float* src = scratch;
             uint32_t k = 0u;
 #pragma unroll 1
             for (; k + 1u < rows; k += 2u, src += 2u * stride) {
                 s0 = fma((Sum)-src[i], (Sum)src[j], s0);
-                s1 = fma((Sum)-src[stride + i], (Sum)src[stride + j], s1);
+                s0 = fma((Sum)-src[stride + i], (Sum)src[stride + j], s0);
             }
             if (k < rows) s0 = fma((Sum)-src[i], (Sum)src[j], s0);
-            if (kKeep && j == 6u) *reinterpret_cast<double*>(block + 8u * i + 6u) = s0 + s1;        // in place of base_g and its pad
-            else entries[lane] = (float)(s0 + s1);
+            if (kKeep && j == 6u) *reinterpret_cast<double*>(block + 8u * i + 6u) = s0;        // in place of base_g and its pad
+            else entries[lane] = (float)(s0);
         }
         __syncwarp();
         float packed[28], a[21];
