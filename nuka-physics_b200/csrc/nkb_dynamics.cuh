@@ -308,14 +308,14 @@ NKB_DEV void stage_accelerations(Env& e, const float (&bias)[NR], bool factor, b
     for (int r = 0; r < NR; ++r) x[r] = dof[r] ? rhs[r] : 0.f;
     if (t.mass_tree != 0u) {
         // factor on the tree's sparsity and solve in the same pass (nkb_tree.cuh); the factor stays for the constraint solve
-        const TreeLane tl = tree_lane(e);
+        const TreeLane<kTreeLevels> tl = tree_lane(e);
         const bool high = NR > 1 && t.floating_root != 0u && l < 6u;         // this lane's joint is its second coordinate
-        TreeRow row;
+        TreeRow<kTreeLevels> row;
         tree_load_row(e, tl, M, ld, row);
         float base_row[kTreeBase], base_x[kTreeBase], joint;
 #pragma unroll
         for (int k = 0; k < kTreeBase; ++k) base_row[k] = NR == 1 ? row.base[k] : t.floating_root != 0u && l < 6u ? M[l * ld + k] : 0.f;
-        tree_solve<NR, true>(e, tl, row, high ? x[NR - 1] : x[0], base_row, x[0], sm_factor(e), joint, base_x);
+        tree_solve<NR, true, kTreeLevels>(e, tl, row, high ? x[NR - 1] : x[0], base_row, x[0], sm_factor(e), joint, base_x);
         tree_scatter<NR>(e, joint, base_x, x);
     } else {
         float* F = sm_factor(e);

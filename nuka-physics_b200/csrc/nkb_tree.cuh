@@ -22,32 +22,57 @@ namespace nkb {
 constexpr int kTreeBase = 6;            // columns of a floating base
 
 // This lane's place in the tree: its joint coordinate (lane, or lane + 32 on the base's lanes of a wide articulation), the
-// number of ancestor joints, the lanes of its descendants, its ancestors' coordinates by depth, one byte each.
+// number of ancestor joints, the lanes of its descendants, its ancestors' coordinates by depth, one byte each; and the tree's depth and
+// row stride in shared memory.
+template <int kLevels>
 struct TreeLane {
-    uint32_t coord, level, desc;
-    uint32_t anc[kTreeLevels / 4];
+    uint32_t coord, level, desc, depth, stride;
+    uint32_t anc[kLevels / 4];
     NKB_DEV uint32_t ancestor(int p) const { return (anc[p >> 2] >> (8 * (p & 3))) & 0xffu; }
+    // the same where p is no constant
+    NKB_DEV uint32_t ancestor_at(int p) const {
+        uint32_t word = anc[0];
+#pragma unroll
+        for (int k = 1; k < kLevels / 4; ++k) if (p >= 4 * k) word = anc[k];
+        return (word >> (8 * (p & 3))) & 0xffu;
+    }
 };
 constexpr uint32_t kTreeNone = 0xffu;   // level of a lane without a joint coordinate
 
-NKB_DEV TreeLane tree_lane(const Env& e) {
-    TreeLane t;
+template <int kLevels = kTreeLevels>
+NKB_DEV TreeLane<kLevels> tree_lane(const Env& e) {
+    TreeLane<kLevels> t;
     const uint32_t* w = e.t->tree_lanes + e.lane * kTreeLaneWords;
     const uint32_t head = __ldg(w);
     t.coord = head & 0xffu; t.level = (head >> 8) & 0xffu;
     t.desc = __ldg(w + 1);
+    t.depth = e.t->tree_depth; t.stride = e.t->tree_stride;
 #pragma unroll
-    for (int k = 0; k < kTreeLevels / 4; ++k) t.anc[k] = __ldg(w + 2 + k);
+    for (int k = 0; k < kLevels / 4; ++k) t.anc[k] = k < kTreeLevels / 4 ? __ldg(w + 2 + k) : 0u;
+    return t;
+}
+// The same in the tree that merge_trees left.
+template <int kLevels>
+NKB_DEV TreeLane<kLevels> merged_lane(const Env& e) {
+    TreeLane<kLevels> t;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(e.sm + e.lay->merged) + e.lane * merged_lane_words(e.t->ndof);
+    t.coord = w[0] & 0xffu; t.level = (w[0] >> 8) & 0xffu;
+    t.desc = w[1];
+    t.depth = e.merged; t.stride = tree_row_stride(e.merged);
+#pragma unroll
+    for (int k = 0; k < kLevels / 4; ++k) t.anc[k] = w[2 + k];
     return t;
 }
 
 // A lane's compressed row.
+template <int kLevels>
 struct TreeRow {
-    float base[kTreeBase], limb[kTreeLevels], diag;
+    float base[kTreeBase], limb[kLevels], diag;
 };
 
 // Row of the lane's coordinate out of a dense symmetric matrix in shared memory (rows of `ld` words, 16-byte aligned).
-NKB_DEV void tree_load_row(const Env& e, const TreeLane& t, const float* matrix, uint32_t ld, TreeRow& row) {
+template <int kLevels>
+NKB_DEV void tree_load_row(const Env& e, const TreeLane<kLevels>& t, const float* matrix, uint32_t ld, TreeRow<kLevels>& row) {
     const float* src = matrix + t.coord * ld;
 #pragma unroll
     for (int k = 0; k < kTreeBase; ++k) row.base[k] = 0.f;
@@ -56,11 +81,11 @@ NKB_DEV void tree_load_row(const Env& e, const TreeLane& t, const float* matrix,
         const float2 hi = *reinterpret_cast<const float2*>(src + 4);
         row.base[0] = lo.x; row.base[1] = lo.y; row.base[2] = lo.z; row.base[3] = lo.w; row.base[4] = hi.x; row.base[5] = hi.y;
     }
-    const int depth = (int)e.t->tree_depth;
+    const int depth = (int)t.depth;
 #pragma unroll
-    for (int p = 0; p < kTreeLevels; ++p) row.limb[p] = 0.f;
+    for (int p = 0; p < kLevels; ++p) row.limb[p] = 0.f;
 #pragma unroll
-    for (int p = 0; p < kTreeLevels; p += 2) {
+    for (int p = 0; p < kLevels; p += 2) {
         if (p >= depth - 1) break;
         row.limb[p] = src[t.ancestor(p)]; row.limb[p + 1] = src[t.ancestor(p + 1)];
     }
@@ -81,11 +106,11 @@ template <int NR> NKB_DEV uint32_t tree_rows(const Env& e) { return NR == 1 ? e.
 // right-hand side and the base's Schur complement in 64 bits: eliminated last, the base gathers the cancellations of all limbs.
 // M^-1 tau against 64 bits, root mean square over 2048 humanoids: 8.0e-7 with approximate roots and 32-bit sums, 5.0e-7 so (the
 // dense factor, base first, 5.1e-7); quadrupeds 1.35e-7 and 0.86e-7 (dense 1.5e-7).  It costs their policy steps 0.7 %.
-template <int NR, bool kKeep>
-NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float rhs, const float (&base_row)[kTreeBase], float base_g,
+template <int NR, bool kKeep, int kLevels>
+NKB_DEV bool tree_solve(const Env& e, const TreeLane<kLevels>& t, TreeRow<kLevels>& row, float rhs, const float (&base_row)[kTreeBase], float base_g,
                         float* scratch, float& x, float (&base_x)[kTreeBase]) {
-    const uint32_t stride = e.t->tree_stride, lane = e.lane;
-    const int depth = (int)e.t->tree_depth;
+    const uint32_t stride = t.stride, lane = e.lane;
+    const int depth = (int)t.depth;
     const uint32_t first = tree_first<NR>(e), rows = tree_rows<NR>(e);
     float* mine = scratch + (lane - first) * stride;
     using Sum = typename std::conditional<kKeep, double, float>::type;
@@ -114,7 +139,7 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float rhs
             out[0] = make_float4(row.base[0], row.base[1], row.base[2], row.base[3]);
             out[1] = make_float4(row.base[4], row.base[5], (float)y, inverse);
 #pragma unroll
-            for (int k = 0; k < kTreeLevels; k += 4) {
+            for (int k = 0; k < kLevels; k += 4) {
                 if (k >= 4 * quads) break;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) row.limb[k + c] *= inverse;
@@ -136,7 +161,7 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float rhs
             row.base[3] = fmaf(-m, b0.w, row.base[3]); row.base[4] = fmaf(-m, b1.x, row.base[4]); row.base[5] = fmaf(-m, b1.y, row.base[5]);
             g = fma((Sum)-m, (Sum)b1.z, g);
 #pragma unroll
-            for (int q = 0; q < kTreeLevels; q += 4) {
+            for (int q = 0; q < kLevels; q += 4) {
                 if (q >= 4 * quads) break;
                 const float4 c4 = *reinterpret_cast<const float4*>(src + 8 + q);
                 row.limb[q] = fmaf(-m, c4.x, row.limb[q]); row.limb[q + 1] = fmaf(-m, c4.y, row.limb[q + 1]);
@@ -200,8 +225,7 @@ NKB_DEV bool tree_solve(const Env& e, const TreeLane& t, TreeRow& row, float rhs
     // joints root to leaf: a depth's solution reaches its descendants by shuffle
 #pragma unroll 1
     for (int p = 0; p < depth - 1; ++p) {
-        const uint32_t word = p < 4 ? t.anc[0] : p < 8 ? t.anc[1] : t.anc[2];
-        const float xp = __shfl_sync(NKB_FULL, (float)(acc * inverse), (word >> (8 * (p & 3))) & 31u);
+        const float xp = __shfl_sync(NKB_FULL, (float)(acc * inverse), t.ancestor_at(p) & 31u);
         if (t.level != kTreeNone && t.level > (uint32_t)p) acc = fma((Sum)-mine[8 + p], (Sum)xp, acc);
     }
     x = (float)(acc * inverse);
@@ -224,7 +248,7 @@ NKB_DEV void tree_scatter(const Env& e, float joint, const float (&base_x)[kTree
 // x = M^-1 g with the kept factor: g and x are the joint lanes' entries, base_g / base_x the base's (lane k of the first six
 // carries base_g of coordinate k; base_x in every lane).
 template <int NR>
-NKB_DEV void tree_mass_solve(const Env& e, const TreeLane& t, float* factor, float g, float base_g, float& x, float (&base_x)[kTreeBase]) {
+NKB_DEV void tree_mass_solve(const Env& e, const TreeLane<kTreeLevels>& t, float* factor, float g, float base_g, float& x, float (&base_x)[kTreeBase]) {
     const uint32_t stride = e.t->tree_stride, lane = e.lane, first = tree_first<NR>(e), rows = tree_rows<NR>(e);
     const int depth = (int)e.t->tree_depth;
     const bool joint = t.level != kTreeNone;
@@ -282,8 +306,7 @@ NKB_DEV void tree_mass_solve(const Env& e, const TreeLane& t, float* factor, flo
     }
 #pragma unroll 1
     for (int p = 0; p < depth - 1; ++p) {
-        const uint32_t word = p < 4 ? t.anc[0] : p < 8 ? t.anc[1] : t.anc[2];
-        const float xp = __shfl_sync(NKB_FULL, acc * inverse, (word >> (8 * (p & 3))) & 31u);
+        const float xp = __shfl_sync(NKB_FULL, acc * inverse, t.ancestor_at(p) & 31u);
         if (joint && t.level > (uint32_t)p) acc = fmaf(-mine[8 + p], xp, acc);
     }
     x = acc * inverse;

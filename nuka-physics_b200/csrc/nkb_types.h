@@ -8,13 +8,22 @@
 
 namespace nkb {
 
+#ifdef __CUDACC__
+#define NKB_HOST_DEVICE __host__ __device__
+#else
+#define NKB_HOST_DEVICE
+#endif
+
 constexpr uint32_t kNoLink = 0xffffffffu;
 constexpr uint32_t kMaxLinks = 32u;     // one warp lane per link
 constexpr uint32_t kMaxDof = 64u;       // a warp lane owns coordinates lane and lane + 32
 constexpr int kTreeLevels = 12;         // joints on one root path that the tree-structured solve covers (a multiple of 4)
 constexpr uint32_t kTreeLaneWords = 2u + kTreeLevels / 4u;   // table words per lane: coordinate and depth, descendants, ancestors
+// Levels that the solve holds in registers: with two coordinates per lane twice as many, for trees joined by contacts (merge_trees).
+template <int NR> constexpr int kSolveLevels = NR > 1 ? 2 * kTreeLevels : kTreeLevels;
+NKB_HOST_DEVICE constexpr uint32_t merged_lane_words(uint32_t ndof) { return 2u + (ndof > 32u ? 2u : 1u) * kTreeLevels / 4u; }
 // Row stride (words) and scratch words of the tree-structured solve for `rows` joint lanes and root paths of `depth` joints.
-inline uint32_t tree_row_stride(uint32_t depth) { return depth <= 5u ? 12u : 20u; }
+NKB_HOST_DEVICE inline uint32_t tree_row_stride(uint32_t depth) { return depth <= 5u ? 12u : depth <= 13u ? 20u : 36u; }
 inline uint32_t tree_scratch_words(uint32_t rows, uint32_t depth) { return rows * tree_row_stride(depth) + 48u + 28u; }
 constexpr uint32_t kMaxBodies = 256u;   // collidable rows per env (the env's shared-memory slice is the practical limit)
 constexpr uint32_t kPtsPerSlot = 4u;
@@ -34,11 +43,6 @@ constexpr uint32_t kHeadStride = 60u;   // words of shared memory per solver hea
 
 // Scratch words of the tree broadphase for B collidable rows (nkb_lbvh.cuh): sorted keys, internal nodes (children, range,
 // box), split table, ready flags and one partner bit row per body.
-#ifdef __CUDACC__
-#define NKB_HOST_DEVICE __host__ __device__
-#else
-#define NKB_HOST_DEVICE
-#endif
 NKB_HOST_DEVICE inline uint32_t lbvh_pow2(uint32_t b) { uint32_t p = 2u; while (p < b) p <<= 1u; return p; }
 NKB_HOST_DEVICE inline uint32_t lbvh_scratch_words(uint32_t B) {
     if (B < 2u) return 0u;
@@ -69,6 +73,7 @@ struct TemplateView {
     const uint32_t *link_leaf;          // L: the deepest joint coordinate on a link's root path, 0xff when there is none
     uint32_t mass_tree;                 // 1: the mass matrix's factor is kept on the tree, 0: dense L D L^T
     const uint32_t *tree_lanes;         // 32 x kTreeLaneWords: a lane's place in the coordinate tree (nkb_tree.cuh)
+    uint32_t merges;                    // 1: a contact can act on two branches of the tree; their envs join the branches (merge_trees)
     uint32_t tree_depth, tree_stride;   // joints on the longest root path (0: deeper than kTreeLevels, dense solve only), row stride
     const float *axis, *offset, *local_quat, *inertia10, *damping, *armature, *frictionloss, *stiffness, *spring_ref;
     const float *limit_lower, *limit_upper, *geom_pos, *geom_quat;
@@ -138,6 +143,7 @@ struct SmemLayout {
     uint32_t cstage;                                            // cache rebuild staging (shares the Jacobian pool, dead by then)
     uint32_t heads, jpool, binfo, chol;                         // solver (chol: the articulation's Newton matrix)
     uint32_t factor_words;                                      // words of the mass matrix's factor
+    uint32_t merged;                                            // lane table of a tree joined by contacts (merged_lane_words x 32)
     // Team mode: `team` warps advance one env; warp 0 leads, the others wait for work (rigid blocks of one colour).
     // team_area: 12 command words, then 4 result words per member.
     uint32_t team, team_area;

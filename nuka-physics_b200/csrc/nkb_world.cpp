@@ -368,8 +368,20 @@ void World::BuildLayout() {
     // controllers of modes 3 and 4 work on the dense factor.
     tv.mass_tree = t.tree_depth != 0u && 2u * t.tree_depth <= n && t.cfg.control_mode != 3u && t.cfg.control_mode != 4u ? 1u : 0u;
     const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
-    s.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
+    // Contacts between two links of which neither is an ancestor of the other join branches of the tree (merge_trees), up to the
+    // levels that the solve holds in registers.
+    tv.merges = 0u;
+    if (t.tree_depth != 0u && !(t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) && std::getenv("NUKA_B200_DENSE") == nullptr)       // tests
+        for (uint32_t key : t.adm_pairs) {
+            const uint32_t a = t.body_to_link[key >> 16], b = t.body_to_link[key & 0xffffu];
+            if (a != kNoLink && b != kNoLink && (t.anc_mask[a] & ~t.anc_mask[b]) != 0u && (t.anc_mask[b] & ~t.anc_mask[a]) != 0u) { tv.merges = 1u; break; }
+        }
+    const uint32_t solve_depth = tv.merges == 0u ? t.tree_depth : static_cast<uint32_t>(n > 32u ? kSolveLevels<2> : kSolveLevels<1>);
+    const uint32_t newton_words = std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, solve_depth) : 0u);
+    const uint32_t merged_words = tv.merges != 0u ? 32u * merged_lane_words(n) : 0u;
+    s.chol = take(newton_words);
     at = std::max(at, dynamics_end);
+    s.merged = take(merged_words);
     s.mass = take(n * s.ld); s.factor_words = tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld;
     s.factor = take(s.factor_words); s.vstride = n > 32u ? 64u : 32u;
     s.vecs = take(7 * s.vstride);
@@ -478,11 +490,12 @@ void World::BuildLayout() {
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
     // Split steps (see image_move): for batches that go over the SMs more than once, 12 envs to an SM and up.  Below, one kernel
-    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.70 ms in one kernel, 1.90
-    // split; 3000: 2.86 and 2.24; 1000 humanoids: 6.30 and 6.85; 2048: 9.08 and 8.41).  With free bodies split steps pay earlier
-    // (1200 quadrupeds with 4 boxes: 4.05 and 3.68; 1776: 4.66 and 4.35; 2400: 5.83 and 5.11); one line serves both.
+    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.47 ms in one kernel, 1.73
+    // split; 10 steps of 2500: 4.63 and 3.77).  Articulations of more than 32 coordinates keep four envs on an SM and go over the SMs
+    // more than once earlier: 7 to an SM and up (1000 humanoids: 3.55 and 2.93; 2048: 5.96 and 3.98).  With free bodies split steps pay
+    // earlier too (1200 quadrupeds with 4 boxes: 4.05 and 3.68; 1776: 4.66 and 4.35; 2400: 5.83 and 5.11) and keep the line of 12.
     stages_ = solve_ = nullptr;
-    bool split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && share > 12u && env_count_ > static_cast<uint32_t>(sms) * most;
+    bool split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && share > (n > 32u && t.n_free == 0u ? 7u : 12u) && env_count_ > static_cast<uint32_t>(sms) * most;
     if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && std::atoi(forced) != 0;
     if (split) {
         stages_ = split_variant(n, t.n_free, control, kPartStages); solve_ = split_variant(n, t.n_free, control, kPartSolve);
@@ -493,7 +506,7 @@ void World::BuildLayout() {
         v = s;
         at = 0;
         v.vel = take(6);
-        v.chol = take(std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : 0u));
+        v.chol = take(newton_words); v.merged = take(merged_words);
         v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(7 * s.vstride);
         v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
         v.cdepth = take(4 * SC);
