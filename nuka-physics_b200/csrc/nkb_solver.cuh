@@ -343,14 +343,15 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
     __syncwarp();
 }
 
-// Incidence lists (heads of each block in head order) and greedy colours.  Without free bodies the articulation is the only block.
+// Incidence lists (heads of each block in head order) and greedy colours.  Without free bodies the articulation is the only block; one
+// of fixed joints alone is none, and rows that act on no block (a fixed link on the ground) are left as they are.
 template <bool kRigid>
 NKB_DEV void index_blocks(Env& e, Tile& tile, bool color) {
     const uint32_t nb = tile.nblocks;
     uint32_t* inc = blk_inc(e, nb);
     uint32_t at = 0u;
 #pragma unroll 1
-    for (uint32_t b = kRigid ? 0u : nb - 1u; b < nb; ++b) {
+    for (uint32_t b = kRigid ? 0u : e.t->B; b < nb; ++b) {
         if (e.lane == 0u) blk_inc_begin(e, nb, b) = at;
         if (kRigid && blk_dim(e, b) == 0u) continue;                // no row acts on a block that does not move
 #pragma unroll 1
@@ -382,7 +383,7 @@ NKB_DEV void index_blocks(Env& e, Tile& tile, bool color) {
         __syncwarp();
     }
     if constexpr (!kRigid) {
-        if (color && e.lane == 0u) { block_order(e, nb)[0] = nb - 1u; block_order(e, nb)[nb] = 1u; }
+        if (color && e.lane == 0u) { block_order(e, nb)[0] = e.t->B; block_order(e, nb)[nb] = nb - e.t->B; }
         __syncwarp();
         return;
     }

@@ -91,3 +91,42 @@ def test_a_world_that_does_not_fit_leaves_no_error_behind(device):
         w.destroy()
     by.synchronize()
     by.destroy()
+
+
+def standing(kind):
+    """A world without a coordinate whose shapes touch the ground: a fixed link, a chain of two, a body of infinite mass."""
+    tb = T.TemplateBuilder(1.0 / 200.0, 6, max_contacts=8)
+    if kind == "body":
+        tb.add_free_body((T.SPHERE, 0.05), np.inf, (np.inf,) * 3, (0.0, 0.0, 0.0495, 1.0, 0.0, 0.0, 0.0))
+    else:
+        root = tb.add_link(None, T.FIXED, mass=1.0, inertia_diag=(0.01, 0.01, 0.01), offset=(0.0, 0.0, 0.0495), shape=(T.SPHERE, 0.05))
+        if kind == "chain":
+            tb.add_link(root, T.FIXED, mass=1.0, inertia_diag=(0.01, 0.01, 0.01), offset=(0.3, 0.0, 0.0), shape=(T.BOX, 0.05, 0.05, 0.05))
+    tb.add_plane()
+    return tb
+
+
+# the position phase descends the same blocks again; no sweep at all goes straight to it
+@pytest.mark.parametrize("vel_iters,pos_iters", [(6, 32), (6, 0), (0, 4)])
+@pytest.mark.parametrize("kind,points", [("link", 1), ("chain", 5), ("body", 1)])
+def test_worlds_without_a_coordinate_stand_still(device, oracle, kind, points, vel_iters, pos_iters):
+    """Contacts that act on no block: the world has heads and nothing that moves."""
+    tb = standing(kind)
+    tb.cfg.update(vel_iters=vel_iters, pos_iters=pos_iters)
+    blob = tb.blob()
+    for E in (1, 37):
+        w, o = nuka.World.create_from_template(device, blob, E), oracle.World(blob, E)
+        assert w.info.dofs_per_env == 0
+        w.forward_kinematics()
+        o.refresh()
+        fields = [F.RIGID_BODY_TRANSFORM] + ([F.ARTICULATION_LINK_POSE, F.LINK_VELOCITY] if kind != "body" else [])
+        before = [w.download(f) for f in fields]
+        for n in (1, 3):
+            w.step_n(n)
+        o.step(4)
+        assert not w.download(F.ENV_STATUS).any() and (w.download(F.CONTACT_COUNT).sum(axis=1) == points).all()
+        assert np.array_equal(w.download(F.CONTACT_COUNT), o.get("contact_count", tb.cfg["max_contacts"]))
+        assert np.array_equal(w.download(F.SOLVER_SWEEPS).ravel(), o.get("solver_sweeps", 1).ravel())
+        for f, a in zip(fields, before):
+            assert np.array_equal(w.download(f), a), f
+        w.destroy()
