@@ -106,9 +106,10 @@ class NukaVecEnv:
 
     def _episode_desc(self, actions):
         """The loop's arrays for the library's episode pass (nuka_b200_world_episode_step), or None where the tensor operations
-        below have to do: a task with a reward or an observation of its own, arrays that are not plain ones of the expected type."""
-        torch, E, nj, own = self._torch, self.num_envs, self.num_joints, type(self)
-        if any(getattr(own, name) is not getattr(NukaVecEnv, name) or name in self.__dict__ for name in ("compute_reward", "_up_axis_z", "_compose")):
+        below have to do: a task with a reward or an observation of its own, replaced methods of the world, arrays that are not plain ones
+        of the expected type."""
+        torch, E, nj = self._torch, self.num_envs, self.num_joints
+        if _replaced(self, _STOCK) or _replaced(self.world, _STOCK_WORLD):
             return None
         if not (self._plain(actions, torch.float32, E, nj) and self._plain(self.last_action, torch.float32, E, nj)
                 and self._plain(self.default_position, torch.float32, nj) and self._plain(self.joint_order, torch.int32, nj)
@@ -175,3 +176,13 @@ class NukaVecEnv:
 
     def close(self):
         self.world.destroy()
+
+
+# The methods whose work the library's episode pass does, as they are defined here: one that was replaced later, in a subclass, on
+# the class itself or on one object, is called instead.
+_STOCK = tuple((name, vars(NukaVecEnv)[name]) for name in ("compute_reward", "_up_axis_z", "_compose"))
+_STOCK_WORLD = tuple((name, vars(World)[name]) for name in ("step_n", "reset_envs_masked", "pack_observations"))
+
+
+def _replaced(obj, stock):
+    return any(getattr(type(obj), name) is not function or name in obj.__dict__ for name, function in stock)

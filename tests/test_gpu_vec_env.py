@@ -101,3 +101,36 @@ def test_episode_pass_equals_the_tensor_operations(device, E, order):
     assert all(a == b + 2 for a, b in launches)               # both forms count the world's launches: actions and verdicts are two more
     for env in envs:
         env.close()
+
+
+@pytest.mark.parametrize("where", ["class", "object", "subclass"])
+def test_a_replaced_reward_is_the_one_that_is_paid(device, monkeypatch, where):
+    torch = pytest.importorskip("torch")
+    mine = lambda self: self._base[:, 2] + 7.0
+    kind = type("Task", (NukaVecEnv,), {"compute_reward": mine}) if where == "subclass" else NukaVecEnv
+    env = kind(device, T.quadruped(0).blob(), 5, decimation=2)
+    env.reset()
+    if where == "class":
+        monkeypatch.setattr(NukaVecEnv, "compute_reward", mine)
+    elif where == "object":
+        env.compute_reward = mine.__get__(env)
+    reward = env.step(torch.zeros((5, 12), device="cuda"))[1]
+    assert torch.equal(reward, mine(env))                            # no env ended: the base is where the reward saw it
+    env.close()
+
+
+@pytest.mark.parametrize("where", ["class", "object"])
+def test_replaced_methods_of_the_world_are_called(device, monkeypatch, where):
+    torch = pytest.importorskip("torch")
+    env, calls = NukaVecEnv(device, T.quadruped(0).blob(), 3), []
+    env.reset()
+    for name in ("step_n", "reset_envs_masked", "pack_observations"):
+        stock = getattr(type(env.world), name)
+        watched = lambda world, *args, stock=stock, name=name: (calls.append(name), stock(world, *args))[1]
+        if where == "class":
+            monkeypatch.setattr(type(env.world), name, watched)
+        else:
+            setattr(env.world, name, watched.__get__(env.world))
+    env.step(torch.zeros((3, 12), device="cuda"))
+    assert calls == ["step_n", "reset_envs_masked", "pack_observations"]
+    env.close()
