@@ -107,7 +107,7 @@ class NukaVecEnv:
     def _episode_desc(self, actions):
         """The loop's arrays for the library's episode pass (nuka_b200_world_episode_step), or None where the tensor operations
         below have to do: a task with a reward or an observation of its own, replaced methods of the world, arrays that are not plain ones
-        of the expected type."""
+        of the expected type, settings that are not plain numbers (a scale per joint, a height per env)."""
         torch, E, nj = self._torch, self.num_envs, self.num_joints
         if _replaced(self, _STOCK) or _replaced(self.world, _STOCK_WORLD):
             return None
@@ -116,7 +116,8 @@ class NukaVecEnv:
                 and self._plain(self.default_targets, torch.float32, E, nj + 1) and self._plain(self.command, torch.float32, 3)
                 and self._plain(self.episode_steps, torch.int32, E) and self._plain(self._done_mask, torch.int32, E)
                 and self._plain(self.obs, torch.float32, E, self.obs_width) and self.last_action.data_ptr() == self._obs_desc.last_action
-                and self._obs_desc.row_stride == 0 and self.max_episode_length < 1 << 31):
+                and self._obs_desc.row_stride == 0 and isinstance(self.max_episode_length, int) and abs(self.max_episode_length) < 1 << 31
+                and all(isinstance(value, (int, float)) for value in (self.action_scale, self.termination_height, self.min_up))):
             return None
         d = self._episode
         d.actions, d.last_action, d.default_position = actions.data_ptr(), self.last_action.data_ptr(), self.default_position.data_ptr()

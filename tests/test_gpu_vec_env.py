@@ -134,3 +134,25 @@ def test_replaced_methods_of_the_world_are_called(device, monkeypatch, where):
     env.step(torch.zeros((3, 12), device="cuda"))
     assert calls == ["step_n", "reset_envs_masked", "pack_observations"]
     env.close()
+
+
+# a value per joint or per env, a device scalar, a float where a count is usual, numpy numbers, a length past 32 bits
+@pytest.mark.parametrize("name,make", [("action_scale", lambda t: t.linspace(0.1, 0.4, 12, device="cuda")), ("action_scale", lambda t: t.tensor(0.3, device="cuda")),
+                                       ("action_scale", lambda t: np.float32(0.25)), ("termination_height", lambda t: t.linspace(0.1, 0.4, 6, device="cuda")),
+                                       ("min_up", lambda t: t.full((6,), 0.9999, device="cuda")), ("max_episode_length", lambda t: 2.0),
+                                       ("max_episode_length", lambda t: np.int64(2)), ("max_episode_length", lambda t: 1 << 40),
+                                       ("max_episode_length", lambda t: t.arange(6, device="cuda"))])
+def test_settings_that_are_no_plain_numbers(device, name, make):
+    torch = pytest.importorskip("torch")
+    envs = [kind(device, T.quadruped(0).blob(), 6, decimation=2) for kind in (NukaVecEnv, OwnReward)]
+    for env in envs:
+        env.reset()
+        setattr(env, name, make(torch))
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for _ in range(3):
+        actions = 0.5 * torch.randn((6, 12), generator=gen, device="cuda")
+        (obs, reward, *flags, info), (obs1, reward1, *flags1, info1) = (env.step(actions) for env in envs)
+        assert torch.equal(obs, obs1) and torch.equal(reward, reward1)
+        assert all(torch.equal(a, b) for a, b in zip(flags + [info["done"]], flags1 + [info1["done"]]))
+    for env in envs:
+        env.close()
