@@ -306,7 +306,10 @@ nuka_result_t nuka_b200_world_pack_observations(nuka_world_handle world, const n
  *     max_episode_length and not terminated; done = either
  *     the done envs are reset (as nuka_b200_world_reset_envs_masked) and their targets, last actions and step counts begin again
  *     every env's observation record goes to device_out and to device_copy (E x width floats each), its last action from this desc
- * All pointers are device memory; none may be NULL. */
+ * All pointers are device memory; none may be NULL.  Refused with nothing launched: NUKA_ERR_NOT_SUPPORTED for worlds without a
+ * floating-base articulation, INVALID_ARG for a null pointer, an observation desc with a reward column, a row stride other than the
+ * record width, a command stride of 1 or 2 or a negative clip, and for capacity_floats (what device_out and device_copy hold, each)
+ * below E x width. */
 typedef struct nuka_b200_episode_desc_t {
     const float* actions;            /* E x nj in the caller's joint order */
     float* last_action;              /* E x nj */
@@ -322,8 +325,7 @@ typedef struct nuka_b200_episode_desc_t {
     int32_t max_episode_length;
 } nuka_b200_episode_desc_t;
 nuka_result_t nuka_b200_world_episode_step(nuka_world_handle world, const nuka_b200_episode_desc_t* desc, const nuka_b200_observation_desc_t* observation,
-                                           uint32_t steps, float* device_out, float* device_copy);
-
+                                           uint32_t steps, float* device_out, float* device_copy, size_t capacity_floats);
 
 /* nuka_world_reset_envs (nuka.h:380-385) with the env set chosen on the device: resets every env whose word in
  * device_mask (E x u32 device memory, read on the world's stream) is non-zero and recomputes their derived poses.

@@ -669,7 +669,7 @@ nuka_result_t nuka_b200_world_pack_observations(nuka_world_handle world, const n
 }
 
 nuka_result_t nuka_b200_world_episode_step(nuka_world_handle world, const nuka_b200_episode_desc_t* desc, const nuka_b200_observation_desc_t* observation,
-                                           uint32_t steps, float* device_out, float* device_copy) {
+                                           uint32_t steps, float* device_out, float* device_copy, size_t capacity_floats) {
     NKB_WORLD(w)
     const uint32_t width = w->ObservationWidth();
     if (width == 0u) { SetError("the world has no actuated joints to observe"); return NUKA_RESULT_NOT_SUPPORTED; }
@@ -681,6 +681,7 @@ nuka_result_t nuka_b200_world_episode_step(nuka_world_handle world, const nuka_b
     if (observation->command == nullptr || (observation->command_stride != 0u && observation->command_stride < 3u)) { SetError("observation command is null or its stride below 3"); return NUKA_RESULT_INVALID_ARG; }
     if (observation->reward != nullptr || (observation->row_stride != 0u && observation->row_stride != width)) { SetError("episode steps write records without a reward column, one behind the other"); return NUKA_RESULT_INVALID_ARG; }
     if (!(observation->clip >= 0.f)) { SetError("clip must not be negative"); return NUKA_RESULT_INVALID_ARG; }
+    if (capacity_floats < static_cast<size_t>(width) * w->env_count()) { SetError("observation buffer is too small"); return NUKA_RESULT_INVALID_ARG; }
     nkb::EpisodeParams p{};
     p.actions = d.actions; p.last_action = d.last_action; p.default_position = d.default_position; p.joint_order = d.joint_order;
     p.default_targets = d.default_targets; p.command = d.command; p.episode_steps = d.episode_steps; p.reward = d.reward;

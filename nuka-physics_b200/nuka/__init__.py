@@ -234,8 +234,11 @@ class World:
     def episode_step(self, desc, observation, steps, out, copy):
         """One pass of an episode loop (nuka_b200_world_episode_step): `desc` an _abi.EpisodeDesc, `observation` from observation_desc,
         `out` and `copy` contiguous CUDA float32 tensors of E x record width."""
-        _check(_abi.lib().nuka_b200_world_episode_step(self._h, ctypes.byref(desc), ctypes.byref(observation), int(steps),
-                                                       ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(copy.data_ptr())))
+        for tensor in (out, copy):
+            if not (tensor.is_cuda and tensor.is_contiguous() and tensor.element_size() == 4 and tensor.is_floating_point()):
+                raise ValueError("out and copy must be contiguous float32 tensors on the GPU")
+        _check(_abi.lib().nuka_b200_world_episode_step(self._h, ctypes.byref(desc), ctypes.byref(observation), steps,
+                                                       ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(copy.data_ptr()), min(out.numel(), copy.numel())))
 
     def reset_envs_masked(self, mask):
         """Resets the envs whose word in `mask` (CUDA tensor of E 32-bit words) is non-zero; stays on the world's stream, no host sync."""

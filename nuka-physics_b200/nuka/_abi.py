@@ -112,7 +112,7 @@ def lib():
     L.nuka_b200_observation_desc_defaults.argtypes = [ctypes.POINTER(ObservationDesc)]
     L.nuka_b200_observation_desc_defaults.restype = None
     L.nuka_b200_world_reset_envs_masked.argtypes = [vp, vp]
-    L.nuka_b200_world_episode_step.argtypes = [vp, ctypes.POINTER(EpisodeDesc), ctypes.POINTER(ObservationDesc), u32, vp, vp]
+    L.nuka_b200_world_episode_step.argtypes = [vp, ctypes.POINTER(EpisodeDesc), ctypes.POINTER(ObservationDesc), u32, vp, vp, sz]
     L.nuka_b200_cook_options_defaults.argtypes = [ctypes.POINTER(CookOptions)]
     L.nuka_b200_cook_options_defaults.restype = None
     L.nuka_b200_scene_cook.argtypes = [ctypes.c_char_p, sz, ctypes.POINTER(CookOptions), vp, sz, ctypes.POINTER(sz)]

@@ -156,3 +156,47 @@ def test_settings_that_are_no_plain_numbers(device, name, make):
         assert all(torch.equal(a, b) for a, b in zip(flags + [info["done"]], flags1 + [info1["done"]]))
     for env in envs:
         env.close()
+
+
+def test_episode_steps_refuse_what_does_not_fit(device):
+    """Each refusal of the library's episode pass, with nothing launched and nothing written."""
+    torch = pytest.importorskip("torch")
+    env = NukaVecEnv(device, T.quadruped(0).blob(), 4)
+    env.reset()
+    world, width = env.world, env.obs_width
+    actions = torch.zeros((4, 12), device="cuda")                    # the desc holds addresses only
+    desc = env._episode_desc(actions)
+    out, copy, flags = torch.full((4, width), 3.0, device="cuda"), torch.full((4, width), 3.0, device="cuda"), torch.zeros((4, 4), device="cuda")
+    desc.reward, desc.terminated, desc.truncated, desc.done = (row.data_ptr() for row in flags)
+    before, observed = world.launch_count(), {name: getattr(env._obs_desc, name) for name in ("command", "command_stride", "reward", "row_stride", "clip")}
+    refused = lambda code=nuka._abi.INVALID_ARG: pytest.raises(nuka.NukaError, check=lambda e: e.code == code)
+    for name in ("actions", "last_action", "default_position", "joint_order", "default_targets", "command", "episode_steps", "reward", "terminated", "truncated",
+                 "done", "done_mask"):
+        kept = getattr(desc, name)
+        setattr(desc, name, None)
+        with refused():
+            world.episode_step(desc, env._obs_desc, 1, out, copy)
+        setattr(desc, name, kept)
+    for name, value in (("command", None), ("command_stride", 2), ("reward", flags.data_ptr()), ("row_stride", width + 1), ("clip", -1.0)):
+        setattr(env._obs_desc, name, value)
+        with refused():
+            world.episode_step(desc, env._obs_desc, 1, out, copy)
+        setattr(env._obs_desc, name, observed[name])
+    for pair in ((out[:3], copy), (out, copy[:3]), (out.view(-1)[:-1], copy)):
+        with refused():
+            world.episode_step(desc, env._obs_desc, 1, *pair)
+    for wrong in (copy.double(), copy.int(), copy.cpu(), torch.zeros((4, 2 * width), device="cuda")[:, ::2]):
+        for pair in ((wrong, copy), (out, wrong)):
+            with pytest.raises(ValueError):
+                world.episode_step(desc, env._obs_desc, 1, *pair)
+    arm = nuka.World.create_from_template(device, T.arm7(0).blob(), 4)
+    with refused(nuka._abi.NOT_SUPPORTED):
+        arm.episode_step(desc, env._obs_desc, 1, out, copy)
+    env.world.synchronize()
+    torch.cuda.synchronize()
+    assert world.launch_count() == before and bool((out == 3.0).all()) and bool((copy == 3.0).all())
+    world.episode_step(desc, env._obs_desc, 1, out, copy)
+    env.world.synchronize()
+    assert world.launch_count() > before and torch.equal(out, copy) and not bool((out == 3.0).any())
+    arm.destroy()
+    env.close()
