@@ -65,9 +65,8 @@ enum { kVecAcc = 0, kVecFree = 1, kVecU = 2, kVecPseudo = 3, kVecTmp = 4, kVecTm
        // Newton-loop scratch shares slots whose other users run before or after the solve
        kVecS0 = kVecTmp, kVecS1 = kVecTmp2, kVecS2 = kVecAcc,
        // the Newton direction is staged after the last read of S0 in an iteration and consumed before the next write
-       kVecD = kVecS0,
-       kVecFixed = 6,          // drive impulses by coordinate (stage_rows)
-       kVecCount = 7 };
+       kVecD = kVecS0, kVecCount = 6 };
+NKB_DEV float* sm_fixed(const Env& e) { return e.sm + e.lay->fixed; }
 
 NKB_DEV uint32_t joint_dofs(uint32_t t) { return (t == kRevolute || t == kPrismatic) ? 1u : t == kFloating ? 6u : t == kSpherical ? 3u : 0u; }
 

@@ -185,9 +185,9 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
     // bounds: its impulse is that bound whatever the velocities do, and it adds no stiffness.  So it is no head of the solve: its impulse
     // waits in a vector by coordinate.
     if (NR > 0) {
-        float* fixed = sm_vec(e, kVecFixed);
+        float* fixed = sm_fixed(e);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) fixed[lane + 32u * r] = 0.f;
+        for (int r = 0; r < NR; ++r) if (lane + 32u * r < n) fixed[lane + 32u * r] = 0.f;
         __syncwarp();
         if (lane < L && joint_dofs(e.jtype) == 1u) fixed[e.link_dof] = fminf(fmaxf(e.drive_command, e.drive_lower), e.drive_upper) * dt;
     }

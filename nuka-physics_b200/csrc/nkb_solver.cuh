@@ -41,7 +41,7 @@ NKB_DEV uint32_t* blk_inc(const Env& e, uint32_t nb) { return sm_binfo(e) + 3u *
 constexpr uint32_t kNoUnitHead = 0xffffu;
 NKB_DEV uint16_t* unit_table(const Env& e, uint32_t nb) { return reinterpret_cast<uint16_t*>(sm_binfo(e) + 3u * nb + 1u + 2u * e.t->head_cap); }
 // moving blocks in descent order, order[nb] = their count
-NKB_DEV uint32_t* block_order(const Env& e, uint32_t nb) { return sm_binfo(e) + 3u * nb + 1u + 2u * e.t->head_cap + 2u * e.vstride; }
+NKB_DEV uint32_t* block_order(const Env& e, uint32_t nb) { return sm_binfo(e) + 3u * nb + 1u + 2u * e.t->head_cap + 3u * e.vstride / 2u; }
 NKB_DEV float* sm_bmass(const Env& e, uint32_t b) { return e.sm + e.lay->bmass + 7u * free_slot(e, b); }
 NKB_DEV float* sm_bfree(const Env& e, uint32_t b) { return e.sm + e.lay->bfree + 6u * free_slot(e, b); }
 NKB_DEV float* sm_bpseudo(const Env& e, uint32_t b) { return e.sm + e.lay->bpseudo + 6u * free_slot(e, b); }
@@ -609,7 +609,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
     float start[NR], fr[NR], u[NR], fixed[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        fixed[r] = position || !coord[r] ? 0.f : sm_vec(e, kVecFixed)[l + 32u * r];
+        fixed[r] = position || !coord[r] ? 0.f : sm_fixed(e)[l + 32u * r];
         start[r] = coord[r] ? velocity[l + 32u * r] : 0.f;
         fr[r] = (coord[r] && !position) ? block_free(e, b)[l + 32u * r] : 0.f;
         u[r] = start[r];
@@ -997,7 +997,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         const double fr = coord[r] && !position ? (double)block_free(e, b)[c] : 0.0;
         dir[r] = u[r] - fr;
         inertial[r] = 0.0; force[r] = 0.f;
-        fixed[r] = position || !coord[r] ? 0.f : sm_vec(e, kVecFixed)[c];
+        fixed[r] = position || !coord[r] ? 0.f : sm_fixed(e)[c];
     }
     bool failure = false;
     float primal = FLT_MAX;
@@ -1954,7 +1954,7 @@ NKB_DEV void measure_articulation(Env& e, Tile& tile, bool reconstruct) {
         for (int r = 0; r < NR; ++r) {
             const uint32_t c = l + 32u * r;
             if (!coord[r]) continue;
-            balance[r] = (double)sm_vec(e, kVecFixed)[c] - mass_row_times(e, c, n4 >> 2, wide);
+            balance[r] = (double)sm_fixed(e)[c] - mass_row_times(e, c, n4 >> 2, wide);
             if (tile.units)
 #pragma unroll 1
                 for (uint32_t slot = 0u; slot < 3u; ++slot) {

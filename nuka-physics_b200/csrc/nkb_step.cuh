@@ -120,7 +120,7 @@ NKB_DEV void stage_readout_drives(Env& e, uint32_t nheads) {
     }
     float applied = 0.f;
     if (e.lane < t.L && joint_dofs(e.jtype) == 1u) {
-        const float impulse = sm_vec(e, kVecFixed)[e.link_dof];
+        const float impulse = sm_fixed(e)[e.link_dof];
         if (impulse != 0.f) { applied = impulse / t.cfg.dt - e.drive_dissipation * e.qd; e.tau += applied; }
     }
     if (e.lane < t.L) e.s->actuator[(size_t)e.env * t.L + e.lane] = applied;
@@ -238,7 +238,7 @@ NKB_DEV void image_move(Env& e, const StepParams& p, float* img, uint32_t nheads
         move(a.pairs, b.pairs, t.slot_cap); move(a.cnormal, b.cnormal, 12u * t.slot_cap); move(a.cfeat, b.cfeat, 8u * t.slot_cap);
         return;
     }
-    if (kLoad || kSet == kBefore) move(a.vecs + b.vstride * kVecFixed, b.vecs + b.vstride * kVecFixed, t.ndof);      // the stages' own
+    if (kLoad || kSet == kBefore) move(a.fixed, b.fixed, t.ndof);      // the stages' own
     move(a.vel, b.vel, t.L != 0u ? 6u : 0u);
     move(a.bvel, b.bvel, 6u * slots);
     move(a.heads, b.heads, kHeadStride * nheads);

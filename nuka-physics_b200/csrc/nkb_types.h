@@ -137,6 +137,7 @@ struct StateView {
 struct SmemLayout {
     uint32_t pose, xrot, xtr, vel, vbias, acc, pbias, ic;       // per link
     uint32_t mass, factor, vecs, vstride;                       // articulation (vstride: words per vector, 32 or 64)
+    uint32_t fixed;                                             // drive impulses by coordinate, ndof words (stage_rows)
     uint32_t bpose, bvel, bwinv, aabb, bmass, bfree, bpseudo;   // bodies
     uint32_t pairs, ccount, cpoint, cnormal, cdepth, cfeat;     // contacts
     uint32_t contacts_far;                                      // contact points and normals live in their read-out arrays

@@ -384,7 +384,7 @@ void World::BuildLayout() {
     s.merged = take(merged_words);
     s.mass = take(n * s.ld); s.factor_words = tv.mass_tree != 0u ? tree_scratch_words(tree_rows, t.tree_depth) : n * s.ld;
     s.factor = take(s.factor_words); s.vstride = n > 32u ? 64u : 32u;
-    s.vecs = take(7 * s.vstride);
+    s.vecs = take(6 * s.vstride); s.fixed = take(n);
     const uint32_t slots = B ? t.n_free + 1u : 0u;
     s.bpose = take(7 * B); s.bvel = take(6 * slots);
     s.bwinv = take(6 * slots); s.bmass = take(7 * slots); s.bfree = take(6 * slots); s.bpseudo = take(6 * slots);
@@ -399,7 +399,8 @@ void World::BuildLayout() {
     s.jpool = take(std::max(std::max(tv.point_cap * 3u * ((n + 3u) & ~3u), stage_cap * 10u + 4u * SC + (4u * S + 31u) / 32u), 6u * B));
     s.cstage = s.jpool; s.aabb = s.jpool;
     const uint32_t nb = B + (n ? 1u : 0u);
-    s.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);      // the unit-row table holds 16-bit head indices
+    const uint32_t block_words = 3 * nb + 1 + 2 * tv.head_cap + 3 * s.vstride / 2 + nb + 1;         // the unit-row table holds 16-bit head indices
+    s.binfo = take(block_words);
     const uint32_t without_points = at;
     s.cpoint = take(12 * SC); s.cnormal = take(12 * SC); s.contacts_far = 0u;      // last: a team's env may leave them out
     // Team mode.  An env of many free bodies fills most of an SM's shared memory by itself, so one warp per env would
@@ -507,12 +508,12 @@ void World::BuildLayout() {
         at = 0;
         v.vel = take(6);
         v.chol = take(newton_words); v.merged = take(merged_words);
-        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(7 * s.vstride);
+        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride); v.fixed = take(n);
         v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
         v.cdepth = take(4 * SC);
         v.heads = take(kHeadStride * tv.head_cap);
         v.jpool = take(tv.point_cap * 3u * ((n + 3u) & ~3u));
-        v.binfo = take(3 * nb + 1 + 2 * tv.head_cap + 2 * s.vstride + nb + 1);
+        v.binfo = take(block_words);
         v.words = at;
         size_t top = 0;
         for (uint32_t w = 1; w <= kWarpsPerBlockMax && w * bytes <= 227u * 1024u; ++w) {

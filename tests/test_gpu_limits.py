@@ -130,3 +130,14 @@ def test_worlds_without_a_coordinate_stand_still(device, oracle, kind, points, v
         for f, a in zip(fields, before):
             assert np.array_equal(w.download(f), a), f
         w.destroy()
+
+
+# slices of exactly the 220 KB that a template may take
+@pytest.mark.parametrize("count,contacts,points", [(40, 325, 564), (41, 331, 560)])
+def test_piles_that_just_fit_are_accepted(device, count, contacts, points):
+    tb = T.box_pile(0, count=count)
+    tb.cfg["max_contacts"], tb.max_points = contacts, points
+    w = nuka.World.create_from_template(device, tb.blob(), 3)
+    w.step_n(40)                                             # they have landed
+    assert not w.download(F.ENV_STATUS).any() and w.download(F.CONTACT_COUNT).sum() > 0
+    w.destroy()
