@@ -323,7 +323,7 @@ const T* World::Upload(const std::vector<T>& v) {
     return p;
 }
 
-void World::BuildLayout() {
+void World::BuildLayout(bool join_branches) {
     const HostTemplate& t = tpl_;
     SmemLayout& s = params_.sm;
     const uint32_t L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
@@ -369,9 +369,10 @@ void World::BuildLayout() {
     tv.mass_tree = t.tree_depth != 0u && 2u * t.tree_depth <= n && t.cfg.control_mode != 3u && t.cfg.control_mode != 4u ? 1u : 0u;
     const uint32_t tree_rows = n > 32u ? 32u : n - (t.floating_root ? 6u : 0u);
     // Contacts between two links of which neither is an ancestor of the other join branches of the tree (merge_trees), up to the
-    // levels that the solve holds in registers.
+    // levels that the solve holds in registers.  A slice that their tables and scratch would take past the limit does without (below):
+    // dense systems where branches touch.
     tv.merges = 0u;
-    if (t.tree_depth != 0u && !(t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) && std::getenv("NUKA_B200_DENSE") == nullptr)       // tests
+    if (join_branches && t.tree_depth != 0u && !(t.adm_pairs.size() == 1 && t.adm_pairs[0] == 0u) && std::getenv("NUKA_B200_DENSE") == nullptr)       // tests
         for (uint32_t key : t.adm_pairs) {
             const uint32_t a = t.body_to_link[key >> 16], b = t.body_to_link[key & 0xffffu];
             if (a != kNoLink && b != kNoLink && (t.anc_mask[a] & ~t.anc_mask[b]) != 0u && (t.anc_mask[b] & ~t.anc_mask[a]) != 0u) { tv.merges = 1u; break; }
@@ -444,6 +445,7 @@ void World::BuildLayout() {
     }
     s.words = at;
     const size_t bytes = static_cast<size_t>(s.words) * 4u;
+    if (bytes > 220u * 1024u && tv.merges != 0u) return BuildLayout(false);
     if (bytes > 220u * 1024u) throw Error(kNotSupported, "template needs more shared memory per env than one SM provides");
     // kernel build (regular or slim) and block shape: what keeps the most warps resident on one SM
     const uint32_t team = s.team;                  // a block holds whole teams: w counts warps, w / team envs

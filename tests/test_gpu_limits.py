@@ -141,3 +141,30 @@ def test_piles_that_just_fit_are_accepted(device, count, contacts, points):
     w.step_n(40)                                             # they have landed
     assert not w.download(F.ENV_STATUS).any() and w.download(F.CONTACT_COUNT).sum() > 0
     w.destroy()
+
+
+# a revolute limb beside one that is fixed to the hub, two and three revolute limbs: spheres at the tips, which can touch across
+# branches, and free ones to fill the slice
+@pytest.mark.parametrize("joints,stub,floating,contacts", [(1, True, True, 433), (2, False, True, 433), (3, True, False, 469)])
+def test_a_slice_that_joined_branches_would_overfill_does_without(device, monkeypatch, joints, stub, floating, contacts):
+    """Near the limit the branches stay apart and the envs where they touch take dense systems, as with joining switched off."""
+    tb = T.TemplateBuilder(1.0 / 200.0, 8, max_contacts=contacts, max_points=contacts)
+    hub = tb.add_link(None, T.FLOATING if floating else T.FIXED, mass=2.0, inertia_diag=(0.02,) * 3, offset=(0.0, 0.0, 1.0))
+    limb = dict(mass=0.3, inertia_diag=(0.001,) * 3, com=(0.0, 0.0, 0.05), shape=(T.SPHERE, 0.05), shape_pos=(0.0, 0.0, 0.1), conaffinity=1)
+    if stub:
+        tb.add_link(hub, T.FIXED, offset=(0.09, 0.0, 0.0), **limb)
+    for k in range(joints):
+        tb.add_link(hub, T.REVOLUTE, axis=(0, 1, 0), offset=(-0.09 * k, 0.0, 0.0), **limb)
+    for k in range(41):
+        tb.add_free_body((T.SPHERE, 0.05), 1.0, (0.001,) * 3, (0.2 * k, 0.0, 3.0, 1.0, 0.0, 0.0, 0.0))
+    tb.add_plane()
+    states = []
+    for dense in (False, True):
+        if dense:
+            monkeypatch.setenv("NUKA_B200_DENSE", "1")
+        w = nuka.World.create_from_template(device, tb.blob(), 3)
+        states.append([w.step_n(4)] + [w.download(f) for f in (F.JOINT_VELOCITY, F.BASE_POSE, F.RIGID_BODY_TRANSFORM, F.CONTACT_COUNT, F.ENV_STATUS)])
+        w.destroy()
+    assert states[0][4].sum() > 0 and not states[0][5].any()
+    for a, b in zip(*states):
+        assert np.array_equal(a, b)
