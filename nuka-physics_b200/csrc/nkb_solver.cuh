@@ -513,8 +513,9 @@ NKB_DEV void line_terms(const HeadRegs& r, float alpha, CSum& rs, float& rc, flo
 
 // Exact line search on the block's one-dimensional model (block_descent_tile.cuh:2048-2125): the first
 // evaluation (alpha = 0) gives the initial slope, the following ones bracket and polish the root.  With at most
-// 32 incident heads each lane keeps its head in registers for the whole search.  `fixed` is the constant impulses' slope.
-NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, float icurv, float fixed, float fixed_size) {
+// 32 incident heads each lane keeps its head in registers for the whole search.  `fixed` is this lane's share of the constant impulses'
+// slope, unrounded like the rows' slopes.
+NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, float icurv, const CSum& fixed, float fixed_size) {
     const uint32_t nb = tile.nblocks;
     const uint32_t* inc = blk_inc(e, nb);
     const uint32_t ib = blk_inc_begin(e, nb, b), ie = blk_inc_begin(e, nb, b + 1u);
@@ -532,7 +533,8 @@ NKB_DEV float search_line(Env& e, const Tile& tile, uint32_t b, float islope, fl
 #pragma unroll 1
         for (uint32_t k = ib + e.lane; k < ie; k += 32u) { const HeadRegs r = load_head(e, inc[k]); line_terms(r, alpha, rs, rc, rm); }
         CSum total = {-rs.value, -rs.error};
-        if (e.lane == 0u) { csum_addp(total, alpha, icurv); csum_add(total, islope); csum_add(total, -fixed); }
+        csum_add(total, -fixed.value); csum_add(total, -fixed.error);
+        if (e.lane == 0u) { csum_addp(total, alpha, icurv); csum_add(total, islope); }
         const float slope = warp_csum_total(total);
         const float curvature = icurv + warp_sum(rc);
         const float magnitude = fabsf(islope) + alpha * icurv + fixed_size + warp_sum(rm);
@@ -857,7 +859,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         tick(e, 20);
         row_steps(e, inc, ib, ie, dim, dvec);
         tick(e, 21);
-        const float alpha = search_line(e, tile, b, islope, icurv, warp_csum_total(fix), warp_sum(fix_size));
+        const float alpha = search_line(e, tile, b, islope, icurv, fix, warp_sum(fix_size));
         tick(e, 22);
         tick_count(e, 23);
         float after[NR];
