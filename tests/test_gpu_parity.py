@@ -112,6 +112,32 @@ def test_joint_accelerations_against_a_64_bit_solve(device, name, bar):
     w.destroy()
 
 
+# more sweeps than one have nothing to do
+@pytest.mark.parametrize("vel_iters", [1, 2, 8])
+def test_drives_of_an_articulation_without_rows_against_a_64_bit_solve(device, vel_iters):
+    """From rest and without gravity a step's velocity is M^-1 (tau dt): the direct solve of row-free articulations against a 64-bit one of
+    the kernel's own M.  The result is held in 32 bits (a rounding of 6e-8) and corrected from 64-bit balances: two roundings in all."""
+    E, tb = 512, T.arm7(0)
+    tb.cfg["vel_iters"] = vel_iters
+    w = nuka.World.create_from_template(device, tb.blob(), E, control_mode=1)
+    assert nuka._abi.lib().nuka_world_set_gravity_z(w._h, 0.0) == 0
+    L, rng = w.info.links_per_env, np.random.default_rng(0)
+    state = T.arm7_state(E, 0)
+    w.upload(F.JOINT_POSITION, state["q"] + (0.3 * rng.normal(size=state["q"].shape)).astype(np.float32))
+    tau = (5.0 * rng.normal(size=(E, L))).astype(np.float32)
+    tau[:, 0] = 0.0
+    w.upload(F.DRIVE_TARGET, tau)
+    w.forward_kinematics(); w.run_stage(1)
+    mass = w.download(F.MASS_MATRIX).reshape(E, L - 1, L - 1).astype(np.float64)
+    w.step()
+    impulse = (tau * np.float32(tb.cfg["dt"]))[:, 1:, None].astype(np.float64)
+    want = np.linalg.solve(mass, impulse)[..., 0]
+    error = np.abs(w.download(F.JOINT_VELOCITY).reshape(E, L)[:, 1:] - want).max(axis=1) / np.abs(want).max(axis=1)
+    assert error.max() < 1.2e-7 and not w.download(F.ENV_STATUS).any()
+    assert (w.download(F.SOLVER_SWEEPS) == 1).all()
+    w.destroy()
+
+
 def test_quadruped_single_step_post_solve(device, oracle):
     E = 256
     q, qdot, base, lv = quad_inputs(E)
