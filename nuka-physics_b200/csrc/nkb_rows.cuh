@@ -1,5 +1,5 @@
-// Warp-per-env constraint heads: contact rows (normal + two tangents per point), joint limit, joint friction and
-// drive rows, chain Jacobians of articulated sides, and the contact warm-start cache.
+// Warp-per-env constraint heads: contact rows (normal + two tangents per point), joint limit and joint friction rows, the
+// drives' constant impulses, chain Jacobians of articulated sides, and the contact warm-start cache.
 // A "head" is one solver row group; its state lives in shared memory as a structure of arrays so that one
 // lane can own one head.  Quantities follow the reference's ops/assemble_rows.cu:406-801 (contact rows),
 // :805-971 (joint rows), :122-186 (chain Jacobians), ops/articulation_types.cuh:193-238 and the warm-start
@@ -181,7 +181,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
         }
     }
     __syncwarp();
-    // joint rows, lane = link: limit lower/upper, dry friction, drive (ops/assemble_rows.cu:805-971).  A drive's row has equal
+    // joint rows, lane = link: limit lower/upper, dry friction (ops/assemble_rows.cu:805-971).  The reference's row of a drive has equal
     // bounds: its impulse is that bound whatever the velocities do, and it adds no stiffness.  So it is no head of the solve: its impulse
     // waits in a vector by coordinate.
     if (NR > 0) {

@@ -568,9 +568,11 @@ NKB_DEV void apply_moves(Env& e, const Tile& tile, uint32_t b, float alpha) {
     __syncwarp();
 }
 
-// Newton steps with exact line search on one block, from where it stands.  A descent ends at the block's minimum wherever it begins, so
-// the reference's search toward the free velocity ahead of the first sweep's Newton steps (block_descent_tile.cuh:2196-2210) is left out:
-// with it a policy step of 1000 quadrupeds took 2 % more line evaluations and time, 4096 quadrupeds with 4 boxes 5 %.  A lane owns coordinates lane + 32 r (r < NR) and the same rows of
+// Newton steps with exact line search on one block, from where it stands.  A descent ends at the block's minimum wherever it begins, to
+// rounding, so the reference's search toward the free velocity ahead of the first sweep's Newton steps (block_descent_tile.cuh:2196-2210)
+// is left out: with it a policy step of 1000 quadrupeds took 2 % more line evaluations and time, 4096 quadrupeds with 4 boxes 5 %.
+// Where sweeps end at their limit, or a comparison picks a contact's axis, an env shows the other rounding amplified; against 64 bits
+// both are as far off (linear velocities of 48-box piles after two steps: relative 1.71e-4 either way).  A lane owns coordinates lane + 32 r (r < NR) and the same rows of
 // the Newton matrix, which lives in the env's shared-memory slice in float4-readable rows; lane k also owns the k-th
 // incident head in the row evaluations and publishes its response through the head's shared-memory fields.
 template <int NR>
@@ -1347,7 +1349,7 @@ struct RigidResult { float momentum, residual; uint32_t status; };
 // of the block's own size (its velocity, its mass, the factorisation) is replicated over the group's lanes in registers, so that
 // neither shared memory nor an exchange sits inside those chains.  Loops run until the last group of the warp is done; a group that
 // is done leaves its state alone.  A body of a 48-box pile has 3.5 rows: sixteen lanes to a body, two bodies to a warp, kept twice the
-// warps busy with the same instructions (1024 such piles 20.1 ms, eight lanes 16.3; 700 of 24 boxes 8.07 and 6.20).
+// warps busy with the same instructions (1024 such piles 20.1 ms, eight lanes 15.5; 700 of 24 boxes 8.07 and 5.85).
 constexpr uint32_t kBodyLanes = 8u, kBodyGroups = 32u / kBodyLanes;
 struct BodyLanes {
     uint32_t j, mask, first;             // lane within the group, the group's lanes, its first lane

@@ -143,8 +143,9 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
     }
 }
 
-// Register cap of the regular builds: they settle at 160 registers without spills, three warps to a scheduler partition.  Which
-// worlds are worth a build of 128 registers and four warps is the slim build's question below.
+// Register cap of the regular builds: one coordinate per lane settles at 167 registers without spills, two at the cap with 16 bytes;
+// three warps to a scheduler partition.  Which worlds are worth a build of 128 registers and four warps is the slim build's question
+// below.
 // NR = coordinates per lane: 1 for articulations of up to 32 coordinates, 2 for up to 64, 0 for worlds without one.
 // kRigid = the world has free rigid bodies; without them the rigid-block solver code is compiled out.
 // Worlds with free bodies are held to fewer resident warps by shared memory than by registers (38 KB per env and more),
@@ -156,9 +157,9 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 #define NKB_MAXNREG_RIGID 224
 #endif
 // The slim build of the same kernel: at 128 registers a fourth warp fits each scheduler partition, so small envs (14 KB
-// of shared memory) reach 16 resident warps per SM instead of 12.  It spills about 150 bytes; a world takes it only where the
-// extra residency is really there (World::BuildLayout).  The stages and the solve of split steps fit 128 registers without
-// spills (one coordinate per lane, no free bodies).
+// of shared memory) reach 16 resident warps per SM instead of 12.  It spills about 250 bytes; a world takes it only where the
+// extra residency is really there (World::BuildLayout).  The stages of split steps fit 128 registers without spills, the solve
+// with 8 bytes (one coordinate per lane, no free bodies).
 // Worlds of bodies only run in teams, two piles to an SM: 168 registers for 12 warps, teams of 6 (1024
 // piles of 48 boxes, 2 steps: 14.5 ms; 128 registers, teams of 8 and 400 bytes of spills, 15.5; 700 of 24 4.82 and 5.85).
 #ifndef NKB_MAXNREG_BODIES

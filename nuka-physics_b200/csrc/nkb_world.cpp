@@ -414,8 +414,10 @@ void World::BuildLayout(bool join_branches) {
         uint32_t team = 1u;
         if (t.n_free >= 8u) {
             // The team size that serves an SM best: envs resident at once (by shared memory, and by the registers that the team's
-            // warps need) times what a team of that size makes of one env.  The lead's share of a step does not shrink: a pile of
-            // 48 boxes takes 1, 1/1.6, 1/2.6 and 1/3.8 of the time with 1, 2, 4 and 8 warps.
+            // warps need) times what a team of that size makes of one env.  The lead's share of a step does not shrink: 1024 piles of
+            // 48 boxes, two to an SM, take 35.9, 21.4, 18.6, 14.7 and 14.4 ms with 1, 2, 3, 4 and 6 warps each (296: 9.84, 6.16, 5.32,
+            // 4.46 and 4.27).  The rate's 0.14 and 0.86 were fitted to helpers that had more to do (1, 1/1.6, 1/2.6 and 1/3.8 with 1,
+            // 2, 4 and 8); shares of 0.2 and 0.8, nearer to these times, make the same choice here.
             const uint32_t warps = 65536u / (32u * std::max(1u, static_cast<uint32_t>(step_kernel_registers(tv, false))));
             auto serve = [&](uint32_t words, uint32_t& size) {
                 double top = 0.0;
@@ -492,11 +494,12 @@ void World::BuildLayout(bool join_branches) {
         const uint32_t grid = static_cast<uint32_t>(sms) * static_cast<uint32_t>(fits[warps_per_block_] / warps_per_block_);
         if (grid != 0u && static_cast<size_t>(grid) * warps_per_block_ < env_count_) grid_ = grid;
     }
-    // Split steps (see image_move): for batches that go over the SMs more than once, 12 envs to an SM and up.  Below, one kernel
-    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.47 ms in one kernel, 1.73
-    // split; 10 steps of 2500: 4.63 and 3.77).  Articulations of more than 32 coordinates keep four envs on an SM and go over the SMs
-    // more than once earlier: 7 to an SM and up (1000 humanoids: 3.55 and 2.93; 2048: 5.96 and 3.98).  With free bodies split steps pay
-    // earlier too (1200 quadrupeds with 4 boxes: 4.05 and 3.68; 1776: 4.66 and 4.35; 2400: 5.83 and 5.11) and keep the line of 12.
+    // Split steps (see image_move): for batches that go over the SMs more than once, more than 12 envs to an SM.  Below, one kernel
+    // is faster: the launches of a step wait for its longest solve (4 steps of 2000 quadrupeds: 1.44 ms in one kernel, 1.68
+    // split; 10 steps of 2500: 4.62 and 3.77).  Articulations of more than 32 coordinates keep four envs on an SM and go over the SMs
+    // more than once earlier: more than 7 to an SM (1100 humanoids: 3.87 and 2.97; 2048: 5.96 and 3.98).  Their forms cross at about 4
+    // (600: 2.62 and 2.60; 740: 3.06 and 2.71; 1000, 7 to an SM: 3.62 and 2.88): the line is a safe one, not the best one.  With free bodies split
+    // steps pay earlier too (1200 quadrupeds with 4 boxes: 4.05 and 3.68; 1776: 4.66 and 4.35; 2400: 5.83 and 5.11) and keep the line of 12.
     stages_ = solve_ = nullptr;
     bool split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && share > (n > 32u && t.n_free == 0u ? 7u : 12u) && env_count_ > static_cast<uint32_t>(sms) * most;
     if (const char* forced = std::getenv("NUKA_B200_SPLIT")) split = team == 1u && s.contacts_far == 0u && n != 0u && SC != 0u && std::atoi(forced) != 0;
