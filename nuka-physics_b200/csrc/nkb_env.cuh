@@ -5,6 +5,10 @@
 
 namespace nkb {
 
+// Whether the articulation's multipliers are known: not in use, before the first descent of a step, after it.
+constexpr uint32_t kMergeUntried = 0xffffffffu;
+enum RowsState : uint32_t { kRowsNone = 0, kRowsFresh = 1, kRowsSettled = 2 };
+
 // Per-warp view of one env: template, state, shared-memory slice and this lane's registers.
 struct Env {
     const TemplateView* t;
@@ -21,7 +25,8 @@ struct Env {
     uint32_t dof_link[2], dof_comp[2];   // comp == kNoLink for scalar joints
     uint32_t status;
     bool branching;          // a contact of this step acts on two branches of the articulation's tree
-    uint32_t merged;         // then: depth of the tree with those branches joined, 0 where that is deeper than the solve's levels
+    uint32_t merged;         // then: depth of the tree with those branches joined, 0 where that is deeper than the solve's levels, kMergeUntried before a descent asks
+    uint32_t by_rows, rows;  // the articulation descends in the space of its rows (RowsState), how many there are
     uint32_t vstride;        // words per shared-memory vector: 32 x coordinates per lane
 #ifdef NKB_STAGE_TAPS
     uint32_t* cyc;           // stage cycle counters of this env, or null
@@ -100,7 +105,7 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
         e.dof_comp[r] = kNoLink;
         if (dof && __ldg(t.jtype + e.dof_link[r]) == kFloating) e.dof_comp[r] = c - __ldg(t.link_dof + e.dof_link[r]);
     }
-    e.status = 0u; e.branching = false; e.merged = 0u;
+    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u;
 #ifdef NKB_STAGE_TAPS
     e.cyc = p.s.dbg_cycles != nullptr ? p.s.dbg_cycles + (size_t)env * 32u : nullptr;
     e.t0 = clock64();

@@ -8,8 +8,7 @@
 // :2493-2595 (dual update), :2379-2489 (momentum balance), :2608-2744 (finish, position marks),
 // :2942-3087 (sweep loop) and ops/block_descent.cu:1734-1753 (position bias).
 #pragma once
-#include "nkb_laws.cuh"
-#include "nkb_rows.cuh"
+#include "nkb_rowspace.cuh"
 
 namespace nkb {
 
@@ -294,11 +293,14 @@ NKB_DEV uint32_t merge_trees(Env& e, uint32_t nheads) {
 }
 
 // Head setup: penalty, response scales (block_descent_tile.cuh:743-797).
-template <int NR>
-NKB_DEV void init_heads(Env& e, const Tile& tile) {
+template <int NR, bool kRows>
+NKB_DEV void init_heads(Env& e, const Tile& tile, bool by_rows) {
     const TemplateView& t = *e.t;
     if constexpr (NR > 0) {
-        if (t.mass_tree == 0u) mass_coupling_dense<NR>(e, tile);
+        bool built = false;
+        if constexpr (kRows) { if (by_rows && t.row_cap != 0u) built = build_rows<NR>(e, tile.nheads); }
+        if (built) e.by_rows = kRowsFresh;
+        else if (t.mass_tree == 0u) mass_coupling_dense<NR>(e, tile);
         else if (e.branching) mass_coupling_branching<NR>(e, tile);
     }
 #pragma unroll 1
@@ -315,7 +317,8 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
             else if (ob == t.B) {
                 if constexpr (NR > 0) {
                     const bool unit = (jo & kUnitRow) != 0u;
-                    if (t.mass_tree != 0u && (unit || !e.branching))
+                    if (kRows && e.by_rows != 0u) c = hf(e, HF_RHO, h);
+                    else if (t.mass_tree != 0u && (unit || !e.branching))
                         c = tree_coupling<NR>(e, sm_factor(e), unit ? nullptr : sm_jpool(e) + jo, unit ? jo & 0xffffu : hu(e, HF_RHO, h), hf(e, HF_UNITV, h));
                     else if (unit) c = mass_coupling_unit<NR>(e, jo & 0xffffu, hf(e, HF_UNITV, h));
                     else c = hf(e, HF_RHO, h);
@@ -341,6 +344,13 @@ NKB_DEV void init_heads(Env& e, const Tile& tile) {
         (void)fl;
     }
     __syncwarp();
+    if constexpr (kRows) {
+        if (e.by_rows != 0u) {
+            bool stiff = false;
+            if (e.lane < e.rows) stiff = !(hf(e, HF_RHO, row_table(e)[e.lane] & 0xffffu) * row_w(e)[e.lane * (row_words(e) + 1u)] <= kRowStiffness);
+            if (__any_sync(NKB_FULL, stiff)) e.by_rows = kRowsNone;
+        }
+    }
 }
 
 // Incidence lists (heads of each block in head order) and greedy colours.  Without free bodies the articulation is the only block; one
@@ -568,6 +578,10 @@ NKB_DEV void apply_moves(Env& e, const Tile& tile, uint32_t b, float alpha) {
     __syncwarp();
 }
 
+// A step from a force within its own rounding, shorter than the velocity tolerance, is the last (`settled`): the force can get no smaller, and
+// M^-1 times its rounding may stay above the tolerance on light links.  Such descents ran all 16 steps, 1e-7 m/s each, 6 % of a quadruped's and the
+// longest of every batch (policy steps of 1000: 1100 us -> 863, rollouts of 2500 3.79 ms -> 2.86).
+//
 // Newton steps with exact line search on one block, from where it stands.  A descent ends at the block's minimum wherever it begins, to
 // rounding, so the reference's search toward the free velocity ahead of the first sweep's Newton steps (block_descent_tile.cuh:2196-2210)
 // is left out: with it a policy step of 1000 quadrupeds took 2 % more line evaluations and time, 4096 quadrupeds with 4 boxes 5 %.
@@ -618,7 +632,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         fr[r] = (coord[r] && !position) ? block_free(e, b)[l + 32u * r] : 0.f;
         u[r] = start[r];
     }
-    bool failure = false;
+    bool failure = false, settled = false;
     float primal = FLT_MAX;
     tick(e, 15);
 #pragma unroll 1
@@ -752,7 +766,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 small &= !coord[r] || fabsf(force[r]) <= kRoundings * FLT_EPSILON * scale[r];
             }
             if (!__all_sync(NKB_FULL, finite)) { failure = true; break; }
-            bool converged = __all_sync(NKB_FULL, small);
+            bool converged = settled = __all_sync(NKB_FULL, small);
             if (converged && tile.tol > 0.f) {
                 solve_block_mass<NR>(e, b, force, d);
                 bool still = true;
@@ -882,7 +896,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) u[r] = after[r];
         apply_moves(e, tile, b, alpha);
-        if (rounded) break;
+        if (rounded || (settled && primal < tile.tol)) break;
     }
 #pragma unroll 1
     for (uint32_t k = ib + l; k < ie; k += 32u) {
@@ -1003,7 +1017,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         inertial[r] = 0.0; force[r] = 0.f;
         fixed[r] = position || !coord[r] ? 0.f : sm_fixed(e)[c];
     }
-    bool failure = false;
+    bool failure = false, settled = false;
     float primal = FLT_MAX;
     tick(e, 15);
 #pragma unroll 1
@@ -1099,7 +1113,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         if (step >= 0) {
             rounded = __all_sync(NKB_FULL, rounded);
             primal = rounded ? 0.f : warp_max_positive(longest);
-            if (!(alpha > 0.f) || rounded || step + 1 == (int)kNewtonSteps) break;
+            if (!(alpha > 0.f) || rounded || (settled && primal < tile.tol) || step + 1 == (int)kNewtonSteps) break;
         }
         ++step;
         // ---- the next Newton system at the new velocity: this lane's row of H, its entry of the force balance ----
@@ -1201,7 +1215,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
             small &= !coord[r] || fabsf(force[r]) <= kRoundings * FLT_EPSILON * scale[r];
         }
         if (!__all_sync(NKB_FULL, finite)) { failure = true; break; }
-        bool converged = __all_sync(NKB_FULL, small);
+        bool converged = settled = __all_sync(NKB_FULL, small);
         if (converged && tile.tol > 0.f) {
             float d[NR];
             solve_block_mass<NR>(e, b, force, d);
@@ -1246,6 +1260,182 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
     if (failure) primal = FLT_MAX;
     tile.residual = fmaxf(tile.residual, fmaxf(primal, coupled ? moved : 0.f));
     __syncwarp();
+}
+
+// The articulation's descent in the space of its rows (nkb_rowspace.cuh): the same model, laws, line search and stopping rules as
+// descend_tree, with a lane to a row.  The first descent of a step starts from the multipliers that the heads start from, whatever the
+// block's velocity is; the later ones from the multipliers that the last one left.
+// A descent in coordinates takes a force for zero within kRoundings of its terms, H's entries times the velocities among them: 10 to 50 times
+// the terms of the rows alone.  What decides is that the force moves no coordinate by the velocity tolerance, there and here; a stricter line
+// here ended sweeps elsewhere than the reference ends them.
+constexpr float kRowRoundings = 16.0f * kRoundings;
+template <int NR>
+NKB_DEV bool descend_rows(Env& e, Tile& tile, bool position) {
+    const TemplateView& t = *e.t;
+    const uint32_t l = e.lane, b = t.B, n = t.ndof, m = e.rows;
+    const bool fresh = !position && e.by_rows == kRowsFresh;
+    float* velocity = block_vel(e, b, position);
+    double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
+    RowLane a = {false, false, l, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    bool coupled = false;
+    uint32_t h = 0u, axis = 0u;
+    if (l < m) {
+        const uint32_t entry = row_table(e)[l], owner = hu(e, HF_OWNER, entry & 0xffffu);
+        h = entry & 0xffffu; axis = entry >> 16;
+        a.live = ((owner & 0xffffu) == b || (owner >> 16) == b) && (axis == 0u || (hu(e, HF_FLAGS, h) & kHeadScalar) == 0u);
+        coupled = a.live && (owner & 0xffffu) != kNoBlock16 && (owner >> 16) != kNoBlock16;
+        a.tangent = axis != 0u;
+        if (a.tangent) a.partner = axis == 1u ? l + 1u : l - 1u;
+        const float4 dual = hq(e, HF_DUAL, h), res = hq(e, HF_RES, h);
+        a.dual = axis == 0u ? dual.x : axis == 1u ? dual.y : dual.z;
+        a.res = axis == 0u ? res.x : axis == 1u ? res.y : res.z;
+        a.rho = dual.w; a.lower = hf(e, HF_LOWER, h); a.upper = hf(e, HF_UPPER, h);
+        // the friction cone's radius follows the head's normal multiplier at the start of the descent
+        a.radius = res.w > 0.f ? (dual.x < 0.0f ? 0.0f : dual.x) * res.w : 0.f;
+    }
+    const uint32_t live = __ballot_sync(NKB_FULL, a.live);
+    coupled = __any_sync(NKB_FULL, coupled);
+    if (live == 0u && !fresh) {                     // nothing holds the block: it is where it ends
+        return true;
+    }
+    double y = a.live ? (fresh ? (a.rho > 0.f ? (double)a.dual : 0.0) : row_y(e)[l]) : 0.0;
+    float move = 0.f;
+    const double begin = y;
+    double travel[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) travel[r] = 0.0;
+    if (fresh) {
+        // from the block's velocity to the one that these multipliers give it
+        row_spread<NR>(e, m, y, travel);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint32_t c = l + 32u * r;
+            if (c < n) travel[r] += (double)row_x(e)[m * t.row_stride + c] - ((double)velocity[c] - (double)block_free(e, b)[c]);
+            wide[c] = travel[r];
+        }
+        __syncwarp();
+        if (a.live) move = (float)row_dot(e, h, axis, wide);
+    }
+    const uint32_t half = m <= 1u ? 0u : min(16u, 1u << (31 - __clz(m - 1u)));         // of the lanes with a row
+    bool failure = false, settled = false, stuck = false;
+    float primal = FLT_MAX;
+    RowResponse at = row_respond(a, move);
+    tick(e, 15);
+    float dy = 0.f, alpha = 0.f;
+    int step = 0;
+#pragma unroll 1
+    for (;; ++step) {
+        const float r = a.live ? (float)((double)at.impulse - y) : 0.f;
+        const float noise = fabsf(at.impulse) + fabsf((float)y) + at.curvature * (fabsf(a.res) + fabsf(move));
+        if (!__all_sync(NKB_FULL, isfinite(r) && isfinite(noise))) { failure = true; break; }
+        settled = __all_sync(NKB_FULL, fabsf(r) <= kRowRoundings * FLT_EPSILON * noise);
+        if (settled) {
+            double d[NR];
+            float longest = 0.f;
+#pragma unroll
+            for (int k = 0; k < NR; ++k) d[k] = 0.0;
+            if (tile.tol > 0.f) {
+                row_spread<NR>(e, m, (double)r, d);
+#pragma unroll
+                for (int k = 0; k < NR; ++k) longest = fmaxf(longest, fabsf((float)d[k]));
+                longest = warp_max_positive(longest);
+            }
+            if (!(tile.tol > 0.f) || longest < tile.tol) { primal = 0.f; break; }
+        }
+        tick(e, 17);
+        // ---- (1 + C W) dy = r ----
+        const float s = row_product(e, m, r);
+        float ra = at.curvature >= FLT_MIN ? at.curvature * rsqrt_normal(at.curvature) : 0.f, rb = 0.f;
+        if (__any_sync(NKB_FULL, at.cross != 0.f)) {
+            const float other = __shfl_sync(NKB_FULL, ra, a.partner);
+            if (at.cross != 0.f) { if (axis == 1u) rb = copysignf(other, at.cross); else ra = 0.f; }
+        }
+        if (!solve_rows<kRowGroups<NR>>(e, m, a.partner, ra, rb, r, s, dy)) { failure = true; break; }
+        tick(e, 19);
+        const float along = row_product(e, m, dy);
+        double decrement = (double)r * (double)along;
+        float icurv = dy * along, unused = 0.f;
+        line_sums(decrement, icurv, unused, half, l);
+        const float initial = -(float)decrement;
+        if (!isfinite(initial) || !(icurv <= FLT_MAX)) { failure = true; break; }
+        tick(e, 20);
+        // ---- exact line search (block_descent_tile.cuh:2048-2125) ----
+        const float aside = __shfl_sync(NKB_FULL, along, a.partner);
+        // rows that hold one another (W r = 0) share their load anew without moving the block: a whole step, nothing to search
+        bool search = initial < 0.f, bounded = false;
+        float low = 0.f, high = 0.f;
+        int trials = 0;
+        alpha = 1.f;
+#pragma unroll 1
+        for (;;) {
+            const float trial = fmaf(alpha, along, move);
+            const double ahead = fma((double)alpha, (double)dy, y);
+            at = row_respond(a, trial);
+            tick_count(e, 28);
+            double slope64 = (ahead - (double)at.impulse) * (double)along;
+            float curvature = fmaf(at.curvature, along, at.cross * aside) * along;
+            float magnitude = (fabsf(at.impulse) + fabsf((float)ahead) + kImpulseRounding * at.curvature * (fabsf(a.res) + fabsf(trial))) * fabsf(along);
+            if (!a.live) { slope64 = 0.0; curvature = 0.f; magnitude = 0.f; }
+            line_sums(slope64, curvature, magnitude, half, l);
+            if (!search) break;
+            const float slope = (float)slope64;
+            curvature += icurv;
+            bool give_up = ++trials >= (int)kLineSteps;
+            if (isfinite(slope) && isfinite(curvature)) {
+                if (fabsf(slope) <= fmaxf(kLineTol * -initial, kRoundings * FLT_EPSILON * magnitude)) break;
+                if (slope < 0.f) low = alpha; else { high = alpha; bounded = true; }
+                give_up |= bounded && high - low <= FLT_EPSILON * high;
+                const float next = alpha - __fdividef(slope, curvature);
+                alpha = next > low && (!bounded || next < high) ? next : bounded ? 0.5f * (low + high) : 2.0f * alpha;
+            } else { high = alpha; bounded = true; alpha = 0.5f * (low + high); }
+            if (give_up) { alpha = low; search = false; }       // one more evaluation, at the point returned
+        }
+        tick(e, 22);
+        tick_count(e, 23);
+        // ---- take the step ----
+        const double after = fma((double)alpha, (double)dy, y);
+        const bool rounded = __all_sync(NKB_FULL, after == y);
+        y = after; move = fmaf(alpha, along, move);
+        if (!(alpha > 0.f) || rounded || settled || step + 1 == (int)kNewtonSteps) {
+            double d[NR];
+            float longest = 0.f;
+#pragma unroll
+            for (int k = 0; k < NR; ++k) d[k] = 0.0;
+            row_spread<NR>(e, m, (double)(alpha * dy), d);
+#pragma unroll
+            for (int k = 0; k < NR; ++k) longest = fmaxf(longest, fabsf((float)d[k]));
+            primal = rounded ? 0.f : warp_max_positive(longest);
+            stuck = !settled && step + 1 == (int)kNewtonSteps;
+            if (!settled || !(alpha > 0.f) || rounded || primal < tile.tol || step + 1 == (int)kNewtonSteps) break;
+        }
+    }
+    // ---- the block's velocity and its rows' residuals at the multipliers found ----
+    if (failure) e.status |= kStatusSolverFailure;
+    row_spread<NR>(e, m, a.live ? y - begin : 0.0, travel);
+    float moved = failure ? FLT_MAX : 0.f;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const uint32_t c = l + 32u * r;
+        wide[c] = c < n ? travel[r] : 0.0;
+        if (c < n) {
+            const float before = velocity[c], now = (float)((double)before + travel[r]);
+            moved = fmaxf(moved, residual_abs(now - before));
+            velocity[c] = now;
+        }
+    }
+    __syncwarp();
+    if (a.live) {
+        hf(e, HF_RES + axis, h) = (float)((double)a.res - row_dot(e, h, axis, wide));
+        row_y(e)[l] = y;
+    }
+    if (!position) e.by_rows = kRowsSettled;
+    moved = warp_max_positive(moved);
+    tile.momentum = fmaxf(tile.momentum, moved);
+    if (failure) primal = FLT_MAX;
+    if (!stuck) tile.residual = fmaxf(tile.residual, fmaxf(primal, coupled ? moved : 0.f));
+    __syncwarp();
+    return !stuck;
 }
 
 // ---- team mode: several warps on one env ---------------------------------------------------------------------------------
@@ -1326,7 +1516,7 @@ NKB_DEV Env bare_env(float* sm, const SmemLayout* lay, const TemplateView* t, co
     e.axis = mk3(0.f, 0.f, 0.f);
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
     e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink;
-    e.status = 0u; e.branching = false; e.merged = 0u; e.vstride = vstride;
+    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u; e.vstride = vstride;
 #ifdef NKB_STAGE_TAPS
     e.cyc = nullptr; e.t0 = 0;
 #endif
@@ -1456,7 +1646,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
         // a block without a push-out row keeps its zero position correction; in the velocity phase an unconstrained block
         // still has to reach its free velocity
         const bool began = have && !(position && count == 0u);
-        bool active = began, coupled = false, failure = false;
+        bool active = began, coupled = false, failure = false, settled = false;
 #pragma unroll 1
         for (uint32_t k = g.j; k < count; k += kBodyLanes) {
             const uint32_t h = inc[k], o = hu(e, HF_OWNER, h);
@@ -1576,7 +1766,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                     }
                     if (step >= 0) {
                         primal = rounded ? 0.f : longest;
-                        active = alpha > 0.f && !rounded && step + 1 < (int)kNewtonSteps;
+                        active = alpha > 0.f && !rounded && !(settled && primal < run.tol) && step + 1 < (int)kNewtonSteps;
                     }
                 }
             }
@@ -1636,6 +1826,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             float inv[6], x[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i) rhs[i] = force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
+            settled = small;
             if (active && small) {
                 bool still = true;
                 if (run.tol > 0.f) {
@@ -1726,21 +1917,28 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
 }
 
 // The articulation's block: on its tree, with the branches joined that a contact acts on; dense where that is too deep.
-template <int NR, bool kRigid>
+template <int NR, bool kRows>
 NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
-    if (e.t->tree_depth != 0u && (!e.branching || e.merged != 0u)) descend_tree<NR>(e, tile, position);
+    if constexpr (kRows) {
+        if (e.by_rows != 0u) {
+            if (descend_rows<NR>(e, tile, position)) return;
+            e.by_rows = kRowsNone;                   // from where the rows left the block
+        }
+    }
+    if (e.branching && e.t->merges != 0u && e.merged == kMergeUntried) e.merged = merge_trees<NR>(e, tile.nheads);
+    if (e.t->tree_depth != 0u && (!e.branching || (e.t->merges != 0u && e.merged != 0u))) descend_tree<NR>(e, tile, position);
     else descend_block<NR>(e, tile, e.t->B, position);
 }
 
 // Blocks descend colour by colour, blocks of one colour in index order (block_descent_tile.cuh:2749-2820).
-template <int NR, bool kRigid>
+template <int NR, bool kRigid, bool kRows>
 NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
     const uint32_t nb = tile.nblocks;
     const uint32_t* order = block_order(e, nb);
     const uint32_t count = order[nb];
     if constexpr (!kRigid) {
 #pragma unroll 1
-        for (uint32_t k = 0u; k < count; ++k) descend_articulation<NR, false>(e, tile, position);
+        for (uint32_t k = 0u; k < count; ++k) descend_articulation<NR, kRows>(e, tile, position);
     } else {
         const uint32_t team = e.lay->team;
         RigidRun run;
@@ -1749,7 +1947,7 @@ NKB_DEV void descend_blocks(Env& e, Tile& tile, bool position) {
 #pragma unroll 1
         for (uint32_t k = 0u; k < count;) {
             const uint32_t b = order[k];
-            if constexpr (NR > 0) { if (b == e.t->B) { descend_articulation<NR, kRigid>(e, tile, position); ++k; continue; } }
+            if constexpr (NR > 0) { if (b == e.t->B) { descend_articulation<NR, kRows>(e, tile, position); ++k; continue; } }
             // the run of rigid blocks that share b's colour (a rigid block's 6 coordinates: one per lane)
             const uint32_t colour = blk_color(e, nb, b);
             uint32_t k_end = k + 1u;
@@ -2005,16 +2203,86 @@ NKB_DEV void measure_articulation(Env& e, Tile& tile, bool reconstruct) {
     }
 }
 
+// The same where the block descends in the space of its rows.  The velocity is first put in balance with the descent's own multipliers
+// (M^-1 J^T carries the factor's rounding, 1e-7 of a term; the balance is taken in 64 bits and costs nothing that the measure would
+// not), then what the physical multipliers differ by is known from the rows.
+template <int NR>
+NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
+    const TemplateView& t = *e.t;
+    const uint32_t l = e.lane, b = t.B, n = t.ndof, m = e.rows, n4 = (n + 3u) & ~3u;
+    float* velocity = block_vel(e, b, false);
+    const float* fr = block_free(e, b);
+    double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
+#pragma unroll
+    for (int r = 0; r < NR; ++r) wide[l + 32u * r] = l + 32u * r < n ? (double)velocity[l + 32u * r] - fr[l + 32u * r] : 0.0;
+    __syncwarp();
+    double balance[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) balance[r] = l + 32u * r < n ? (double)sm_fixed(e)[l + 32u * r] - mass_row_times(e, l + 32u * r, n4 >> 2, wide) : 0.0;
+#pragma unroll 1
+    for (uint32_t k = 0u; k < m; ++k) {
+        const uint32_t entry = row_table(e)[k], h = entry & 0xffffu, jo = hu(e, HF_JOFF, h);
+        const double y = row_y(e)[k];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint32_t c = l + 32u * r;
+            if (c >= n) continue;
+            if (!(jo & kUnitRow)) balance[r] = fma((double)sm_jpool(e)[jo + (entry >> 16) * n4 + c], y, balance[r]);
+            else if (c == (jo & 0xffffu)) balance[r] = fma((double)hf(e, HF_UNITV, h), y, balance[r]);
+        }
+    }
+    float force[NR], dir[NR];
+    bool ok = true;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) { force[r] = (float)balance[r]; dir[r] = 0.f; ok &= fabs(balance[r]) <= FLT_MAX; }
+    const bool finite = __all_sync(NKB_FULL, ok);
+    float residual = FLT_MAX;
+    if (finite) {
+        solve_block_mass<NR>(e, b, force, dir);
+        double lag[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) lag[r] = 0.0;
+        const uint32_t entry = l < m ? row_table(e)[l] : 0u;
+        row_spread<NR>(e, m, l < m ? (double)comp(head_lambda(e, entry & 0xffffu), (int)(entry >> 16)) - row_y(e)[l] : 0.0, lag);
+        float worst = 0.f;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint32_t c = l + 32u * r;
+            if (c < n) {
+                worst = fmaxf(worst, isfinite(dir[r]) && isfinite((float)lag[r]) ? fabsf((float)lag[r]) : FLT_MAX);
+                if (reconstruct) dir[r] += (float)lag[r];
+                velocity[c] += dir[r];
+            }
+            wide[c] = c < n ? (double)dir[r] : 0.0;
+        }
+        residual = warp_max_positive(worst);
+        __syncwarp();
+        if (l < m) {
+            const uint32_t h = entry & 0xffffu, axis = entry >> 16;
+            hf(e, HF_RES + axis, h) = (float)((double)hf(e, HF_RES + axis, h) - row_dot(e, h, axis, wide));
+            if (reconstruct) row_y(e)[l] = (double)comp(head_lambda(e, h), (int)axis);
+        }
+        __syncwarp();
+    }
+    tile.residual = fmaxf(tile.residual, residual);
+    if (reconstruct && finite) tile.momentum = fmaxf(tile.momentum, residual);
+}
+
 // Momentum balance of every moving block against the physical multipliers (block_descent_tile.cuh:2379-2489).
-template <int NR, bool kRigid>
+template <int NR, bool kRigid, bool kRows>
 NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
     if constexpr (kRigid) measure_bodies(e, tile, reconstruct);
-    if constexpr (NR > 0) measure_articulation<NR>(e, tile, reconstruct);
+    if constexpr (NR > 0) {
+        if constexpr (kRows) { if (e.by_rows != 0u) { measure_rows<NR>(e, tile, reconstruct); return; } }
+        measure_articulation<NR>(e, tile, reconstruct);
+    }
 }
 
 // The whole constraint solve of one env.  On entry the heads are built, the articulation's post-dynamics
 // velocity is in (e.qd, sm_vel(root)) and free-body velocities are in sm_bvel.
-template <int NR, bool kRigid>
+// kRows: contacts can act on the articulation, so that its descent in the space of its rows is compiled in.
+template <int NR, bool kRigid, bool kRows>
 NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
     const TemplateView& t = *e.t;
     const uint32_t l = e.lane, B = t.B, n = NR > 0 ? t.ndof : 0u;
@@ -2073,8 +2341,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
         }
     }
     __syncwarp();
-    init_heads<NR>(e, tile);
-    if constexpr (NR > 0) { if (e.branching && t.merges != 0u) e.merged = merge_trees<NR>(e, nheads); }
+    init_heads<NR, kRows>(e, tile, kRigid || nheads != 0u);
     tick(e, 8);
     float rows[3] = {0.f, 0.f, 0.f};
     float cls[4] = {0.f, 0.f, 0.f, 0.f};
@@ -2170,12 +2437,14 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
                 }
                 push = __any_sync(NKB_FULL, push); coupled = __any_sync(NKB_FULL, coupled);
                 __syncwarp();
-                if (push) { phase = kPhasePosition; reindex = true; positions = coupled ? t.cfg.pos_iters : 1u; pushes = 0u; }
+                if (push) {
+                    if (NR > 0 && e.by_rows != 0u) { if (l < e.rows) row_y(e)[l] = 0.0; __syncwarp(); }
+                    phase = kPhasePosition; reindex = true; positions = coupled ? t.cfg.pos_iters : 1u; pushes = 0u; }
             }
             continue;
         }
         if (phase == kPhaseVelocity) { ++sweeps; tile.momentum = 0.f; tile.residual = 0.f; }
-        if (!linear) descend_blocks<NR, kRigid>(e, tile, phase == kPhasePosition);
+        if (!linear) descend_blocks<NR, kRigid, kRows>(e, tile, phase == kPhasePosition);
         if (phase == kPhasePosition) {
             if (++pushes >= positions) { phase = kPhaseDone; continue; }
         } else tick(e, 10);
@@ -2192,7 +2461,7 @@ NKB_DEV void stage_solve(Env& e, uint32_t nheads) {
             else if (stage == 1) run = worst_row < tile.tol && tile.residual >= tile.tol && tile.residual < FLT_MAX;
             if (stage == 1 && !run) break;
             const bool reconstruct = stage == 1 || (linear && stage == 0);
-            if (run) { measure_primals<NR, kRigid>(e, tile, reconstruct); tick(e, 25); tick_count(e, 27); }
+            if (run) { measure_primals<NR, kRigid, kRows>(e, tile, reconstruct); tick(e, 25); tick_count(e, 27); }
             if (linear && !(tile.residual < FLT_MAX)) { e.status |= kStatusSolverFailure; break; }
             if (reconstruct) {
                 if (!(tile.residual < FLT_MAX)) break;

@@ -313,7 +313,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             tick(e, 13);
             if (kPart == kPartStages ? p.last != 0u : step == p.steps) return;
         }
-        e.status = 0u; e.branching = false; e.merged = 0u;
+        e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone;
         if (p.mode == kModeRefresh) {
             if (has_bodies) stage_store_bodies(e, false);
             if (has_artic) {
@@ -378,7 +378,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
       }
-        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid>(e, nheads);
+        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid, NR != 0 && kPart != kPartBare>(e, nheads);
         if constexpr (kPart == kPartSolve) {
             image_move<false, kAfter>(e, p, img, nheads);
             __stcg(reinterpret_cast<float*>(lanes + lane), e.qd);

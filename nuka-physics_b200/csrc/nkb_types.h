@@ -24,6 +24,11 @@ template <int NR> constexpr int kSolveLevels = NR > 1 ? 2 * kTreeLevels : kTreeL
 NKB_HOST_DEVICE constexpr uint32_t merged_lane_words(uint32_t ndof) { return 2u + (ndof > 32u ? 2u : 1u) * kTreeLevels / 4u; }
 // Row stride (words) and scratch words of the tree-structured solve for `rows` joint lanes and root paths of `depth` joints.
 NKB_HOST_DEVICE inline uint32_t tree_row_stride(uint32_t depth) { return depth <= 5u ? 12u : depth <= 13u ? 20u : 36u; }
+// Groups of three rows that a descent in the rows' space holds in registers
+template <int NR> constexpr int kRowGroups = NR > 1 ? 6 : 5;
+// The rows' space (nkb_rowspace.cuh): M^-1 J^T of `rows` rows and the drives, J M^-1 J^T, the row table; then the multipliers, 64 bits each
+NKB_HOST_DEVICE constexpr uint32_t row_space_head(uint32_t rows, uint32_t stride) { return ((rows + 1u) * stride + rows * (rows | 1u) + rows + 3u) & ~3u; }
+inline uint32_t row_space_words(uint32_t rows, uint32_t stride) { return rows == 0u ? 0u : row_space_head(rows, stride) + 2u * rows; }
 inline uint32_t tree_scratch_words(uint32_t rows, uint32_t depth) { return rows * tree_row_stride(depth) + 48u + 28u; }
 constexpr uint32_t kMaxBodies = 256u;   // collidable rows per env (the env's shared-memory slice is the practical limit)
 constexpr uint32_t kPtsPerSlot = 4u;
@@ -74,6 +79,7 @@ struct TemplateView {
     uint32_t mass_tree;                 // 1: the mass matrix's factor is kept on the tree, 0: dense L D L^T
     const uint32_t *tree_lanes;         // 32 x kTreeLaneWords: a lane's place in the coordinate tree (nkb_tree.cuh)
     uint32_t merges;                    // 1: a contact can act on two branches of the tree; their envs join the branches (merge_trees)
+    uint32_t row_cap, row_stride;       // rows of the articulation that its descent in their space holds (0: in coordinates), words per row (nkb_rowspace.cuh)
     uint32_t tree_depth, tree_stride;   // joints on the longest root path (0: deeper than kTreeLevels, dense solve only), row stride
     const float *axis, *offset, *local_quat, *inertia10, *damping, *armature, *frictionloss, *stiffness, *spring_ref;
     const float *limit_lower, *limit_upper, *geom_pos, *geom_quat;

@@ -323,7 +323,7 @@ const T* World::Upload(const std::vector<T>& v) {
     return p;
 }
 
-void World::BuildLayout(bool join_branches) {
+void World::BuildLayout(bool join_branches, bool rows) {
     const HostTemplate& t = tpl_;
     SmemLayout& s = params_.sm;
     const uint32_t L = t.L, B = t.B, n = t.ndof, S = t.cfg.max_contacts;
@@ -378,7 +378,12 @@ void World::BuildLayout(bool join_branches) {
             if (a != kNoLink && b != kNoLink && (t.anc_mask[a] & ~t.anc_mask[b]) != 0u && (t.anc_mask[b] & ~t.anc_mask[a]) != 0u) { tv.merges = 1u; break; }
         }
     const uint32_t solve_depth = tv.merges == 0u ? t.tree_depth : static_cast<uint32_t>(n > 32u ? kSolveLevels<2> : kSolveLevels<1>);
-    const uint32_t newton_words = std::max(n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, solve_depth) : 0u);
+    // Rows of the articulation that its descent in their space holds.
+    tv.row_stride = s.ld;
+    tv.row_cap = 0u;
+    if (rows && tv.mass_tree != 0u && std::getenv("NUKA_B200_DENSE") == nullptr) tv.row_cap = std::min(3u * static_cast<uint32_t>(n > 32u ? kRowGroups<2> : kRowGroups<1>), 3u * tv.point_cap + t.joint_rows);
+    if (const char* forced = std::getenv("NUKA_B200_ROWS")) tv.row_cap = std::min(tv.row_cap, static_cast<uint32_t>(std::atoi(forced)));       // tests
+    const uint32_t newton_words = std::max({row_space_words(tv.row_cap, tv.row_stride), n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, solve_depth) : 0u});
     const uint32_t merged_words = tv.merges != 0u ? 32u * merged_lane_words(n) : 0u;
     s.chol = take(newton_words);
     at = std::max(at, dynamics_end);
@@ -447,7 +452,8 @@ void World::BuildLayout(bool join_branches) {
     }
     s.words = at;
     const size_t bytes = static_cast<size_t>(s.words) * 4u;
-    if (bytes > 220u * 1024u && tv.merges != 0u) return BuildLayout(false);
+    if (bytes > 220u * 1024u && tv.row_cap != 0u) return BuildLayout(join_branches, false);
+    if (bytes > 220u * 1024u && tv.merges != 0u) return BuildLayout(false, rows);
     if (bytes > 220u * 1024u) throw Error(kNotSupported, "template needs more shared memory per env than one SM provides");
     // kernel build (regular or slim) and block shape: what keeps the most warps resident on one SM
     const uint32_t team = s.team;                  // a block holds whole teams: w counts warps, w / team envs

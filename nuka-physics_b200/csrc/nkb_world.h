@@ -98,7 +98,7 @@ private:
     template <typename T> T* Alloc(size_t count, bool zero = true);
     template <typename T> const T* Upload(const std::vector<T>& v);
     void Check(cudaError_t err, const char* what);
-    void BuildLayout(bool join_branches = true);
+    void BuildLayout(bool join_branches = true, bool rows = true);
     void Seed();
 
     int device_;

@@ -1,0 +1,46 @@
+"""The articulation's descent in the space of its constraint rows against the one in its coordinates."""
+import numpy as np
+import pytest
+
+from nuka import Field as F, templates as T
+from test_gpu_merged_tree import star
+from test_gpu_variants import create, outputs
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(name, E):
+    rng = np.random.Generator(np.random.PCG64(len(name)))
+    if name == "quadruped":
+        return T.quadruped(0), T.quadruped_state(E, 0)
+    limbs, depth, floating, joint = {"limits": (2, 2, True, dict(limits=(-0.1, 0.1), frictionloss=0.02)),       # 12 rows of joints, with a contact the 15 that fit
+                                     "fixed": (4, 2, False, {}), "deep": (3, 5, True, {}),
+                                     "wide": (5, 6, True, {})}[name]                                              # two coordinates per lane
+    n = limbs * depth
+    q = np.zeros((E, n + 1), np.float32)
+    q[:, 1:] = 0.25 * rng.standard_normal((E, n))
+    state = {"q": q, "qdot": np.zeros_like(q)}
+    state["qdot"][:, 1:] = rng.standard_normal((E, n))
+    if floating:
+        state["base_pose"] = np.zeros((E, 7), np.float32)
+        state["base_pose"][:, 2:4] = 1.0
+    return star(limbs, depth, floating, **joint), state
+
+
+# Every row that fits; 14 and 4 rows at most, no multiples of the three that a contact has (envs with more take the coordinates);
+# split steps.  The bars of one step's velocities against the reference: 1e-5 of max(|v|, 1).  A sweep ends an env's solve where its
+# rows' residual falls below 1e-5 m/s, so two roundings can end it a sweep apart, which moves a light joint at the end of a limb by
+# that residual over its lever of 0.04 m: up to 3e-4 rad/s per row, of which a tip has three.
+@pytest.mark.parametrize("name", ["quadruped", "limits", "fixed", "deep", "wide"])
+@pytest.mark.parametrize("forced", [{}, {"ROWS": 14}, {"ROWS": 4}, {"SPLIT": 1}], ids=["all", "14", "4", "split"])
+def test_rows_equal_coordinates(device, name, forced):
+    E = 96
+    tb, state = scene(name, E)
+    rows = outputs(create(device, tb, state, E, **forced), (1,))
+    coordinates = outputs(create(device, tb, state, E, ROWS=0), (1,))
+    assert rows["CONTACT_COUNT"].sum() > 0 and rows["ENV_STATUS"].max() == 0 and coordinates["ENV_STATUS"].max() == 0
+    got, want = rows["JOINT_VELOCITY"].astype(np.float64), coordinates["JOINT_VELOCITY"].astype(np.float64)
+    assert np.array_equal(got, want) == (name == "limits" and forced.get("ROWS") == 4)          # the other route, where the joints' rows leave room
+    error = np.abs(got - want).max(axis=1) / np.maximum(np.abs(want).max(axis=1), 1.0)
+    assert np.percentile(error, 95) < 1e-5 and error.max() < 1e-3, (float(np.percentile(error, 95)), float(error.max()))
+    assert (rows["SOLVER_SWEEPS"] == coordinates["SOLVER_SWEEPS"]).mean() > 0.95
