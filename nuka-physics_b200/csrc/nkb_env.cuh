@@ -27,6 +27,8 @@ struct Env {
     bool branching;          // a contact of this step acts on two branches of the articulation's tree
     uint32_t merged;         // then: depth of the tree with those branches joined, 0 where that is deeper than the solve's levels, kMergeUntried before a descent asks
     uint32_t by_rows, rows;  // the articulation descends in the space of its rows (RowsState), how many there are
+    float* pool;             // where stage_rows leaves the contact rows' Jacobians
+    uint32_t reach;          // contact heads that act on the articulation; the others have no rows there
     uint32_t vstride;        // words per shared-memory vector: 32 x coordinates per lane
 #ifdef NKB_STAGE_TAPS
     uint32_t* cyc;           // stage cycle counters of this env, or null
@@ -105,7 +107,7 @@ NKB_DEV void env_begin(Env& e, const StepParams& p, float* sm, uint32_t env, uin
         e.dof_comp[r] = kNoLink;
         if (dof && __ldg(t.jtype + e.dof_link[r]) == kFloating) e.dof_comp[r] = c - __ldg(t.link_dof + e.dof_link[r]);
     }
-    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u;
+    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u; e.reach = 0u; e.pool = sm + p.sm.jpool;
 #ifdef NKB_STAGE_TAPS
     e.cyc = p.s.dbg_cycles != nullptr ? p.s.dbg_cycles + (size_t)env * 32u : nullptr;
     e.t0 = clock64();

@@ -147,16 +147,22 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
                 }
             }
         }
-        float* pool = sm_jpool(e);
+        float* pool = e.pool;
+        e.reach = 0u;
 #pragma unroll 1
         for (uint32_t h = 0u; h < ncontact; ++h) {
             const uint32_t ref = hu(e, HF_REF, h), la = ref >> 16, lb = hu(e, HF_JOFF, h) & 0xffffu;
+            if (la == 0xffffu && lb == 0xffffu) {                    // between bodies: no row here
+                __syncwarp();
+                if (lane == 0u) { hu(e, HF_JOFF, h) = 0u; hu(e, HF_RHO, h) = 0xffu; }
+                continue;
+            }
             if (la != 0xffffu && lb != 0xffffu) {
                 const uint32_t ma = __ldg(t.anc_mask + la), mb = __ldg(t.anc_mask + lb);
                 e.branching |= (ma & ~mb) != 0u && (mb & ~ma) != 0u;
             }
             __syncwarp();      // every lane has read the side-b link before lane 0 replaces it with the pool offset
-            const uint32_t n4 = (n + 3u) & ~3u, joff = h * 3u * n4;
+            const uint32_t n4 = (n + 3u) & ~3u, joff = e.reach++ * 3u * n4;
             const V3 point = ld3(sm_cpoint(e, ref & 0xffffu));
             const V3 dirs[3] = {hf3(e, HF_N, h), hf3(e, HF_T1, h), hf3(e, HF_T2, h)};
 #pragma unroll

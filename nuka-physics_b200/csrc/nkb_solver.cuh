@@ -1516,7 +1516,7 @@ NKB_DEV Env bare_env(float* sm, const SmemLayout* lay, const TemplateView* t, co
     e.axis = mk3(0.f, 0.f, 0.f);
     e.drive_command = e.drive_dissipation = e.drive_lower = e.drive_upper = 0.f;
     e.dof_link[0] = e.dof_link[1] = 0u; e.dof_comp[0] = e.dof_comp[1] = kNoLink;
-    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u; e.vstride = vstride;
+    e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.rows = 0u; e.reach = 0u; e.pool = sm + lay->jpool; e.vstride = vstride;
 #ifdef NKB_STAGE_TAPS
     e.cyc = nullptr; e.t0 = 0;
 #endif

@@ -148,8 +148,8 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 // below.
 // NR = coordinates per lane: 1 for articulations of up to 32 coordinates, 2 for up to 64, 0 for worlds without one.
 // kRigid = the world has free rigid bodies; without them the rigid-block solver code is compiled out.
-// Worlds with free bodies are held to fewer resident warps by shared memory than by registers (38 KB per env and more),
-// so their variants take a wider cap: no spills, and a team of 8 warps still fits the register file.
+// Whole steps with free bodies are held to fewer resident warps by shared memory than by registers, so they take a wider cap: no
+// spills, and a team of 8 warps still fits the register file.
 #ifndef NKB_MAXNREG
 #define NKB_MAXNREG 176
 #endif
@@ -164,6 +164,11 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 // piles of 48 boxes, 2 steps: 14.5 ms; 128 registers, teams of 8 and 400 bytes of spills, 15.5; 700 of 24 4.82 and 5.85).
 #ifndef NKB_MAXNREG_BODIES
 #define NKB_MAXNREG_BODIES 168
+#endif
+// The parts of split steps, where slices are small: three warps to a partition (solves of quadrupeds with boxes at 224 registers and
+// no spills, two: 5.22 ms; at 168 and 150 bytes, three: 4.74).
+#ifndef NKB_MAXNREG_SPLIT
+#define NKB_MAXNREG_SPLIT 168
 #endif
 #ifndef NKB_MAXNREG_SLIM
 #define NKB_MAXNREG_SLIM 128
@@ -247,7 +252,7 @@ NKB_DEV void image_move(Env& e, const StepParams& p, float* img, uint32_t nheads
         move(a.mass, b.mass, t.ndof * b.ld); move(a.factor, b.factor, b.factor_words);
         move(a.bwinv, b.bwinv, 6u * slots);
         move(a.cdepth, b.cdepth, 4u * t.slot_cap);
-        move(a.jpool, b.jpool, 3u * n4 * min(nheads, t.point_cap));
+        if (kLoad) move(a.jpool, b.jpool, 3u * n4 * e.reach);            // the stages write it in place
     } else {
         move(a.vecs + b.vstride * kVecPseudo, b.vecs + b.vstride * kVecPseudo, t.ndof);
         move(a.bpseudo, b.bpseudo, 6u * slots);
@@ -273,11 +278,12 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
         img = p.image + (size_t)(env - p.image_first) * p.image_stride;
         lanes = reinterpret_cast<float4*>(img + p.image_stride - kImageLaneWords);
         tail = reinterpret_cast<uint32_t*>(lanes + 32);
+        if (kPart == kPartStages) e.pool = img + p.im.jpool;            // nothing here reads the rows
         if (resumed) {
             const float4 mine = __ldcg(lanes + lane);
             const uint4 words = __ldcg(reinterpret_cast<const uint4*>(tail));
             e.qd = mine.x; e.qdd = mine.y; e.tau = mine.z; e.drive_dissipation = mine.w;
-            e.status = lane == 0u ? words.x : 0u; nheads = words.y; e.branching = words.z != 0u;
+            e.status = lane == 0u ? words.x : 0u; nheads = words.y; e.branching = words.z != 0u; e.reach = words.w;
             image_move<true, kPart == kPartSolve ? kBefore : kAfter>(e, p, img, nheads);
             if (kPart == kPartStages) image_move<true, kAside>(e, p, img, nheads);
             __syncwarp();
@@ -374,7 +380,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             image_move<false, kBefore>(e, p, img, nheads); image_move<false, kAside>(e, p, img, nheads);
             __stcg(lanes + lane, make_float4(e.qd, e.qdd, e.tau, e.drive_dissipation));
             const uint32_t st = __reduce_or_sync(NKB_FULL, e.status);
-            if (lane == 0u) __stcg(reinterpret_cast<uint4*>(tail), make_uint4(st, nheads, e.branching ? 1u : 0u, 0u));
+            if (lane == 0u) __stcg(reinterpret_cast<uint4*>(tail), make_uint4(st, nheads, e.branching ? 1u : 0u, e.reach));
             return;
         }
       }
@@ -471,13 +477,19 @@ NKB_DEV void team_helper(float* sm, const SmemLayout& shared_layout, const Templ
 // Block layout: blockDim.x / 32 warps, `team` consecutive warps per env (one unless the world runs in team mode); an
 // env's shared-memory slice is shared by its team.
 template <int NR, bool kRigid, bool kSlim, bool kControl, int kPart>
-__global__ void __maxnreg__(NR == 0 ? NKB_MAXNREG_BODIES : kRigid ? NKB_MAXNREG_RIGID : (kSlim ? NKB_MAXNREG_SLIM : NKB_MAXNREG)) step_kernel(const __grid_constant__ StepParams p) {
+__global__ void __maxnreg__(NR == 0 ? NKB_MAXNREG_BODIES : kSlim ? NKB_MAXNREG_SLIM : kSplitPart<kPart> ? NKB_MAXNREG_SPLIT : kRigid ? NKB_MAXNREG_RIGID : NKB_MAXNREG) step_kernel(const __grid_constant__ StepParams p) {
     extern __shared__ __align__(16) float smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t team = kRigid ? p.sm.team : 1u;
     const uint32_t slot = warp / team, member = warp - slot * team;
     uint32_t env = blockIdx.x * ((blockDim.x >> 5) / team) + slot;
     if constexpr (kSplitPart<kPart>) env = p.first + env < p.end ? p.first + env : 0xffffffffu;
+    if constexpr (kPart == kPartSolve) {
+        if (p.tier != kTierAll && env != 0xffffffffu) {
+            const uint4 words = __ldcg(reinterpret_cast<const uint4*>(p.image + (size_t)(env - p.image_first + 1u) * p.image_stride - 4u));
+            if ((words.y <= p.tier_heads && words.w <= p.tier_reach) != (p.tier == kTierSmall)) return;
+        }
+    }
     float* sm = smem + (size_t)slot * p.sm.words;
     if constexpr (kRigid) {
         // team mode: every lead zeroes its team's sequence numbers before any helper looks (a block-wide barrier, passed by

@@ -169,6 +169,9 @@ constexpr uint32_t kImageLaneWords = 4u * 32u + 4u;     // an image's tail: four
 
 enum StepMode : uint32_t { kModeStep = 0, kModeDynamicsOnly = 1, kModeCollideOnly = 2, kModeRefresh = 3 };
 
+// Which envs a launch of solves takes: all, those whose heads and rows fit the small slice, the others.
+enum SolveTier : uint32_t { kTierAll = 0, kTierSmall = 1, kTierLarge = 2 };
+
 struct StepParams {
     TemplateView t;
     StateView s;
@@ -184,6 +187,7 @@ struct StepParams {
     float* image;
     uint32_t image_stride;
     uint32_t first, end, image_first;   // the envs of this launch, the env the images start with
+    uint32_t tier, tier_heads, tier_reach;   // part 2 (SolveTier): heads and contacts of the articulation that the small slice holds
     uint32_t resume, last;              // part 1: finish the step whose solve is done first; stop there
     SmemLayout im;
     // Env selection of a refresh launch (null: every env).  sel_ids lists sel_count envs, one warp each; sel_mask is

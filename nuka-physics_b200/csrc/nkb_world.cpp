@@ -398,7 +398,8 @@ void World::BuildLayout(bool join_branches, bool rows) {
     const uint32_t SC = tv.slot_cap;
     s.pairs = take(SC); s.ccount = take(SC); s.cdepth = take(4 * SC); s.cfeat = take(8 * SC);                       // cfeat: contact identity words
     // before the heads exist the region serves the tree broadphase and then the narrowphase as scratch
-    s.heads = take(std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kTeamMax : 1u)) : 0u));
+    const uint32_t heads_words = std::max(kHeadStride * tv.head_cap, SC != 0u ? std::max(lbvh_scratch_words(B), manifold_scratch_words(B, t.n_free != 0u ? kTeamMax : 1u)) : 0u);
+    s.heads = take(heads_words);
     // the Jacobian pool also holds the AABBs (dead once the narrowphase is done) and, after the solve, the cache staging
     // entries, owner marks and retained bits
     const uint32_t stage_cap = std::min(tv.point_cap, 4u * SC);
@@ -514,18 +515,50 @@ void World::BuildLayout(bool join_branches, bool rows) {
     }
     if (stages_ != nullptr) {
         // the solve's slice: what it reads and its own scratch, nothing of the kinematics and the contacts
-        SmemLayout& v = solve_sm_;
-        v = s;
-        at = 0;
-        v.vel = take(6);
-        v.chol = take(newton_words); v.merged = take(merged_words);
-        v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride); v.fixed = take(n);
-        v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
-        v.cdepth = take(4 * SC);
-        v.heads = take(kHeadStride * tv.head_cap);
-        v.jpool = take(tv.point_cap * 3u * ((n + 3u) & ~3u));
-        v.binfo = take(block_words);
-        v.words = at;
+        auto solve_slice = [&](SmemLayout& v, uint32_t heads, uint32_t reach) {
+            v = s;
+            at = 0;
+            v.vel = take(6);
+            v.chol = take(newton_words); v.merged = take(merged_words);
+            v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride); v.fixed = take(n);
+            v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bmass = take(7 * slots); v.bfree = take(6 * slots); v.bpseudo = take(6 * slots);
+            v.cdepth = take(4 * SC);
+            v.heads = take(kHeadStride * heads);
+            v.jpool = take(reach * 3u * ((n + 3u) & ~3u));
+            v.binfo = take(block_words - 2 * (tv.head_cap - heads));
+            v.words = at;
+        };
+        solve_slice(solve_sm_, tv.head_cap, tv.point_cap);
+        // A slice is sized for every contact that the template admits; a step has a few of them.  Envs whose heads and rows fit a small
+        // slice are solved in it, more of them to an SM, the others in a launch behind that is empty as a rule: as many contacts of the
+        // articulation as its rows' space holds, five of a free body.  2048 humanoids, 4 steps: 50 KB, 4 to an SM, 2.53 ms; 22 KB, 10 to an SM,
+        // 1.96.  4096 quadrupeds with 4 boxes: 8 to an SM 5.35 ms, 12 in 4.74.  Where registers hold the same number anyway, or the batch fits the large slices at once, there is one.
+        small_heads_ = std::min(tv.head_cap, (tv.row_cap / 3u + t.joint_rows + 5u * t.n_free + 3u) & ~3u);
+        small_reach_ = std::min(tv.point_cap, tv.row_cap / 3u);
+        small_sm_.words = 0u;
+        if (tv.row_cap != 0u && std::getenv("NUKA_B200_ONE_TIER") == nullptr) {          // tests
+            solve_slice(small_sm_, small_heads_, small_reach_);
+            const int many = solve_->resident_blocks(1, small_sm_.words * 4u), few = solve_->resident_blocks(1, solve_sm_.words * 4u);
+            const bool worth = 4 * many >= 5 * few && env_count_ > static_cast<uint32_t>(sms * few);
+            if (!worth && std::getenv("NUKA_B200_TWO_TIERS") == nullptr) small_sm_.words = 0u;
+        }
+        // the stages' slice: no solver's scratch, and the rows' Jacobians go where the solve loads them from
+        {
+            SmemLayout& v = stages_sm_;
+            v = s;
+            at = 0;
+            v.pose = take(7 * L); v.vel = take(6 * L);
+            v.xrot = take(9 * L); v.xtr = take(3 * L); v.acc = take(6 * L); v.pbias = take(6 * L); v.ic = take(10 * L); v.chol = v.merged = v.xrot;
+            v.mass = take(n * s.ld); v.factor = take(s.factor_words); v.vecs = take(6 * s.vstride); v.fixed = take(n);
+            v.bpose = take(7 * B); v.bvel = take(6 * slots); v.bwinv = take(6 * slots); v.bpseudo = take(6 * slots); v.bmass = v.bfree = v.bpseudo;
+            v.pairs = take(SC); v.ccount = take(SC); v.cdepth = take(4 * SC); v.cfeat = take(8 * SC);
+            v.heads = take(heads_words);
+            v.jpool = v.cstage = v.aabb = take(std::max(stage_cap * 10u + 4u * SC + (4u * S + 31u) / 32u, 6u * B));
+            v.cpoint = take(12 * SC); v.cnormal = take(12 * SC);
+            v.binfo = v.jpool;
+            v.words = at;
+        }
+        const size_t bytes = static_cast<size_t>(stages_sm_.words) * 4u;
         size_t top = 0;
         for (uint32_t w = 1; w <= kWarpsPerBlockMax && w * bytes <= 227u * 1024u; ++w) {
             const size_t r = static_cast<size_t>(stages_->resident_blocks(w, w * bytes)) * w;
@@ -533,8 +566,8 @@ void World::BuildLayout(bool join_branches, bool rows) {
         }
     }
     if (std::getenv("NUKA_B200_DEBUG_LAYOUT") != nullptr) {
-        if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %d registers, %u warps per block; solve %u B, %d registers, %d resident\n", stages_->registers(), stages_warps_,
-                                             solve_sm_.words * 4u, solve_->registers(), solve_->resident_blocks(1, solve_sm_.words * 4u));
+        if (stages_ != nullptr) std::fprintf(stderr, "[nuka_b200] split: stages %u B, %d registers, %u warps per block; solve %u B, %d registers, %d resident; small %u B, %d resident\n", stages_sm_.words * 4u, stages_->registers(), stages_warps_,
+                                             solve_sm_.words * 4u, solve_->registers(), solve_->resident_blocks(1, solve_sm_.words * 4u), small_sm_.words * 4u, small_sm_.words != 0u ? solve_->resident_blocks(1, small_sm_.words * 4u) : 0);
         std::fprintf(stderr, "[nuka_b200] %zu B of shared memory per env, %d registers per thread%s; resident warps per SM by block size:", bytes,
                      step_kernel_registers(tv, slim_), slim_ ? " (slim build)" : "");
         for (uint32_t w = 1; w <= kWarpsPerBlockMax; ++w) std::fprintf(stderr, " %u:%zu", w, fits[w]);
@@ -815,12 +848,21 @@ void World::EnqueueSteps(uint32_t n) {
                 p.first = done + static_cast<uint32_t>(static_cast<uint64_t>(round) * c / kChunks);
                 p.end = done + static_cast<uint32_t>(static_cast<uint64_t>(round) * (c + 1u) / kChunks);
                 StepParams v = p;
-                v.sm = solve_sm_;
+                v.sm = solve_sm_; v.tier = kTierAll;
+                p.sm = stages_sm_;
                 for (uint32_t k = 0; k <= n; ++k) {
                     p.resume = k != 0u ? 1u : 0u; p.last = k == n ? 1u : 0u;
                     Check(stages_->launch(p, stages_warps_, stream), "step stages launch");
                     ++launches_;
                     if (k == n) break;
+                    if (small_sm_.words != 0u) {
+                        StepParams few = v;
+                        few.sm = small_sm_; few.t.head_cap = small_heads_;
+                        few.tier = kTierSmall; v.tier = kTierLarge;
+                        few.tier_heads = v.tier_heads = small_heads_; few.tier_reach = v.tier_reach = small_reach_;
+                        Check(solve_->launch(few, 1u, stream), "step solve launch");
+                        ++launches_;
+                    }
                     Check(solve_->launch(v, 1u, stream), "step solve launch");
                     ++launches_;
                 }

@@ -114,7 +114,9 @@ private:
     // split steps (null variants: steps run in one kernel): the kernels, the solve's own shared-memory layout, block size of the
     // stages, the envs' images between launches
     const StepVariant *stages_ = nullptr, *solve_ = nullptr;
-    SmemLayout solve_sm_{};
+    SmemLayout solve_sm_{}, stages_sm_{};
+    SmemLayout small_sm_{};            // the solves' small slice (words 0: none), and what it holds
+    uint32_t small_heads_ = 0, small_reach_ = 0;
     uint32_t stages_warps_ = 1;
     uint32_t image_envs_ = 0;                  // envs the image buffer holds: larger batches go in rounds
     static constexpr uint32_t kChunks = 3u;    // parts of a round, each on a stream of its own

@@ -4,7 +4,7 @@ import pytest
 
 from nuka import Field as F, templates as T
 from test_gpu_merged_tree import star
-from test_gpu_variants import create, outputs
+from test_gpu_variants import assert_same, create, outputs
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,20 @@ def test_rows_equal_coordinates(device, name, forced):
     error = np.abs(got - want).max(axis=1) / np.maximum(np.abs(want).max(axis=1), 1.0)
     assert np.percentile(error, 95) < 1e-5 and error.max() < 1e-3, (float(np.percentile(error, 95)), float(error.max()))
     assert (rows["SOLVER_SWEEPS"] == coordinates["SOLVER_SWEEPS"]).mean() > 0.95
+
+
+# Solves in two slices against one, and against whole steps: the same bits.  With four rows the small slice holds one contact, so that both
+# slices have envs to solve; with free bodies one that touches nothing counts as well
+@pytest.mark.parametrize("name", ["quadruped", "boxes", "wide"])
+@pytest.mark.parametrize("rows", [4, 64])
+def test_small_and_large_slices_equal_whole_steps(device, name, rows):
+    E = 300
+    if name == "boxes":
+        tb, state = T.quadruped(0, boxes=2), T.quadruped_state(E, 0)
+    else:
+        tb, state = scene(name, E)
+    whole, one, two = (outputs(create(device, tb, state, E, ROWS=rows, **forced), (2, 1))
+                       for forced in (dict(SPLIT=0), dict(SPLIT=1, ONE_TIER=1), dict(SPLIT=1, TWO_TIERS=1)))
+    assert two["CONTACT_COUNT"].sum() > 0
+    assert_same(whole, one)
+    assert_same(one, two)
