@@ -276,6 +276,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
 
 NKB_DEV uint32_t head_pair(const Env& e, uint32_t h) { return sm_pairs(e)[(hu(e, HF_REF, h) & 0xffffu) >> 2]; }
 
+constexpr uint32_t kCacheChunk = 4u;           // entries per lane that a search of the cache loads at once
 // Warm start (phase 0): a contact head takes the multipliers of the cached point with the same identity.
 // Range form: this warp takes the heads first, first + stride, ... (a head's match reads earlier heads and the cache and
 // writes only the head's own dual).
@@ -302,14 +303,22 @@ NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t 
             }
             dup |= __any_sync(NKB_FULL, same);
         }
-        if (dup) continue;
+        if (dup) { if (e.lane == 0u) hu(e, HF_FLAGS, h) |= kHeadDuplicate; continue; }
         uint32_t found = 0xffffffffu;
+        // a chunk's pairs are loaded at once: one after another, a pile of 48 boxes waited 8 k cycles per head for them
 #pragma unroll 1
-        for (uint32_t base = 0u; base < npts && found == 0xffffffffu; base += 32u) {
-            const uint32_t c = base + e.lane;
-            const bool hit = c < npts && cache[c].pair == pair && cache[c].feature == feat && cache[c].age < 2u;
-            const uint32_t m = __ballot_sync(NKB_FULL, hit);
-            if (m != 0u) found = base + (uint32_t)__ffs(m) - 1u;
+        for (uint32_t base = 0u; base < npts && found == 0xffffffffu; base += 32u * kCacheChunk) {
+            uint32_t pairs[kCacheChunk];
+#pragma unroll
+            for (uint32_t k = 0u; k < kCacheChunk; ++k) { const uint32_t c = base + 32u * k + e.lane; pairs[k] = c < npts ? cache[c].pair : 0xffffffffu; }
+#pragma unroll
+            for (uint32_t k = 0u; k < kCacheChunk; ++k) {
+                if (found != 0xffffffffu || !__any_sync(NKB_FULL, pairs[k] == pair)) continue;
+                const uint32_t c = base + 32u * k + e.lane;
+                const bool hit = pairs[k] == pair && cache[c].feature == feat && cache[c].age < 2u;
+                const uint32_t m = __ballot_sync(NKB_FULL, hit);
+                if (m != 0u) found = base + 32u * k + (uint32_t)__ffs(m) - 1u;
+            }
         }
         if (found == 0xffffffffu) continue;
         if (e.lane == 0u) {
@@ -327,7 +336,7 @@ NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t 
     __syncwarp();
 }
 
-// Marks of the cache rebuild: the first current point of each identity owns its cache entry; an entry of age 0 that no current
+// Marks of the cache rebuild: the first current point of each identity (the warm start marked the others) owns its cache entry; an entry of age 0 that no current
 // point matches is retained (one bit each, behind the owners).  Range form over the contact heads first, first + stride, ... (a
 // head's test reads earlier heads and writes its own point's mark) and over the entries' words of bits likewise.  Walking all
 // heads for every live entry was the longest part of the rebuild on a team's lead (48-box piles, 1024 envs: 20.5 ms before, 19.9).
@@ -336,40 +345,36 @@ NKB_DEV void cache_owners_range(Env& e, uint32_t ncontact, uint32_t first, uint3
     const uint32_t stage_cap = min(t.point_cap, t.slot_cap * 4u);
     uint32_t* owner = reinterpret_cast<uint32_t*>(reinterpret_cast<CacheEntry*>(e.sm + e.lay->cstage) + stage_cap);
 #pragma unroll 1
-    for (uint32_t h = first; h < ncontact; h += stride) {
-        const uint32_t at = hu(e, HF_REF, h) & 0xffffu;
-        const uint32_t pair = head_pair(e, h);
-        const uint32_t* f = sm_cfeat(e, at);
-        bool dup = false;
-#pragma unroll 1
-        for (uint32_t base = 0u; base < h; base += 32u) {
-            const uint32_t j = base + e.lane;
-            bool same = false;
-            if (j < h) { const uint32_t* g = sm_cfeat(e, hu(e, HF_REF, j) & 0xffffu); same = head_pair(e, j) == pair && g[0] == f[0] && g[1] == f[1]; }
-            dup |= __any_sync(NKB_FULL, same);
-        }
-        if (!dup && e.lane == 0u) owner[at] = h;
-    }
+    for (uint32_t h = 32u * first + e.lane; h < ncontact; h += 32u * stride)
+        if ((hu(e, HF_FLAGS, h) & kHeadDuplicate) == 0u) owner[hu(e, HF_REF, h) & 0xffffu] = h;
     const uint32_t npts = t.cfg.max_contacts * 4u;
     const CacheEntry* cache = e.s->cache + (size_t)e.env * npts;
     uint32_t* retained = owner + t.slot_cap * 4u;
 #pragma unroll 1
     for (uint32_t word = first; 32u * word < npts; word += stride) {
         const uint32_t c = 32u * word + e.lane;
-        bool keep = false;
-        if (c < npts) {
-            const uint32_t pair = cache[c].pair;
-            const unsigned long long feature = cache[c].feature;
-            keep = pair != 0xffffffffu && cache[c].age < 1u;
-#pragma unroll 1
-            for (uint32_t h = 0u; h < ncontact && keep; ++h) {
+        const uint32_t pair = c < npts ? cache[c].pair : 0xffffffffu;
+        bool keep = pair != 0xffffffffu && cache[c].age < 1u;
+        uint32_t m = __ballot_sync(NKB_FULL, keep);
+        if (m != 0u) {
+            const unsigned long long feature = keep ? cache[c].feature : 0ull;
+#pragma unroll 4
+            for (uint32_t h = 0u; h < ncontact; ++h) {
                 const uint32_t* f = sm_cfeat(e, hu(e, HF_REF, h) & 0xffffu);
-                if (head_pair(e, h) == pair && (((unsigned long long)f[1] << 32) | f[0]) == feature) keep = false;
+                keep = keep && !(head_pair(e, h) == pair && (((unsigned long long)f[1] << 32) | f[0]) == feature);
             }
+            // the first of equal entries stays: the few that are left are looked for by all lanes
+            m = __ballot_sync(NKB_FULL, keep);
 #pragma unroll 1
-            for (uint32_t d = 0u; d < c && keep; ++d) if (cache[d].pair == pair && cache[d].feature == feature) keep = false;
+            for (uint32_t left = m; left != 0u; left &= left - 1u) {
+                const uint32_t lane = (uint32_t)__ffs(left) - 1u, at = 32u * word + lane, wanted = __shfl_sync(NKB_FULL, pair, lane);
+                const unsigned long long identity = __shfl_sync(NKB_FULL, feature, lane);
+                bool earlier = false;
+#pragma unroll 4
+                for (uint32_t d = e.lane; d < at; d += 32u) if (cache[d].pair == wanted) earlier |= cache[d].feature == identity;
+                if (__any_sync(NKB_FULL, earlier)) m &= ~(1u << lane);
+            }
         }
-        const uint32_t m = __ballot_sync(NKB_FULL, keep);
         if (e.lane == 0u) retained[word] = m;
     }
     __syncwarp();

@@ -43,7 +43,8 @@ enum : uint32_t { kStatusPairOverflow = 1u << 0, kStatusDofOverflow = 1u << 2, k
 // head flags
 enum : uint32_t { kHeadContact = 1u << 0, kHeadContactNormal = 1u << 1, kHeadSpeculative = 1u << 2,
                   kHeadVelocityOnly = 1u << 3, kHeadLimit = 1u << 5, kHeadFriction = 1u << 6,
-                  kHeadScalar = 1u << 7 /* position pass: only the normal axis */ };
+                  kHeadScalar = 1u << 7 /* position pass: only the normal axis */,
+                  kHeadDuplicate = 1u << 8 /* an earlier contact point of this step has the same identity */ };
 constexpr uint32_t kHeadStride = 60u;   // words of shared memory per solver head: groups of four, 28 mod 32 for conflict-free vector access
 
 // Scratch words of the tree broadphase for B collidable rows (nkb_lbvh.cuh): sorted keys, internal nodes (children, range,
