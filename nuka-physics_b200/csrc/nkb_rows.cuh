@@ -197,6 +197,7 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
         __syncwarp();
         if (lane < L && joint_dofs(e.jtype) == 1u) fixed[e.link_dof] = fminf(fmaxf(e.drive_command, e.drive_lower), e.drive_upper) * dt;
     }
+    if (t.joint_rows != 0u)
 #pragma unroll 1
     for (uint32_t kind = 0u; kind < 3u; ++kind) {
         bool emit = false;

@@ -296,6 +296,7 @@ NKB_DEV uint32_t merge_trees(Env& e, uint32_t nheads) {
 template <int NR, bool kRows>
 NKB_DEV void init_heads(Env& e, const Tile& tile, bool by_rows) {
     const TemplateView& t = *e.t;
+    if (tile.nheads == 0u && !by_rows) return;
     if constexpr (NR > 0) {
         bool built = false;
         if constexpr (kRows) { if (by_rows && t.row_cap != 0u) built = build_rows<NR>(e, tile.nheads); }
@@ -358,6 +359,16 @@ NKB_DEV void init_heads(Env& e, const Tile& tile, bool by_rows) {
 template <bool kRigid>
 NKB_DEV void index_blocks(Env& e, Tile& tile, bool color) {
     const uint32_t nb = tile.nblocks;
+    if (!kRigid && tile.nheads == 0u) {                 // the articulation alone, no row on it
+        if (e.lane == 0u) {
+            if (nb != e.t->B) blk_inc_begin(e, nb, e.t->B) = 0u;
+            blk_inc_begin(e, nb, nb) = 0u;
+            block_order(e, nb)[0] = e.t->B; block_order(e, nb)[nb] = nb - e.t->B;
+        }
+        tile.units = false;
+        __syncwarp();
+        return;
+    }
     uint32_t* inc = blk_inc(e, nb);
     uint32_t at = 0u;
 #pragma unroll 1
@@ -2004,6 +2015,8 @@ struct DualMomentum { float t, beta; };
 
 // Dual update over every head (block_descent_tile.cuh:2493-2595); returns the residual classes.
 NKB_DEV void update_duals(Env& e, const Tile& tile, DualMomentum* mom, bool velocity, bool commit, float out[3]) {
+    out[0] = out[1] = out[2] = 0.f;
+    if (tile.nheads == 0u) return;
     float cn = 0.f, ct = 0.f, cj = 0.f;
     double restart = 0.0;
 #pragma unroll 1

@@ -73,6 +73,7 @@ struct TemplateView {
     uint32_t L, B, ndof, max_depth, n_excluded, floating_root;
     uint32_t head_cap;          // solver heads per env held in shared memory
     uint32_t point_cap;         // contact points per env that get rows
+    uint32_t joint_rows;        // limit and dry-friction rows of the joints
     uint32_t slot_cap;          // candidate slots one step can fill: min(max_contacts, admissible pairs)
     const uint32_t *parent, *jtype, *depth, *child_begin, *children, *link_dof, *link_body, *geom_kind, *limit_flags;
     const uint32_t *dof_link, *anc_mask;

@@ -343,6 +343,7 @@ void World::BuildLayout(bool join_branches, bool rows) {
         // bounds the head records and Jacobian pool in shared memory; the template may ask for more than the default
         tv.point_cap = std::min(total, t.max_points != 0u ? t.max_points : 128u);
     }
+    tv.joint_rows = t.joint_rows;
     tv.head_cap = (tv.point_cap + t.joint_rows + 3u) & ~3u;
     if (tv.head_cap == 0u) tv.head_cap = 4u;
     if (t.cfg.control_mode == 4u) {
