@@ -2218,7 +2218,8 @@ NKB_DEV void measure_articulation(Env& e, Tile& tile, bool reconstruct) {
 
 // The same where the block descends in the space of its rows.  The velocity is first put in balance with the descent's own multipliers
 // (M^-1 J^T carries the factor's rounding, 1e-7 of a term; the balance is taken in 64 bits and costs nothing that the measure would
-// not), then what the physical multipliers differ by is known from the rows.
+// not), then what the physical multipliers differ by is known from the rows: a reconstruction, which
+// follows a measure, only adds it.
 template <int NR>
 NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
     const TemplateView& t = *e.t;
@@ -2226,10 +2227,13 @@ NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
     float* velocity = block_vel(e, b, false);
     const float* fr = block_free(e, b);
     double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
+    double balance[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) balance[r] = 0.0;
+    if (!reconstruct) {
 #pragma unroll
     for (int r = 0; r < NR; ++r) wide[l + 32u * r] = l + 32u * r < n ? (double)velocity[l + 32u * r] - fr[l + 32u * r] : 0.0;
     __syncwarp();
-    double balance[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) balance[r] = l + 32u * r < n ? (double)sm_fixed(e)[l + 32u * r] - mass_row_times(e, l + 32u * r, n4 >> 2, wide) : 0.0;
 #pragma unroll 1
@@ -2244,6 +2248,7 @@ NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
             else if (c == (jo & 0xffffu)) balance[r] = fma((double)hf(e, HF_UNITV, h), y, balance[r]);
         }
     }
+    }
     float force[NR], dir[NR];
     bool ok = true;
 #pragma unroll
@@ -2251,7 +2256,7 @@ NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
     const bool finite = __all_sync(NKB_FULL, ok);
     float residual = FLT_MAX;
     if (finite) {
-        solve_block_mass<NR>(e, b, force, dir);
+        if (!reconstruct) solve_block_mass<NR>(e, b, force, dir);
         double lag[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) lag[r] = 0.0;
