@@ -15,7 +15,9 @@
 // What bounds it is the chain of one warp: build_rows over the joints, one after another, solve_rows over groups of three rows, the
 // line search.  In coordinates (descend_tree) a Newton system was an assembly over the heads, an elimination over the tree's levels and the
 // base's six, and a product with M: 6.6 k cycles on a quadruped alone, here 2.5 k.  Policy steps of 4096 quadrupeds 2050 -> 1750 us, of
-// 16 384 7.44 -> 6.27 ms, of 2048 humanoids 3.68 -> 2.53 ms, a rollout of 2500 2.81 -> 2.35 ms.
+// 16 384 7.44 -> 6.27 ms, of 2048 humanoids 3.68 -> 2.53 ms, a rollout of 2500 2.81 -> 2.35 ms.  A batch at rest, one Newton step to a descent, pays for
+// W (4096 standing quadrupeds 0.263 -> 0.312 ms); taking coordinates for the envs whose rows are within 0.01 m/s of their target has the warps of an
+// SM run both codes out of one instruction cache: 0.285 ms there, and 16 384 quadrupeds 6.2 -> 10.7 ms.
 #pragma once
 #include "nkb_laws.cuh"
 #include "nkb_rows.cuh"

@@ -1927,7 +1927,8 @@ NKB_DEV void team_fork(Env& e, uint32_t op, uint32_t count, Work&& work) {
     }
 }
 
-// The articulation's block: on its tree, with the branches joined that a contact acts on; dense where that is too deep.
+// The articulation's block: in the space of its rows; else on its tree, with the branches joined that a contact acts on; dense where that is
+// too deep.
 template <int NR, bool kRows>
 NKB_DEV void descend_articulation(Env& e, Tile& tile, bool position) {
     if constexpr (kRows) {
