@@ -4,7 +4,7 @@
 // unknowns are the m multipliers y of the rows that act on the articulation, not its n coordinates.  With W = J M^-1 J^T a Newton
 // step of the block's problem, H d = J^T (f - y) with H = M + J^T C J, is d = M^-1 J^T dy with (1 + C W) dy = f - y; the rows move
 // by W dy, the line's slope at step a is sum (y + a dy - f(a)) (W dy), its curvature dy^T W dy + (W dy)^T C (W dy).  Nothing inside
-// the loop is as wide as the articulation: a robot on two feet has 6 rows and 18 coordinates, a humanoid 35, and a contact between
+// the loop is as wide as the articulation: a humanoid on two feet has 6 rows and 35 coordinates, and a contact between
 // two limbs adds three rows instead of joining branches of the tree.  C = R R^T with one column of R per row that responds (a
 // sliding contact has one for both tangents), and dy = (f - y) + R w with (1 + R^T W R) w = - R^T W (f - y): symmetric, every
 // pivot at least 1, and only as wide as the rows that respond.
@@ -12,12 +12,10 @@
 // M^-1 J^T and W are built once a step from the mass matrix's factor, a lane to a row (build_rows); W's diagonal is also the rows'
 // response that the penalties want.  Envs with more rows than solve_rows holds (row_cap) take the descents in coordinates.
 //
-// What bounds it is the chain of one warp: build_rows over the joints, one after another, solve_rows over groups of three rows, the
-// line search.  In coordinates (descend_tree) a Newton system was an assembly over the heads, an elimination over the tree's levels and the
-// base's six, and a product with M: 6.6 k cycles on a quadruped alone, here 2.5 k.  Policy steps of 4096 quadrupeds 2050 -> 1750 us, of
-// 16 384 7.44 -> 6.27 ms, of 2048 humanoids 3.68 -> 2.53 ms, a rollout of 2500 2.81 -> 2.35 ms.  A batch at rest, one Newton step to a descent, pays for
-// W (4096 standing quadrupeds 0.263 -> 0.312 ms); taking coordinates for the envs whose rows are within 0.01 m/s of their target has the warps of an
-// SM run both codes out of one instruction cache: 0.285 ms there, and 16 384 quadrupeds 6.2 -> 10.7 ms.
+// It is taken by articulations of more than 32 coordinates: 2048 humanoids, 4 steps, 1.85 ms (in coordinates 3.20).  Up to 32 the descent in
+// coordinates stays: a quadruped's 18 make a system about as cheap as W, and an env at rest, one Newton step to a descent, would pay for building
+// W (4096 standing quadrupeds 198 us against 183).
+// What bounds it is the chain of one warp: build_rows over the joints, one after another, solve_rows over groups of three rows, the line search.
 #pragma once
 #include "nkb_laws.cuh"
 #include "nkb_rows.cuh"

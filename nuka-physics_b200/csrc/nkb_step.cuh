@@ -384,7 +384,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             return;
         }
       }
-        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid, NR != 0 && kPart != kPartBare>(e, nheads);
+        if constexpr (kPart != kPartStages) stage_solve<NR, kRigid, NR == 2 && kPart != kPartBare>(e, nheads);
         if constexpr (kPart == kPartSolve) {
             image_move<false, kAfter>(e, p, img, nheads);
             __stcg(reinterpret_cast<float*>(lanes + lane), e.qd);

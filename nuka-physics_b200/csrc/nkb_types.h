@@ -25,7 +25,7 @@ NKB_HOST_DEVICE constexpr uint32_t merged_lane_words(uint32_t ndof) { return 2u 
 // Row stride (words) and scratch words of the tree-structured solve for `rows` joint lanes and root paths of `depth` joints.
 NKB_HOST_DEVICE inline uint32_t tree_row_stride(uint32_t depth) { return depth <= 5u ? 12u : depth <= 13u ? 20u : 36u; }
 // Groups of three rows that a descent in the rows' space holds in registers
-template <int NR> constexpr int kRowGroups = NR > 1 ? 6 : 5;
+constexpr int kRowGroups = 6;
 // The rows' space (nkb_rowspace.cuh): M^-1 J^T of `rows` rows and the drives, J M^-1 J^T, the row table; then the multipliers, 64 bits each
 NKB_HOST_DEVICE constexpr uint32_t row_space_head(uint32_t rows, uint32_t stride) { return ((rows + 1u) * stride + rows * (rows | 1u) + rows + 3u) & ~3u; }
 inline uint32_t row_space_words(uint32_t rows, uint32_t stride) { return rows == 0u ? 0u : row_space_head(rows, stride) + 2u * rows; }

@@ -379,10 +379,10 @@ void World::BuildLayout(bool join_branches, bool rows) {
             if (a != kNoLink && b != kNoLink && (t.anc_mask[a] & ~t.anc_mask[b]) != 0u && (t.anc_mask[b] & ~t.anc_mask[a]) != 0u) { tv.merges = 1u; break; }
         }
     const uint32_t solve_depth = tv.merges == 0u ? t.tree_depth : static_cast<uint32_t>(n > 32u ? kSolveLevels<2> : kSolveLevels<1>);
-    // Rows of the articulation that its descent in their space holds.
+    // Rows of the articulation that its descent in their space holds; only where a lane has two coordinates (nkb_rowspace.cuh)
     tv.row_stride = s.ld;
     tv.row_cap = 0u;
-    if (rows && tv.mass_tree != 0u && std::getenv("NUKA_B200_DENSE") == nullptr) tv.row_cap = std::min(3u * static_cast<uint32_t>(n > 32u ? kRowGroups<2> : kRowGroups<1>), 3u * tv.point_cap + t.joint_rows);
+    if (rows && n > 32u && tv.mass_tree != 0u && std::getenv("NUKA_B200_DENSE") == nullptr) tv.row_cap = std::min(3u * static_cast<uint32_t>(kRowGroups), 3u * tv.point_cap + t.joint_rows);
     if (const char* forced = std::getenv("NUKA_B200_ROWS")) tv.row_cap = std::min(tv.row_cap, static_cast<uint32_t>(std::atoi(forced)));       // tests
     const uint32_t newton_words = std::max({row_space_words(tv.row_cap, tv.row_stride), n * pad_ld(n), t.tree_depth != 0u ? tree_scratch_words(tree_rows, solve_depth) : 0u});
     const uint32_t merged_words = tv.merges != 0u ? 32u * merged_lane_words(n) : 0u;
@@ -531,13 +531,14 @@ void World::BuildLayout(bool join_branches, bool rows) {
         };
         solve_slice(solve_sm_, tv.head_cap, tv.point_cap);
         // A slice is sized for every contact that the template admits; a step has a few of them.  Envs whose heads and rows fit a small
-        // slice are solved in it, more of them to an SM, the others in a launch behind that is empty as a rule: as many contacts of the
-        // articulation as its rows' space holds, five of a free body.  2048 humanoids, 4 steps: 50 KB, 4 to an SM, 2.53 ms; 22 KB, 10 to an SM,
+        // slice are solved in it, more of them to an SM, the others in a launch behind that is empty as a rule: five or six contacts
+        // of the articulation, five of a free body.  2048 humanoids, 4 steps: 50 KB, 4 to an SM, 2.53 ms; 22 KB, 10 to an SM,
         // 1.96.  4096 quadrupeds with 4 boxes: 8 to an SM 5.35 ms, 12 in 4.74.  Where registers hold the same number anyway, or the batch fits the large slices at once, there is one.
-        small_heads_ = std::min(tv.head_cap, (tv.row_cap / 3u + t.joint_rows + 5u * t.n_free + 3u) & ~3u);
-        small_reach_ = std::min(tv.point_cap, tv.row_cap / 3u);
+        small_reach_ = std::min(tv.point_cap, n > 32u ? 6u : 5u);
+        if (const char* forced = std::getenv("NUKA_B200_SMALL_REACH")) small_reach_ = std::min(small_reach_, static_cast<uint32_t>(std::atoi(forced)));       // tests
+        small_heads_ = std::min(tv.head_cap, (small_reach_ + t.joint_rows + 5u * t.n_free + 3u) & ~3u);
         small_sm_.words = 0u;
-        if (tv.row_cap != 0u && std::getenv("NUKA_B200_ONE_TIER") == nullptr) {          // tests
+        if (std::getenv("NUKA_B200_ONE_TIER") == nullptr) {          // tests
             solve_slice(small_sm_, small_heads_, small_reach_);
             const int many = solve_->resident_blocks(1, small_sm_.words * 4u), few = solve_->resident_blocks(1, solve_sm_.words * 4u);
             const bool worth = 4 * many >= 5 * few && env_count_ > static_cast<uint32_t>(sms * few);
