@@ -2221,84 +2221,18 @@ NKB_DEV void measure_articulation(Env& e, Tile& tile, bool reconstruct) {
     }
 }
 
-// The same where the block descends in the space of its rows.  The velocity is first put in balance with the descent's own multipliers
-// (M^-1 J^T carries the factor's rounding, 1e-7 of a term; the balance is taken in 64 bits and costs nothing that the measure would
-// not), then what the physical multipliers differ by is known from the rows: a reconstruction, which
-// follows a measure, only adds it.
-template <int NR>
-NKB_DEV void measure_rows(Env& e, Tile& tile, bool reconstruct) {
-    const TemplateView& t = *e.t;
-    const uint32_t l = e.lane, b = t.B, n = t.ndof, m = e.rows, n4 = (n + 3u) & ~3u;
-    float* velocity = block_vel(e, b, false);
-    const float* fr = block_free(e, b);
-    double* wide = reinterpret_cast<double*>(sm_vec(e, kVecS0));       // spans S0 and S1
-    double balance[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r) balance[r] = 0.0;
-    if (!reconstruct) {
-#pragma unroll
-    for (int r = 0; r < NR; ++r) wide[l + 32u * r] = l + 32u * r < n ? (double)velocity[l + 32u * r] - fr[l + 32u * r] : 0.0;
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < NR; ++r) balance[r] = l + 32u * r < n ? (double)sm_fixed(e)[l + 32u * r] - mass_row_times(e, l + 32u * r, n4 >> 2, wide) : 0.0;
-#pragma unroll 1
-    for (uint32_t k = 0u; k < m; ++k) {
-        const uint32_t entry = row_table(e)[k], h = entry & 0xffffu, jo = hu(e, HF_JOFF, h);
-        const double y = row_y(e)[k];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const uint32_t c = l + 32u * r;
-            if (c >= n) continue;
-            if (!(jo & kUnitRow)) balance[r] = fma((double)sm_jpool(e)[jo + (entry >> 16) * n4 + c], y, balance[r]);
-            else if (c == (jo & 0xffffu)) balance[r] = fma((double)hf(e, HF_UNITV, h), y, balance[r]);
-        }
-    }
-    }
-    float force[NR], dir[NR];
-    bool ok = true;
-#pragma unroll
-    for (int r = 0; r < NR; ++r) { force[r] = (float)balance[r]; dir[r] = 0.f; ok &= fabs(balance[r]) <= FLT_MAX; }
-    const bool finite = __all_sync(NKB_FULL, ok);
-    float residual = FLT_MAX;
-    if (finite) {
-        if (!reconstruct) solve_block_mass<NR>(e, b, force, dir);
-        double lag[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) lag[r] = 0.0;
-        const uint32_t entry = l < m ? row_table(e)[l] : 0u;
-        row_spread<NR>(e, m, l < m ? (double)comp(head_lambda(e, entry & 0xffffu), (int)(entry >> 16)) - row_y(e)[l] : 0.0, lag);
-        float worst = 0.f;
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const uint32_t c = l + 32u * r;
-            if (c < n) {
-                worst = fmaxf(worst, isfinite(dir[r]) && isfinite((float)lag[r]) ? fabsf((float)lag[r]) : FLT_MAX);
-                if (reconstruct) dir[r] += (float)lag[r];
-                velocity[c] += dir[r];
-            }
-            wide[c] = c < n ? (double)dir[r] : 0.0;
-        }
-        residual = warp_max_positive(worst);
-        __syncwarp();
-        if (l < m) {
-            const uint32_t h = entry & 0xffffu, axis = entry >> 16;
-            hf(e, HF_RES + axis, h) = (float)((double)hf(e, HF_RES + axis, h) - row_dot(e, h, axis, wide));
-            if (reconstruct) row_y(e)[l] = (double)comp(head_lambda(e, h), (int)axis);
-        }
-        __syncwarp();
-    }
-    tile.residual = fmaxf(tile.residual, residual);
-    if (reconstruct && finite) tile.momentum = fmaxf(tile.momentum, residual);
-}
-
 // Momentum balance of every moving block against the physical multipliers (block_descent_tile.cuh:2379-2489).
 template <int NR, bool kRigid, bool kRows>
 NKB_DEV void measure_primals(Env& e, Tile& tile, bool reconstruct) {
     if constexpr (kRigid) measure_bodies(e, tile, reconstruct);
     if constexpr (NR > 0) {
-        if constexpr (kRows) { if (e.by_rows != 0u) { measure_rows<NR>(e, tile, reconstruct); return; } }
         measure_articulation<NR>(e, tile, reconstruct);
+        if constexpr (kRows) {
+            if (reconstruct && e.by_rows != 0u) {          // the velocity is the physical multipliers' now
+                if (e.lane < e.rows) { const uint32_t entry = row_table(e)[e.lane]; row_y(e)[e.lane] = (double)comp(head_lambda(e, entry & 0xffffu), (int)(entry >> 16)); }
+                __syncwarp();
+            }
+        }
     }
 }
 
