@@ -28,7 +28,7 @@ def scene(name, E):
     return star(limbs, depth, floating, **joint), state
 
 
-# Articulations of more than 32 coordinates; up to that many the coordinates serve.  Every row that fits; 14 and 4 rows at most, no multiples of the three that a contact has (envs with more take the coordinates);
+# Every row that fits; 14 and 4 rows at most, no multiples of the three that a contact has (envs with more take the coordinates);
 # split steps.  The bars of one step's velocities against the reference: 1e-5 of max(|v|, 1).  A sweep ends an env's solve where its
 # rows' residual falls below 1e-5 m/s, so two roundings can end it a sweep apart, which moves a light joint at the end of a limb by
 # that residual over its lever of 0.04 m: up to 3e-4 rad/s per row, of which a tip has three.
@@ -41,10 +41,7 @@ def test_rows_equal_coordinates(device, name, forced):
     coordinates = outputs(create(device, tb, state, E, ROWS=0), (1,))
     assert rows["CONTACT_COUNT"].sum() > 0 and rows["ENV_STATUS"].max() == 0 and coordinates["ENV_STATUS"].max() == 0
     got, want = rows["JOINT_VELOCITY"].astype(np.float64), coordinates["JOINT_VELOCITY"].astype(np.float64)
-    if name != "wide":                        # up to 32 coordinates: no rows' space, whatever is asked for
-        assert np.array_equal(got, want)
-        return
-    assert not np.array_equal(got, want)                                                        # the other route
+    assert np.array_equal(got, want) == (name != "wide")          # the other route, which up to 32 coordinates do not take
     error = np.abs(got - want).max(axis=1) / np.maximum(np.abs(want).max(axis=1), 1.0)
     assert np.percentile(error, 95) < 1e-5 and error.max() < 1e-3, (float(np.percentile(error, 95)), float(error.max()))
     assert (rows["SOLVER_SWEEPS"] == coordinates["SOLVER_SWEEPS"]).mean() > 0.95
@@ -62,11 +59,28 @@ def test_balance_of_descents_by_rows_is_measured(device, name):
     assert (want > 0).sum() > 20 and not ((got == 0) & (want > 0)).any(), (int(((got == 0) & (want > 0)).sum()), float(want.max()))
 
 
-# Solves in two slices against one, and against whole steps: the same bits.  A small slice with room for one contact of the articulation
+# Solves in two slices against one, and against whole steps: the same bits.  With four rows the small slice holds one contact, so that both
+# slices have envs to solve; with free bodies one that touches nothing counts as well
+@pytest.mark.parametrize("name", ["quadruped", "boxes", "wide"])
+@pytest.mark.parametrize("rows", [4, 64])
+def test_small_and_large_slices_equal_whole_steps(device, name, rows):
+    E = 300
+    if name == "boxes":
+        tb, state = T.quadruped(0, boxes=2), T.quadruped_state(E, 0)
+    else:
+        tb, state = scene(name, E)
+    whole, one, two = (outputs(create(device, tb, state, E, ROWS=rows, **forced), (2, 1))
+                       for forced in (dict(SPLIT=0), dict(SPLIT=1, ONE_TIER=1), dict(SPLIT=1, TWO_TIERS=1)))
+    assert two["CONTACT_COUNT"].sum() > 0
+    assert_same(whole, one)
+    assert_same(one, two)
+
+
+# The same with the shapes read from the printed layout.  A small slice with room for one contact of the articulation
 # leaves both slices envs to solve (with free bodies one that touches nothing counts as well); the usual one; with four rows in the rows' space
 @pytest.mark.parametrize("name", ["quadruped", "boxes", "wide"])
 @pytest.mark.parametrize("small", [{"SMALL_REACH": 1}, {}, {"ROWS": 4}], ids=["one", "usual", "rows"])
-def test_small_and_large_slices_equal_whole_steps(device, capfd, name, small):
+def test_envs_on_both_sides_of_the_small_slice(device, capfd, name, small):
     E = 300
     if name == "boxes":
         tb, state = T.quadruped(0, boxes=2), T.quadruped_state(E, 0)
