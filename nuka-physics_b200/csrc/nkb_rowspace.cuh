@@ -12,7 +12,7 @@
 // M^-1 J^T and W are built once a step from the mass matrix's factor, a lane to a row (build_rows); W's diagonal is also the rows'
 // response that the penalties want.  Envs with more rows than solve_rows holds (row_cap) take the descents in coordinates.
 //
-// It is taken by articulations of more than 32 coordinates: 2048 humanoids, 4 steps, 1.85 ms (in coordinates 3.20).  Up to 32 the descent in
+// It is taken by articulations of more than 32 coordinates: 2048 humanoids, 4 steps, 1.97 ms (in coordinates 3.50).  Up to 32 the descent in
 // coordinates stays: a quadruped's 18 make a system about as cheap as W, and an env at rest, one Newton step to a descent, would pay for building
 // W (4096 standing quadrupeds 198 us against 183).
 // What bounds it is the chain of one warp: build_rows over the joints, one after another, solve_rows over groups of three rows, the line search.

@@ -1,4 +1,6 @@
 """The articulation's descent in the space of its constraint rows against the one in its coordinates."""
+import os
+
 import numpy as np
 import pytest
 
@@ -45,6 +47,21 @@ def test_rows_equal_coordinates(device, name, forced):
     error = np.abs(got - want).max(axis=1) / np.maximum(np.abs(want).max(axis=1), 1.0)
     assert np.percentile(error, 95) < 1e-5 and error.max() < 1e-3, (float(np.percentile(error, 95)), float(error.max()))
     assert (rows["SOLVER_SWEEPS"] == coordinates["SOLVER_SWEEPS"]).mean() > 0.95
+
+
+# One step against a 64-bit evaluation of the same inputs (golden/wide_exact.npz: the oracle's sources with double for float).  The descent by
+# rows may be no less exact than the one in coordinates.  The envs are the same, so what a mean over 512 of them can differ by is a few per cent.
+def test_rows_are_as_exact_as_coordinates(device):
+    E = 512
+    tb, state = scene("wide", E)
+    want = np.load(os.path.join(os.path.dirname(__file__), "golden", "wide_exact.npz"))["qdot"]
+    errors = []
+    for forced in ({}, {"ROWS": 0}):
+        out = outputs(create(device, tb, state, E, **forced), (1,))
+        touched = (out["CONTACT_COUNT"].reshape(E, -1) > 0).any(axis=1)
+        error = np.abs(out["JOINT_VELOCITY"].reshape(E, -1).astype(np.float64) - want).max(axis=1) / np.maximum(np.abs(want).max(axis=1), 1.0)
+        errors.append(np.exp(np.log(error[touched] + 1e-12).mean()))
+    assert errors[0] != errors[1] and errors[0] < 1.05 * errors[1], errors
 
 
 # The last residual is the momentum balance at the velocity found, whichever space the descent took: no 32-bit velocity is in exact balance
