@@ -148,7 +148,6 @@ NKB_DEV uint32_t stage_rows(Env& e, uint32_t pair_count) {
             }
         }
         float* pool = e.pool;
-        e.reach = 0u;
 #pragma unroll 1
         for (uint32_t h = 0u; h < ncontact; ++h) {
             const uint32_t ref = hu(e, HF_REF, h), la = ref >> 16, lb = hu(e, HF_JOFF, h) & 0xffffu;
@@ -280,7 +279,7 @@ NKB_DEV uint32_t head_pair(const Env& e, uint32_t h) { return sm_pairs(e)[(hu(e,
 constexpr uint32_t kCacheChunk = 4u;           // entries per lane that a search of the cache loads at once
 // Warm start (phase 0): a contact head takes the multipliers of the cached point with the same identity.
 // Range form: this warp takes the heads first, first + stride, ... (a head's match reads earlier heads and the cache and
-// writes only the head's own dual).
+// writes only the head's own dual and duplicate flag).
 NKB_DEV void warm_start_range(Env& e, uint32_t nheads, uint32_t first, uint32_t stride) {
     const TemplateView& t = *e.t;
     const uint32_t npts = t.cfg.max_contacts * 4u;

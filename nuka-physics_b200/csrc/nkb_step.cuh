@@ -319,7 +319,7 @@ NKB_DEV void advance_env(const StepParams& p, float* sm, uint32_t env, uint32_t 
             tick(e, 13);
             if (kPart == kPartStages ? p.last != 0u : step == p.steps) return;
         }
-        e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone;
+        e.status = 0u; e.branching = false; e.merged = kMergeUntried; e.by_rows = kRowsNone; e.reach = 0u;
         if (p.mode == kModeRefresh) {
             if (has_bodies) stage_store_bodies(e, false);
             if (has_artic) {

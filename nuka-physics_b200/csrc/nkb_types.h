@@ -167,7 +167,7 @@ struct SmemLayout {
 // a step in one launch of a world without contacts.
 enum StepPart : int { kPartWhole = 0, kPartStages = 1, kPartSolve = 2, kPartBare = 3 };
 template <int kPart> constexpr bool kSplitPart = kPart == kPartStages || kPart == kPartSolve;
-constexpr uint32_t kImageLaneWords = 4u * 32u + 4u;     // an image's tail: four words per lane, then status, heads, branching
+constexpr uint32_t kImageLaneWords = 4u * 32u + 4u;     // an image's tail: four words per lane, then status, heads, branching, reach (contact heads with rows)
 
 enum StepMode : uint32_t { kModeStep = 0, kModeDynamicsOnly = 1, kModeCollideOnly = 2, kModeRefresh = 3 };
 
