@@ -10,7 +10,7 @@
 // pivot at least 1, and only as wide as the rows that respond.
 //
 // M^-1 J^T and W are built once a step from the mass matrix's factor, a lane to a row (build_rows); W's diagonal is also the rows'
-// response that the penalties want.  Envs with more rows than solve_rows holds (row_cap) take the descents in coordinates.
+// response that the penalties want.  Envs with more rows than solve_rows holds (row_cap), or a response below zero, take the descents in coordinates.
 //
 // It is taken by articulations of more than 32 coordinates: 2048 humanoids, 4 steps, 1.97 ms (in coordinates 3.50).  Up to 32 the descent in
 // coordinates stays: a quadruped's 18 make a system about as cheap as W, and an env at rest, one Newton step to a descent, would pay for building
@@ -54,7 +54,7 @@ NKB_DEV double row_dot(const Env& e, uint32_t h, uint32_t axis, const double* v)
 }
 
 // Numbers the rows that act on the articulation (three per contact head, then one per joint row), solves M x = J^T for each and
-// for the drives' impulses, and multiplies out W.  False where there are more rows than the slice holds.
+// for the drives' impulses, and multiplies out W.  False where there are more rows than the slice holds, or a response is below zero.
 // A lane walks the tree for its row: joints from the last to the first push their share to the base and to their ancestors, then
 // the base's 6 x 6, then joints from the first to the last; the factor's rows are read by all lanes at once.
 template <int NR>
@@ -182,8 +182,10 @@ NKB_DEV bool build_rows(Env& e, uint32_t nheads) {
         }
     __syncwarp();
     // W, lane = row: J_l X_j, three j at a time (a contact's rows)
+    const uint32_t entry = l < m ? table[l] : 0u, h = entry & 0xffffu;
+    const float* diagonal = row_w(e) + l * (row_words(e) + 1u);
     if (l < m) {
-        const uint32_t entry = table[l], h = entry & 0xffffu, jo = hu(e, HF_JOFF, h), at = jo & 0xffffu;
+        const uint32_t jo = hu(e, HF_JOFF, h), at = jo & 0xffffu;
         const bool unit = (jo & kUnitRow) != 0u;
         const float4* j4 = reinterpret_cast<const float4*>(sm_jpool(e) + (unit ? 0u : jo)) + (entry >> 16) * chunks;
         const float value = unit ? hf(e, HF_UNITV, h) : 0.f;
@@ -207,9 +209,11 @@ NKB_DEV bool build_rows(Env& e, uint32_t nheads) {
             if (j + 1u < m) mine[j + 1u] = s1;
             if (j + 2u < m) mine[j + 2u] = s2;
         }
-        if ((entry >> 16) == 0u) hf(e, HF_RHO, h) = mine[l];          // the response of the head's normal row (init_heads)
         row_y(e)[l] = 0.0;
     }
+    // W's diagonal is a sum of both signs: a response that rounds below zero, which init_heads takes for a failure, is one for the coordinates
+    if (__any_sync(NKB_FULL, l < m && !(*diagonal >= 0.f))) return false;
+    if (l < m && (entry >> 16) == 0u) hf(e, HF_RHO, h) = *diagonal;          // the response of the head's normal row (init_heads)
     __syncwarp();
     return true;
 }
