@@ -589,11 +589,9 @@ NKB_DEV void apply_moves(Env& e, const Tile& tile, uint32_t b, float alpha) {
     __syncwarp();
 }
 
-// A step from a force within its own rounding, shorter than the velocity tolerance, is the last (`settled`): the force can get no smaller, and
-// M^-1 times its rounding may stay above the tolerance on light links.  Such descents ran all 16 steps, 1e-7 m/s each, 6 % of a quadruped's and the
-// longest of every batch (policy steps of 1000: 1100 us -> 863, rollouts of 2500 3.79 ms -> 2.86).
-// On the articulation's tree the second such step is the last (1 % slower): with the first, one env of a reference trajectory of quadrupeds is 1.1e-4
-// off after 40 steps, with the second 5e-5, with all sixteen 4e-5.
+// A descent whose force is within its own rounding while M^-1 times that rounding stays above the tolerance (light links) goes on to the step limit,
+// 1e-7 m/s a step.  Ending it there is no less exact against 64 bits and up to 1.3 times faster (rollouts of 2500 quadrupeds), but such steps move
+// single envs across the edge of a contact: one batch of six was 3.5e-3 from the results with all steps, piles 0.3 in one box.  It is not done.
 //
 // Newton steps with exact line search on one block, from where it stands.  A descent ends at the block's minimum wherever it begins, to
 // rounding, so the reference's search toward the free velocity ahead of the first sweep's Newton steps (block_descent_tile.cuh:2196-2210)
@@ -645,7 +643,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
         fr[r] = (coord[r] && !position) ? block_free(e, b)[l + 32u * r] : 0.f;
         u[r] = start[r];
     }
-    bool failure = false, settled = false;
+    bool failure = false;
     float primal = FLT_MAX;
     tick(e, 15);
 #pragma unroll 1
@@ -779,7 +777,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
                 small &= !coord[r] || fabsf(force[r]) <= kRoundings * FLT_EPSILON * scale[r];
             }
             if (!__all_sync(NKB_FULL, finite)) { failure = true; break; }
-            bool converged = settled = __all_sync(NKB_FULL, small);
+            bool converged = __all_sync(NKB_FULL, small);
             if (converged && tile.tol > 0.f) {
                 solve_block_mass<NR>(e, b, force, d);
                 bool still = true;
@@ -909,7 +907,7 @@ NKB_DEV void descend_block(Env& e, Tile& tile, uint32_t b, bool position) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) u[r] = after[r];
         apply_moves(e, tile, b, alpha);
-        if (rounded || (settled && primal < tile.tol)) break;
+        if (rounded) break;
     }
 #pragma unroll 1
     for (uint32_t k = ib + l; k < ie; k += 32u) {
@@ -1031,7 +1029,6 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         fixed[r] = position || !coord[r] ? 0.f : sm_fixed(e)[c];
     }
     bool failure = false;
-    int settled = 0;
     float primal = FLT_MAX;
     tick(e, 15);
 #pragma unroll 1
@@ -1127,7 +1124,7 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         if (step >= 0) {
             rounded = __all_sync(NKB_FULL, rounded);
             primal = rounded ? 0.f : warp_max_positive(longest);
-            if (!(alpha > 0.f) || rounded || (settled > 1 && primal < tile.tol) || step + 1 == (int)kNewtonSteps) break;
+            if (!(alpha > 0.f) || rounded || step + 1 == (int)kNewtonSteps) break;
         }
         ++step;
         // ---- the next Newton system at the new velocity: this lane's row of H, its entry of the force balance ----
@@ -1230,7 +1227,6 @@ NKB_DEV void descend_tree(Env& e, Tile& tile, bool position) {
         }
         if (!__all_sync(NKB_FULL, finite)) { failure = true; break; }
         bool converged = __all_sync(NKB_FULL, small);
-        settled = converged ? settled + 1 : 0;
         if (converged && tile.tol > 0.f) {
             float d[NR];
             solve_block_mass<NR>(e, b, force, d);
@@ -1711,7 +1707,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
         // a block without a push-out row keeps its zero position correction; in the velocity phase an unconstrained block
         // still has to reach its free velocity
         const bool began = have && !(position && count == 0u);
-        bool active = began, coupled = false, failure = false, settled = false;
+        bool active = began, coupled = false, failure = false;
 #pragma unroll 1
         for (uint32_t k = g.j; k < count; k += kBodyLanes) {
             const uint32_t h = inc[k], o = hu(e, HF_OWNER, h);
@@ -1831,7 +1827,7 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
                     }
                     if (step >= 0) {
                         primal = rounded ? 0.f : longest;
-                        active = alpha > 0.f && !rounded && !(settled && primal < run.tol) && step + 1 < (int)kNewtonSteps;
+                        active = alpha > 0.f && !rounded && step + 1 < (int)kNewtonSteps;
                     }
                 }
             }
@@ -1891,7 +1887,6 @@ NKB_DEV RigidResult descend_bodies(const RigidRun& run, uint32_t k_begin, uint32
             float inv[6], x[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i) rhs[i] = force[i] = __shfl_sync(NKB_FULL, own, g.first + i);
-            settled = small;
             if (active && small) {
                 bool still = true;
                 if (run.tol > 0.f) {
