@@ -166,7 +166,7 @@ NKB_DEV void stage_store_bodies(Env& e, bool velocities) {
 #define NKB_MAXNREG_BODIES 168
 #endif
 // The parts of split steps, where slices are small: three warps to a partition (solves of quadrupeds with boxes at 224 registers and
-// no spills, two: 5.22 ms; at 168 and 150 bytes, three: 4.74).
+// no spills, two: 5.97 ms; at 168, three: 5.41).
 #ifndef NKB_MAXNREG_SPLIT
 #define NKB_MAXNREG_SPLIT 168
 #endif

@@ -532,8 +532,8 @@ void World::BuildLayout(bool join_branches, bool rows) {
         solve_slice(solve_sm_, tv.head_cap, tv.point_cap);
         // A slice is sized for every contact that the template admits; a step has a few of them.  Envs whose heads and rows fit a small
         // slice are solved in it, more of them to an SM, the others in a launch behind that is empty as a rule: five or six contacts
-        // of the articulation, five of a free body.  2048 humanoids, 4 steps: 50 KB, 4 to an SM, 2.53 ms; 22 KB, 10 to an SM,
-        // 1.96.  4096 quadrupeds with 4 boxes: 8 to an SM 5.35 ms, 12 in 4.74.  Where registers hold the same number anyway, or the batch fits the large slices at once, there is one.
+        // of the articulation, five of a free body.  2048 humanoids, 4 steps: 50 KB, 4 to an SM, 2.37 ms; 22 KB, 10 to an SM,
+        // 1.96.  4096 quadrupeds with 4 boxes: 8 to an SM 6.21 ms, 12 in 5.41.  Where registers hold the same number anyway, or the batch fits the large slices at once, there is one.
         small_reach_ = std::min(tv.point_cap, n > 32u ? 6u : 5u);
         if (const char* forced = std::getenv("NUKA_B200_SMALL_REACH")) small_reach_ = std::min(small_reach_, static_cast<uint32_t>(std::atoi(forced)));       // tests
         small_heads_ = std::min(tv.head_cap, (small_reach_ + t.joint_rows + 5u * t.n_free + 3u) & ~3u);
